@@ -764,6 +764,50 @@ constexpr int RR_THREADS = 1024;            // resolve: one block per frame
 constexpr int RR_WARPS = RR_THREADS / 32;
 constexpr int RR_ILP = 2;                  // resolve: listed entries per lane in flight together
 
+// True when no sample point of the triangle can be a fragment, decided without evaluating one:
+// its box has at most 2 x 2 sample points, each of which lies outside the corners' range by
+// more than RC_MARGIN in x or in y, and the triangle is not a sliver.
+// Why no evaluation could accept such a point (u = 2^-24; l0 = |b - a|, l1 = |c - a|, s the sine
+// between them, D = (l0 l1 s)^2 the exact denominator; the corner differences carry one rounding
+// each): a point outside the range by M in one coordinate, of a triangle at most 2 wide, has a
+// barycentric coordinate of at most -e, e = M / 4 (1 - 1e-4). FP32 forms na and nb within
+// 13 u l1^2 l0 l2 and 13 u l0^2 l1 l2 and the denominator within 13 u l0^2 l1^2, l2 <= 2.83 the
+// distance of the point from a. alpha (beta) <= -e then gives na (nb) the wrong sign, and
+// alpha + beta >= 1 + e leaves the rounded sum above 1, whenever min(l0, l1) s^3 > 153 u / e =
+// 2.4e-3; the test below asks for 5.5e-3 (squared: RC_SLIVER). Any NaN fails a comparison here and
+// takes the full path, as do boxes outside the domain.
+constexpr float RC_MARGIN = 1.0f / 64.0f;
+constexpr float RC_SLIVER = 3e-5f;
+
+__device__ __forceinline__ bool no_sample_inside(float bx, float by, float cx, float cy, float ax, float ay)
+{
+    const float xmax = fmaxf(fmaxf(bx, cx), ax), xmin = fminf(fminf(bx, cx), ax);
+    const float ymax = fmaxf(fmaxf(by, cy), ay), ymin = fminf(fminf(by, cy), ay);
+    const float xhi = ceilf(xmax), yhi = ceilf(ymax), xlo = floorf(xmin), ylo = floorf(ymin);
+    const bool dom = xlo >= 0.0f && ylo >= 0.0f && xhi <= 65535.0f && yhi <= 65535.0f && xhi - xlo <= 2.0f &&
+                     yhi - ylo <= 2.0f;
+    // columns xlo and xlo + 1 (rows alike): outside by more than the margin, or not sampled
+    const float x1 = xlo + 1.0f, y1 = ylo + 1.0f;
+    const bool xout = xmin - xlo > RC_MARGIN && (x1 >= xhi || x1 - xmax > RC_MARGIN);
+    const bool yout = ymin - ylo > RC_MARGIN && (y1 >= yhi || y1 - ymax > RC_MARGIN);
+    const float v0x = bx - ax, v1x = cx - ax, v0y = by - ay, v1y = cy - ay;
+    const float d00 = v0x * v0x + v0y * v0y, d01 = v0x * v1x + v0y * v1y, d11 = v1x * v1x + v1y * v1y;
+    const float q = d00 * d11, denom = q - d01 * d01;
+    const bool wide = (denom * denom) * (denom * fminf(d00, d11)) > RC_SLIVER * ((q * q) * q);
+    return dom && (xout || yout) && wide;
+}
+
+// A dense face mesh has about 25 triangles per visible fragment, most of them smaller than a
+// pixel, so the pass is bound by the instructions spent on triangles without a sample
+// point. Each warp therefore first tests its triangles with no_sample_inside (about 55
+// instructions instead of about 230) and queues the others' corners in shared memory; a full
+// warp's worth of queued triangles is then evaluated densely. Two triangles per lane have
+// their gathers in flight together. 1,024 frames of the 53,490-vertex model in one launch:
+// 1,192 -> 697 us (0.68 us per frame); 174 -> 106 us averaged over the rounds of that fit.
+constexpr int RD_WARPS = RD_THREADS / 32;
+constexpr int RD_ILP = 2;                   // triangles per lane and step
+constexpr int RD_QUEUE = 32 * (RD_ILP + 1); // a warp's queue: what a step adds to a remainder below 32
+
 __global__ void __launch_bounds__(RD_THREADS) k_raster_depth(DModel m, DBatch b)
 {
     if ((int)blockIdx.y >= active_n(b)) return;
@@ -771,6 +815,10 @@ __global__ void __launch_bounds__(RD_THREADS) k_raster_depth(DModel m, DBatch b)
     const FrameCtl &ctl = b.ctl[f];
     if (!ctl.render) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) prof_count(b, KID_RASTER);
+    __shared__ float4 s_qa[RD_WARPS][RD_QUEUE];     // bx, by, cx, cy
+    __shared__ float4 s_qb[RD_WARPS][RD_QUEUE];     // ax, ay, camera Z of b, triangle id (bits)
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    float4 *qa = s_qa[warp], *qb = s_qb[warp];
     const uint32_t tag = TAG_MAX - (ctl.epoch + 1);
     const float4 *pj = b.proj + (size_t)f * m.V;
     unsigned long long *zb = b.zbuf + (size_t)f * NPIX;
@@ -781,20 +829,49 @@ __global__ void __launch_bounds__(RD_THREADS) k_raster_depth(DModel m, DBatch b)
     const int per_block = (T + gridDim.x - 1) / gridDim.x;
     const int s_begin = blockIdx.x * per_block, s_end = min(T, s_begin + per_block);
     uint32_t flags = 0;
-    for (int s = s_begin + (int)threadIdx.x; s < s_end; s += RD_THREADS) {
-        const int4 tq = __ldg(m.tlo4 + s);
-        const int idx = tq.w;
-        const float4 pb = __ldg(pj + tq.x);
-        const float4 pc = __ldg(pj + tq.y);
-        const float4 pa = __ldg(pj + tq.z);
-        const unsigned long long key = zkey(tag, pb.z, idx);
-        const int nf = tri_samples(pb.x, pb.y, pc.x, pc.y, pa.x, pa.y, x0, y0, flags,
+    int queued = 0;                                 // entries of the warp's queue
+    auto evaluate = [&](int e) {
+        const float4 A = qa[e], B = qb[e];
+        const int idx = __float_as_int(B.w);
+        const unsigned long long key = zkey(tag, B.z, idx);
+        const int nf = tri_samples(A.x, A.y, A.z, A.w, B.x, B.y, x0, y0, flags,
                                    [&](int, uint32_t px, float, float) { atomicMin(zb + px, key); });
         if (nf) {
-            if (!(pb.z > 0.0f)) flags |= FLAG_OUT_OF_DOMAIN;
+            if (!(B.z > 0.0f)) flags |= FLAG_OUT_OF_DOMAIN;
             atomicOr(mask + (idx >> 5), 1u << (idx & 31));
         }
+    };
+    for (int base = s_begin + warp * 32 * RD_ILP; base < s_end; base += RD_THREADS * RD_ILP) {
+        int4 tq[RD_ILP];
+        float4 pb[RD_ILP], pc[RD_ILP], pa[RD_ILP];
+#pragma unroll
+        for (int h = 0; h < RD_ILP; ++h) tq[h] = __ldg(m.tlo4 + min(base + 32 * h + lane, T - 1));
+#pragma unroll
+        for (int h = 0; h < RD_ILP; ++h) {
+            pb[h] = __ldg(pj + tq[h].x);
+            pc[h] = __ldg(pj + tq[h].y);
+            pa[h] = __ldg(pj + tq[h].z);
+        }
+#pragma unroll
+        for (int h = 0; h < RD_ILP; ++h) {
+            const bool take = base + 32 * h + lane < s_end &&
+                              !no_sample_inside(pb[h].x, pb[h].y, pc[h].x, pc[h].y, pa[h].x, pa[h].y);
+            const unsigned msk = __ballot_sync(0xffffffffu, take);
+            if (take) {
+                const int e = queued + __popc(msk & ((1u << lane) - 1u));
+                qa[e] = make_float4(pb[h].x, pb[h].y, pc[h].x, pc[h].y);
+                qb[e] = make_float4(pa[h].x, pa[h].y, pb[h].z, __int_as_float(tq[h].w));
+            }
+            queued += __popc(msk);
+        }
+        __syncwarp();
+        while (queued >= 32) {
+            queued -= 32;
+            evaluate(queued + lane);
+            __syncwarp();
+        }
     }
+    if (lane < queued) evaluate(lane);
     if (flags) atomicOr(&b.ctl[f].flags, flags);
 }
 
