@@ -485,7 +485,7 @@ tdi_status normal_equations(const Launch &L, const Cfg &c, int stage)
     }
     TDI_TRY(launch(L.bt, KID_BARRIER, k_barrier_full, dim3(L.A()), dim3(256), L.smem_bar(), L.s, L.m, L.b,
                    (int)(stage == ST_FINETUNE)));
-    TDI_TRY(launch(L.bt, KID_SOLVE, L.m.KT <= 96 ? k_solve_t<6> : k_solve_t<8>, dim3(L.A()), dim3(SV_THREADS),
+    TDI_TRY(launch(L.bt, KID_SOLVE, sv_blocks(L.m.KT) == 6 ? k_solve_t<6> : k_solve_t<8>, dim3(L.A()), dim3(SV_THREADS),
                    L.smem_solve(), L.s, L.m, L.b, c, stage));
     return TDI_OK;
 }

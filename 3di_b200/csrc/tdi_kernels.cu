@@ -3,6 +3,7 @@
 // contraction, so each per-fragment quantity is bit-identical to the CPU oracle's.
 #include "tdi_internal.cuh"
 #include "tdi_async.cuh"
+#include "tdi_cholesky.cuh"
 
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
@@ -2340,181 +2341,34 @@ __global__ void __launch_bounds__(256) k_barrier_full(DModel m, DBatch b, int ft
 }
 
 // ------------------------------------------------------------------------------------------
-// FP64 Cholesky solve (solver.h:70-105, cuSOLVER DPOTRF/DPOTRS in the reference) of the shape
-// system, one block per frame, then the first trial of the line search.
-//
-// Arithmetic (shared with the oracle's solve_shape): pivots l_jj = sqrt(s_j) with reciprocal
-// r_j = 1 / l_jj; L(i,j) = t_ij * r_j, where t_ij is a_ij minus L(i,k) L(j,k) for k = 0, 1, ...
-// in increasing k (each product and difference rounded); forward y_i = (g_i - sum_k L(i,k) y_k)
-// * r_i with terms in increasing k; back x_i = (y_i - sum_k L(k,i) x_k) * r_i with terms in
-// decreasing k. (cuSOLVER's order is the library's; the reciprocal is one rounding per column.)
-//
-// The lower triangle is held in registers: thread (tr, tc) = (tid % 16, tid / 16) owns the
-// entries (i, l) with i = tr + 16a, l = tc + 16b, i >= l. Step j: every thread reads column j
-// as its owners left it in shared memory (pivot included) and r_j as the pivot's owner formed
-// it, forms the scaled entries it needs, and subtracts L(i,j) L(l,j) from its entries right of
-// column j: the register block holding column j + 1 first, after which the owners of column
-// j + 1 store it and the owner of its pivot forms l and r for the next step while the other
-// blocks are updated. Each entry so receives its updates in increasing j, the sequence of the
-// oracle's left-looking dot products. One barrier per step; the two substitutions run in one
-// warp, four rows per lane, the newly known value broadcast by shuffle.
-//
-// The steps run in groups of 16 columns, one group per register block, each group its own
-// instantiation. Every register block is then named by a compile-time index, and the finished
-// blocks are skipped without tests. Selecting the next column's block at run time instead moved
-// the whole block array into local memory (a 288-byte stack frame). Keeping it in registers
-// while updating every block under run-time tests measured slower still: 1.59 µs per
-// evaluation, against 1.10 µs with the stack and 0.96 µs in groups. The substitutions with the
-// reciprocals in registers and no stores inside the passes took it to 0.90 µs, and the pivot
-// formed one step ahead by its owner to 0.86 µs.
+// FP64 Cholesky solve (solver.h:70-105) of the shape system, one block per frame
+// (tdi_cholesky.cuh), then the first trial of the line search.
 
-constexpr int SV_THREADS = 256;
-constexpr int SV_MAXN = 128;
+constexpr int SV_THREADS = CH_THREADS;
 
-__host__ __device__ __forceinline__ size_t solve_smem(int n)
-{
-    return ((size_t)n * n + 4 * SV_MAXN + 2) * sizeof(double);
-}
-
-// One substitution pass of the warp: rows i = lane + 32 q (q < 4) start from t[q]; for each
-// step k (ascending when FWD, descending otherwise) the owner of row k (lane k % 32) forms
-// x_k = t_k r_k from its own registers and broadcasts it, and every row i after k in that
-// order subtracts coef(i, k) x_k. The steps run in four segments of 32 with the row slot q a
-// compile-time index, and nothing is stored inside the pass, so that the coefficient loads of
-// later steps can be issued early. x of the lane's own rows ends in xm[].
-template <bool FWD>
-__device__ __forceinline__ void sv_substitute(int n, double (&t)[4], const double (&rm)[4], double (&xm)[4],
-                                              const double *Lf)
-{
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int s = 0; s < 4; ++s) {
-        const int q = FWD ? s : 3 - s;
-        if (32 * q >= n) continue;
-#pragma unroll 4
-        for (int u = 0; u < 32; ++u) {
-            const int kk = FWD ? u : 31 - u;
-            const int k = 32 * q + kk;
-            if (k >= n) { if (FWD) break; else continue; }
-            const double xo = t[q] * rm[q];             // meaningful in the owner lane
-            if (lane == kk) xm[q] = xo;
-            const double xk = __shfl_sync(0xffffffffu, xo, kk);
-#pragma unroll
-            for (int qq = 0; qq < 4; ++qq) {
-                if (FWD ? qq < q : qq > q) continue;
-                const int i = lane + 32 * qq;
-                // forward: L(i,k) for i > k (column k); back: L(k,i) for i < k (column i)
-                if (FWD ? (i > k && i < n) : (i < k)) t[qq] -= (FWD ? Lf[(size_t)k * n + i] : Lf[(size_t)i * n + k]) * xk;
-            }
-        }
-    }
-}
-
-// The trailing update of step j (column j scaled into ci, cl), with column j + 1 in register
-// block B: the blocks (a, B) first; then the owners of column j + 1 store it, and the owner of
-// its pivot forms l = sqrt(s) and r = 1 / l (both correctly rounded) for the next step while
-// the other blocks (a, bb > B) are updated. Blocks left of B receive no more updates.
-template <int RB, int B>
-__device__ __forceinline__ void sv_update(double (&v)[RB][RB], const double (&ci)[RB], const double (&cl)[RB],
-                                          int tr, int tc, int j, int n, double *rn, double *Lf, double *rv)
-{
-#pragma unroll
-    for (int a = B; a < RB; ++a) {
-        const int i = tr + 16 * a, l = tc + 16 * B;
-        if (l > j && i >= l && i < n) v[a][B] -= ci[a] * cl[B];
-    }
-    const int jn = j + 1;
-    if (jn < n && tc == (jn & 15)) {
-#pragma unroll
-        for (int a = B; a < RB; ++a) {
-            const int i = tr + 16 * a;
-            if (i >= jn && i < n) rn[i] = v[a][B];
-        }
-        if (tr == (jn & 15)) {
-            const double sn = v[B][B];
-            if (sn > 0.0) {
-                const double ln = sqrt(sn);
-                Lf[(size_t)jn * n + jn] = ln;
-                rv[jn] = __drcp_rn(ln);
-            }
-        }
-    }
-#pragma unroll
-    for (int a = B + 1; a < RB; ++a)
-#pragma unroll
-        for (int bb = B + 1; bb <= a; ++bb) {
-            const int i = tr + 16 * a, l = tc + 16 * bb;
-            if (l > j && i >= l && i < n) v[a][bb] -= ci[a] * cl[bb];
-        }
-}
-
-// Steps j of column group J (columns 16 J .. 16 J + 15), then the next group; false when a
-// pivot is not positive (every thread reads the same pivot, so all return together). Blocks
-// left of group J (bb < J) and rows above it (a < J) are finished: their columns l < 16 J <= j
-// receive no more updates, so they are skipped statically.
-template <int RB, int J>
-__device__ __forceinline__ bool sv_factor(double (&v)[RB][RB], double *raw, double *Lf, double *rv,
-                                          int tr, int tc, int tid, int n)
-{
-    const int jend = min(n, 16 * J + 16);
-    for (int j = 16 * J; j < jend; ++j) {
-        const double *rj = raw + (j & 1) * SV_MAXN;
-        const double sj = rj[j];
-        if (!(sj > 0.0)) return false;
-        const double r = rv[j];                          // formed by the pivot's owner in step j - 1
-        if (tid > j && tid < n) Lf[(size_t)j * n + tid] = rj[tid] * r;
-        double ci[RB], cl[RB];
-#pragma unroll
-        for (int a = J; a < RB; ++a) {
-            const int i = tr + 16 * a, l = tc + 16 * a;
-            ci[a] = (i > j && i < n) ? rj[i] * r : 0.0;
-            cl[a] = (l > j && l < n) ? rj[l] * r : 0.0;
-        }
-        double *rn = raw + ((j + 1) & 1) * SV_MAXN;
-        if (j < 16 * J + 15) sv_update<RB, J>(v, ci, cl, tr, tc, j, n, rn, Lf, rv);
-        else sv_update<RB, (J + 1 < RB ? J + 1 : J)>(v, ci, cl, tr, tc, j, n, rn, Lf, rv);
-        __syncthreads();
-    }
-    if constexpr (J + 1 < RB) return sv_factor<RB, J + 1>(v, raw, Lf, rv, tr, tc, tid, n);
-    else return true;
-}
+__host__ __device__ __forceinline__ int sv_blocks(int n) { return n < 96 ? 6 : 8; }   // register blocks: n < 16 of them
+// the solve, then the direction and the gradient (floats) and their products (doubles)
+__host__ __device__ __forceinline__ size_t solve_smem(int n) { return chol_smem(n, sv_blocks(n)); }
 
 template <int RB>
 __device__ __forceinline__ void solve_frame(const DModel &m, const DBatch &b, const Cfg &c, int stage, int f,
                                             FrameCtl &ctl, double *sm)
 {
     const int n = m.KT, KTP = m.KTP, K = m.K;
-    const int tid = threadIdx.x, tr = tid & 15, tc = tid >> 4;
-    double *Lf = sm;                     // [n][n] column-major: the factor, for the substitutions
-    double *raw = Lf + (size_t)n * n;    // [2][SV_MAXN] column j before its scaling (by step parity)
-    double *rv = raw + 2 * SV_MAXN;      // [SV_MAXN] reciprocal pivots
-    double *yv = rv + SV_MAXN;           // [SV_MAXN] forward, then back results
+    const int tid = threadIdx.x;
     const float *H = b.H + (size_t)f * KTP * KTP;
     const float *gv = b.g + (size_t)f * KTP;
-    double v[RB][RB];
+    float *d = b.d + (size_t)f * KTP;
     const double lam_d = (double)c.damping;      // damped solve: H + lambda I (0: undamped)
-#pragma unroll
-    for (int a = 0; a < RB; ++a)
-#pragma unroll
-        for (int bb = 0; bb < RB; ++bb) {
-            const int i = tr + 16 * a, l = tc + 16 * bb;
-            v[a][bb] = (i < n && l < n && i >= l) ? (double)H[(size_t)l * KTP + i] : 0.0;
-            if (i == l && i < n) v[a][bb] += lam_d;
-        }
-    // column 0 before scaling, pivot included
-#pragma unroll
-    for (int a = 0; a < RB; ++a)
-        if (tc == 0 && tr + 16 * a < n) raw[tr + 16 * a] = v[a][0];
-    if (tid == 0 && v[0][0] > 0.0) {
-        const double l0 = sqrt(v[0][0]);
-        Lf[0] = l0;
-        rv[0] = __drcp_rn(l0);
-    }
-    __syncthreads();
-    // Columns in register-block groups J (columns 16 J .. 16 J + 15), one instantiation per
-    // group, so that every register block is named by a compile-time index.
-    if (!sv_factor<RB, 0>(v, raw, Lf, rv, tr, tc, tid, n)) {    // block-uniform: the same pivot everywhere
-        float *d = b.d + (size_t)f * KTP;
+    double *xs;
+    const bool ok = chol_solve<RB, false>(
+        n, sm,
+        [&](int i, int l) {
+            const double h = (double)H[(size_t)l * KTP + i];
+            return i == l ? h + lam_d : h;
+        },
+        [&](int l) { return (double)gv[l]; }, xs);
+    if (!ok) {                                   // block-uniform
         for (int i = tid; i < n; i += SV_THREADS) d[i] = __int_as_float(0x7fc00000);
         if (tid == 0) {
             ctl.flags |= FLAG_CHOL_FAILED | FLAG_NAN_DIRECTION;
@@ -2522,33 +2376,15 @@ __device__ __forceinline__ void solve_frame(const DModel &m, const DBatch &b, co
         }
         return;
     }
-    // forward and back substitution in one warp
-    if (tid < 32) {
-        double t[4], rm[4], xm[4];
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int i = tid + 32 * q;
-            t[q] = i < n ? (double)gv[i] : 0.0;
-            rm[q] = i < n ? rv[i] : 0.0;
-            xm[q] = 0.0;
-        }
-        sv_substitute<true>(n, t, rm, xm, Lf);
-        // y_i = t_i r_i: the value the owner of row i broadcast at step i
-#pragma unroll
-        for (int q = 0; q < 4; ++q) t[q] = xm[q];
-        sv_substitute<false>(n, t, rm, xm, Lf);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int i = tid + 32 * q;
-            if (i < n) yv[i] = xm[q];
-        }
+    // direction, its slope and the first trial point (the factor's memory is free again)
+    double *prod = sm;
+    float *dsm = reinterpret_cast<float *>(sm + n);
+    if (tid < n) {
+        const float dv = (float)(-xs[tid]);
+        d[tid] = dv;
+        dsm[tid] = dv;
+        prod[tid] = (double)dv * (double)gv[tid];
     }
-    __syncthreads();
-    const double y = tid < n ? yv[tid] : 0.0;
-    // direction, its slope and the first trial point
-    float *d = b.d + (size_t)f * KTP;
-    float *dsm = reinterpret_cast<float *>(raw);
-    if (tid < n) { const float dv = (float)(-y); d[tid] = dv; dsm[tid] = dv; }
     __syncthreads();
     if (isnan(dsm[0])) {
         if (tid == 0) {
@@ -2564,7 +2400,8 @@ __device__ __forceinline__ void solve_frame(const DModel &m, const DBatch &b, co
     for (int a = tid; a < n_upd; a += SV_THREADS) xl[a] = x[a] + t * dsm[a];
     if (tid == 0) {
         double dg = 0.0;
-        for (int a = 0; a < n; ++a) dg += (double)dsm[a] * (double)gv[a];
+#pragma unroll 8
+        for (int a = 0; a < n; ++a) dg += prod[a];       // (the products are exact)
         ctl.l2base = (float)dg;
         ctl.mode = M_TRIAL;
         ctl.t = t;
@@ -2578,10 +2415,10 @@ __device__ __forceinline__ void solve_frame(const DModel &m, const DBatch &b, co
     }
 }
 
-// RB = 6 register blocks for up to 96 unknowns, 8 up to 128: one kernel each, so that the
+// RB = 6 register blocks for up to 95 unknowns, 8 up to 127: one kernel each, so that the
 // smaller system is not held to the larger one's register count
 template <int RB>
-__global__ void __launch_bounds__(SV_THREADS) k_solve_t(DModel m, DBatch b, Cfg c, int stage)
+__global__ void __launch_bounds__(SV_THREADS, RB == 6 ? 2 : 1) k_solve_t(DModel m, DBatch b, Cfg c, int stage)
 {
     if ((int)blockIdx.x >= active_n(b)) return;
     const int f = b.act[blockIdx.x];
