@@ -277,8 +277,11 @@ tdi_status set_attrs()
 {
     static bool done = false;
     if (done) return TDI_OK;
-    TDI_CUDA(cudaFuncSetAttribute(k_render, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    TDI_CUDA(cudaFuncSetAttribute(k_render_t<512>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   RENDER_SMEM_FLOATS * (int)sizeof(float)));
+    TDI_CUDA(cudaFuncSetAttribute(k_render_t<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  RENDER_SMEM_FLOATS * (int)sizeof(float)));
+    TDI_CUDA(cudaFuncSetAttribute(k_light_fit, cudaFuncAttributeMaxDynamicSharedMemorySize, LIGHT_SMEM));
     TDI_CUDA(cudaFuncSetAttribute(k_neighbours, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)neigh_smem()));
     TDI_CUDA(cudaFuncSetAttribute(k_vertex_t<VT_FPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
@@ -296,9 +299,8 @@ tdi_status set_attrs()
     return TDI_OK;
 }
 
-// Vertex stage grid: frame tiles of nf frames x vertex-tile groups, about VT_BLOCKS_PER_SM
-// blocks per SM.
-dim3 vertex_grid(const DModel &m, int frames, int nf = VT_F)
+// SMs of the current device (148 on B200).
+int sm_count()
 {
     static int sms = 0;
     if (!sms) {
@@ -306,6 +308,14 @@ dim3 vertex_grid(const DModel &m, int frames, int nf = VT_F)
         cudaGetDevice(&dev);
         if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
     }
+    return sms;
+}
+
+// Vertex stage grid: frame tiles of nf frames x vertex-tile groups, about VT_BLOCKS_PER_SM
+// blocks per SM.
+dim3 vertex_grid(const DModel &m, int frames, int nf = VT_F)
+{
+    const int sms = sm_count();
     // the kernel splits the blocks between frame tiles and vertex stripes by the number of
     // frames that render, which is at most `frames`
     const long ftiles = std::max(1, (frames + nf - 1) / nf);
@@ -331,12 +341,7 @@ tdi_status launch_vertex(B *bt, const DModel &m, const DBatch &d, cudaStream_t s
 // Tensor-core vertex stage: one block per SM, split between frame tiles and vertex stripes.
 dim3 vertex_tc_grid(const DModel &m, int frames)
 {
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-    }
+    const int sms = sm_count();
     const long ftiles = std::max(1, (frames + VC_F - 1) / VC_F);
     const long ntiles = (m.V + VC_V - 1) / VC_V;
     return dim3((unsigned)std::max(ftiles, std::min((long)sms, ftiles * ntiles)));
@@ -346,12 +351,7 @@ dim3 vertex_tc_grid(const DModel &m, int frames)
 // launch still spreads over every SM (about five resident blocks per SM).
 unsigned raster_blocks(int frames)
 {
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        cudaGetDevice(&dev);
-        if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) sms = 148;
-    }
+    const int sms = sm_count();
     const int want = (5 * sms + std::max(frames, 1) - 1) / std::max(frames, 1);
     return (unsigned)std::max(RD_BLOCKS, std::min(RD_MAX_BLOCKS, want));
 }
@@ -381,6 +381,7 @@ DBatch batch_view(const tdi_batch *bt, int f0, int nf)
     DBatch v = a;
     v.F = nf;
     v.target = a.target + F0 * NPIX;
+    v.tgn = a.tgn + F0 * NPIX;
     v.xl = a.xl + F0 * NL; v.yl = a.yl + F0 * NL;
     v.bounds = a.bounds + F0 * 4 * NL;
     v.face_size = a.face_size + F0;
@@ -459,10 +460,12 @@ tdi_status geometry(const Launch &L, const Cfg &c, int stage)
     return TDI_OK;
 }
 
-tdi_status render(const Launch &L, const Cfg &c, int stage)
+tdi_status render(const Launch &L, const Cfg &c)
 {
-    return launch(L.bt, KID_RENDER, k_render, dim3(L.A()), dim3(RENDER_THREADS),
-                  RENDER_SMEM_FLOATS * sizeof(float), L.s, L.m, L.b, c, stage);
+    // 1,024 threads per frame while every frame can have an SM to itself, else two blocks of 512 per SM
+    const bool wide = L.A() <= sm_count();
+    return launch(L.bt, KID_RENDER, wide ? k_render_t<1024> : k_render_t<512>, dim3(L.A()), dim3(wide ? 1024 : 512),
+                  RENDER_SMEM_FLOATS * sizeof(float), L.s, L.m, L.b, c);
 }
 
 tdi_status normal_equations(const Launch &L, const Cfg &c, int stage)
@@ -490,27 +493,29 @@ tdi_status normal_equations(const Launch &L, const Cfg &c, int stage)
     return TDI_OK;
 }
 
-// One round of a stage for the frames of b (launched on s).
-tdi_status stage_round(tdi_batch *bt, const Cfg &c, int stage, const DBatch &b, cudaStream_t s, long round)
+// One round of a shape stage for the frames of b (launched on s).
+tdi_status stage_round(tdi_batch *bt, const Cfg &c, int stage, const DBatch &b, cudaStream_t s)
 {
     const DModel &m = bt->m->d;
     Launch L{bt, m, b, s, b.F};
     TDI_TRY(launch(bt, 0, k_prepare, L.wblocks(), dim3(128), 0, s, m, b, stage));
-    if (stage == ST_LAMBDA) {
-        if (round == 0) {
-            TDI_TRY(geometry(L, c, stage));
-            TDI_TRY(launch(bt, KID_NEIGHBOURS, k_neighbours, dim3(L.A()), dim3(1024), L.smem_neigh(), s, b, 1));
-        }
-        TDI_TRY(render(L, c, stage));
-        TDI_TRY(launch(bt, 0, k_decide_lambda, L.ablocks(), dim3(128), 0, s, m, b, c));
-        TDI_TRY(launch(bt, 0, k_lambda_jac, dim3(L.A()), dim3(256), 0, s, m, b, c));
-    } else {
-        TDI_TRY(geometry(L, c, stage));
-        TDI_TRY(render(L, c, stage));
-        TDI_TRY(launch(bt, 0, k_decide_shape, L.ablocks(), dim3(128), 0, s, m, b, c, stage));
-        TDI_TRY(normal_equations(L, c, stage));
-    }
-    return TDI_OK;
+    TDI_TRY(geometry(L, c, stage));
+    TDI_TRY(render(L, c));
+    TDI_TRY(launch(bt, 0, k_decide_shape, L.ablocks(), dim3(128), 0, s, m, b, c, stage));
+    return normal_equations(L, c, stage);
+}
+
+// The whole light fit of a lane's running frames: their raster and neighbour maps, then every
+// frame's line search in one launch.
+tdi_status light_fit(tdi_batch *bt, const Cfg &c, const DBatch &b, cudaStream_t s, long max_rounds)
+{
+    const DModel &m = bt->m->d;
+    Launch L{bt, m, b, s, b.F};
+    TDI_TRY(launch(bt, 0, k_prepare, L.wblocks(), dim3(128), 0, s, m, b, (int)ST_LAMBDA));
+    TDI_TRY(geometry(L, c, ST_LAMBDA));
+    TDI_TRY(launch(bt, KID_NEIGHBOURS, k_neighbours, dim3(L.A()), dim3(1024), L.smem_neigh(), s, b, 1));
+    return launch(bt, 0, k_light_fit, dim3(L.A()), dim3(LIGHT_THREADS), (size_t)LIGHT_SMEM, s, m, b,
+                  c, max_rounds);
 }
 
 // Rounds replayed from CUDA graphs. A graph holds GRAPH_ROUNDS rounds of a stage, each followed by
@@ -544,7 +549,7 @@ tdi_status stage_graph(tdi_batch *bt, const Cfg &c, int stage, int lane, int tie
     TDI_CUDA(cudaStreamBeginCapture(ln.s, cudaStreamCaptureModeThreadLocal));
     tdi_status st = TDI_OK;
     for (int r = 0; r < GRAPH_ROUNDS && st == TDI_OK; ++r) {
-        st = stage_round(bt, c, stage, gv, ln.s, 1 + r);
+        st = stage_round(bt, c, stage, gv, ln.s);
         if (st == TDI_OK)
             st = launch(bt, 0, k_compact_active, dim3(1), dim3(1024), 0, ln.s, (const DBatch)gv, ln.d_count);
     }
@@ -563,31 +568,23 @@ tdi_status stage_graph(tdi_batch *bt, const Cfg &c, int stage, int lane, int tie
     return TDI_OK;
 }
 
-// A stage with its rounds replayed from graphs (no live profiling): every lane's replay is
-// enqueued on its stream before any lane's count is read back.
-tdi_status run_stage_graphs(tdi_batch *bt, const Cfg &c, int stage, int nlanes)
+// Starts a stage: every lane's running frames counted (lanes' streams are waited for).
+tdi_status stage_begin(tdi_batch *bt, const Cfg &c, int stage, int nlanes)
 {
-    const DModel &m = bt->m->d;
     for (int l = 0; l < nlanes; ++l) {
         tdi_lane &ln = bt->lanes[l];
-        TDI_TRY(launch(bt, 0, k_stage_start, dim3((ln.d.F + 127) / 128), dim3(128), 0, ln.s, m, ln.d, c, stage));
+        TDI_TRY(launch(bt, 0, k_stage_start, dim3((ln.d.F + 127) / 128), dim3(128), 0, ln.s, bt->m->d, ln.d, c, stage));
         TDI_TRY(lane_compact(bt, ln));
     }
     for (int l = 0; l < nlanes; ++l) TDI_TRY(lane_count(bt->lanes[l]));
-    const long max_rounds = stage == ST_LAMBDA ? 8L * c.max_iters_lambda + 16
-                                               : 16L * (stage == ST_RIGID ? c.max_iters_rigid : c.max_iters_finetune) + 16;
+    return TDI_OK;
+}
+
+// A shape stage with its rounds replayed from graphs (no live profiling): every lane's replay is
+// enqueued on its stream before any lane's count is read back.
+tdi_status run_stage_graphs(tdi_batch *bt, const Cfg &c, int stage, int nlanes, long max_rounds)
+{
     long round[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    if (stage == ST_LAMBDA) {                   // the light fit's first round also rasterises
-        for (int l = 0; l < nlanes; ++l) {
-            tdi_lane &ln = bt->lanes[l];
-            if (ln.n <= 0) continue;
-            TDI_TRY(stage_round(bt, c, stage, ln.d, ln.s, 0));
-            TDI_TRY(lane_compact(bt, ln));
-            round[l] = 1;
-        }
-        for (int l = 0; l < nlanes; ++l)
-            if (round[l]) TDI_TRY(lane_count(bt->lanes[l]));
-    }
     for (;;) {
         bool launched[8] = {false, false, false, false, false, false, false, false}, any = false;
         for (int l = 0; l < nlanes; ++l) {
@@ -612,23 +609,22 @@ tdi_status run_stage_graphs(tdi_batch *bt, const Cfg &c, int stage, int nlanes)
 // the lanes' rounds are enqueued on their own streams before any lane is waited for.
 tdi_status run_stage_lanes(tdi_batch *bt, const Cfg &c, int stage, int nlanes)
 {
-    if (!c.host_rounds && bt->prof_id == 0) return run_stage_graphs(bt, c, stage, nlanes);
-    const DModel &m = bt->m->d;
-    for (int l = 0; l < nlanes; ++l) {
-        tdi_lane &ln = bt->lanes[l];
-        TDI_TRY(launch(bt, 0, k_stage_start, dim3((ln.d.F + 127) / 128), dim3(128), 0, ln.s, m, ln.d, c, stage));
-        TDI_TRY(lane_compact(bt, ln));
+    TDI_TRY(stage_begin(bt, c, stage, nlanes));
+    if (stage == ST_LAMBDA) {
+        for (int l = 0; l < nlanes; ++l)
+            if (bt->lanes[l].n > 0)
+                TDI_TRY(light_fit(bt, c, bt->lanes[l].d, bt->lanes[l].s, 8L * c.max_iters_lambda + 16));
+        return TDI_OK;
     }
-    for (int l = 0; l < nlanes; ++l) TDI_TRY(lane_count(bt->lanes[l]));
-    const long max_rounds = stage == ST_LAMBDA ? 8L * c.max_iters_lambda + 16
-                                               : 16L * (stage == ST_RIGID ? c.max_iters_rigid : c.max_iters_finetune) + 16;
+    const long max_rounds = 16L * (stage == ST_RIGID ? c.max_iters_rigid : c.max_iters_finetune) + 16;
+    if (!c.host_rounds && bt->prof_id == 0) return run_stage_graphs(bt, c, stage, nlanes, max_rounds);
     for (long round = 0; round < max_rounds; ++round) {
         bool any = false;
         for (int l = 0; l < nlanes; ++l) {
             tdi_lane &ln = bt->lanes[l];
             if (ln.n <= 0) continue;
             any = true;
-            TDI_TRY(stage_round(bt, c, stage, ln.d, ln.s, round));
+            TDI_TRY(stage_round(bt, c, stage, ln.d, ln.s));
             TDI_TRY(lane_compact(bt, ln));
         }
         if (!any) break;
@@ -814,7 +810,7 @@ tdi_status tdi_batch_create(tdi_model *m, int32_t max_frames, tdi_batch **out)
     int32_t *x0y0;
     tdi_status st = TDI_OK;
 #define A(ptr, n) if (st == TDI_OK) st = dalloc(b->allocs, &ptr, (n))
-    A(target, F * NPIX); A(b->target_raw, F * NPIX); A(b->prep, F); A(xl, F * NL); A(yl, F * NL);
+    A(target, F * NPIX); A(d.tgn, F * NPIX); A(b->target_raw, F * NPIX); A(b->prep, F); A(xl, F * NL); A(yl, F * NL);
     A(bounds, F * 4 * NL); A(fs, F); A(cam, F * 4); A(x0y0, F * 2); A(Lint, F);
     A(d.x, F * KTP); A(d.x_ls, F * KTP); A(d.xe, F * KTP);
     A(d.lam, F * 4); A(d.lam_ls, F * 4); A(d.lame, F * 4); A(d.dlam, F * 4); A(d.glam, F * 4);
@@ -985,6 +981,7 @@ static tdi_status blur_targets(tdi_batch *b, const Cfg &c, cudaStream_t s)
     TDI_TRY(launch(b, 0, k_blur_rows_full, blocks, dim3(256), 0, s, (const float *)b->target_raw, b->d.img, c, b->d.F));
     // img holds 2*NPIX floats per frame; the row pass above used the first F*NPIX floats
     TDI_TRY(launch(b, 0, k_blur_cols_full, blocks, dim3(256), 0, s, (const float *)b->d.img, (float *)b->d.target, c, b->d.F));
+    TDI_TRY(launch(b, 0, k_target_grad, blocks, dim3(256), 0, s, (const float *)b->d.target, b->d.tgn, b->d.F));
     return TDI_OK;
 }
 
@@ -1101,7 +1098,7 @@ tdi_status tdi_batch_evaluate(tdi_batch *b, const tdi_fit_config *cfg, int32_t f
     if (n == 0) return TDI_OK;
     TDI_TRY(launch(b, 0, k_prepare, L.wblocks(), dim3(128), 0, s, m, d, stage));
     TDI_TRY(geometry(L, c, stage));
-    TDI_TRY(render(L, c, stage));
+    TDI_TRY(render(L, c));
     TDI_TRY(launch(b, 0, k_decide_shape, L.ablocks(), dim3(128), 0, s, m, d, c, stage));
     TDI_TRY(normal_equations(L, c, stage));
     TDI_TRY(launch(b, 0, k_scalars, L.fblocks(), dim3(128), 0, s, d, b->scalars));

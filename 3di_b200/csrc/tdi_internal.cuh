@@ -106,6 +106,7 @@ struct DBatch {
     int32_t F;               // frames in this batch
     // inputs
     const float *target;     // [F][NPIX] blurred crops
+    float2 *tgn;             // [F][NPIX] their normalised gradients
     const float *xl, *yl;    // [F][NL]
     const float *bounds;     // [F][4][NL]
     const float *face_size;  // [F]

@@ -1276,205 +1276,257 @@ __device__ __forceinline__ void neighbour_pixels(int p, int &kr, int &kl, int &k
 // Region of the render: the fragment box + 8 px, or the whole crop when the fragments touch
 // its border (a border pixel's neighbour is pixel 0). Blur taps are summed in ascending
 // offset order with zeros outside the region (rows along y, then columns along x).
-// The region buffers carry KRAD zero lines on the blurred side, so the taps need no bounds
-// test: A[xl][KRAD + yl] (pitch rh + 2 KRAD) holds the shaded image and later the blurred
-// one, B[KRAD + xl][yl] (pitch rh) the row pass. They live in shared memory when they fit,
-// else in the frame's global buffer. Fragment gathers are issued RENDER_U at a time before
-// their results are stored.
+// The region buffers carry zero lines on the blurred side, so the taps need no bounds test:
+// A[xl][RPAD + yl] (pitch pb + 2 RPAD) holds the shaded image and later the blurred one,
+// B[KRAD + xl][yl] (pitch pb, rh rounded up to even) the row pass. They live in shared memory
+// when they fit, else in the frame's global buffer.
+// Each blur thread forms a run of outputs along the taps' direction from a sliding window (a
+// value is read (RUN + 14) / RUN times instead of 15) on two lines at once, with packed FP32
+// products and sums (each half rounds as the scalar operation does). Runs of 9 along y put a
+// warp's lanes on distinct banks; the last run of a line is moved back to end at the line's end
+// (its first outputs are formed twice, with the same values).
 
-constexpr int RENDER_THREADS = 512;
-constexpr int RENDER_SMEM_FLOATS = 27 * 1024;     // padded region buffers (108 KB): two blocks per SM
-constexpr int RENDER_U = 2;                       // fragments whose gathers are in flight together
-constexpr int RENDER_GU = 2;                      // the same in the gradient pass (8 loads each)
+constexpr int LIGHT_THREADS = 1024;               // the light fit's renders
+constexpr int RENDER_SMEM_FLOATS = 27 * 1024;     // padded region buffers (108 KB)
+constexpr int RENDER_GU = 4;                      // fragments in flight in the gradient pass
 constexpr int RENDER_SU = 4;                      // the same when shading from the resolve's terms
-constexpr int RIMG = 2 * DIM * (DIM + 2 * KRAD);  // per-frame floats of the global fallback
+constexpr int RPAD = 8;                           // zero columns left and right of A's lines (KRAD used)
+constexpr int RUN_Y = 9, RUN_X = 8;               // outputs per thread and line of the row and column pass
+constexpr int RIMG = 2 * DIM * (DIM + 2 * RPAD);  // per-frame floats of the global fallback
 
-__host__ __device__ __forceinline__ int region_floats(int rw, int rh)
+struct Region {
+    int rx0, ry0, rw, rh, pb, ph;
+    float *A, *B;
+    __device__ __forceinline__ int at(int p) const { return ((p >> 8) - rx0) * ph + RPAD + ((p & 255) - ry0); }
+};
+
+// The frame's region; its buffers at smem when they fit, else in the frame's global buffer.
+__device__ __forceinline__ Region make_region(const FrameCtl &ctl, float *smem, float *global)
 {
-    return rw * (rh + 2 * KRAD) + (rw + 2 * KRAD) * rh;
+    const bool border = ctl.bbox[0] < 1 || ctl.bbox[1] > DIM - 2 || ctl.bbox[2] < 1 || ctl.bbox[3] > DIM - 2;
+    Region r;
+    r.rx0 = border ? 0 : max(0, ctl.bbox[0] - 8);
+    r.ry0 = border ? 0 : max(0, ctl.bbox[2] - 8);
+    r.rw = (border ? DIM - 1 : min(DIM - 1, ctl.bbox[1] + 8)) - r.rx0 + 1;
+    r.rh = (border ? DIM - 1 : min(DIM - 1, ctl.bbox[3] + 8)) - r.ry0 + 1;
+    r.pb = (r.rh + 1) & ~1;
+    r.ph = r.pb + 2 * RPAD;
+    // (an odd region's last row pair reads one line past A: B's first)
+    r.A = r.rw * r.ph + (r.rw + 2 * KRAD) * r.pb <= RENDER_SMEM_FLOATS ? smem : global;
+    r.B = r.A + r.rw * r.ph;
+    return r;
 }
 
-template <bool SMEM>
-__device__ __forceinline__ void render_region(const DModel &m, const DBatch &b, const Cfg &c, int stage,
-                                              int f, FrameCtl &ctl, float *A, float *B, int rx0,
-                                              int ry0, int rw, int rh, double *s_red)
+// A zeroed; with pads, B's zero lines too (they stay zero).
+template <int NT>
+__device__ __forceinline__ void region_clear(const Region &r, bool pads)
 {
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    constexpr int NW = RENDER_THREADS / 32;
-    const int N = ctl.N;
-    const int ph = rh + 2 * KRAD;
-    for (int i = tid; i < rw * ph; i += RENDER_THREADS) A[i] = 0.0f;
-    for (int i = tid; i < KRAD * rh; i += RENDER_THREADS) { B[i] = 0.0f; B[(KRAD + rw) * rh + i] = 0.0f; }
-    __syncthreads();
-    const float4 *geo = b.geo + (size_t)f * m.V;
-    const float *R = b.R + f * 9;
-    const float *xsrc = stage == ST_LAMBDA ? b.x : b.xe;
-    const float *tau = xsrc + (size_t)f * m.KTP + m.K;
-    const float *lam = (stage == ST_LAMBDA && ctl.mode == M_TRIAL) ? b.lam_ls + f * 4 : b.lam + f * 4;
-    const float Lint = b.Lint[f];
-    const Fragment *frags = b.frag + (size_t)f * NMAX;
-    auto at = [&](int p) { return ((p >> 8) - rx0) * ph + KRAD + ((p & 255) - ry0); };
-    if (stage == ST_LAMBDA || ctl.shade_cached) {
-        // Each fragment's unit normal, n . p and interpolated albedo depend only on the geometry
-        // of the raster: the resolve forms them (shc, sht) for every raster that renders, and
-        // the light fit, which moves only the light, keeps them for all its renders and for
-        // k_lambda_jac (a render that finds them missing forms them itself). A render forms
-        // only the rotated light R^T (lambda - tau), once, and the same FP32 operations as
-        // shade(): Id = (n0 q0 + n1 q1) + n2 q2 - n.p, I = t + (L t) Id.
-        float4 *shc = b.shc + (size_t)f * NMAX;
-        float *sht = b.sht + (size_t)f * NMAX;
-        const bool cached = ctl.shade_cached != 0;
-        const float d0 = lam[0] - tau[0], d1 = lam[1] - tau[1], d2 = lam[2] - tau[2];
-        const float q0 = (R[0] * d0 + R[1] * d1) + R[2] * d2;
-        const float q1 = (R[3] * d0 + R[4] * d1) + R[5] * d2;
-        const float q2 = (R[6] * d0 + R[7] * d1) + R[8] * d2;
-        if (cached) {
-            // RENDER_SU fragments per thread: each one's pixel word and shading terms are loaded
-            // together (the terms are indexed by the fragment, not by its contents)
-            for (int n0 = tid; n0 < N; n0 += RENDER_THREADS * RENDER_SU) {
-                uint32_t po[RENDER_SU];
-                float4 sn[RENDER_SU];
-                float t[RENDER_SU];
+    float2 *A = reinterpret_cast<float2 *>(r.A);
+    for (int i = threadIdx.x; i < r.rw * (r.ph >> 1); i += NT) A[i] = make_float2(0.0f, 0.0f);
+    if (pads)
+        for (int i = threadIdx.x; i < KRAD * r.pb; i += NT) {
+            r.B[i] = 0.0f;
+            r.B[(KRAD + r.rw) * r.pb + i] = 0.0f;
+        }
+}
+
+__device__ __forceinline__ float2 fmul2(float2 a, float2 b)
+{
+    float2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;"
+        : "=l"(reinterpret_cast<unsigned long long &>(d))
+        : "l"(reinterpret_cast<const unsigned long long &>(a)), "l"(reinterpret_cast<const unsigned long long &>(b)));
+    return d;
+}
+
+// 1 in both halves, from a value the compiler cannot know (normal_eq is 0 or 1). Packed products and
+// packed sums are contracted into packed fused multiply-adds by the assembler, .rn or not (measured:
+// every result equals fma's); a sum written as fma(p, 1, s) with an unknown 1 keeps the product's
+// own rounding and rounds as p + s.
+__device__ __forceinline__ float2 packed_one(const Cfg &c)
+{
+    const float u = __int_as_float(0x3f800000 | (c.normal_eq & 2));
+    return make_float2(u, u);
+}
+
+// Row pass A -> B, column pass B -> A (the shaded image in A, then the blurred one).
+template <int NT>
+__device__ __forceinline__ void region_blur(const Region &r, const Cfg &c)
+{
+    const int tid = threadIdx.x;
+    const float2 one = packed_one(c);
+    float2 tap[NTAPS];                                   // tap[j]: the weight of offset j - KRAD, in both halves
 #pragma unroll
-                for (int u = 0; u < RENDER_SU; ++u) {
-                    const int n = n0 + u * RENDER_THREADS;
-                    po[u] = 0u;
-                    if (n < N) {
-                        po[u] = frags[n].pix_owner;
-                        sn[u] = shc[n];
-                        t[u] = sht[n];
-                    }
-                }
+    for (int j = 0; j < NTAPS; ++j) tap[j] = make_float2(c.taps[2 * KRAD - j], c.taps[2 * KRAD - j]);
+    {
+        const int nrun = (r.rh + RUN_Y - 1) / RUN_Y, npair = (r.rw + 1) >> 1;
+        for (int i = tid; i < npair * nrun; i += NT) {
+            const int xl = i / nrun, y0 = min((i - xl * nrun) * RUN_Y, r.rh - RUN_Y);
+            const float *a0 = r.A + 2 * xl * r.ph + RPAD - KRAD + y0, *a1 = a0 + r.ph;   // a0[t] = A(2 xl, y0 - KRAD + t)
+            float2 s[RUN_Y];
 #pragma unroll
-                for (int u = 0; u < RENDER_SU; ++u)
-                    if (po[u] & 0x80000000u) {
-                        const float Id = ((sn[u].x * q0 + sn[u].y * q1) + sn[u].z * q2) - sn[u].w;
-                        A[at(po[u] & 0xFFFF)] = t[u] + (Lint * t[u]) * Id;
-                    }
+            for (int o = 0; o < RUN_Y; ++o) s[o] = make_float2(0.0f, 0.0f);
+#pragma unroll
+            for (int t = 0; t < RUN_Y + 2 * KRAD; ++t) {
+                const float2 v = make_float2(a0[t], a1[t]);
+#pragma unroll
+                for (int o = 0; o < RUN_Y; ++o)
+                    if (t >= o && t - o <= 2 * KRAD) s[o] = ffma2(fmul2(tap[t - o], v), one, s[o]);
             }
-        } else
-        for (int n = tid; n < N; n += RENDER_THREADS) {
-            const Fragment fr = frags[n];
-            const Shading s = shade(m, geo, fr, R, tau, lam, Lint);
-            const float4 sn = make_float4(s.nn[0], s.nn[1], s.nn[2],
-                                          (s.nn[0] * s.p[0] + s.nn[1] * s.p[1]) + s.nn[2] * s.p[2]);
-            const float t = s.t;
-            shc[n] = sn;
-            sht[n] = t;
-            if (fr.pix_owner & 0x80000000u) {
-                const float Id = ((sn.x * q0 + sn.y * q1) + sn.z * q2) - sn.w;
-                A[at(fr.pix_owner & 0xFFFF)] = t + (Lint * t) * Id;
+            float *q = r.B + (KRAD + 2 * xl) * r.pb + y0;
+#pragma unroll
+            for (int o = 0; o < RUN_Y; ++o) q[o] = s[o].x;
+            if (2 * xl + 1 < r.rw) {
+#pragma unroll
+                for (int o = 0; o < RUN_Y; ++o) q[r.pb + o] = s[o].y;
             }
         }
-        if (tid == 0) ctl.shade_cached = 1;
-    } else
-    for (int n0 = tid; n0 < N; n0 += RENDER_THREADS * RENDER_U) {
-        Fragment fr[RENDER_U];
+    }
+    __syncthreads();
+    {
+        const int nrun = (r.rw + RUN_X - 1) / RUN_X, npair = r.pb >> 1;
+        for (int i = tid; i < npair * nrun; i += NT) {
+            const int g = i / npair, yl = 2 * (i - g * npair), x0 = min(g * RUN_X, r.rw - RUN_X);
+            const float *bp = r.B + x0 * r.pb + yl;                    // bp[t pb] = B(x0 - KRAD + t, yl)
+            float2 s[RUN_X];
 #pragma unroll
-        for (int u = 0; u < RENDER_U; ++u) {
-            const int n = n0 + u * RENDER_THREADS;
-            fr[u] = n < N ? frags[n] : Fragment{0u, 0, 0.0f, 0.0f};
-        }
-        float tex[RENDER_U];
-        int idx[RENDER_U];
+            for (int o = 0; o < RUN_X; ++o) s[o] = make_float2(0.0f, 0.0f);
 #pragma unroll
-        for (int u = 0; u < RENDER_U; ++u) {
-            idx[u] = -1;
-            tex[u] = 0.0f;
-            if (fr[u].pix_owner & 0x80000000u) {
-                tex[u] = shade(m, geo, fr[u], R, tau, lam, Lint).tex;
-                idx[u] = at(fr[u].pix_owner & 0xFFFF);
+            for (int t = 0; t < RUN_X + 2 * KRAD; ++t) {
+                const float2 v = *reinterpret_cast<const float2 *>(bp + t * r.pb);
+#pragma unroll
+                for (int o = 0; o < RUN_X; ++o)
+                    if (t >= o && t - o <= 2 * KRAD) s[o] = ffma2(fmul2(tap[t - o], v), one, s[o]);
             }
+            float *q = r.A + x0 * r.ph + RPAD + yl;
+#pragma unroll
+            for (int o = 0; o < RUN_X; ++o) *reinterpret_cast<float2 *>(q + o * r.ph) = s[o];
         }
-#pragma unroll
-        for (int u = 0; u < RENDER_U; ++u)
-            if (idx[u] >= 0) A[idx[u]] = tex[u];
     }
     __syncthreads();
-    const uint32_t mgh = 0xFFFFFFFFu / (uint32_t)rh + 1u;   // i / rh = umulhi(i, mgh) for i <= 2^16
-    // rows: along the contiguous (y) index
-    for (int i = tid; i < rw * rh; i += RENDER_THREADS) {
-        const int xl = (int)__umulhi((uint32_t)i, mgh), yl = i - xl * rh;
-        const float *a = A + xl * ph + yl;               // a[KRAD + j] = A(xl, yl + j)
-        float s = 0.0f;
+}
+
+// The rotated light R^T (lambda - tau) of a render.
+__device__ __forceinline__ void light_terms(const float *R, const float *tau, const float *lam, float (&q)[3])
+{
+    const float d0 = lam[0] - tau[0], d1 = lam[1] - tau[1], d2 = lam[2] - tau[2];
+    q[0] = (R[0] * d0 + R[1] * d1) + R[2] * d2;
+    q[1] = (R[3] * d0 + R[4] * d1) + R[5] * d2;
+    q[2] = (R[6] * d0 + R[7] * d1) + R[8] * d2;
+}
+
+// Owners shaded into the cleared region. Each fragment's unit normal, n . p and interpolated
+// albedo depend only on the geometry of the raster: the resolve forms them (shc, sht) for every
+// raster that renders. A render forms the rotated light once and the same FP32 operations as
+// shade(): Id = (n0 q0 + n1 q1) + n2 q2 - n.p, I = t + (L t) Id. RENDER_SU fragments per thread:
+// each one's pixel word and shading terms are loaded together.
+template <int NT>
+__device__ __forceinline__ void region_shade(const Region &r, const Fragment *frags, const float4 *shc,
+                                             const float *sht, int N, const float (&q)[3], float Lint)
+{
+    for (int n0 = threadIdx.x; n0 < N; n0 += NT * RENDER_SU) {
+        uint32_t po[RENDER_SU];
+        float4 sn[RENDER_SU];
+        float t[RENDER_SU];
 #pragma unroll
-        for (int j = -KRAD; j <= KRAD; ++j) s = s + c.taps[KRAD - j] * a[KRAD + j];
-        B[(KRAD + xl) * rh + yl] = s;
-    }
-    __syncthreads();
-    // columns: along the strided (x) index
-    for (int i = tid; i < rw * rh; i += RENDER_THREADS) {
-        const int xl = (int)__umulhi((uint32_t)i, mgh), yl = i - xl * rh;
-        const float *bp = B + xl * rh + yl;              // bp[(KRAD + j) * rh] = B(xl + j, yl)
-        float s = 0.0f;
-#pragma unroll
-        for (int j = -KRAD; j <= KRAD; ++j) s = s + c.taps[KRAD - j] * bp[(KRAD + j) * rh];
-        A[xl * ph + KRAD + yl] = s;
-    }
-    __syncthreads();
-    const float *tgt = b.target + (size_t)f * NPIX;
-    float *fg = b.fgrad + (size_t)f * 5 * NMAX;
-    double corr = 0.0;
-    for (int n0 = tid; n0 < N; n0 += RENDER_THREADS * RENDER_GU) {
-        int pv[RENDER_GU];
-#pragma unroll
-        for (int u = 0; u < RENDER_GU; ++u) {
-            const int n = n0 + u * RENDER_THREADS;
-            pv[u] = n < N ? (int)(frags[n].pix_owner & 0xFFFF) : -1;
-        }
-        float rv[RENDER_GU][4], tv[RENDER_GU][4];
-#pragma unroll
-        for (int u = 0; u < RENDER_GU; ++u) {
-            rv[u][0] = rv[u][1] = rv[u][2] = rv[u][3] = 0.0f;
-            tv[u][0] = tv[u][1] = tv[u][2] = tv[u][3] = 0.0f;
-            if (pv[u] >= 0) {                  // (pixel 0 lies outside a region that is not the crop)
-                int kr, kl, kd, ku;
-                neighbour_pixels(pv[u], kr, kl, kd, ku);
-                rv[u][0] = A[at(kr)]; rv[u][1] = A[at(kl)]; rv[u][2] = A[at(kd)]; rv[u][3] = A[at(ku)];
-                tv[u][0] = tgt[kr]; tv[u][1] = tgt[kl]; tv[u][2] = tgt[kd]; tv[u][3] = tgt[ku];
+        for (int u = 0; u < RENDER_SU; ++u) {
+            const int n = n0 + u * NT;
+            po[u] = 0u;
+            if (n < N) {
+                po[u] = frags[n].pix_owner;
+                sn[u] = shc[n];
+                t[u] = sht[n];
             }
         }
 #pragma unroll
-        for (int u = 0; u < RENDER_GU; ++u) {
-            if (pv[u] < 0) break;
-            const int n = n0 + u * RENDER_THREADS;
-            float gx, gy, h, gxn, gyn, sx, sy, sh, sxn, syn;
-            grad_of(rv[u][0], rv[u][1], rv[u][2], rv[u][3], gx, gy, h, gxn, gyn);
-            grad_of(tv[u][0], tv[u][1], tv[u][2], tv[u][3], sx, sy, sh, sxn, syn);
-            fg[n] = gx; fg[NMAX + n] = gy; fg[2 * NMAX + n] = h;
-            fg[3 * NMAX + n] = sxn; fg[4 * NMAX + n] = syn;
-            corr += (double)gxn * (double)sxn + (double)gyn * (double)syn;
-        }
-    }
-    for (int o = 16; o > 0; o >>= 1) corr += __shfl_down_sync(0xffffffffu, corr, o);
-    if (lane == 0) s_red[warp] = corr;
-    __syncthreads();
-    if (tid == 0) {
-        double s = 0.0;
-        for (int w = 0; w < NW; ++w) s += s_red[w];
-        ctl.corr = s;
+        for (int u = 0; u < RENDER_SU; ++u)
+            if (po[u] & 0x80000000u) {
+                const float Id = ((sn[u].x * q[0] + sn[u].y * q[1]) + sn[u].z * q[2]) - sn[u].w;
+                r.A[r.at(po[u] & 0xFFFF)] = t[u] + (Lint * t[u]) * Id;
+            }
     }
 }
 
-__global__ void __launch_bounds__(RENDER_THREADS, 2) k_render(DModel m, DBatch b, Cfg c, int stage)
+// FP64 sum of a block's values: shuffles, then the warps in order; the total in thread 0.
+template <int NT>
+__device__ __forceinline__ double render_sum(double v, double *s_red)
+{
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = v;
+    __syncthreads();
+    double s = 0.0;
+    if (threadIdx.x == 0)
+        for (int w = 0; w < NT / 32; ++w) s += s_red[w];
+    return s;
+}
+
+// Normalised gradients of the blurred targets at every pixel, once per fit: a render reads one
+// 8-byte value per fragment instead of forming them from four gathered pixels.
+__global__ void k_target_grad(const float *target, float2 *tgn, int F)
+{
+    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (size_t)F * NPIX) return;
+    const int p = (int)(i & (NPIX - 1));
+    const float *t = target + (i - p);
+    int kr, kl, kd, ku;
+    neighbour_pixels(p, kr, kl, kd, ku);
+    float gx, gy, h;
+    float2 g;
+    grad_of(t[kr], t[kl], t[kd], t[ku], gx, gy, h, g.x, g.y);
+    tgn[i] = g;
+}
+
+// NT threads per frame: 512 (two blocks per SM) for full rounds, 1,024 when the frames do not
+// fill the SMs and a block's own latency is the round's.
+template <int NT>
+__global__ void __launch_bounds__(NT, 1024 / NT) k_render_t(DModel m, DBatch b, Cfg c)
 {
     if ((int)blockIdx.x >= active_n(b)) return;
     const int f = b.act[blockIdx.x];
     FrameCtl &ctl = b.ctl[f];
     if (!ctl.render) return;
-    if (threadIdx.x == 0) prof_count(b, KID_RENDER);
+    const int tid = threadIdx.x;
+    if (tid == 0) prof_count(b, KID_RENDER);
     extern __shared__ __align__(16) float rsm[];
-    __shared__ double s_red[RENDER_THREADS / 32];
-    const bool border = ctl.bbox[0] < 1 || ctl.bbox[1] > DIM - 2 || ctl.bbox[2] < 1 || ctl.bbox[3] > DIM - 2;
-    const int rx0 = border ? 0 : max(0, ctl.bbox[0] - 8), rx1 = border ? DIM - 1 : min(DIM - 1, ctl.bbox[1] + 8);
-    const int ry0 = border ? 0 : max(0, ctl.bbox[2] - 8), ry1 = border ? DIM - 1 : min(DIM - 1, ctl.bbox[3] + 8);
-    const int rw = rx1 - rx0 + 1, rh = ry1 - ry0 + 1;
-    if (region_floats(rw, rh) <= RENDER_SMEM_FLOATS) {
-        render_region<true>(m, b, c, stage, f, ctl, rsm, rsm + rw * (rh + 2 * KRAD), rx0, ry0, rw, rh, s_red);
-    } else {
-        float *g = b.img + (size_t)f * RIMG;
-        render_region<false>(m, b, c, stage, f, ctl, g, g + rw * (rh + 2 * KRAD), rx0, ry0, rw, rh, s_red);
+    __shared__ double s_red[NT / 32];
+    const Region r = make_region(ctl, rsm, b.img + (size_t)f * RIMG);
+    const int N = ctl.N;
+    const Fragment *frags = b.frag + (size_t)f * NMAX;
+    region_clear<NT>(r, true);
+    float q[3];
+    light_terms(b.R + f * 9, b.xe + (size_t)f * m.KTP + m.K, b.lam + f * 4, q);
+    __syncthreads();
+    region_shade<NT>(r, frags, b.shc + (size_t)f * NMAX, b.sht + (size_t)f * NMAX, N, q, b.Lint[f]);
+    __syncthreads();
+    region_blur<NT>(r, c);
+    const float2 *tgn = b.tgn + (size_t)f * NPIX;
+    float *fg = b.fgrad + (size_t)f * 5 * NMAX;
+    double corr = 0.0;
+    for (int n0 = tid; n0 < N; n0 += NT * RENDER_GU) {
+        int pv[RENDER_GU];
+        float2 tg[RENDER_GU];
+#pragma unroll
+        for (int u = 0; u < RENDER_GU; ++u) {
+            const int n = n0 + u * NT;
+            pv[u] = n < N ? (int)(frags[n].pix_owner & 0xFFFF) : -1;
+        }
+#pragma unroll
+        for (int u = 0; u < RENDER_GU; ++u) tg[u] = pv[u] >= 0 ? tgn[pv[u]] : make_float2(0.0f, 0.0f);
+#pragma unroll
+        for (int u = 0; u < RENDER_GU; ++u) {
+            if (pv[u] < 0) break;
+            const int n = n0 + u * NT;
+            int kr, kl, kd, ku;                // (pixel 0 lies outside a region that is not the crop)
+            neighbour_pixels(pv[u], kr, kl, kd, ku);
+            float gx, gy, h, gxn, gyn;
+            grad_of(r.A[r.at(kr)], r.A[r.at(kl)], r.A[r.at(kd)], r.A[r.at(ku)], gx, gy, h, gxn, gyn);
+            fg[n] = gx; fg[NMAX + n] = gy; fg[2 * NMAX + n] = h;
+            fg[3 * NMAX + n] = tg[u].x; fg[4 * NMAX + n] = tg[u].y;
+            corr += (double)gxn * (double)tg[u].x + (double)gyn * (double)tg[u].y;
+        }
     }
+    const double total = render_sum<NT>(corr, s_red);
+    if (tid == 0) ctl.corr = total;
 }
 
 // ------------------------------------------------------------------------------------------
@@ -1516,39 +1568,6 @@ __global__ void k_decide_shape(DModel m, DBatch b, Cfg c, int stage)
         ctl.need_jac = 1;
     } else {
         shape_reject(m, b, c, f, stage);
-    }
-}
-
-// Light fit (model_fitter.cu:981-1073): objective -corr; Armijo test with alpha = beta = 0.5.
-__global__ void k_decide_lambda(DModel m, DBatch b, Cfg c)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= active_n(b)) return;
-    const int f = b.act[i];
-    FrameCtl &ctl = b.ctl[f];
-    if (!ctl.active) return;
-    if (ctl.flags & (FLAG_RENDER_SKIPPED | FLAG_OVERFLOW)) { ctl.active = 0; return; }
-    if (!ctl.render) return;
-    const float obj = -(float)ctl.corr;
-    if (ctl.mode == M_FULL) {
-        ctl.obj0 = obj;
-        ctl.iters_lambda++;
-        ctl.need_jac = 1;
-        return;
-    }
-    ctl.inner++;
-    float l2 = ctl.l2base;
-    l2 = l2 * (0.5f * ctl.t);
-    if (obj < ctl.obj0 + l2) {
-        for (int j = 0; j < 3; ++j) b.lam[f * 4 + j] = b.lam_ls[f * 4 + j];
-        ctl.obj0 = obj;
-        if (ctl.iters_lambda >= c.max_iters_lambda) { ctl.active = 0; return; }
-        ctl.iters_lambda++;
-        ctl.need_jac = 1;
-    } else {
-        ctl.t = ctl.t * 0.5f;
-        if (ctl.t < 0.01f) { ctl.active = 0; return; }
-        for (int j = 0; j < 3; ++j) b.lam_ls[f * 4 + j] = b.lam[f * 4 + j] + ctl.t * b.dlam[f * 4 + j];
     }
 }
 
@@ -2430,149 +2449,286 @@ __global__ void __launch_bounds__(SV_THREADS, RB == 6 ? 2 : 1) k_solve_t(DModel 
 }
 
 // ------------------------------------------------------------------------------------------
-// Light system (derivative_computer.cu:235-312): dI/dlambda = L t (R n), chain rule, 3x3
-// normal equations in FP64, Cholesky, first trial. One block per frame.
+// Light fit (model_fitter.cu:981-1073), one block per frame, every render and decision of the
+// frame's line search in one launch: objective -corr, Armijo test with alpha = beta = 0.5, the light
+// system (derivative_computer.cu:235-312) as dI/dlambda = L t (R n), chain rule, 3x3 normal
+// equations in FP64, Cholesky.
+//
+// The fit moves only the light: the raster, its neighbour maps, every fragment's dI/dlambda and
+// so the neighbour differences of the chain rule stay as they are. They are formed once (32
+// bytes per fragment, LightTerm); the shading terms and pixel positions stay in shared memory when
+// they fit beside the region. An iteration is a render (shade, blur, gradients) whose
+// gradient pass also sums the light system: nearly every trial is accepted (151 of 159 in a
+// long fit), so a second pass over the fragments only for accepted trials costs more.
+// It is bound by the latency of one block (a fit of 160 iterations in a batch of 77 decides the
+// launch). As rounds over all frames, four launches each, that light fit took 6.7 ms; with a
+// 512-thread block per frame and a separate pass for the system 2.8 ms; this form 1.8 ms
+// (3.8 ms of a 1,024-frame fit, most of it one frame of 270 iterations).
 
-constexpr int LJ_U = 4;   // fragments per thread whose gathers are in flight together
+struct __align__(16) LightTerm {
+    float dh[3], dv[3];      // differences of dI/dlambda between the right/left, below/above neighbours
+    float sxn, syn;          // normalised target gradient
+};
 
-__global__ void __launch_bounds__(256) k_lambda_jac(DModel m, DBatch b, Cfg c)
+struct LightSearch {
+    double corr;
+    float obj0, l2base, t, lam[3], dlam[3], glam[3];
+    int iters, inner, trials;
+};
+
+constexpr int LIGHT_SMEM = 216 * 1024;       // the region, then 24 bytes per fragment when they fit
+constexpr int LF_SUMS = 10;                  // the correlation, 6 entries of H's upper triangle, 3 of the right-hand side
+
+__device__ __forceinline__ int light_region_bytes(const Region &r) { return (r.rw * r.ph + (r.rw + 2 * KRAD) * r.pb) * 4; }
+
+// d = -(H^-1 g) of the 3x3 light system in the oracle's order (upper triangle of H in row order);
+// NaN when a pivot is not positive.
+__device__ __forceinline__ void light_solve(const float (&h)[6], const float (&g)[3], float (&d)[3])
 {
+    const double a00 = h[0], a10 = h[1], a20 = h[2], a11 = h[3], a21 = h[4], a22 = h[5];
+    bool ok = a00 > 0.0;
+    const double l00 = sqrt(a00), l10 = a10 / l00, l20 = a20 / l00;
+    const double s1 = a11 - l10 * l10;
+    ok = ok && s1 > 0.0;
+    const double l11 = sqrt(s1), l21 = (a21 - l20 * l10) / l11;
+    const double s2 = (a22 - l20 * l20) - l21 * l21;
+    ok = ok && s2 > 0.0;
+    const double l22 = sqrt(s2);
+    const double y0 = (double)g[0] / l00, y1 = ((double)g[1] - l10 * y0) / l11;
+    const double y2 = (((double)g[2] - l20 * y0) - l21 * y1) / l22;
+    const double x2 = y2 / l22, x1 = (y1 - l21 * x2) / l11, x0 = ((y0 - l10 * x1) - l20 * x2) / l00;
+    const float nan = __int_as_float(0x7fc00000);
+    d[0] = ok ? (float)(-x0) : nan;
+    d[1] = ok ? (float)(-x1) : nan;
+    d[2] = ok ? (float)(-x2) : nan;
+}
+
+__global__ void __launch_bounds__(LIGHT_THREADS, 1) k_light_fit(DModel m, DBatch b, Cfg c, long max_rounds)
+{
+    constexpr int NT = LIGHT_THREADS;
     if ((int)blockIdx.x >= active_n(b)) return;
     const int f = b.act[blockIdx.x];
     FrameCtl &ctl = b.ctl[f];
-    if (!ctl.need_jac) return;
-    __shared__ double s_red[8][12];
-    __shared__ double s_L[9], s_y[3];
-    __shared__ float s_g[3];
-    const int tid = threadIdx.x, N = ctl.N;
-    const float4 *geo = b.geo + (size_t)f * m.V;
-    const float *R = b.R + f * 9;
-    const float *tau = b.x + (size_t)f * m.KTP + m.K;
-    const float *lam = b.lam + f * 4;
-    const float Lint = b.Lint[f];
+    if (!ctl.active) return;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (ctl.flags & (FLAG_RENDER_SKIPPED | FLAG_OVERFLOW)) {
+        if (tid == 0) ctl.active = 0;
+        return;
+    }
+    if (!ctl.render) return;
+    extern __shared__ __align__(16) float rsm[];
+    __shared__ double s_sum[NT / 32][LF_SUMS];
+    __shared__ double s_tot[LF_SUMS];
+    __shared__ float s_q[3];                 // the rotated light of the next render
+    __shared__ float s_lam[3];               // and the light itself
+    __shared__ float s_R[9], s_tau[3];
+    __shared__ LightSearch st;               // thread 0's, written back when the fit ends
+    __shared__ int s_next;                   // after a render: 0 = done, 1 = another trial
+    const Region r = make_region(ctl, rsm, b.img + (size_t)f * RIMG);
+    const int N = ctl.N;
     const Fragment *frags = b.frag + (size_t)f * NMAX;
-    float *Jl = b.J + (size_t)f * NMAX * m.KTP;   // rows of pitch 4
-    // fragments LJ_U at a time, their gathers issued together (each thread still takes its
-    // fragments in ascending order, so the FP64 sums below keep their order)
-    for (int n0 = tid; n0 < N; n0 += 256 * LJ_U) {
-        Fragment fr[LJ_U];
+    const float4 *shc = b.shc + (size_t)f * NMAX;
+    const float *sht = b.sht + (size_t)f * NMAX;
+    const float Lint = b.Lint[f];
+    // shading terms and region positions (-1: not the pixel's owner) in shared memory when they fit
+    const int rbytes = r.A == rsm ? (light_region_bytes(r) + 15) & ~15 : 0;
+    const bool cached = rbytes + N * 24 <= LIGHT_SMEM;
+    float4 *c_sn = reinterpret_cast<float4 *>(reinterpret_cast<char *>(rsm) + rbytes);
+    float *c_t = reinterpret_cast<float *>(c_sn + N);
+    int *c_at = reinterpret_cast<int *>(c_t + N);
+    if (tid < 9) s_R[tid] = b.R[f * 9 + tid];
+    if (tid < 3) {
+        s_tau[tid] = b.x[(size_t)f * m.KTP + m.K + tid];
+        const float v = b.lam[f * 4 + tid];
+        s_lam[tid] = v;
+        st.lam[tid] = v;
+        st.dlam[tid] = st.glam[tid] = 0.0f;
+    }
+    if (tid == 0) {
+        st.obj0 = st.l2base = 0.0f;
+        st.t = 1.0f;
+        st.iters = ctl.iters_lambda;
+        st.inner = ctl.inner;
+        st.trials = 0;
+    }
+    region_clear<NT>(r, true);
+    __syncthreads();
+    // the terms (in the Jacobian's buffer), and while they are formed the rows dI/dlambda
+    LightTerm *terms = reinterpret_cast<LightTerm *>(b.J + (size_t)f * NMAX * m.KTP);
+    float4 *rows = reinterpret_cast<float4 *>(b.fgrad + (size_t)f * 5 * NMAX);
+    for (int n = tid; n < N; n += NT) {
+        const float4 sn = shc[n];
+        const float t = sht[n];
+        const float Lt = Lint * t;
+        const float r0 = Lt * sn.x, r1 = Lt * sn.y, r2 = Lt * sn.z;
+        float v[3];
 #pragma unroll
-        for (int u = 0; u < LJ_U; ++u) {
-            const int n = n0 + u * 256;
-            fr[u] = n < N ? frags[n] : Fragment{0u, 0, 0.0f, 0.0f};
-        }
-        float rr[LJ_U][3];
-#pragma unroll
-        for (int u = 0; u < LJ_U; ++u) {
-            float nn[3], t;
-            if (ctl.shade_cached) {
-                // the light fit's render of this geometry formed them (k_render)
-                const int n = min(n0 + u * 256, N - 1);
-                const float4 sn = b.shc[(size_t)f * NMAX + n];
-                nn[0] = sn.x; nn[1] = sn.y; nn[2] = sn.z;
-                t = b.sht[(size_t)f * NMAX + n];
-            } else {
-                const Shading sh = shade(m, geo, fr[u], R, tau, lam, Lint);
-                nn[0] = sh.nn[0]; nn[1] = sh.nn[1]; nn[2] = sh.nn[2];
-                t = sh.t;
-            }
-            const float Lt = Lint * t;
-            const float r0 = Lt * nn[0], r1 = Lt * nn[1], r2 = Lt * nn[2];
-#pragma unroll
-            for (int j = 0; j < 3; ++j) rr[u][j] = (r0 * R[j] + r1 * R[j + 3]) + r2 * R[j + 6];
-        }
-#pragma unroll
-        for (int u = 0; u < LJ_U; ++u) {
-            const int n = n0 + u * 256;
-            if (n >= N) break;
-            *reinterpret_cast<float4 *>(Jl + (size_t)n * 4) = make_float4(rr[u][0], rr[u][1], rr[u][2], 0.0f);
+        for (int j = 0; j < 3; ++j) v[j] = (r0 * s_R[j] + r1 * s_R[j + 3]) + r2 * s_R[j + 6];
+        rows[n] = make_float4(v[0], v[1], v[2], 0.0f);
+        if (cached) {
+            const uint32_t po = frags[n].pix_owner;
+            c_sn[n] = sn;
+            c_t[n] = t;
+            c_at[n] = r.at(po & 0xFFFF) | (int)(po & 0x80000000u);
         }
     }
     __syncthreads();
+    const float2 *tgn = b.tgn + (size_t)f * NPIX;
     const int32_t *nb = b.nb + (size_t)f * 4 * NMAX;
-    const float *fg = b.fgrad + (size_t)f * 5 * NMAX;
-    double acc[12];
-    for (int q = 0; q < 12; ++q) acc[q] = 0.0;
-    for (int n0 = tid; n0 < N; n0 += 256 * LJ_U) {
-        float4 jr[LJ_U][4];
-#pragma unroll
-        for (int u = 0; u < LJ_U; ++u) {
-            const int n = n0 + u * 256;
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                jr[u][q] = n < N ? *reinterpret_cast<const float4 *>(Jl + (size_t)nb[q * NMAX + n] * 4) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int n = tid; n < N; n += NT) {
+        const float4 k0 = rows[nb[n]], k1 = rows[nb[NMAX + n]], k2 = rows[nb[2 * NMAX + n]], k3 = rows[nb[3 * NMAX + n]];
+        const float2 tg = tgn[frags[n].pix_owner & 0xFFFF];
+        LightTerm t;
+        t.dh[0] = k1.x - k0.x; t.dh[1] = k1.y - k0.y; t.dh[2] = k1.z - k0.z;
+        t.dv[0] = k3.x - k2.x; t.dv[1] = k3.y - k2.y; t.dv[2] = k3.z - k2.z;
+        t.sxn = tg.x; t.syn = tg.y;
+        terms[n] = t;
+    }
+    if (tid == 0) {
+        float q[3];
+        light_terms(s_R, s_tau, s_lam, q);
+        for (int j = 0; j < 3; ++j) s_q[j] = q[j];
+    }
+    __syncthreads();
+    // a border pixel's neighbours wrap to pixel 0; elsewhere they lie beside it in the region
+    const bool border = r.rw == DIM && r.rh == DIM;
+    for (long round = 0; round < max_rounds; ++round) {
+        const float q[3] = {s_q[0], s_q[1], s_q[2]};
+        if (cached) {
+            for (int n = tid; n < N; n += NT) {
+                const int at = c_at[n];
+                if (at < 0) {
+                    const float4 sn = c_sn[n];
+                    const float t = c_t[n];
+                    const float Id = ((sn.x * q[0] + sn.y * q[1]) + sn.z * q[2]) - sn.w;
+                    r.A[at & 0x7FFFFFFF] = t + (Lint * t) * Id;
+                }
+            }
+        } else {
+            region_shade<NT>(r, frags, shc, sht, N, q, Lint);
         }
+        __syncthreads();
+        region_blur<NT>(r, c);
+        double acc[LF_SUMS];
 #pragma unroll
-        for (int u = 0; u < LJ_U; ++u) {
-            const int n = n0 + u * 256;
-            if (n >= N) break;
-            const float gx = fg[n], gy = fg[NMAX + n], h = fg[2 * NMAX + n];
+        for (int e = 0; e < LF_SUMS; ++e) acc[e] = 0.0;
+        for (int n = tid; n < N; n += NT) {
+            const LightTerm t = terms[n];
+            float v[4];
+            if (cached && !border) {
+                const int at = c_at[n] & 0x7FFFFFFF;
+                v[0] = r.A[at + r.ph]; v[1] = r.A[at - r.ph]; v[2] = r.A[at + 1]; v[3] = r.A[at - 1];
+            } else {
+                int kr, kl, kd, ku;
+                neighbour_pixels((int)(frags[n].pix_owner & 0xFFFF), kr, kl, kd, ku);
+                v[0] = r.A[r.at(kr)]; v[1] = r.A[r.at(kl)]; v[2] = r.A[r.at(kd)]; v[3] = r.A[r.at(ku)];
+            }
+            float gx, gy, h, gxn, gyn;
+            grad_of(v[0], v[1], v[2], v[3], gx, gy, h, gxn, gyn);
             const float pre = (float)(1.0 / (0.001 + (double)(h * h * h)));
-            float ox[3], oy[3];
-            const float k0[3] = {jr[u][0].x, jr[u][0].y, jr[u][0].z}, k1[3] = {jr[u][1].x, jr[u][1].y, jr[u][1].z};
-            const float k2[3] = {jr[u][2].x, jr[u][2].y, jr[u][2].z}, k3[3] = {jr[u][3].x, jr[u][3].y, jr[u][3].z};
+            const float diffx = 2 * gx, diffy = 2 * gy;
+            double ox[3], oy[3];
 #pragma unroll
             for (int j = 0; j < 3; ++j) {
-                const float vv[4] = {k0[j], k1[j], k2[j], k3[j]};
-                chain_value(vv, pre, 2 * gx, 2 * gy, ox[j], oy[j]);
+                const float X = (-diffy) * (-t.dh[j]) - (-diffx) * (-t.dv[j]);
+                ox[j] = (double)(((-pre) * (-diffy)) * X);
+                oy[j] = (double)((pre * (-diffx)) * X);
             }
-            const double sx = fg[3 * NMAX + n], sy = fg[4 * NMAX + n];
-            for (int a = 0; a < 3; ++a) {
-                acc[9 + a] += sx * ox[a] + sy * oy[a];
-                for (int bb = 0; bb < 3; ++bb) acc[a * 3 + bb] += (double)ox[a] * ox[bb] + (double)oy[a] * oy[bb];
+            // (the products of floats are exact in FP64: a fused multiply-add rounds as their sum)
+            const double sx = t.sxn, sy = t.syn;
+            acc[0] += fma((double)gxn, sx, (double)gyn * sy);
+            acc[1] += fma(ox[0], ox[0], oy[0] * oy[0]);
+            acc[2] += fma(ox[0], ox[1], oy[0] * oy[1]);
+            acc[3] += fma(ox[0], ox[2], oy[0] * oy[2]);
+            acc[4] += fma(ox[1], ox[1], oy[1] * oy[1]);
+            acc[5] += fma(ox[1], ox[2], oy[1] * oy[2]);
+            acc[6] += fma(ox[2], ox[2], oy[2] * oy[2]);
+            acc[7] += fma(sx, ox[0], sy * oy[0]);
+            acc[8] += fma(sx, ox[1], sy * oy[1]);
+            acc[9] += fma(sx, ox[2], sy * oy[2]);
+        }
+#pragma unroll
+        for (int e = 0; e < LF_SUMS; ++e) {
+            double v = acc[e];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if (lane == 0) s_sum[warp][e] = v;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            if (lane < LF_SUMS) {
+                double v = 0.0;
+#pragma unroll
+                for (int w = 0; w < NT / 32; ++w) v += s_sum[w][lane];
+                s_tot[lane] = v;
+            }
+            __syncwarp();
+            if (lane == 0) {
+                st.corr = s_tot[0];
+                const float obj = -(float)s_tot[0];
+                int next = 2;                            // accepted: a new direction
+                if (round == 0) {
+                    st.obj0 = obj;
+                    st.iters++;
+                } else {
+                    st.inner++;
+                    float l2 = st.l2base;
+                    l2 = l2 * (0.5f * st.t);
+                    if (obj < st.obj0 + l2) {
+                        for (int j = 0; j < 3; ++j) st.lam[j] = s_lam[j];
+                        st.obj0 = obj;
+                        if (st.iters >= c.max_iters_lambda) next = 0; else st.iters++;
+                    } else {
+                        next = 1;
+                        st.t = st.t * 0.5f;
+                        if (st.t < 0.01f) next = 0;
+                        else
+                            for (int j = 0; j < 3; ++j) s_lam[j] = st.lam[j] + st.t * st.dlam[j];
+                    }
+                }
+                if (next == 2) {
+                    float h[6], g[3], dl[3];
+                    for (int e = 0; e < 6; ++e) h[e] = (float)s_tot[1 + e];
+                    for (int j = 0; j < 3; ++j) g[j] = (float)(-s_tot[7 + j]);
+                    light_solve(h, g, dl);
+                    const float l2 = (float)((double)dl[0] * g[0] + (double)dl[1] * g[1] + (double)dl[2] * g[2]);
+                    st.l2base = l2;
+                    st.trials = 1;
+                    st.t = 1.0f;
+                    for (int j = 0; j < 3; ++j) {
+                        st.dlam[j] = dl[j];
+                        st.glam[j] = g[j];
+                        s_lam[j] = st.lam[j] + 1.0f * dl[j];
+                    }
+                    // the first trial's -g.d test (model_fitter.cu:1044-1048) does not depend on the trial
+                    next = !((double)(-l2) < 0.0003 || !(l2 == l2));
+                }
+                float qn[3];
+                light_terms(s_R, s_tau, s_lam, qn);
+                for (int j = 0; j < 3; ++j) s_q[j] = qn[j];
+                s_next = next;
             }
         }
+        region_clear<NT>(r, false);          // for the next render (the gradients are read)
+        __syncthreads();
+        if (!s_next) break;
     }
-    for (int q = 0; q < 12; ++q)
-        for (int o = 16; o > 0; o >>= 1) acc[q] += __shfl_down_sync(0xffffffffu, acc[q], o);
-    if ((tid & 31) == 0)
-        for (int q = 0; q < 12; ++q) s_red[tid >> 5][q] = acc[q];
-    __syncthreads();
-    if (tid != 0) return;
-    double tot[12];
-    for (int q = 0; q < 12; ++q) { tot[q] = 0.0; for (int w = 0; w < 8; ++w) tot[q] += s_red[w][q]; }
-    float Hf[9];
-    for (int i = 0; i < 9; ++i) Hf[i] = (float)tot[i];
-    for (int i = 0; i < 3; ++i) s_g[i] = (float)(-tot[9 + i]);
-    // 3x3 Cholesky in the oracle's order (single thread)
-    int ok = 1;
-    for (int i = 0; i < 9; ++i) s_L[i] = (double)Hf[i];
-    for (int j = 0; j < 3 && ok; ++j) {
-        double s = s_L[j * 3 + j];
-        for (int k = 0; k < j; ++k) s -= s_L[k * 3 + j] * s_L[k * 3 + j];
-        if (!(s > 0.0)) { ok = 0; break; }
-        const double ljj = sqrt(s);
-        s_L[j * 3 + j] = ljj;
-        for (int i = j + 1; i < 3; ++i) {
-            double t = s_L[j * 3 + i];
-            for (int k = 0; k < j; ++k) t -= s_L[k * 3 + i] * s_L[k * 3 + j];
-            s_L[j * 3 + i] = t / ljj;
+    if (tid == 0) {
+        ctl.active = 0;
+        ctl.need_jac = 0;
+        ctl.corr = st.corr;
+        ctl.obj0 = st.obj0;
+        ctl.iters_lambda = st.iters;
+        ctl.inner = st.inner;
+        ctl.l2base = st.l2base;
+        ctl.t = st.t;
+        if (st.trials) ctl.mode = M_TRIAL;
+        for (int j = 0; j < 3; ++j) {
+            b.lam[f * 4 + j] = st.lam[j];
+            b.lam_ls[f * 4 + j] = s_lam[j];
+            if (st.trials) { b.dlam[f * 4 + j] = st.dlam[j]; b.glam[f * 4 + j] = st.glam[j]; }
         }
     }
-    float dl[3];
-    if (ok) {
-        for (int i = 0; i < 3; ++i) {
-            double t = (double)s_g[i];
-            for (int k = 0; k < i; ++k) t -= s_L[k * 3 + i] * s_y[k];
-            s_y[i] = t / s_L[i * 3 + i];
-        }
-        for (int i = 2; i >= 0; --i) {
-            double t = s_y[i];
-            for (int k = i + 1; k < 3; ++k) t -= s_L[i * 3 + k] * s_y[k];
-            s_y[i] = t / s_L[i * 3 + i];
-        }
-        for (int i = 0; i < 3; ++i) dl[i] = (float)(-s_y[i]);
-    } else {
-        for (int i = 0; i < 3; ++i) dl[i] = __int_as_float(0x7fc00000);
-    }
-    for (int j = 0; j < 3; ++j) { b.dlam[f * 4 + j] = dl[j]; b.glam[f * 4 + j] = s_g[j]; }
-    const float l2 = (float)((double)dl[0] * s_g[0] + (double)dl[1] * s_g[1] + (double)dl[2] * s_g[2]);
-    ctl.l2base = l2;
-    ctl.mode = M_TRIAL;
-    ctl.t = 1.0f;
-    for (int j = 0; j < 3; ++j) b.lam_ls[f * 4 + j] = lam[j] + 1.0f * dl[j];
-    // the first trial's -g.d test (model_fitter.cu:1044-1048) does not depend on the trial
-    if ((double)(-l2) < 0.0003 || !(l2 == l2)) ctl.active = 0;
 }
 
 // Unblurred image and owner-triangle map of every rendering frame (renderer.cu:635-696).
