@@ -85,11 +85,6 @@ __global__ void k_blur_cols_full(const float *src, float *dst, Cfg c, int F)
     dst[i] = acc;
 }
 
-__global__ void k_set_render(DBatch b, int frame)
-{
-    for (int f = threadIdx.x; f < b.F; f += blockDim.x) b.ctl[f].render = (f == frame);
-}
-
 __global__ void k_scalars(DBatch b, double *out)   // [F][4]
 {
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
@@ -290,7 +285,6 @@ tdi_status set_attrs()
     TDI_CUDA(cudaFuncSetAttribute(k_solve_t<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     TDI_CUDA(cudaFuncSetAttribute(k_solve_t<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     TDI_CUDA(cudaFuncSetAttribute(k_normal_eq, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    TDI_CUDA(cudaFuncSetAttribute(k_precheck, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     TDI_CUDA(cudaFuncSetAttribute(k_normal_eq_tc<NE_GRP>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM));
     TDI_CUDA(cudaFuncSetAttribute(k_normal_eq_tc<TC_MAXN / 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM));
     TDI_CUDA(cudaFuncSetAttribute(k_vertex_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vc_smem(VC_MAXK)));
@@ -347,15 +341,6 @@ dim3 vertex_tc_grid(const DModel &m, int frames)
     return dim3((unsigned)std::max(ftiles, std::min((long)sms, ftiles * ntiles)));
 }
 
-// Blocks per frame of the depth pass: 16, or more when few frames run, so that a short
-// launch still spreads over every SM (about five resident blocks per SM).
-unsigned raster_blocks(int frames)
-{
-    const int sms = sm_count();
-    const int want = (5 * sms + std::max(frames, 1) - 1) / std::max(frames, 1);
-    return (unsigned)std::max(RD_BLOCKS, std::min(RD_MAX_BLOCKS, want));
-}
-
 struct Launch {
     tdi_batch *bt;
     const DModel &m;
@@ -368,8 +353,6 @@ struct Launch {
     size_t smem_solve() const { return solve_smem(m.KT); }
     dim3 fblocks() const { return dim3((F + 127) / 128); }
     int A() const { return b.nact; }                      // frames active this round
-    dim3 ablocks() const { return dim3((A() + 127) / 128); }
-    dim3 wblocks() const { return dim3((A() + 3) / 4); }      // a warp per active frame, 128 threads
 };
 
 // View of frames [f0, f0 + nf) of a batch: every per-frame array starts at frame f0.
@@ -398,7 +381,8 @@ DBatch batch_view(const tdi_batch *bt, int f0, int nf)
     v.act = a.act + F0;
     v.nact = 0;
     v.rlist = a.rlist + F0;
-    v.rcount = a.rcount + F0;
+    v.jlist = a.jlist + F0;
+    v.rcount = a.rcount + 2 * F0;
     v.geo = a.geo + F0 * m.V; v.proj = a.proj + F0 * m.V;
     v.zbuf = a.zbuf + F0 * NPIX;
     v.tri_mask = a.tri_mask + F0 * mask_words(m.T);
@@ -444,28 +428,38 @@ tdi_status compact_active(tdi_batch *bt, cudaStream_t s, int *n)
     return TDI_OK;
 }
 
+// The evaluation points of the active frames and the list of those that render; with check, a
+// trial's pre-render decisions (a rejected trial skips the vertex stage and the raster).
+tdi_status points(const Launch &L, const Cfg &c, int stage, int check)
+{
+    return launch(L.bt, 0, k_point, dim3(std::max(L.A(), 1)), dim3(PT_THREADS), point_smem(L.m.K, L.m.KTP), L.s, L.m,
+                  L.b, c, stage, check);
+}
+
+// Visibility of the rendering frames from their projections.
+tdi_status raster(const Launch &L)
+{
+    TDI_TRY(launch(L.bt, KID_RASTER, k_raster_depth, dim3(raster_grid(L.A())), dim3(RD_THREADS), 0, L.s, L.m, L.b));
+    return launch(L.bt, KID_RESOLVE, k_raster_resolve, dim3(L.A()), dim3(RR_THREADS), 0, L.s, L.m, L.b);
+}
+
 tdi_status geometry(const Launch &L, const Cfg &c, int stage)
 {
-    // the pre-render checks need only the landmarks: a rejected trial skips the vertex stage
-    TDI_TRY(launch(L.bt, 0, k_precheck, dim3((L.A() + PC_WARPS - 1) / PC_WARPS), dim3(PC_WARPS * 32),
-                   precheck_smem(L.m.K, L.m.KP), L.s, L.m, L.b, c, stage));
-    TDI_TRY(launch(L.bt, 0, k_compact_render, dim3(1), dim3(1024), 0, L.s, L.b));
+    TDI_TRY(points(L, c, stage, stage != ST_LAMBDA));
     if (c.vertex_stage == 1)
         TDI_TRY(launch(L.bt, KID_VERTEX, k_vertex_tc, vertex_tc_grid(L.m, L.A()), dim3(VC_THREADS), vc_smem(L.m.K),
                        L.s, L.m, L.b, reinterpret_cast<const __nv_bfloat16 *>(L.m.Etc)));
     else
         TDI_TRY(launch_vertex(L.bt, L.m, L.b, L.s, L.A()));
-    TDI_TRY(launch(L.bt, KID_RASTER, k_raster_depth, dim3(raster_blocks(L.A()), L.A()), dim3(RD_THREADS), 0, L.s, L.m, L.b));
-    TDI_TRY(launch(L.bt, KID_RESOLVE, k_raster_resolve, dim3(L.A()), dim3(RR_THREADS), 0, L.s, L.m, L.b));
-    return TDI_OK;
+    return raster(L);
 }
 
-tdi_status render(const Launch &L, const Cfg &c)
+tdi_status render(const Launch &L, const Cfg &c, int stage)
 {
     // 1,024 threads per frame while every frame can have an SM to itself, else two blocks of 512 per SM
     const bool wide = L.A() <= sm_count();
     return launch(L.bt, KID_RENDER, wide ? k_render_t<1024> : k_render_t<512>, dim3(L.A()), dim3(wide ? 1024 : 512),
-                  RENDER_SMEM_FLOATS * sizeof(float), L.s, L.m, L.b, c);
+                  RENDER_SMEM_FLOATS * sizeof(float), L.s, L.m, L.b, c, stage);
 }
 
 tdi_status normal_equations(const Launch &L, const Cfg &c, int stage)
@@ -496,12 +490,9 @@ tdi_status normal_equations(const Launch &L, const Cfg &c, int stage)
 // One round of a shape stage for the frames of b (launched on s).
 tdi_status stage_round(tdi_batch *bt, const Cfg &c, int stage, const DBatch &b, cudaStream_t s)
 {
-    const DModel &m = bt->m->d;
-    Launch L{bt, m, b, s, b.F};
-    TDI_TRY(launch(bt, 0, k_prepare, L.wblocks(), dim3(128), 0, s, m, b, stage));
+    Launch L{bt, bt->m->d, b, s, b.F};
     TDI_TRY(geometry(L, c, stage));
-    TDI_TRY(render(L, c));
-    TDI_TRY(launch(bt, 0, k_decide_shape, L.ablocks(), dim3(128), 0, s, m, b, c, stage));
+    TDI_TRY(render(L, c, stage));
     return normal_equations(L, c, stage);
 }
 
@@ -511,18 +502,18 @@ tdi_status light_fit(tdi_batch *bt, const Cfg &c, const DBatch &b, cudaStream_t 
 {
     const DModel &m = bt->m->d;
     Launch L{bt, m, b, s, b.F};
-    TDI_TRY(launch(bt, 0, k_prepare, L.wblocks(), dim3(128), 0, s, m, b, (int)ST_LAMBDA));
     TDI_TRY(geometry(L, c, ST_LAMBDA));
     TDI_TRY(launch(bt, KID_NEIGHBOURS, k_neighbours, dim3(L.A()), dim3(1024), L.smem_neigh(), s, b, 1));
     return launch(bt, 0, k_light_fit, dim3(L.A()), dim3(LIGHT_THREADS), (size_t)LIGHT_SMEM, s, m, b,
                   c, max_rounds);
 }
 
-// Rounds replayed from CUDA graphs. A graph holds GRAPH_ROUNDS rounds of a stage, each followed by
-// the compaction of the active frames into the device count that the next round's kernels
-// read; grids are sized for a capacity tier (the smallest of 32, 128, 512 or the batch that
-// holds the frames still running: the count only falls during a stage), and blocks past the
-// device count return at once. The host reads the count once per replay instead of once per
+// Rounds replayed from CUDA graphs. A graph holds GRAPH_ROUNDS rounds of a stage, then the
+// compaction of the active frames into the device count that the next replay's kernels read
+// (within a replay a frame that has ended is skipped by its flag: every kernel after k_point works
+// on the round's own lists); grids are sized for a capacity tier (the smallest of 32, 128, 512 or
+// the batch that holds the frames still running: the count only falls during a stage), and
+// blocks past the device counts return at once. The host reads the count once per replay instead of once per
 // round. Graphs are built on first use and kept per (stage, tier, frames, configuration).
 constexpr int GRAPH_ROUNDS = 16;
 
@@ -548,11 +539,8 @@ tdi_status stage_graph(tdi_batch *bt, const Cfg &c, int stage, int lane, int tie
     const int64_t before = bt->launches;
     TDI_CUDA(cudaStreamBeginCapture(ln.s, cudaStreamCaptureModeThreadLocal));
     tdi_status st = TDI_OK;
-    for (int r = 0; r < GRAPH_ROUNDS && st == TDI_OK; ++r) {
-        st = stage_round(bt, c, stage, gv, ln.s);
-        if (st == TDI_OK)
-            st = launch(bt, 0, k_compact_active, dim3(1), dim3(1024), 0, ln.s, (const DBatch)gv, ln.d_count);
-    }
+    for (int r = 0; r < GRAPH_ROUNDS && st == TDI_OK; ++r) st = stage_round(bt, c, stage, gv, ln.s);
+    if (st == TDI_OK) st = launch(bt, 0, k_compact_active, dim3(1), dim3(1024), 0, ln.s, (const DBatch)gv, ln.d_count);
     cudaGraph_t graph = nullptr;
     const cudaError_t ec = cudaStreamEndCapture(ln.s, &graph);
     const int64_t kernels = bt->launches - before;
@@ -815,7 +803,7 @@ tdi_status tdi_batch_create(tdi_model *m, int32_t max_frames, tdi_batch **out)
     A(d.x, F * KTP); A(d.x_ls, F * KTP); A(d.xe, F * KTP);
     A(d.lam, F * 4); A(d.lam_ls, F * 4); A(d.lame, F * 4); A(d.dlam, F * 4); A(d.glam, F * 4);
     A(d.d, F * KTP); A(d.g, F * KTP); A(d.H, F * KTP * KTP); A(d.R, F * 9); A(d.dR, F * 27);
-    A(d.ctl, F); A(d.act, F); A(d.rlist, F); A(d.rcount, F); A(d.geo, F * (size_t)md.V); A(d.proj, F * (size_t)md.V); A(d.zbuf, F * NPIX); A(d.tri_mask, F * (size_t)mask_words(md.T)); A(d.tri_list, F * (size_t)md.T); A(d.frag, F * NMAX);
+    A(d.ctl, F); A(d.act, F); A(d.rlist, F); A(d.jlist, F); A(d.rcount, 2 * F); A(d.geo, F * (size_t)md.V); A(d.proj, F * (size_t)md.V); A(d.zbuf, F * NPIX); A(d.tri_mask, F * (size_t)mask_words(md.T)); A(d.tri_list, F * (size_t)md.T); A(d.frag, F * NMAX);
     A(d.fgrad, F * 5 * NMAX); A(d.nb, F * 4 * NMAX); A(d.shc, F * NMAX); A(d.sht, F * NMAX);
     A(d.J, F * NMAX * KTP); b->ne_frame_doubles = NE_MAXCH * std::max((size_t)ne_part_stride((int)KTP), (tc_part_bytes(md.KT) + 7) / 8);
     A(d.ne_part, F * b->ne_frame_doubles); A(d.err, 1); A(d.img, F * RIMG); A(b->scalars, F * 4); A(b->d_count, 2);
@@ -1096,10 +1084,8 @@ tdi_status tdi_batch_evaluate(tdi_batch *b, const tdi_fit_config *cfg, int32_t f
     int n = 0;
     TDI_TRY(compact_active(b, s, &n));
     if (n == 0) return TDI_OK;
-    TDI_TRY(launch(b, 0, k_prepare, L.wblocks(), dim3(128), 0, s, m, d, stage));
     TDI_TRY(geometry(L, c, stage));
-    TDI_TRY(render(L, c));
-    TDI_TRY(launch(b, 0, k_decide_shape, L.ablocks(), dim3(128), 0, s, m, d, c, stage));
+    TDI_TRY(render(L, c, stage));
     TDI_TRY(normal_equations(L, c, stage));
     TDI_TRY(launch(b, 0, k_scalars, L.fblocks(), dim3(128), 0, s, d, b->scalars));
     TDI_CUDA(cudaStreamSynchronize(s));
@@ -1290,11 +1276,9 @@ static tdi_status adj_forward(tdi_batch *b, const Cfg &c, const float *x, const 
     int n = 0;
     TDI_TRY(compact_active(b, s, &n));
     if (n > 0) {
-        TDI_TRY(launch(b, 0, k_prepare, Lc.wblocks(), dim3(128), 0, s, m, d, (int)ST_RIGID));
-        TDI_TRY(launch(b, 0, k_compact_render, dim3(1), dim3(1024), 0, s, (const DBatch)d));
+        TDI_TRY(points(Lc, c, ST_RIGID, 0));
         TDI_TRY(launch_vertex(b, m, d, s, n));
-        TDI_TRY(launch(b, KID_RASTER, k_raster_depth, dim3(raster_blocks(n), n), dim3(RD_THREADS), 0, s, m, d));
-        TDI_TRY(launch(b, KID_RESOLVE, k_raster_resolve, dim3(n), dim3(RR_THREADS), 0, s, m, d));
+        TDI_TRY(raster(Lc));
     }
     const size_t np = (size_t)F * NPIX;
     const dim3 pb((unsigned)((np + 255) / 256));
@@ -1472,11 +1456,11 @@ tdi_status tdi_batch_raster(tdi_batch *b, int32_t frame, const float *xp, const 
     TDI_CUDA(cudaMemcpy((void *)(d.x0y0 + 2 * frame), o, sizeof(o), cudaMemcpyHostToDevice));
     uint32_t zero = 0;
     TDI_CUDA(cudaMemcpy(&d.ctl[frame].flags, &zero, sizeof(zero), cudaMemcpyHostToDevice));
-    TDI_CUDA(cudaMemcpy(d.act, &frame, sizeof(int32_t), cudaMemcpyHostToDevice));
+    const int32_t one[2] = {1, 0};               // the only frame of the round's list
+    TDI_CUDA(cudaMemcpy(d.rlist, &frame, sizeof(int32_t), cudaMemcpyHostToDevice));
+    TDI_CUDA(cudaMemcpy(d.rcount, one, sizeof(one), cudaMemcpyHostToDevice));
     d.nact = 1;
-    TDI_TRY(launch(b, 0, k_set_render, dim3(1), dim3(256), 0, (cudaStream_t)0, d, (int)frame));
-    TDI_TRY(launch(b, KID_RASTER, k_raster_depth, dim3(raster_blocks(1), 1), dim3(RD_THREADS), 0, (cudaStream_t)0, m, d));
-    TDI_TRY(launch(b, KID_RESOLVE, k_raster_resolve, dim3(1), dim3(RR_THREADS), 0, (cudaStream_t)0, m, d));
+    TDI_TRY(raster(Launch{b, m, d, (cudaStream_t)0, d.F}));
     TDI_CUDA(cudaDeviceSynchronize());
     FrameCtl ctl;
     TDI_CUDA(cudaMemcpy(&ctl, d.ctl + frame, sizeof(FrameCtl), cudaMemcpyDeviceToHost));
@@ -1500,11 +1484,9 @@ tdi_status tdi_batch_render(tdi_batch *b, float *images, int32_t *tri_map, void 
     int n = 0;
     TDI_TRY(compact_active(b, s, &n));
     if (n > 0) {
-        TDI_TRY(launch(b, 0, k_prepare, L.wblocks(), dim3(128), 0, s, m, d, (int)ST_RIGID));
-        TDI_TRY(launch(b, 0, k_compact_render, dim3(1), dim3(1024), 0, s, (const DBatch)d));
+        TDI_TRY(points(L, c, ST_RIGID, 0));
         TDI_TRY(launch_vertex(b, m, d, s, n));
-        TDI_TRY(launch(b, KID_RASTER, k_raster_depth, dim3(raster_blocks(n), n), dim3(RD_THREADS), 0, s, m, d));
-        TDI_TRY(launch(b, KID_RESOLVE, k_raster_resolve, dim3(n), dim3(RR_THREADS), 0, s, m, d));
+        TDI_TRY(raster(L));
     }
     float *img = d.img;                                   // [F][NPIX] image, then [F][NPIX] map
     int32_t *map = reinterpret_cast<int32_t *>(d.img + (size_t)d.F * NPIX);

@@ -61,7 +61,6 @@ struct FrameCtl {
     int32_t bbox[4];     // fragment pixel box of the last raster: xmin, xmax, ymin, ymax
     float objective;     // last accepted objective
     int32_t stage_ok;    // result of the last shape fit (outer > NITERS_SUCCESS)
-    int32_t shade_cached;// the light fit's per-fragment shading terms (shc, sht) hold this raster's
 };
 
 struct Fragment {        // one surviving fragment, in slot order
@@ -124,7 +123,8 @@ struct DBatch {
     int32_t nact;            // entries of act (host-driven rounds)
     const int32_t *dnact;    // when set: entries of act read from device memory (rounds in a CUDA graph)
     int32_t *rlist;          // [F] frames of act that render this round (after the pre-checks)
-    int32_t *rcount;         // [F]: rcount[0] = entries of rlist (one counter per view)
+    int32_t *jlist;          // [F] frames whose point was accepted: they get their normal equations
+    int32_t *rcount;         // [F][2]: entries of rlist and jlist (the first pair of a view counts)
     // per-render working set
     float4 *geo;             // [F][V]: X0, Y0, Z0 and the albedo of the vertex (slot order)
     float4 *proj;            // [F][V]: xp, yp, camera Z, 0 -- what the raster gathers

@@ -92,19 +92,6 @@ __device__ __forceinline__ int active_n(const DBatch &b) { return b.dnact ? *b.d
 
 __device__ __forceinline__ bool shape_stage(int stage) { return stage != ST_LAMBDA; }
 
-// Writes x_ls = x + t*d over the first n_upd entries; returns false when tau_z < 0 (the
-// reference's line search then breaks without terminating, and every later outer
-// iteration repeats the same trial: the frame is stuck at x, model_fitter.cu:255-259).
-__device__ bool set_trial(const DModel &m, const DBatch &b, int f, int n_upd)
-{
-    const float *x = b.x + (size_t)f * m.KTP;
-    const float *d = b.d + (size_t)f * m.KTP;
-    float *xl = b.x_ls + (size_t)f * m.KTP;
-    const float t = b.ctl[f].t;
-    for (int a = 0; a < n_upd; ++a) xl[a] = x[a] + t * d[a];
-    return !(xl[m.K + 2] < 0.0f);
-}
-
 __device__ void end_shape_stage(const Cfg &c, FrameCtl &ctl, int stage, int outer)
 {
     ctl.active = 0;
@@ -114,27 +101,44 @@ __device__ void end_shape_stage(const Cfg &c, FrameCtl &ctl, int stage, int oute
     if (stage == ST_RIGID) ctl.stage_ok = outer > c.niters_success;
 }
 
-// Line-search rejection (model_fitter.cu:325-355): shrink t, stop below the threshold,
-// otherwise place the next trial.
-__device__ void shape_reject(const DModel &m, const DBatch &b, const Cfg &c, int f, int stage)
+// Line-search rejection (model_fitter.cu:325-355) by a whole block: shrink t, stop below the
+// threshold, otherwise place the next trial x_ls = x + t d over the entries the stage updates. A
+// trial with tau_z < 0 ends the stage: the reference's line search then breaks without terminating,
+// and every later outer iteration repeats the same trial (the frame is stuck at x,
+// model_fitter.cu:255-259). s_t: a shared float.
+__device__ void shape_reject(const DModel &m, const DBatch &b, const Cfg &c, int f, int stage, float *s_t)
 {
     FrameCtl &ctl = b.ctl[f];
     const int maxit = stage == ST_RIGID ? c.max_iters_rigid : c.max_iters_finetune;
-    ctl.t = ctl.t * 0.8f;
-    if (ctl.t < 0.075f) {
-        end_shape_stage(c, ctl, stage, ctl.outer < maxit ? ctl.outer + 1 : ctl.outer);
-        return;
+    if (threadIdx.x == 0) {
+        const float t = ctl.t * 0.8f;
+        ctl.t = t;
+        *s_t = t;
+        if (t < 0.075f) end_shape_stage(c, ctl, stage, ctl.outer < maxit ? ctl.outer + 1 : ctl.outer);
     }
+    __syncthreads();
+    const float t = *s_t;
+    if (t < 0.075f) return;
     const int n_upd = stage == ST_FINETUNE ? m.K : m.KT;
-    if (!set_trial(m, b, f, n_upd)) {
+    const float *x = b.x + (size_t)f * m.KTP, *d = b.d + (size_t)f * m.KTP;
+    float *xl = b.x_ls + (size_t)f * m.KTP;
+    for (int a = threadIdx.x; a < n_upd; a += blockDim.x) xl[a] = x[a] + t * d[a];
+    __syncthreads();
+    if (threadIdx.x == 0 && xl[m.K + 2] < 0.0f) {
         ctl.flags |= FLAG_STUCK_NEG_TZ;
         end_shape_stage(c, ctl, stage, maxit);
     }
 }
 
+// Lists of a round, built by atomic appends (a kernel's result does not depend on their order): the
+// frames that render, and those whose accepted point gets its normal equations.
+__device__ __forceinline__ int render_n(const DBatch &b) { return b.rcount[0]; }
+__device__ __forceinline__ int jac_n(const DBatch &b) { return b.rcount[1]; }
+
 __global__ void k_stage_start(DModel m, DBatch b, Cfg c, int stage)
 {
     int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f == 0) b.rcount[0] = b.rcount[1] = 0;
     if (f >= b.F) return;
     FrameCtl &ctl = b.ctl[f];
     const bool dead = (ctl.flags & (FLAG_RENDER_SKIPPED | FLAG_OVERFLOW)) != 0;
@@ -153,32 +157,6 @@ __global__ void k_stage_start(DModel m, DBatch b, Cfg c, int stage)
     // finetune keeps the line-search state the last shape fit left.
     if (stage == ST_RIGID || stage == ST_LAMBDA) {
         for (int a = 0; a < m.KT; ++a) b.x_ls[(size_t)f * m.KTP + a] = b.x[(size_t)f * m.KTP + a];
-    }
-}
-
-// Evaluation point, rotation and render flag of every active frame.
-__global__ void k_prepare(DModel m, DBatch b, int stage)
-{
-    // a warp per frame: the lanes copy the evaluation point, lane 0 forms R(u) and dR/du
-    const int i = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
-    if (i >= active_n(b)) return;
-    const int f = b.act[i];
-    FrameCtl &ctl = b.ctl[f];
-    const bool active = ctl.active != 0;
-    const bool full = ctl.mode == M_FULL;
-    __syncwarp();
-    if (lane == 0) {
-        ctl.need_jac = 0;
-        if (!active) ctl.render = 0;
-    }
-    if (!active) return;
-    const float *src = (full || stage == ST_LAMBDA) ? b.x : b.x_ls;
-    float *xe = b.xe + (size_t)f * m.KTP;
-    for (int a = lane; a < m.KT; a += 32) xe[a] = src[(size_t)f * m.KTP + a];
-    __syncwarp();
-    if (lane == 0) {
-        rotation(xe + m.K + 3, b.R + f * 9, b.dR + f * 27);
-        ctl.render = 1;
     }
 }
 
@@ -448,113 +426,143 @@ __device__ __forceinline__ void landmark_G(const DModel &m, const DBatch &b, int
     G[3] = 0.0f - ((yproj - bnd[3 * NL + i] * fs) - yl);
 }
 
-// Face-size check (renderer.cu:838-857), barrier objective and the pre-render decisions of
-// a trial (model_fitter.cu:237-300): tau_z, face size, NaN barrier, then -g.d < 3e-4.
-// Both need only the 51 landmark vertices, so they run before the vertex stage: the landmark
-// object points and projections are formed here with the vertex stage's arithmetic (the same
-// values bit for bit), and a trial rejected here costs no vertex stage and no raster.
-constexpr int PC_WARPS = 8;                      // frames per block (a warp each)
-constexpr int PC_LM = 5;                         // per landmark: X0, Y0, Z0, xp, yp
+// The evaluation point of every active frame, one block per frame: the state x or x_ls, R(u) and
+// dR/du; with check, the face-size check (renderer.cu:838-857), the barrier objective and the
+// pre-render decisions of a trial (model_fitter.cu:237-300): tau_z, face size, NaN barrier, then
+// -g.d < 3e-4. These need only the 51 landmark vertices, so they run before the vertex stage: the
+// landmark object points and projections are formed here with the vertex stage's arithmetic (the
+// same values bit for bit), and a trial rejected here costs no vertex stage and no raster. Frames
+// that go on are appended to the round's list.
+// Latency-bound (every frame has its block): a thread per landmark coordinate runs one fused
+// multiply-add chain with its basis row loaded ahead, another warp forms the rotation meanwhile,
+// the logarithms spread over the block. As a warp per frame with the landmark rows staged per
+// block, the rotation and the list in launches of their own, a round spent 31 us here;
+// 8 us in this form (77 frames).
+constexpr int PT_THREADS = 192;
+constexpr int PT_E4 = 10;                        // 16-byte loads of a basis row in flight
 
-// Shared memory of k_precheck (floats): the landmarks' basis rows (pitch 3 KP + 1, staged once
-// per block for all its frames), per warp the frame's coefficients, the barrier terms and
-// the landmark points.
-__host__ __device__ __forceinline__ size_t precheck_smem(int K, int KP)
+__host__ __device__ __forceinline__ size_t point_smem(int K, int KTP)
 {
-    return ((size_t)NL * (3 * KP + 1) + (size_t)PC_WARPS * (KP + 2 * K + 4 * NL + NL * PC_LM)) * sizeof(float);
+    return ((size_t)KTP + 4 + 2 * K + 4 * NL) * sizeof(float);   // the state (padded), the barrier terms
 }
 
-__global__ void __launch_bounds__(PC_WARPS * 32) k_precheck(DModel m, DBatch b, Cfg c, int stage)
+__global__ void __launch_bounds__(PT_THREADS) k_point(DModel m, DBatch b, Cfg c, int stage, int check)
 {
-    extern __shared__ float psm[];
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int K = m.K, KP = m.KP, EP = 3 * KP + 1;
-    const int nterm = 2 * K + 4 * NL;
-    float *Es = psm;                                       // [NL][EP]
-    float *xs = Es + (size_t)NL * EP + (size_t)warp * KP;  // [KP] this warp's coefficients
-    float *pterm = Es + (size_t)NL * EP + (size_t)PC_WARPS * KP;   // [PC_WARPS][nterm]
-    float *lm = pterm + PC_WARPS * nterm + warp * NL * PC_LM;
-    // the 51 landmark basis rows, once for the block's frames
-    if ((int)(blockIdx.x * PC_WARPS) >= active_n(b)) return;
-    for (int q = threadIdx.x; q < NL * 3 * KP; q += PC_WARPS * 32) {
-        const int li = q / (3 * KP), o = q - li * 3 * KP;
-        Es[li * EP + o] = m.E[(size_t)m.lis[li] * 3 * KP + o];
+    extern __shared__ __align__(16) float psm[];
+    __shared__ float s_R[9], s_dR[27], s_lm[NL][3], s_xp[NL], s_yp[NL], s_t;
+    __shared__ double s_ob[PT_THREADS / 32];
+    __shared__ int s_go;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (blockIdx.x == 0 && tid == 0) b.rcount[1] = 0;     // the last round's normal equations are done
+    if ((int)blockIdx.x >= active_n(b)) return;
+    const int f = b.act[blockIdx.x];
+    FrameCtl &ctl = b.ctl[f];
+    const bool active = ctl.active != 0, full = ctl.mode == M_FULL;
+    __syncthreads();                             // (every thread has read the flags)
+    if (tid == 0) {
+        ctl.need_jac = 0;
+        if (!active) ctl.render = 0;
+    }
+    if (!active) return;
+    const int K = m.K, KP = m.KP, KT = m.KT;
+    float *xs = psm, *term = psm + m.KTP + 4;
+    const float *src = (full || stage == ST_LAMBDA ? b.x : b.x_ls) + (size_t)f * m.KTP;
+    float *xe = b.xe + (size_t)f * m.KTP;
+    for (int a = tid; a < KT; a += PT_THREADS) {
+        const float v = src[a];
+        xs[a] = v;
+        xe[a] = v;
     }
     __syncthreads();
-    const int i = blockIdx.x * PC_WARPS + warp;
-    if (i >= active_n(b)) return;
-    const int f = b.act[i];
-    FrameCtl &ctl = b.ctl[f];
-    if (!ctl.active || !ctl.render) return;
-    const float *x = b.xe + (size_t)f * m.KTP;
-    const float *R = b.R + f * 9;
-    for (int k = lane; k < K; k += 32) xs[k] = x[k];
-    __syncwarp();
-    {
-        const float *tau = x + K;
-        const float *cam = b.cam + f * 4;
-        for (int li = lane; li < NL; li += 32) {
-            const int v = m.lis[li];
-            const float *er = Es + li * EP;
-            float a0 = 0.0f, a1 = 0.0f, a2 = 0.0f;
-            for (int k = 0; k < K; ++k) {
-                const float xk = xs[k];
-                a0 = fmaf(er[k], xk, a0);
-                a1 = fmaf(er[KP + k], xk, a1);
-                a2 = fmaf(er[2 * KP + k], xk, a2);
-            }
-            const float X0 = m.mean[v] + a0, Y0 = m.mean[m.V + v] + a1, Z0 = m.mean[2 * m.V + v] + a2;
-            const float X3 = ((R[0] * X0 + R[3] * Y0) + R[6] * Z0) + tau[0];
-            const float Y3 = ((R[1] * X0 + R[4] * Y0) + R[7] * Z0) + tau[1];
-            const float Z3 = ((R[2] * X0 + R[5] * Y0) + R[8] * Z0) + tau[2];
-            float *o = lm + li * PC_LM;
-            o[0] = X0; o[1] = Y0; o[2] = Z0;
-            o[3] = (cam[0] * X3) / Z3 + cam[2];
-            o[4] = (cam[1] * Y3) / Z3 + cam[3];
-        }
+    if (warp == PT_THREADS / 32 - 1) {
+        if (lane == 0) rotation(xs + K + 3, s_R, s_dR);
         __syncwarp();
+        if (lane < 9) b.R[f * 9 + lane] = s_R[lane];
+        if (lane < 27) b.dR[f * 27 + lane] = s_dR[lane];
+        if (!check) {
+            if (lane == 0) {
+                ctl.render = 1;
+                b.rlist[atomicAdd(b.rcount, 1)] = f;
+            }
+            return;
+        }
+    } else {
+        if (!check) return;
+        if (tid < 3 * NL) {
+            const int li = tid / 3, cc = tid - 3 * li, v = m.lis[li];
+            const float4 *e4 = reinterpret_cast<const float4 *>(m.E + ((size_t)v * 3 + cc) * KP);
+            float acc = 0.0f;
+            for (int k0 = 0; k0 < K; k0 += 4 * PT_E4) {
+                float4 e[PT_E4];
+#pragma unroll
+                for (int u = 0; u < PT_E4; ++u) e[u] = k0 + 4 * u < K ? __ldg(e4 + (k0 >> 2) + u) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+                for (int u = 0; u < PT_E4; ++u) {
+                    const int k = k0 + 4 * u;
+                    if (k < K) acc = fmaf(e[u].x, xs[k], acc);
+                    if (k + 1 < K) acc = fmaf(e[u].y, xs[k + 1], acc);
+                    if (k + 2 < K) acc = fmaf(e[u].z, xs[k + 2], acc);
+                    if (k + 3 < K) acc = fmaf(e[u].w, xs[k + 3], acc);
+                }
+            }
+            s_lm[li][cc] = m.mean[(size_t)cc * m.V + v] + acc;
+        }
     }
-    const float d_iod = fabsf(lm[9 * PC_LM + 3] - lm[0 * PC_LM + 3]);
-    const float d_lem = fabsf(lm[0 * PC_LM + 4] - lm[40 * PC_LM + 4]);
-    const float d_rem = fabsf(lm[9 * PC_LM + 4] - lm[40 * PC_LM + 4]);
-    const double lim = (double)c.ref_face_size * 2;
-    const int face_ok = !((double)d_iod > lim || (double)d_lem > lim || (double)d_rem > lim);
-    if (!shape_stage(stage)) {
-        if (lane == 0) ctl.face_ok = face_ok;
-        return;
-    }
-    float *t = pterm + warp * nterm;
+    // the expression bounds' terms need only the state
     const bool ft = stage == ST_FINETUNE;
-    const float *lb = m.eps_b + (ft ? 2 : 0) * m.K;
-    const float *ub = m.eps_b + (ft ? 3 : 1) * m.K;
-    for (int k = lane; k < m.K; k += 32) {
-        const float fub = x[k] - ub[k];
-        const float flb = lb[k] - x[k];
-        t[2 * k] = -(float)log((double)(-flb));
-        t[2 * k + 1] = -(float)log((double)(-fub));
-    }
-    for (int li = lane; li < NL; li += 32) {
+    const float *lb = m.eps_b + (ft ? 2 : 0) * K, *ub = m.eps_b + (ft ? 3 : 1) * K;
+    __syncthreads();
+    const float *tau = xs + K;
+    const float *cam = b.cam + f * 4;
+    if (tid < NL) {
+        const float X0 = s_lm[tid][0], Y0 = s_lm[tid][1], Z0 = s_lm[tid][2];
+        const float X3 = ((s_R[0] * X0 + s_R[3] * Y0) + s_R[6] * Z0) + tau[0];
+        const float Y3 = ((s_R[1] * X0 + s_R[4] * Y0) + s_R[7] * Z0) + tau[1];
+        const float Z3 = ((s_R[2] * X0 + s_R[5] * Y0) + s_R[8] * Z0) + tau[2];
+        s_xp[tid] = (cam[0] * X3) / Z3 + cam[2];
+        s_yp[tid] = (cam[1] * Y3) / Z3 + cam[3];
         float G[4];
-        landmark_G(m, b, f, x, R, li, lm + li * PC_LM, G);
-        for (int sset = 0; sset < 4; ++sset) t[2 * m.K + sset * NL + li] = -(float)log((double)G[sset]);
+        landmark_G(m, b, f, xs, s_R, tid, s_lm[tid], G);
+        for (int s = 0; s < 4; ++s) term[2 * K + s * NL + tid] = G[s];
+    } else {
+        for (int k = tid - NL; k < K; k += PT_THREADS - NL) {
+            const float fub = xs[k] - ub[k];
+            const float flb = lb[k] - xs[k];
+            term[2 * k] = -flb;
+            term[2 * k + 1] = -fub;
+        }
     }
-    __syncwarp();
-    if (lane != 0) return;
-    ctl.face_ok = face_ok;
+    __syncthreads();
     double ob = 0.0;
-    for (int q = 0; q < nterm; ++q) ob += (double)t[q];
-    ctl.obj_b = (float)ob;
-    if (ctl.mode != M_TRIAL) return;
-    if (!face_ok || isnan(ob)) {
-        ctl.render = 0;
-        shape_reject(m, b, c, f, stage);
-        return;
+    for (int q = tid; q < 2 * K + 4 * NL; q += PT_THREADS) ob += (double)(-(float)log((double)term[q]));
+    for (int o = 16; o > 0; o >>= 1) ob += __shfl_down_sync(0xffffffffu, ob, o);
+    if (lane == 0) s_ob[warp] = ob;
+    __syncthreads();
+    if (tid == 0) {
+        const float d_iod = fabsf(s_xp[9] - s_xp[0]);
+        const float d_lem = fabsf(s_yp[0] - s_yp[40]);
+        const float d_rem = fabsf(s_yp[9] - s_yp[40]);
+        const double lim = (double)c.ref_face_size * 2;
+        const int face_ok = !((double)d_iod > lim || (double)d_lem > lim || (double)d_rem > lim);
+        ob = 0.0;
+        for (int w = 0; w < PT_THREADS / 32; ++w) ob += s_ob[w];
+        ctl.face_ok = face_ok;
+        ctl.obj_b = (float)ob;
+        int go = 1;                              // 0: the trial is rejected; -1: the stage ends
+        if (!full) {
+            if (!face_ok || isnan(ob)) go = 0;
+            else if ((double)(-ctl.l2base) < 0.0003) go = -1;
+        }
+        ctl.render = go > 0;
+        if (go > 0) b.rlist[atomicAdd(b.rcount, 1)] = f;
+        if (go < 0) {
+            const int maxit = stage == ST_RIGID ? c.max_iters_rigid : c.max_iters_finetune;
+            end_shape_stage(c, ctl, stage, ctl.outer < maxit ? ctl.outer + 1 : ctl.outer);
+        }
+        s_go = go;
     }
-    if ((double)(-ctl.l2base) < 0.0003) {
-        ctl.render = 0;
-        const int maxit = stage == ST_RIGID ? c.max_iters_rigid : c.max_iters_finetune;
-        end_shape_stage(c, ctl, stage, ctl.outer < maxit ? ctl.outer + 1 : ctl.outer);
-    }
+    __syncthreads();
+    if (s_go == 0) shape_reject(m, b, c, f, stage, &s_t);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -760,7 +768,8 @@ __device__ __forceinline__ bool survives(unsigned long long k, uint32_t tag, uin
 
 constexpr int RD_THREADS = 256;             // depth pass: threads per block
 constexpr int RD_BLOCKS = 16;               // depth pass: blocks per frame (at least)
-constexpr int RD_MAX_BLOCKS = 256;          // depth pass: blocks per frame when few frames render
+constexpr int RD_MAX_BLOCKS = 128;          // depth pass: blocks per frame when few frames render
+constexpr int RD_SPREAD = 2400;             // blocks that fill the SMs twice over
 constexpr int RR_THREADS = 1024;            // resolve: one block per frame
 constexpr int RR_WARPS = RR_THREADS / 32;
 constexpr int RR_ILP = 2;                  // resolve: listed entries per lane in flight together
@@ -798,6 +807,18 @@ __device__ __forceinline__ bool no_sample_inside(float bx, float by, float cx, f
     return dom && (xout || yout) && wide;
 }
 
+// Blocks per frame for rc rendering frames, and the largest grid up to `frames` of them can ask for.
+__host__ __device__ __forceinline__ int raster_parts(int rc)
+{
+    const int p = RD_SPREAD / rc;
+    return p < RD_BLOCKS ? RD_BLOCKS : p > RD_MAX_BLOCKS ? RD_MAX_BLOCKS : p;
+}
+inline int raster_grid(int frames)
+{
+    const int spread = frames * RD_MAX_BLOCKS < RD_SPREAD ? frames * RD_MAX_BLOCKS : RD_SPREAD;
+    return frames * RD_BLOCKS > spread ? frames * RD_BLOCKS : spread;
+}
+
 // A dense face mesh has about 25 triangles per visible fragment, most of them smaller than a
 // pixel, so the pass is bound by the instructions spent on triangles without a sample
 // point. Each warp therefore first tests its triangles with no_sample_inside (about 55
@@ -811,11 +832,15 @@ constexpr int RD_QUEUE = 32 * (RD_ILP + 1); // a warp's queue: what a step adds 
 
 __global__ void __launch_bounds__(RD_THREADS) k_raster_depth(DModel m, DBatch b)
 {
-    if ((int)blockIdx.y >= active_n(b)) return;
-    const int f = b.act[blockIdx.y];
+    // the blocks are split between the frames that render: RD_BLOCKS each, or more when few do
+    const int rc = render_n(b);
+    if (rc == 0) return;
+    const int parts = raster_parts(rc);
+    const int fi = blockIdx.x / parts, part = blockIdx.x - fi * parts;
+    if (fi >= rc) return;
+    const int f = b.rlist[fi];
     const FrameCtl &ctl = b.ctl[f];
-    if (!ctl.render) return;
-    if (blockIdx.x == 0 && threadIdx.x == 0) prof_count(b, KID_RASTER);
+    if (part == 0 && threadIdx.x == 0) prof_count(b, KID_RASTER);
     __shared__ float4 s_qa[RD_WARPS][RD_QUEUE];     // bx, by, cx, cy
     __shared__ float4 s_qb[RD_WARPS][RD_QUEUE];     // ax, ay, camera Z of b, triangle id (bits)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -827,8 +852,8 @@ __global__ void __launch_bounds__(RD_THREADS) k_raster_depth(DModel m, DBatch b)
     const int x0 = b.x0y0[2 * f], y0 = b.x0y0[2 * f + 1];
     const int T = m.T;
     // each block a contiguous range of the Morton order
-    const int per_block = (T + gridDim.x - 1) / gridDim.x;
-    const int s_begin = blockIdx.x * per_block, s_end = min(T, s_begin + per_block);
+    const int per_block = (T + parts - 1) / parts;
+    const int s_begin = part * per_block, s_end = min(T, s_begin + per_block);
     uint32_t flags = 0;
     int queued = 0;                                 // entries of the warp's queue
     auto evaluate = [&](int e) {
@@ -909,10 +934,9 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t *s_w, uint32
 
 __global__ void __launch_bounds__(RR_THREADS) k_raster_resolve(DModel m, DBatch b)
 {
-    if ((int)blockIdx.x >= active_n(b)) return;
-    const int f = b.act[blockIdx.x];
+    if ((int)blockIdx.x >= render_n(b)) return;
+    const int f = b.rlist[blockIdx.x];
     FrameCtl &ctl = b.ctl[f];
-    if (!ctl.render) return;
     if (threadIdx.x == 0) prof_count(b, KID_RESOLVE);
     __shared__ uint32_t s_w[RR_WARPS + 1];
     __shared__ uint32_t s_cnt[RR_WARPS][NTMP];   // survivors per warp and row
@@ -1191,7 +1215,6 @@ __global__ void __launch_bounds__(RR_THREADS) k_raster_resolve(DModel m, DBatch 
         ctl.epoch = epoch == TAG_MAX ? 0u : epoch;
         ctl.flags |= fl;
         ctl.renders += 1;
-        ctl.shade_cached = (fl & (FLAG_RENDER_SKIPPED | FLAG_OVERFLOW)) ? 0 : 1;
         for (int q = 0; q < 4; ++q) ctl.bbox[q] = s_bbox[q];
         if (s_bbox[1] >= 0 && (s_bbox[0] < 1 || s_bbox[1] > DIM - 2 || s_bbox[2] < 1 || s_bbox[3] > DIM - 2))
             ctl.flags |= FLAG_OUT_OF_DOMAIN;
@@ -1479,16 +1502,21 @@ __global__ void k_target_grad(const float *target, float2 *tgn, int F)
 // NT threads per frame: 512 (two blocks per SM) for full rounds, 1,024 when the frames do not
 // fill the SMs and a block's own latency is the round's.
 template <int NT>
-__global__ void __launch_bounds__(NT, 1024 / NT) k_render_t(DModel m, DBatch b, Cfg c)
+__global__ void __launch_bounds__(NT, 1024 / NT) k_render_t(DModel m, DBatch b, Cfg c, int stage)
 {
-    if ((int)blockIdx.x >= active_n(b)) return;
-    const int f = b.act[blockIdx.x];
+    if ((int)blockIdx.x >= render_n(b)) return;
+    const int f = b.rlist[blockIdx.x];
     FrameCtl &ctl = b.ctl[f];
-    if (!ctl.render) return;
     const int tid = threadIdx.x;
+    if (!ctl.render) {                           // the resolve refused the raster
+        if (tid == 0) end_shape_stage(c, ctl, stage, ctl.outer);
+        return;
+    }
     if (tid == 0) prof_count(b, KID_RENDER);
     extern __shared__ __align__(16) float rsm[];
     __shared__ double s_red[NT / 32];
+    __shared__ int s_take;
+    __shared__ float s_t;
     const Region r = make_region(ctl, rsm, b.img + (size_t)f * RIMG);
     const int N = ctl.N;
     const Fragment *frags = b.frag + (size_t)f * NMAX;
@@ -1526,48 +1554,40 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_render_t(DModel m, DBatch b, 
         }
     }
     const double total = render_sum<NT>(corr, s_red);
-    if (tid == 0) ctl.corr = total;
-}
-
-// ------------------------------------------------------------------------------------------
-// Decisions after a render.
-
-// Shape fits (model_fitter.cu:215-356): objective -(tau*corr - barrier); Armijo test.
-__global__ void k_decide_shape(DModel m, DBatch b, Cfg c, int stage)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= active_n(b)) return;
-    const int f = b.act[i];
-    FrameCtl &ctl = b.ctl[f];
-    if (!ctl.active) return;
-    const int maxit = stage == ST_RIGID ? c.max_iters_rigid : c.max_iters_finetune;
-    if (ctl.flags & (FLAG_RENDER_SKIPPED | FLAG_OVERFLOW)) {
-        end_shape_stage(c, ctl, stage, ctl.outer);
-        return;
+    // The decision (model_fitter.cu:215-356): objective -(tau*corr - barrier); Armijo test.
+    if (tid == 0) {
+        const int maxit = stage == ST_RIGID ? c.max_iters_rigid : c.max_iters_finetune;
+        const float tau_img = 5.0f * 5.0f;
+        ctl.corr = total;
+        float gc = tau_img * (float)total;
+        gc = gc + (-ctl.obj_b);
+        const float obj = -gc;
+        int take = 1, jac = 1;                   // the point is kept; it gets its normal equations
+        if (ctl.mode == M_FULL) {
+            take = 2;                            // (already x)
+        } else {
+            ctl.inner++;
+            float l2 = ctl.l2base;
+            l2 = l2 * (0.4f * ctl.t);
+            if (obj < ctl.obj0 + l2) {
+                if (ctl.outer >= maxit) { end_shape_stage(c, ctl, stage, ctl.outer); jac = 0; }
+                else ctl.outer++;
+            } else {
+                take = jac = 0;
+            }
+        }
+        if (take) { ctl.obj0 = obj; ctl.objective = obj; }
+        if (jac) {
+            ctl.need_jac = 1;
+            b.jlist[atomicAdd(b.rcount + 1, 1)] = f;
+        }
+        s_take = take;
     }
-    if (!ctl.render) return;
-    const float tau_img = 5.0f * 5.0f;
-    float gc = tau_img * (float)ctl.corr;
-    gc = gc + (-ctl.obj_b);
-    const float obj = -gc;
-    if (ctl.mode == M_FULL) {
-        ctl.obj0 = obj;
-        ctl.objective = obj;
-        ctl.need_jac = 1;
-        return;
-    }
-    ctl.inner++;
-    float l2 = ctl.l2base;
-    l2 = l2 * (0.4f * ctl.t);
-    if (obj < ctl.obj0 + l2) {
-        for (int a = 0; a < m.KT; ++a) b.x[(size_t)f * m.KTP + a] = b.x_ls[(size_t)f * m.KTP + a];
-        ctl.obj0 = obj;
-        ctl.objective = obj;
-        if (ctl.outer >= maxit) { end_shape_stage(c, ctl, stage, ctl.outer); return; }
-        ctl.outer++;
-        ctl.need_jac = 1;
-    } else {
-        shape_reject(m, b, c, f, stage);
+    __syncthreads();
+    if (s_take == 1) {
+        for (int a = tid; a < m.KT; a += NT) b.x[(size_t)f * m.KTP + a] = b.x_ls[(size_t)f * m.KTP + a];
+    } else if (s_take == 0) {
+        shape_reject(m, b, c, f, stage, &s_t);
     }
 }
 
@@ -1599,8 +1619,8 @@ __device__ __forceinline__ uint32_t cnt_at(const uint32_t *cnt, int p)
 
 __global__ void __launch_bounds__(1024) k_neighbours(DBatch b, int all_frames)
 {
-    if ((int)blockIdx.x >= active_n(b)) return;
-    const int f = b.act[blockIdx.x];
+    if ((int)blockIdx.x >= (all_frames ? render_n(b) : jac_n(b))) return;
+    const int f = (all_frames ? b.rlist : b.jlist)[blockIdx.x];
     FrameCtl &ctl = b.ctl[f];
     if (!(all_frames ? ctl.render : ctl.need_jac)) return;
     if (threadIdx.x == 0) prof_count(b, KID_NEIGHBOURS);
@@ -1797,10 +1817,9 @@ constexpr int JAC_BPF = 32;                  // blocks per frame
 
 __global__ void __launch_bounds__(JAC_THREADS, 4) k_jacobian(DModel m, DBatch b)
 {
-    if ((int)blockIdx.y >= active_n(b)) return;
-    const int f = b.act[blockIdx.y];
+    if ((int)blockIdx.y >= jac_n(b)) return;
+    const int f = b.jlist[blockIdx.y];
     const FrameCtl &ctl = b.ctl[f];
-    if (!ctl.need_jac) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) prof_count(b, KID_JACOBIAN);
     __shared__ float4 s_w[JAC_CH];           // al, be, ga, gx
     __shared__ float4 s_v[JAC_CH];           // vx, vy, vz, gy
@@ -2033,10 +2052,9 @@ __device__ __forceinline__ void ne_pairs(double (&acc)[NE_TPW][2], const double 
 
 __global__ void __launch_bounds__(NE_THREADS, 2) k_normal_eq(DModel m, DBatch b)
 {
-    if ((int)blockIdx.y >= active_n(b)) return;
-    const int f = b.act[blockIdx.y];
+    if ((int)blockIdx.y >= jac_n(b)) return;
+    const int f = b.jlist[blockIdx.y];
     const FrameCtl &ctl = b.ctl[f];
-    if (!ctl.need_jac) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) prof_count(b, KID_NORMAL_EQ);
     extern __shared__ __align__(16) double nesd[];  // rows [2][2*NE_SUB][NE_PD]
     const int KTP = m.KTP, KT = m.KT;
@@ -2127,10 +2145,9 @@ __global__ void __launch_bounds__(NE_THREADS, 2) k_normal_eq(DModel m, DBatch b)
 // Sum of the chunk partials in chunk order: H = tau*S, g = -tau*(column KT of S).
 __global__ void __launch_bounds__(NE_THREADS) k_normal_eq_reduce(DModel m, DBatch b)
 {
-    if ((int)blockIdx.y >= active_n(b)) return;
-    const int f = b.act[blockIdx.y];
+    if ((int)blockIdx.y >= jac_n(b)) return;
+    const int f = b.jlist[blockIdx.y];
     const FrameCtl &ctl = b.ctl[f];
-    if (!ctl.need_jac) return;
     const int KTP = m.KTP, KT = m.KT;
     const int stride = ne_part_stride8();
     const int nch = (ctl.N + NE_CH - 1) / NE_CH;
@@ -2188,10 +2205,8 @@ __device__ __forceinline__ void bar_hessian(double (&acc)[NE_TPW][2], const floa
 
 __global__ void __launch_bounds__(256) k_barrier_full(DModel m, DBatch b, int ft_bounds)
 {
-    if ((int)blockIdx.x >= active_n(b)) return;
-    const int f = b.act[blockIdx.x];
-    const FrameCtl &ctl = b.ctl[f];
-    if (!ctl.need_jac) return;
+    if ((int)blockIdx.x >= jac_n(b)) return;
+    const int f = b.jlist[blockIdx.x];
     if (threadIdx.x == 0) prof_count(b, KID_BARRIER);
     extern __shared__ float bsm[];
     const int KT = m.KT, KTP = m.KTP, K = m.K;
@@ -2439,10 +2454,10 @@ __device__ __forceinline__ void solve_frame(const DModel &m, const DBatch &b, co
 template <int RB>
 __global__ void __launch_bounds__(SV_THREADS, RB == 6 ? 2 : 1) k_solve_t(DModel m, DBatch b, Cfg c, int stage)
 {
-    if ((int)blockIdx.x >= active_n(b)) return;
-    const int f = b.act[blockIdx.x];
+    if (blockIdx.x == 0 && threadIdx.x == 0) b.rcount[0] = 0;    // the round's renders are done
+    if ((int)blockIdx.x >= jac_n(b)) return;
+    const int f = b.jlist[blockIdx.x];
     FrameCtl &ctl = b.ctl[f];
-    if (!ctl.need_jac) return;
     if (threadIdx.x == 0) prof_count(b, KID_SOLVE);
     extern __shared__ double ssm[];
     solve_frame<RB>(m, b, c, stage, f, ctl, ssm);
@@ -2506,16 +2521,14 @@ __device__ __forceinline__ void light_solve(const float (&h)[6], const float (&g
 __global__ void __launch_bounds__(LIGHT_THREADS, 1) k_light_fit(DModel m, DBatch b, Cfg c, long max_rounds)
 {
     constexpr int NT = LIGHT_THREADS;
-    if ((int)blockIdx.x >= active_n(b)) return;
-    const int f = b.act[blockIdx.x];
+    if ((int)blockIdx.x >= render_n(b)) return;
+    const int f = b.rlist[blockIdx.x];
     FrameCtl &ctl = b.ctl[f];
-    if (!ctl.active) return;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (ctl.flags & (FLAG_RENDER_SKIPPED | FLAG_OVERFLOW)) {
+    if (!ctl.render) {                           // the resolve refused the raster
         if (tid == 0) ctl.active = 0;
         return;
     }
-    if (!ctl.render) return;
     extern __shared__ __align__(16) float rsm[];
     __shared__ double s_sum[NT / 32][LF_SUMS];
     __shared__ double s_tot[LF_SUMS];
@@ -2757,39 +2770,6 @@ __global__ void k_paint(DModel m, DBatch b, float *images, int32_t *tri_map)
         images[(size_t)f * NPIX + p] = s.tex;
         tri_map[(size_t)f * NPIX + p] = fr.tri;
     }
-}
-
-// Frames of the active list that render this round, in ascending order (one block).
-__global__ void __launch_bounds__(1024) k_compact_render(DBatch b)
-{
-    __shared__ int s_warp[32];
-    __shared__ int s_base;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0) s_base = 0;
-    __syncthreads();
-    const int na = active_n(b);
-    for (int i0 = 0; i0 < na; i0 += 1024) {
-        const int i = i0 + tid;
-        const int f = i < na ? b.act[i] : -1;
-        const int r = f >= 0 && b.ctl[f].render;
-        const unsigned mask = __ballot_sync(0xffffffffu, r);
-        if (lane == 0) s_warp[warp] = __popc(mask);
-        __syncthreads();
-        if (tid < 32) {
-            int v = s_warp[tid], incl = v;
-            for (int o = 1; o < 32; o <<= 1) {
-                const int t = __shfl_up_sync(0xffffffffu, incl, o);
-                if (tid >= o) incl += t;
-            }
-            s_warp[tid] = incl - v;
-        }
-        __syncthreads();
-        if (r) b.rlist[s_base + s_warp[warp] + __popc(mask & ((1u << lane) - 1u))] = f;
-        __syncthreads();
-        if (tid == 1023) s_base += s_warp[31] + __popc(mask);
-        __syncthreads();
-    }
-    if (tid == 0) b.rcount[0] = s_base;
 }
 
 // Frames still running the current stage, in ascending order (one block, block-wide scan).

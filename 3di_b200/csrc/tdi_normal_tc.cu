@@ -107,10 +107,9 @@ __device__ __forceinline__ uint32_t pack2(__nv_bfloat16 a, __nv_bfloat16 b)
 template <int GRP>
 __global__ void __launch_bounds__(TC_THREADS, 3) k_normal_eq_tc(DModel m, DBatch b)
 {
-    if ((int)blockIdx.y >= active_n(b)) return;
-    const int f = b.act[blockIdx.y];
+    if ((int)blockIdx.y >= jac_n(b)) return;
+    const int f = b.jlist[blockIdx.y];
     const FrameCtl &ctl = b.ctl[f];
-    if (!ctl.need_jac) return;
     const int N = ctl.N;
     const int nch = (N + NE_CH - 1) / NE_CH;
     if ((int)blockIdx.x >= nch) return;                  // the whole block leaves together
@@ -260,10 +259,9 @@ constexpr int TC_RBLOCKS = 4;
 
 __global__ void __launch_bounds__(256) k_normal_eq_tc_reduce(DModel m, DBatch b)
 {
-    if ((int)blockIdx.y >= active_n(b)) return;
-    const int f = b.act[blockIdx.y];
+    if ((int)blockIdx.y >= jac_n(b)) return;
+    const int f = b.jlist[blockIdx.y];
     const FrameCtl &ctl = b.ctl[f];
-    if (!ctl.need_jac) return;
     const int KTP = m.KTP, KT = m.KT, PK = tc_pitch(KT);
     const int nch = (ctl.N + NE_CH - 1) / NE_CH;
     const size_t pstride = tc_part_bytes(KT) / sizeof(float);
