@@ -277,6 +277,7 @@ tdi_status set_attrs()
     TDI_CUDA(cudaFuncSetAttribute(k_render_t<1024>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   RENDER_SMEM_FLOATS * (int)sizeof(float)));
     TDI_CUDA(cudaFuncSetAttribute(k_light_fit, cudaFuncAttributeMaxDynamicSharedMemorySize, LIGHT_SMEM));
+    TDI_CUDA(cudaFuncSetAttribute(k_raster_resolve, cudaFuncAttributeMaxDynamicSharedMemorySize, RR_SMEM));
     TDI_CUDA(cudaFuncSetAttribute(k_neighbours, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)neigh_smem()));
     TDI_CUDA(cudaFuncSetAttribute(k_vertex_t<VT_FPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
@@ -385,8 +386,8 @@ DBatch batch_view(const tdi_batch *bt, int f0, int nf)
     v.rcount = a.rcount + 2 * F0;
     v.geo = a.geo + F0 * m.V; v.proj = a.proj + F0 * m.V;
     v.zbuf = a.zbuf + F0 * NPIX;
-    v.tri_mask = a.tri_mask + F0 * mask_words(m.T);
-    v.tri_list = a.tri_list + F0 * m.T;
+    v.ccount = a.ccount + F0;
+    if (a.tri_work) v.tri_work = a.tri_work + F0 * resolve_words(m.T);
     v.frag = a.frag + F0 * NMAX;
     v.fgrad = a.fgrad + F0 * 5 * NMAX;
     v.nb = a.nb + F0 * 4 * NMAX;
@@ -440,7 +441,10 @@ tdi_status points(const Launch &L, const Cfg &c, int stage, int check)
 tdi_status raster(const Launch &L)
 {
     TDI_TRY(launch(L.bt, KID_RASTER, k_raster_depth, dim3(raster_grid(L.A())), dim3(RD_THREADS), 0, L.s, L.m, L.b));
-    return launch(L.bt, KID_RESOLVE, k_raster_resolve, dim3(L.A()), dim3(RR_THREADS), 0, L.s, L.m, L.b);
+    TDI_TRY(launch(L.bt, KID_RESOLVE, k_raster_resolve, dim3(L.A()), dim3(RR_THREADS), resolve_smem(L.m.T), L.s,
+                   L.m, L.b));
+    return launch(L.bt, 0, k_raster_slots, dim3(std::min(L.A() * RS_PARTS, 8 * sm_count())), dim3(RS_THREADS), 0, L.s,
+                  L.m, L.b);
 }
 
 tdi_status geometry(const Launch &L, const Cfg &c, int stage)
@@ -803,7 +807,7 @@ tdi_status tdi_batch_create(tdi_model *m, int32_t max_frames, tdi_batch **out)
     A(d.x, F * KTP); A(d.x_ls, F * KTP); A(d.xe, F * KTP);
     A(d.lam, F * 4); A(d.lam_ls, F * 4); A(d.lame, F * 4); A(d.dlam, F * 4); A(d.glam, F * 4);
     A(d.d, F * KTP); A(d.g, F * KTP); A(d.H, F * KTP * KTP); A(d.R, F * 9); A(d.dR, F * 27);
-    A(d.ctl, F); A(d.act, F); A(d.rlist, F); A(d.jlist, F); A(d.rcount, 2 * F); A(d.geo, F * (size_t)md.V); A(d.proj, F * (size_t)md.V); A(d.zbuf, F * NPIX); A(d.tri_mask, F * (size_t)mask_words(md.T)); A(d.tri_list, F * (size_t)md.T); A(d.frag, F * NMAX);
+    A(d.ctl, F); A(d.act, F); A(d.rlist, F); A(d.jlist, F); A(d.rcount, 2 * F); A(d.geo, F * (size_t)md.V); A(d.proj, F * (size_t)md.V); A(d.zbuf, F * NPIX); A(d.ccount, F); if (!resolve_smem(md.T)) A(d.tri_work, F * (size_t)resolve_words(md.T)); A(d.frag, F * NMAX);
     A(d.fgrad, F * 5 * NMAX); A(d.nb, F * 4 * NMAX); A(d.shc, F * NMAX); A(d.sht, F * NMAX);
     A(d.J, F * NMAX * KTP); b->ne_frame_doubles = NE_MAXCH * std::max((size_t)ne_part_stride((int)KTP), (tc_part_bytes(md.KT) + 7) / 8);
     A(d.ne_part, F * b->ne_frame_doubles); A(d.err, 1); A(d.img, F * RIMG); A(b->scalars, F * 4); A(b->d_count, 2);
@@ -814,7 +818,7 @@ tdi_status tdi_batch_create(tdi_model *m, int32_t max_frames, tdi_batch **out)
     if (cudaMemset(d.zbuf, 0xFF, F * NPIX * sizeof(unsigned long long)) != cudaSuccess ||
         cudaMemset(d.ctl, 0, F * sizeof(FrameCtl)) != cudaSuccess ||
         cudaMemset(d.err, 0, sizeof(int32_t)) != cudaSuccess ||
-        cudaMemset(d.tri_mask, 0, F * mask_words(md.T) * sizeof(uint32_t)) != cudaSuccess ||
+        cudaMemset(d.ccount, 0, F * sizeof(int32_t)) != cudaSuccess ||
         cudaMemset(d.x, 0, F * KTP * sizeof(float)) != cudaSuccess ||
         cudaMemset(d.x_ls, 0, F * KTP * sizeof(float)) != cudaSuccess ||
         cudaMemset(d.J, 0, F * NMAX * KTP * sizeof(float)) != cudaSuccess ||

@@ -61,6 +61,7 @@ struct FrameCtl {
     int32_t bbox[4];     // fragment pixel box of the last raster: xmin, xmax, ymin, ymax
     float objective;     // last accepted objective
     int32_t stage_ok;    // result of the last shape fit (outer > NITERS_SUCCESS)
+    int32_t slots;       // the resolve left the candidate of every slot (k_raster_slots copies them)
 };
 
 struct Fragment {        // one surviving fragment, in slot order
@@ -129,8 +130,9 @@ struct DBatch {
     float4 *geo;             // [F][V]: X0, Y0, Z0 and the albedo of the vertex (slot order)
     float4 *proj;            // [F][V]: xp, yp, camera Z, 0 -- what the raster gathers
     unsigned long long *zbuf;// [F][NPIX]
-    uint32_t *tri_mask;      // [F][ceil(T/32)] triangles with fragments in the raster in flight
-    int32_t *tri_list;       // [F][T] triangles with fragments, ascending
+    int32_t *ccount;         // [F] candidates of the raster in flight
+    uint32_t *tri_work;      // [F][resolve_words(T)] the resolve's bit sets for meshes too large for
+                             // shared memory (else null)
     Fragment *frag;          // [F][NMAX]
     float *fgrad;            // [F][5][NMAX]: gx, gy, h, gxs_n, gys_n
     int32_t *nb;             // [F][4][NMAX]: kl, kr, ka, kb

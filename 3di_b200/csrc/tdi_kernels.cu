@@ -569,16 +569,16 @@ __global__ void __launch_bounds__(PT_THREADS) k_point(DModel m, DBatch b, Cfg c,
 // Visibility (get_pixels_to_render + keep_only_minZ + remove_if, funcs.cu:900-1029,
 // renderer.cu:650-680) in two kernels.
 //
-// k_raster_depth: every triangle enumerates its <= 4 fragments in bounding-box order and
-// folds a 64-bit key [epoch tag | depth bits | triangle id] into the frame's z-buffer with
-// atomicMin; triangles with fragments set their bit in the frame's triangle mask. The
-// z-buffer does not depend on the visiting order, so triangles are visited in Morton order
-// of their centroids and their corners (vertex slots) lie close in memory.
+// k_raster_depth: every triangle enumerates its <= 4 fragments in bounding-box order, folds a
+// 64-bit key [epoch tag | depth bits | triangle id] into the frame's z-buffer with atomicMin
+// and appends the fragment to the frame's candidates. Neither depends on the visiting
+// order, so triangles are visited in Morton order of their centroids and their corners (vertex
+// slots) lie close in memory.
 //
-// k_raster_resolve, one block per frame: lists the masked triangles in ascending order
-// (clearing the mask), counts the survivors of every slot row (depth equal to the pixel
-// minimum), and writes them in slot order (row r, then triangle). The pixel owner is the
-// minimum key (smallest triangle among depth ties). Slot 0 is dropped, as remove_if(is_zero)
+// k_raster_resolve, one block per frame: the candidates whose depth equals their pixel's minimum
+// survive. Slot order is (row r, then triangle): every survivor sets its bit in one bit set per
+// row over the triangles, and its slot is the number of bits before its own. The pixel owner is
+// the minimum key (smallest triangle among depth ties). Slot 0 is dropped, as remove_if(is_zero)
 // does. The epoch tag makes earlier renders' keys lose to this one's without clearing the
 // z-buffer; it is cleared once the tag range is used up.
 
@@ -754,6 +754,15 @@ __device__ __forceinline__ void shade_geometry(const float4 &gb, const float4 &g
     t = (gb.w * al + gc.w * be) + ga4.w * ga;
 }
 
+// The shading inputs of a fragment as records: (unit normal, n . p), and the albedo t.
+__device__ __forceinline__ float4 shade_record(const float4 &gb, const float4 &gc, const float4 &ga, float al, float be,
+                                               float &t)
+{
+    float nn[3], p[3];
+    shade_geometry(gb, gc, ga, al, be, nn, p, t);
+    return make_float4(nn[0], nn[1], nn[2], (nn[0] * p[0] + nn[1] * p[1]) + nn[2] * p[2]);
+}
+
 __device__ __forceinline__ unsigned long long zkey(uint32_t tag, float Z, int tri)
 {
     return ((unsigned long long)tag << (31 + TRI_BITS)) |
@@ -767,44 +776,76 @@ __device__ __forceinline__ bool survives(unsigned long long k, uint32_t tag, uin
 }
 
 constexpr int RD_THREADS = 256;             // depth pass: threads per block
-constexpr int RD_BLOCKS = 16;               // depth pass: blocks per frame (at least)
+constexpr int RD_BLOCKS = 8;                // depth pass: blocks per frame (at least)
 constexpr int RD_MAX_BLOCKS = 128;          // depth pass: blocks per frame when few frames render
 constexpr int RD_SPREAD = 2400;             // blocks that fill the SMs twice over
 constexpr int RR_THREADS = 1024;            // resolve: one block per frame
 constexpr int RR_WARPS = RR_THREADS / 32;
-constexpr int RR_ILP = 2;                  // resolve: listed entries per lane in flight together
+constexpr int RR_U = 4;                     // resolve: candidates per thread in flight together
+constexpr int RD_CAND = 640;                // depth pass: candidates a block collects before it appends them
 
-// True when no sample point of the triangle can be a fragment, decided without evaluating one:
-// its box has at most 2 x 2 sample points, each of which lies outside the corners' range by
-// more than RC_MARGIN in x or in y, and the triangle is not a sliver.
+// A fragment of the raster in flight. Candidates of a frame lie in its Jacobian buffer (idle
+// between the solve and the next accepted point), CandidateSpan of them at most; a frame with more
+// takes the resolve's general path.
+struct __align__(16) Candidate {
+    uint32_t pix_row;                       // pixel | row << 16
+    int32_t tri;
+    float al, be;
+};
+
+struct CandidateSpan {
+    Candidate *c;
+    float4 *sn;                             // shading inputs: unit normal and n . p
+    float *t;                               // and interpolated albedo
+    float *z;                               // camera Z of the triangle's first corner
+    int cap;
+};
+
+__device__ __forceinline__ CandidateSpan candidates(const DModel &m, const DBatch &b, int f)
+{
+    CandidateSpan s;
+    const size_t bytes = (size_t)NMAX * m.KTP * sizeof(float);
+    s.cap = (int)(bytes / (sizeof(Candidate) + sizeof(float4) + 2 * sizeof(float)));
+    s.c = reinterpret_cast<Candidate *>(b.J + (size_t)f * NMAX * m.KTP);
+    s.sn = reinterpret_cast<float4 *>(s.c + s.cap);
+    s.t = reinterpret_cast<float *>(s.sn + s.cap);
+    s.z = s.t + s.cap;
+    return s;
+}
+
+// True when no sample point of the triangle can be a fragment, decided without evaluating one: the
+// box has a single sample column (or row), and it lies left of (above) every corner by a gap that
+// rounding cannot bridge for a triangle of this shape. (With two columns the second lies inside the
+// corners' range.)
 // Why no evaluation could accept such a point (u = 2^-24; l0 = |b - a|, l1 = |c - a|, s the sine
 // between them, D = (l0 l1 s)^2 the exact denominator; the corner differences carry one rounding
-// each): a point outside the range by M in one coordinate, of a triangle at most 2 wide, has a
-// barycentric coordinate of at most -e, e = M / 4 (1 - 1e-4). FP32 forms na and nb within
-// 13 u l1^2 l0 l2 and 13 u l0^2 l1 l2 and the denominator within 13 u l0^2 l1^2, l2 <= 2.83 the
-// distance of the point from a. alpha (beta) <= -e then gives na (nb) the wrong sign, and
-// alpha + beta >= 1 + e leaves the rounded sum above 1, whenever min(l0, l1) s^3 > 153 u / e =
-// 2.4e-3; the test below asks for 5.5e-3 (squared: RC_SLIVER). Any NaN fails a comparison here and
-// takes the full path, as do boxes outside the domain.
-constexpr float RC_MARGIN = 1.0f / 64.0f;
-constexpr float RC_SLIVER = 3e-5f;
+// each): a point outside the range by g in a coordinate in which the triangle is at most 1 wide has
+// a barycentric coordinate of at most -e, e = g / 2 (1 - 1e-3). FP32 forms na and nb within
+// 13 u l1^2 l0 l2 and 13 u l0^2 l1 l2 and the denominator within 13 u l0^2 l1^2, l2 <= 3.2 the
+// distance of the point from a (the triangle is at most 2 wide in the other coordinate). alpha
+// (beta) <= -e then gives na (nb) the wrong sign, and alpha + beta >= 1 + e leaves the rounded sum
+// above 1, whenever g min(l0, l1) s^3 > 2 x 173 u (1 + 1e-3) = 2.1e-5; the test below asks for
+// 4.5e-5 (squared: RC_SHAPE), and for a gap that is large against the rounding of the differences
+// (RC_GAP). Any NaN makes the shape test fail and takes the full path, as do boxes outside
+// the domain.
+constexpr float RC_GAP = 1.0f / 4096.0f;
+constexpr float RC_SHAPE = 2.025e-9f;
 
 __device__ __forceinline__ bool no_sample_inside(float bx, float by, float cx, float cy, float ax, float ay)
 {
     const float xmax = fmaxf(fmaxf(bx, cx), ax), xmin = fminf(fminf(bx, cx), ax);
     const float ymax = fmaxf(fmaxf(by, cy), ay), ymin = fminf(fminf(by, cy), ay);
-    const float xhi = ceilf(xmax), yhi = ceilf(ymax), xlo = floorf(xmin), ylo = floorf(ymin);
-    const bool dom = xlo >= 0.0f && ylo >= 0.0f && xhi <= 65535.0f && yhi <= 65535.0f && xhi - xlo <= 2.0f &&
-                     yhi - ylo <= 2.0f;
-    // columns xlo and xlo + 1 (rows alike): outside by more than the margin, or not sampled
-    const float x1 = xlo + 1.0f, y1 = ylo + 1.0f;
-    const bool xout = xmin - xlo > RC_MARGIN && (x1 >= xhi || x1 - xmax > RC_MARGIN);
-    const bool yout = ymin - ylo > RC_MARGIN && (y1 >= yhi || y1 - ymax > RC_MARGIN);
+    const bool dom = fminf(xmin, ymin) >= 0.0f && fmaxf(xmax, ymax) <= 65535.0f &&
+                     fmaxf(xmax - xmin, ymax - ymin) <= 2.0f;
+    const float xlo = floorf(xmin), ylo = floorf(ymin);
+    const float gx = xmax <= xlo + 1.0f ? xmin - xlo : 0.0f;
+    const float gy = ymax <= ylo + 1.0f ? ymin - ylo : 0.0f;
+    const float g = fmaxf(gx, gy);
     const float v0x = bx - ax, v1x = cx - ax, v0y = by - ay, v1y = cy - ay;
     const float d00 = v0x * v0x + v0y * v0y, d01 = v0x * v1x + v0y * v1y, d11 = v1x * v1x + v1y * v1y;
     const float q = d00 * d11, denom = q - d01 * d01;
-    const bool wide = (denom * denom) * (denom * fminf(d00, d11)) > RC_SLIVER * ((q * q) * q);
-    return dom && (xout || yout) && wide;
+    const bool shape = (denom * denom) * (denom * fminf(d00, d11)) * (g * g) > RC_SHAPE * ((q * q) * q);
+    return dom && g > RC_GAP && shape;
 }
 
 // Blocks per frame for rc rendering frames, and the largest grid up to `frames` of them can ask for.
@@ -821,13 +862,16 @@ inline int raster_grid(int frames)
 
 // A dense face mesh has about 25 triangles per visible fragment, most of them smaller than a
 // pixel, so the pass is bound by the instructions spent on triangles without a sample
-// point. Each warp therefore first tests its triangles with no_sample_inside (about 55
-// instructions instead of about 230) and queues the others' corners in shared memory; a full
-// warp's worth of queued triangles is then evaluated densely. Two triangles per lane have
-// their gathers in flight together. 1,024 frames of the 53,490-vertex model in one launch:
-// 1,192 -> 697 us (0.68 us per frame); 174 -> 106 us averaged over the rounds of that fit.
+// point. Each warp therefore first tests its triangles with no_sample_inside (about 50
+// instructions instead of about 230) and queues the others' corners in shared memory (12-15% of the
+// 53,490-vertex mesh's); a full warp's worth of queued triangles is then evaluated densely. RD_ILP
+// triangles per lane have their gathers in flight together (1,024 frames in one launch: 1 875 us,
+// 2 707, 3 671; a fifth block per SM needs 48 registers and spills, 953).
+// 1,024 frames of the 53,490-vertex model in one launch: 1,192 us with every sample evaluated in
+// place, 671 with the queue, the candidates and their shading inputs included (which the resolve
+// formed before). What is left is issue (0.68 per cycle) and the latency of the gathers.
 constexpr int RD_WARPS = RD_THREADS / 32;
-constexpr int RD_ILP = 2;                   // triangles per lane and step
+constexpr int RD_ILP = 3;                   // triangles per lane and step
 constexpr int RD_QUEUE = 32 * (RD_ILP + 1); // a warp's queue: what a step adds to a remainder below 32
 
 __global__ void __launch_bounds__(RD_THREADS) k_raster_depth(DModel m, DBatch b)
@@ -842,15 +886,34 @@ __global__ void __launch_bounds__(RD_THREADS) k_raster_depth(DModel m, DBatch b)
     const FrameCtl &ctl = b.ctl[f];
     if (part == 0 && threadIdx.x == 0) prof_count(b, KID_RASTER);
     __shared__ float4 s_qa[RD_WARPS][RD_QUEUE];     // bx, by, cx, cy
-    __shared__ float4 s_qb[RD_WARPS][RD_QUEUE];     // ax, ay, camera Z of b, triangle id (bits)
+    __shared__ float4 s_qb[RD_WARPS][RD_QUEUE];     // ax, ay, camera Z of b, place in the Morton order (bits)
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     float4 *qa = s_qa[warp], *qb = s_qb[warp];
     const uint32_t tag = TAG_MAX - (ctl.epoch + 1);
     const float4 *pj = b.proj + (size_t)f * m.V;
     unsigned long long *zb = b.zbuf + (size_t)f * NPIX;
-    uint32_t *mask = b.tri_mask + (size_t)f * mask_words(m.T);
     const int x0 = b.x0y0[2 * f], y0 = b.x0y0[2 * f + 1];
     const int T = m.T;
+    // candidates are collected per block and appended together: one global counter update per
+    // block. Their shading inputs are formed then, for every render of this raster: here the corners'
+    // geometry lies close together in Morton order and the gathers are spread over all SMs.
+    __shared__ Candidate s_cand[RD_CAND];
+    __shared__ float s_cz[RD_CAND];
+    __shared__ int s_cs[RD_CAND];
+    const CandidateSpan cs = candidates(m, b, f);
+    const float4 *geo = b.geo + (size_t)f * m.V;
+    auto append = [&](int g, const Candidate &cd, float z, int place) {
+        if (g >= cs.cap) return;
+        const int4 tq = __ldg(m.tlo4 + place);
+        float t;
+        cs.sn[g] = shade_record(__ldg(geo + tq.x), __ldg(geo + tq.y), __ldg(geo + tq.z), cd.al, cd.be, t);
+        cs.t[g] = t;
+        cs.c[g] = cd;
+        cs.z[g] = z;
+    };
+    __shared__ int s_nc, s_base;
+    if (threadIdx.x == 0) s_nc = 0;
+    __syncthreads();
     // each block a contiguous range of the Morton order
     const int per_block = (T + parts - 1) / parts;
     const int s_begin = part * per_block, s_end = min(T, s_begin + per_block);
@@ -858,14 +921,22 @@ __global__ void __launch_bounds__(RD_THREADS) k_raster_depth(DModel m, DBatch b)
     int queued = 0;                                 // entries of the warp's queue
     auto evaluate = [&](int e) {
         const float4 A = qa[e], B = qb[e];
-        const int idx = __float_as_int(B.w);
+        const int place = __float_as_int(B.w), idx = __ldg(&m.tlo4[place].w);
         const unsigned long long key = zkey(tag, B.z, idx);
         const int nf = tri_samples(A.x, A.y, A.z, A.w, B.x, B.y, x0, y0, flags,
-                                   [&](int, uint32_t px, float, float) { atomicMin(zb + px, key); });
-        if (nf) {
-            if (!(B.z > 0.0f)) flags |= FLAG_OUT_OF_DOMAIN;
-            atomicOr(mask + (idx >> 5), 1u << (idx & 31));
-        }
+                                   [&](int r, uint32_t px, float al, float be) {
+                                       atomicMin(zb + px, key);
+                                       const Candidate cd{px | ((uint32_t)r << 16), idx, al, be};
+                                       const int k = atomicAdd(&s_nc, 1);
+                                       if (k < RD_CAND) {
+                                           s_cand[k] = cd;
+                                           s_cz[k] = B.z;
+                                           s_cs[k] = place;
+                                       } else {
+                                           append(atomicAdd(b.ccount + f, 1), cd, B.z, place);
+                                       }
+                                   });
+        if (nf && !(B.z > 0.0f)) flags |= FLAG_OUT_OF_DOMAIN;
     };
     for (int base = s_begin + warp * 32 * RD_ILP; base < s_end; base += RD_THREADS * RD_ILP) {
         int4 tq[RD_ILP];
@@ -886,7 +957,7 @@ __global__ void __launch_bounds__(RD_THREADS) k_raster_depth(DModel m, DBatch b)
             if (take) {
                 const int e = queued + __popc(msk & ((1u << lane) - 1u));
                 qa[e] = make_float4(pb[h].x, pb[h].y, pc[h].x, pc[h].y);
-                qb[e] = make_float4(pa[h].x, pa[h].y, pb[h].z, __int_as_float(tq[h].w));
+                qb[e] = make_float4(pa[h].x, pa[h].y, pb[h].z, __int_as_float(base + 32 * h + lane));
             }
             queued += __popc(msk);
         }
@@ -899,6 +970,11 @@ __global__ void __launch_bounds__(RD_THREADS) k_raster_depth(DModel m, DBatch b)
     }
     if (lane < queued) evaluate(lane);
     if (flags) atomicOr(&b.ctl[f].flags, flags);
+    __syncthreads();
+    const int nc = min(s_nc, RD_CAND);
+    if (threadIdx.x == 0 && nc) s_base = atomicAdd(b.ccount + f, nc);
+    __syncthreads();
+    for (int e = threadIdx.x; e < nc; e += RD_THREADS) append(s_base + e, s_cand[e], s_cz[e], s_cs[e]);
 }
 
 // Block-wide exclusive scan of one value per thread (RR_THREADS threads); returns the
@@ -932,293 +1008,186 @@ __device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t *s_w, uint32
     return off;
 }
 
+// Words of the resolve's working set: NTMP bit sets over the triangles and as many offsets. In shared
+// memory when they fit (two blocks per SM for 106,466 triangles), else in the frame's buffer.
+constexpr int RR_SMEM = 224 * 1024;
+__host__ __device__ __forceinline__ int resolve_words(int T) { return 2 * NTMP * mask_words(T); }
+__host__ __device__ __forceinline__ size_t resolve_smem(int T)
+{
+    const size_t bytes = (size_t)resolve_words(T) * sizeof(uint32_t);
+    return bytes <= RR_SMEM ? bytes : 0;
+}
+
+// What bounds it is latency (a candidate's record, then its pixel's key, twice), so RR_U candidates
+// per thread are in flight together. Listing the triangles with fragments from a bit mask,
+// re-evaluating their samples, staging the survivors and forming their shading inputs here took 40 us
+// for 77 frames (319 us for 1,024); most of it was gathering the corners' geometry through one
+// SM, which the depth pass's blocks now do with their candidates. 16 us (176) with
+// k_raster_slots.
 __global__ void __launch_bounds__(RR_THREADS) k_raster_resolve(DModel m, DBatch b)
 {
     if ((int)blockIdx.x >= render_n(b)) return;
     const int f = b.rlist[blockIdx.x];
     FrameCtl &ctl = b.ctl[f];
     if (threadIdx.x == 0) prof_count(b, KID_RESOLVE);
+    extern __shared__ __align__(16) uint32_t rrs[];
     __shared__ uint32_t s_w[RR_WARPS + 1];
-    __shared__ uint32_t s_cnt[RR_WARPS][NTMP];   // survivors per warp and row
-    __shared__ uint32_t s_off[RR_WARPS][NTMP];   // exclusive offsets of the warps per row
-    __shared__ uint32_t s_row[NTMP + 1];         // row bases; s_row[NTMP] = total
     __shared__ int s_bbox[4];
-    __shared__ uint32_t s_flags;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const unsigned lt_mask = (1u << lane) - 1u;
-    const int T = m.T;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int T = m.T, W = mask_words(T);
+    uint32_t *bits = resolve_smem(T) ? rrs : b.tri_work + (size_t)f * resolve_words(T);   // [NTMP][W]
+    uint32_t *pre = bits + NTMP * W;                                                       // bits before each word
     const uint32_t epoch = ctl.epoch + 1;
     const uint32_t tag = TAG_MAX - epoch;
     unsigned long long *zb = b.zbuf + (size_t)f * NPIX;
-    uint32_t *mask = b.tri_mask + (size_t)f * mask_words(T);
-    int32_t *list = b.tri_list + (size_t)f * T;
     const float4 *pj = b.proj + (size_t)f * m.V;
+    const float4 *geo = b.geo + (size_t)f * m.V;
     const int x0 = b.x0y0[2 * f], y0 = b.x0y0[2 * f + 1];
+    const CandidateSpan cs = candidates(m, b, f);
+    const int nc = b.ccount[f];
+    const bool listed = nc <= cs.cap;
     if (tid == 0) {
-        s_flags = 0;
         s_bbox[0] = s_bbox[2] = 1 << 30;
         s_bbox[1] = s_bbox[3] = -1;
     }
-
-    // list of the masked triangles, ascending: each thread a contiguous run of mask words
-    const int W = mask_words(T);
-    const int wpt = (W + RR_THREADS - 1) / RR_THREADS;
-    const int w_begin = min(W, tid * wpt), w_end = min(W, w_begin + wpt);
-    uint32_t nz = 0;
-    for (int w = w_begin; w < w_end; ++w) nz += __popc(__ldcg(mask + w));
-    uint32_t L;
-    uint32_t pos = block_scan(nz, s_w, &L);
-    for (int w = w_begin; w < w_end; ++w) {
-        uint32_t bits = __ldcg(mask + w);
-        if (bits) mask[w] = 0u;
-        while (bits) {
-            const int bit = __ffs(bits) - 1;
-            bits &= bits - 1u;
-            list[pos++] = w * 32 + bit;
-        }
-    }
+    for (int w = tid; w < NTMP * W; w += RR_THREADS) bits[w] = 0u;
     __syncthreads();
-    // list entries per warp, contiguous; lanes take consecutive entries
-    const int per_e = (int)(((L + RR_WARPS * 32 - 1) / (RR_WARPS * 32)) * 32);
-    const int e_begin = min((int)L, warp * per_e);
-    const int e_end = min((int)L, e_begin + per_e);
-
-    // Survivors of every listed triangle, per slot row and warp. When the frame's per-warp,
-    // per-row staging fits the gradient buffer (unused until the render), the survivors are
-    // formed once here and copied to their slots after the scan; otherwise the triangles are
-    // evaluated a second time in the write pass.
-    Fragment *stage = reinterpret_cast<Fragment *>(b.fgrad + (size_t)f * 5 * NMAX);
-    const bool one_pass = (size_t)RR_WARPS * NTMP * per_e * sizeof(Fragment) <= (size_t)5 * NMAX * sizeof(float);
-    Fragment *wstage = stage + (size_t)warp * NTMP * per_e;     // [NTMP][per_e] of this warp
-    int bx0 = 1 << 30, bx1 = -1, by0 = 1 << 30, by1 = -1;
-    // one listed triangle: survivor flags, owners, pixels and barycentrics of its samples
-    auto evaluate = [&](int e, bool (&sv)[NTMP], bool (&own)[NTMP], uint32_t (&pix)[NTMP],
-                        float (&al)[NTMP], float (&be)[NTMP]) -> int {
-        const int idx = __ldcg(list + e);
-        const int4 tc = __ldg(m.tl4 + idx);
-        const float4 pb = __ldg(pj + tc.x);
-        const float4 pc = __ldg(pj + tc.y);
-        const float4 pa = __ldg(pj + tc.z);
-        const uint32_t zbits = __float_as_uint(pb.z) & 0x7FFFFFFFu;
-        const unsigned long long mykey = zkey(tag, pb.z, idx);
-        uint32_t fl2 = 0;
-        tri_samples(pb.x, pb.y, pc.x, pc.y, pa.x, pa.y, x0, y0, fl2, [&](int r, uint32_t px, float a, float bb) {
-            const unsigned long long k = __ldcg(zb + px);
-            sv[r] = survives(k, tag, zbits) && !(r == 0 && idx == 0);
-            own[r] = (k == mykey);
-            pix[r] = px; al[r] = a; be[r] = bb;
-        });
-        return idx;
+    // visit(c, z, key, i): every candidate with its pixel's key and its place in the list
+    auto for_candidates = [&](auto &&visit) {
+        if (listed) {
+            for (int i0 = tid; i0 < nc; i0 += RR_THREADS * RR_U) {
+                Candidate cd[RR_U];
+                float z[RR_U];
+                unsigned long long key[RR_U];
+#pragma unroll
+                for (int u = 0; u < RR_U; ++u) {
+                    const int i = i0 + u * RR_THREADS;
+                    if (i < nc) { cd[u] = cs.c[i]; z[u] = cs.z[i]; }
+                }
+#pragma unroll
+                for (int u = 0; u < RR_U; ++u)
+                    if (i0 + u * RR_THREADS < nc) key[u] = __ldcg(zb + (cd[u].pix_row & 0xFFFFu));
+#pragma unroll
+                for (int u = 0; u < RR_U; ++u)
+                    if (i0 + u * RR_THREADS < nc) visit(cd[u], z[u], key[u], i0 + u * RR_THREADS);
+            }
+        } else {
+            // more candidates than the buffer holds: every triangle's samples again
+            for (int idx = tid; idx < T; idx += RR_THREADS) {
+                const int4 tc = __ldg(m.tl4 + idx);
+                const float4 pb = __ldg(pj + tc.x), pc = __ldg(pj + tc.y), pa = __ldg(pj + tc.z);
+                uint32_t fl2 = 0;
+                tri_samples(pb.x, pb.y, pc.x, pc.y, pa.x, pa.y, x0, y0, fl2, [&](int r, uint32_t px, float al, float be) {
+                    visit(Candidate{px | ((uint32_t)r << 16), idx, al, be}, pb.z, __ldcg(zb + px), -1);
+                });
+            }
+        }
     };
-    uint32_t cnt[NTMP] = {0, 0, 0, 0};
-    if (one_pass) {
-        // RR_ILP entries per lane and step (entries base + 32 h + lane), in phases: all their
-        // triangles' corners, all sample sets, all z-buffer keys, then the survivors entry by
-        // entry in entry order, so that the dependent loads of the entries overlap
-        for (int base = e_begin; base < e_end; base += 32 * RR_ILP) {
-            int idx[RR_ILP];
-            int4 tq[RR_ILP];
-            float4 pb[RR_ILP], pc[RR_ILP], pa[RR_ILP];
-#pragma unroll
-            for (int h = 0; h < RR_ILP; ++h) {
-                const int e = base + 32 * h + lane;
-                idx[h] = e < e_end ? __ldcg(list + e) : -1;
-            }
-#pragma unroll
-            for (int h = 0; h < RR_ILP; ++h) tq[h] = __ldg(m.tl4 + (idx[h] >= 0 ? idx[h] : 0));
-#pragma unroll
-            for (int h = 0; h < RR_ILP; ++h) {
-                pb[h] = __ldg(pj + tq[h].x);
-                pc[h] = __ldg(pj + tq[h].y);
-                pa[h] = __ldg(pj + tq[h].z);
-            }
-            uint32_t pix[RR_ILP][NTMP];
-            float al[RR_ILP][NTMP], be[RR_ILP][NTMP];
-            int nf[RR_ILP];
-#pragma unroll
-            for (int h = 0; h < RR_ILP; ++h) {
-                nf[h] = 0;
-                if (idx[h] >= 0) {
-                    uint32_t fl2 = 0;
-                    nf[h] = tri_samples(pb[h].x, pb[h].y, pc[h].x, pc[h].y, pa[h].x, pa[h].y, x0, y0, fl2,
-                                        [&](int r, uint32_t px, float a, float bb) {
-                                            pix[h][r] = px; al[h][r] = a; be[h][r] = bb;
-                                        });
-                }
-            }
-            unsigned long long key[RR_ILP][NTMP];
-#pragma unroll
-            for (int h = 0; h < RR_ILP; ++h)
-#pragma unroll
-                for (int r = 0; r < NTMP; ++r) key[h][r] = r < nf[h] ? __ldcg(zb + pix[h][r]) : 0ull;
-#pragma unroll
-            for (int h = 0; h < RR_ILP; ++h) {
-                const uint32_t zbits = __float_as_uint(pb[h].z) & 0x7FFFFFFFu;
-                const unsigned long long mykey = zkey(tag, pb[h].z, idx[h]);
-#pragma unroll
-                for (int r = 0; r < NTMP; ++r) {
-                    const bool sv = r < nf[h] && survives(key[h][r], tag, zbits) && !(r == 0 && idx[h] == 0);
-                    const unsigned msk = __ballot_sync(0xffffffffu, sv);
-                    if (sv) {
-                        Fragment fr;
-                        fr.pix_owner = pix[h][r] | (key[h][r] == mykey ? 0x80000000u : 0u);
-                        fr.tri = idx[h];
-                        fr.al = al[h][r];
-                        fr.be = be[h][r];
-                        wstage[(size_t)r * per_e + cnt[r] + __popc(msk & lt_mask)] = fr;
-                        const int px = (int)(pix[h][r] >> 8), py = (int)(pix[h][r] & 255);
-                        bx0 = min(bx0, px); bx1 = max(bx1, px);
-                        by0 = min(by0, py); by1 = max(by1, py);
-                    }
-                    cnt[r] += __popc(msk);
-                }
-            }
-        }
-    } else {
-        // counts only; the survivors are formed again in the write pass
-        for (int base = e_begin; base < e_end; base += 32) {
-            const int e = base + lane;
-            bool sv[NTMP] = {false, false, false, false};
-            bool own[NTMP] = {false, false, false, false};
-            uint32_t pix[NTMP] = {0, 0, 0, 0};
-            float al[NTMP] = {0.0f, 0.0f, 0.0f, 0.0f}, be[NTMP] = {0.0f, 0.0f, 0.0f, 0.0f};
-            if (e < e_end) evaluate(e, sv, own, pix, al, be);
-#pragma unroll
-            for (int r = 0; r < NTMP; ++r) cnt[r] += __popc(__ballot_sync(0xffffffffu, sv[r]));
-        }
-    }
-    if (lane == 0)
-        for (int r = 0; r < NTMP; ++r) s_cnt[warp][r] = cnt[r];
-    __syncthreads();
-    if (warp == 0) {
-        // per row: exclusive scan over the warps (lane = warp index)
-        uint32_t rowsum[NTMP];
-#pragma unroll
-        for (int r = 0; r < NTMP; ++r) {
-            const uint32_t v = lane < RR_WARPS ? s_cnt[lane][r] : 0u;
-            uint32_t inc = v;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t t = __shfl_up_sync(0xffffffffu, inc, o);
-                if (lane >= o) inc += t;
-            }
-            if (lane < RR_WARPS) s_off[lane][r] = inc - v;
-            rowsum[r] = __shfl_sync(0xffffffffu, inc, 31);
-        }
-        if (lane == 0) {
-            uint32_t acc = 0;
-            for (int r = 0; r < NTMP; ++r) { s_row[r] = acc; acc += rowsum[r]; }
-            s_row[NTMP] = acc;
-            ctl.N = (int)min(acc, (uint32_t)NMAX);
-            uint32_t fl = 0;
-            if (acc > (uint32_t)NMAX) fl |= FLAG_OVERFLOW;
-            if (acc < 1000u || acc > 52000u) fl |= FLAG_RENDER_SKIPPED;
-            if (acc > 25600u) fl |= FLAG_OUT_OF_DOMAIN;
-            s_flags = fl;
-        }
-    }
-    __syncthreads();
-
-    // survivors in slot order (row, then triangle)
-    uint32_t wbase[NTMP];
-#pragma unroll
-    for (int r = 0; r < NTMP; ++r) wbase[r] = s_row[r] + s_off[warp][r];
-    Fragment *out = b.frag + (size_t)f * NMAX;
-    if (one_pass) {
-#pragma unroll
-        for (int r = 0; r < NTMP; ++r)
-            for (uint32_t k = lane; k < cnt[r]; k += 32) {
-                const uint32_t p = wbase[r] + k;
-                if (p < (uint32_t)NMAX) out[p] = wstage[(size_t)r * per_e + k];
-            }
-    } else {
-        uint32_t run[NTMP] = {0, 0, 0, 0};
-        for (int base = e_begin; base < e_end; base += 32) {
-            const int e = base + lane;
-            bool sv[NTMP] = {false, false, false, false};
-            bool own[NTMP] = {false, false, false, false};
-            uint32_t pix[NTMP] = {0, 0, 0, 0};
-            float al[NTMP] = {0.0f, 0.0f, 0.0f, 0.0f}, be[NTMP] = {0.0f, 0.0f, 0.0f, 0.0f};
-            int idx = -1;
-            if (e < e_end) idx = evaluate(e, sv, own, pix, al, be);
-#pragma unroll
-            for (int r = 0; r < NTMP; ++r) {
-                const unsigned msk = __ballot_sync(0xffffffffu, sv[r]);
-                if (sv[r]) {
-                    const uint32_t p = wbase[r] + run[r] + __popc(msk & lt_mask);
-                    if (p < (uint32_t)NMAX) {
-                        Fragment fr;
-                        fr.pix_owner = pix[r] | (own[r] ? 0x80000000u : 0u);
-                        fr.tri = idx;
-                        fr.al = al[r];
-                        fr.be = be[r];
-                        out[p] = fr;
-                    }
-                    const int px = (int)(pix[r] >> 8), py = (int)(pix[r] & 255);
-                    bx0 = min(bx0, px); bx1 = max(bx1, px);
-                    by0 = min(by0, py); by1 = max(by1, py);
-                }
-                run[r] += __popc(msk);
-            }
-        }
-    }
-    if (bx1 >= 0) {
+    auto survivor = [&](const Candidate &c, float z, unsigned long long key) -> bool {
+        return survives(key, tag, __float_as_uint(z) & 0x7FFFFFFFu) && !(c.tri == 0 && (c.pix_row >> 16) == 0);
+    };
+    int bx0 = 1 << 30, bx1 = -1, by0 = 1 << 30, by1 = -1;
+    for_candidates([&](const Candidate &c, float z, unsigned long long key, int) {
+        if (!survivor(c, z, key)) return;
+        atomicOr(bits + (c.pix_row >> 16) * W + (c.tri >> 5), 1u << (c.tri & 31));
+        const int px = (int)((c.pix_row >> 8) & 255u), py = (int)(c.pix_row & 255u);
+        bx0 = min(bx0, px); bx1 = max(bx1, px);
+        by0 = min(by0, py); by1 = max(by1, py);
+    });
+    bx0 = __reduce_min_sync(0xffffffffu, bx0); bx1 = __reduce_max_sync(0xffffffffu, bx1);
+    by0 = __reduce_min_sync(0xffffffffu, by0); by1 = __reduce_max_sync(0xffffffffu, by1);
+    if (lane == 0 && bx1 >= 0) {
         atomicMin(&s_bbox[0], bx0); atomicMax(&s_bbox[1], bx1);
         atomicMin(&s_bbox[2], by0); atomicMax(&s_bbox[3], by1);
     }
     __syncthreads();
-    // Shading inputs of every fragment for the renders of this raster: unit normal and n . p
-    // (shc), interpolated albedo (sht), formed by shade_geometry as shade() forms them, so that
-    // the renders shade from coalesced records instead of gathering the triangle corners (R,
-    // tau and the light enter per render). RR_ILP fragments per thread have their loads in
-    // flight together. (A separate kernel of 8 blocks per frame measured slower: 38.7 us per
-    // launch against the 28 us this adds to the resolve, whose other phases it overlaps.)
-    if (!(s_flags & (FLAG_RENDER_SKIPPED | FLAG_OVERFLOW))) {
-        const int Nf = (int)min(s_row[NTMP], (uint32_t)NMAX);
-        const float4 *geo = b.geo + (size_t)f * m.V;
-        float4 *shc = b.shc + (size_t)f * NMAX;
-        float *sht = b.sht + (size_t)f * NMAX;
-        for (int p0 = tid; p0 < Nf; p0 += RR_THREADS * RR_ILP) {
-            Fragment fr[RR_ILP];
-            int4 tq[RR_ILP];
-            float4 gb[RR_ILP], gc[RR_ILP], ga[RR_ILP];
-#pragma unroll
-            for (int h = 0; h < RR_ILP; ++h) {
-                const int p = p0 + h * RR_THREADS;
-                fr[h] = p < Nf ? out[p] : Fragment{0u, 0, 0.0f, 0.0f};
-            }
-#pragma unroll
-            for (int h = 0; h < RR_ILP; ++h) tq[h] = __ldg(m.tl4 + fr[h].tri);
-#pragma unroll
-            for (int h = 0; h < RR_ILP; ++h) {
-                gb[h] = geo[tq[h].x];
-                gc[h] = geo[tq[h].y];
-                ga[h] = geo[tq[h].z];
-            }
-#pragma unroll
-            for (int h = 0; h < RR_ILP; ++h) {
-                const int p = p0 + h * RR_THREADS;
-                if (p >= Nf) continue;
-                float nn[3], pp[3], t;
-                shade_geometry(gb[h], gc[h], ga[h], fr[h].al, fr[h].be, nn, pp, t);
-                shc[p] = make_float4(nn[0], nn[1], nn[2], (nn[0] * pp[0] + nn[1] * pp[1]) + nn[2] * pp[2]);
-                sht[p] = t;
-            }
-        }
+    // bits before every word, in slot order (row by row): each thread a contiguous run of words
+    const int wpt = (NTMP * W + RR_THREADS - 1) / RR_THREADS;
+    const int w_begin = min(NTMP * W, tid * wpt), w_end = min(NTMP * W, w_begin + wpt);
+    uint32_t nz = 0;
+    for (int w = w_begin; w < w_end; ++w) nz += __popc(bits[w]);
+    uint32_t total;
+    uint32_t run = block_scan(nz, s_w, &total);
+    for (int w = w_begin; w < w_end; ++w) {
+        pre[w] = run;
+        run += __popc(bits[w]);
     }
+    __syncthreads();
+    uint32_t fl = 0;
+    if (total > (uint32_t)NMAX) fl |= FLAG_OVERFLOW;
+    if (total < 1000u || total > 52000u) fl |= FLAG_RENDER_SKIPPED;
+    if (total > 25600u) fl |= FLAG_OUT_OF_DOMAIN;
+    const bool refused = (fl & (FLAG_RENDER_SKIPPED | FLAG_OVERFLOW)) != 0;
+    // Every survivor's slot: the candidate of each slot for k_raster_slots, or (when the candidates
+    // did not fit) the fragment itself with its shading inputs.
+    Fragment *out = b.frag + (size_t)f * NMAX;
+    float4 *shc = b.shc + (size_t)f * NMAX;
+    float *sht = b.sht + (size_t)f * NMAX;
+    uint32_t *slot = reinterpret_cast<uint32_t *>(b.nb + (size_t)f * 4 * NMAX);
+    for_candidates([&](const Candidate &c, float z, unsigned long long key, int i) {
+        if (!survivor(c, z, key)) return;
+        const int w = (int)(c.pix_row >> 16) * W + (c.tri >> 5);
+        const uint32_t p = pre[w] + __popc(bits[w] & ((1u << (c.tri & 31)) - 1u));
+        if (p >= (uint32_t)NMAX) return;
+        const uint32_t owner = key == zkey(tag, z, c.tri) ? 0x80000000u : 0u;
+        if (i >= 0) {
+            slot[p] = (uint32_t)i | owner;
+            return;
+        }
+        const Fragment fr{(c.pix_row & 0xFFFFu) | owner, c.tri, c.al, c.be};
+        const int4 tq = __ldg(m.tl4 + c.tri);
+        float t;
+        out[p] = fr;
+        shc[p] = shade_record(geo[tq.x], geo[tq.y], geo[tq.z], c.al, c.be, t);
+        sht[p] = t;
+    });
     if (epoch == TAG_MAX) {
         // tag range used up: the next raster starts from a cleared z-buffer
+        __syncthreads();
         for (int p = tid; p < NPIX; p += RR_THREADS) zb[p] = ~0ull;
     }
     if (tid == 0) {
-        const uint32_t fl = s_flags;
+        ctl.N = (int)min(total, (uint32_t)NMAX);
         ctl.epoch = epoch == TAG_MAX ? 0u : epoch;
         ctl.flags |= fl;
         ctl.renders += 1;
         for (int q = 0; q < 4; ++q) ctl.bbox[q] = s_bbox[q];
         if (s_bbox[1] >= 0 && (s_bbox[0] < 1 || s_bbox[1] > DIM - 2 || s_bbox[2] < 1 || s_bbox[3] > DIM - 2))
             ctl.flags |= FLAG_OUT_OF_DOMAIN;
-        if (fl & (FLAG_RENDER_SKIPPED | FLAG_OVERFLOW)) ctl.render = 0;
+        if (refused) ctl.render = 0;
+        ctl.slots = listed;
+        b.ccount[f] = 0;                     // (every thread has read it: barriers above)
+    }
+}
+
+// The fragments of a raster in slot order with their shading inputs for its renders (unit normal and
+// n . p in shc, interpolated albedo in sht, so that the renders shade from coalesced records;
+// R, tau and the light enter per render). Slot order follows the triangle numbering, which has
+// nothing to do with the order in which candidates were found: three scattered records per
+// fragment, which took one SM 17 us per frame inside the resolve and here are spread over RS_PARTS
+// blocks per frame.
+constexpr int RS_THREADS = 256, RS_PARTS = 16;
+
+__global__ void __launch_bounds__(RS_THREADS) k_raster_slots(DModel m, DBatch b)
+{
+    const int rc = render_n(b);
+    for (int it = blockIdx.x; it < rc * RS_PARTS; it += gridDim.x) {
+        const int f = b.rlist[it / RS_PARTS];
+        const FrameCtl &ctl = b.ctl[f];
+        if (!ctl.slots) continue;
+        const int N = ctl.N;
+        const CandidateSpan cs = candidates(m, b, f);
+        const uint32_t *slot = reinterpret_cast<const uint32_t *>(b.nb + (size_t)f * 4 * NMAX);
+        for (int p = (it % RS_PARTS) * RS_THREADS + threadIdx.x; p < N; p += RS_PARTS * RS_THREADS) {
+            const uint32_t s = slot[p];
+            const int i = (int)(s & 0x7FFFFFFFu);
+            const Candidate c = cs.c[i];
+            const float4 sn = cs.sn[i];
+            const float t = cs.t[i];
+            b.frag[(size_t)f * NMAX + p] = Fragment{(c.pix_row & 0xFFFFu) | (s & 0x80000000u), c.tri, c.al, c.be};
+            b.shc[(size_t)f * NMAX + p] = sn;
+            b.sht[(size_t)f * NMAX + p] = t;
+        }
     }
 }
 

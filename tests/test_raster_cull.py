@@ -6,24 +6,24 @@ import numpy as np
 import pytest
 
 F32 = np.float32
-MARGIN, SLIVER = F32(1.0 / 64.0), F32(3e-5)
+GAP, SHAPE = F32(1.0 / 4096.0), F32(2.025e-9)
 
 
 def culled(bx, by, cx, cy, ax, ay):
     """The device rule, restated."""
-    xmax, xmin = np.maximum(np.maximum(bx, cx), ax), np.minimum(np.minimum(bx, cx), ax)
-    ymax, ymin = np.maximum(np.maximum(by, cy), ay), np.minimum(np.minimum(by, cy), ay)
-    xhi, yhi, xlo, ylo = np.ceil(xmax), np.ceil(ymax), np.floor(xmin), np.floor(ymin)
-    dom = (xlo >= 0) & (ylo >= 0) & (xhi <= 65535) & (yhi <= 65535) & (xhi - xlo <= 2) & (yhi - ylo <= 2)
-    x1, y1 = xlo + F32(1), ylo + F32(1)
-    xout = (xmin - xlo > MARGIN) & ((x1 >= xhi) | (x1 - xmax > MARGIN))
-    yout = (ymin - ylo > MARGIN) & ((y1 >= yhi) | (y1 - ymax > MARGIN))
+    xmax, xmin = np.fmax(np.fmax(bx, cx), ax), np.fmin(np.fmin(bx, cx), ax)
+    ymax, ymin = np.fmax(np.fmax(by, cy), ay), np.fmin(np.fmin(by, cy), ay)
+    xlo, ylo = np.floor(xmin), np.floor(ymin)
+    dom = (np.fmin(xmin, ymin) >= 0) & (np.fmax(xmax, ymax) <= 65535) & (np.fmax(xmax - xmin, ymax - ymin) <= 2)
+    gx = np.where(xmax <= xlo + F32(1), xmin - xlo, F32(0))
+    gy = np.where(ymax <= ylo + F32(1), ymin - ylo, F32(0))
+    g = np.fmax(gx, gy)
     v0x, v1x, v0y, v1y = bx - ax, cx - ax, by - ay, cy - ay
     d00, d01, d11 = v0x * v0x + v0y * v0y, v0x * v1x + v0y * v1y, v1x * v1x + v1y * v1y
     q = d00 * d11
     den = q - d01 * d01
-    wide = (den * den) * (den * np.minimum(d00, d11)) > SLIVER * ((q * q) * q)
-    return dom & (xout | yout) & wide
+    shape = (den * den) * (den * np.minimum(d00, d11)) * (g * g) > SHAPE * ((q * q) * q)
+    return dom & (g > GAP) & shape
 
 
 def accepted(bx, by, cx, cy, ax, ay):
@@ -34,8 +34,8 @@ def accepted(bx, by, cx, cy, ax, ay):
     d00, d01, d11 = v0x * v0x + v0y * v0y, v0x * v1x + v0y * v1y, v1x * v1x + v1y * v1y
     den = d00 * d11 - d01 * d01
     hit = np.zeros(bx.shape, bool)
-    for i in range(2):
-        for j in range(2):
+    for i in range(4):
+        for j in range(4):
             x, y = xlo + F32(i), ylo + F32(j)
             d20, d21 = v0x * (x - ax) + v0y * (y - ay), v1x * (x - ax) + v1y * (y - ay)
             al, be = (d11 * d20 - d01 * d21) / den, (d00 * d21 - d01 * d20) / den
