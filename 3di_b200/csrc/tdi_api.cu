@@ -282,7 +282,8 @@ tdi_status set_attrs()
                                   (int)neigh_smem()));
     TDI_CUDA(cudaFuncSetAttribute(k_vertex_t<VT_FPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     TDI_CUDA(cudaFuncSetAttribute(k_vertex_t<VT_FPT_SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    TDI_CUDA(cudaFuncSetAttribute(k_barrier_full, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    TDI_CUDA(cudaFuncSetAttribute(k_barrier_full<NE_P8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    TDI_CUDA(cudaFuncSetAttribute(k_barrier_full<BAR_WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     TDI_CUDA(cudaFuncSetAttribute(k_solve_t<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     TDI_CUDA(cudaFuncSetAttribute(k_solve_t<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     TDI_CUDA(cudaFuncSetAttribute(k_normal_eq, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
@@ -350,7 +351,8 @@ struct Launch {
     int F;
     size_t smem_neigh() const { return neigh_smem(); }
     size_t smem_ne() const { return (size_t)2 * 2 * NE_SUB * NE_PD * sizeof(double); }
-    size_t smem_bar() const { return (size_t)4 * NL * NE_P8 * sizeof(float); }
+    int bar_width() const { return m.KT <= NE_P8 - 1 ? NE_P8 : BAR_WIDE; }
+    size_t smem_bar() const { return (size_t)4 * NL * bar_width() * sizeof(float); }
     size_t smem_solve() const { return solve_smem(m.KT); }
     dim3 fblocks() const { return dim3((F + 127) / 128); }
     int A() const { return b.nact; }                      // frames active this round
@@ -484,7 +486,7 @@ tdi_status normal_equations(const Launch &L, const Cfg &c, int stage)
         TDI_TRY(launch(L.bt, KID_NORMAL_EQ, k_normal_eq, dim3(NE_BPF, L.A()), dim3(NE_THREADS), L.smem_ne(), L.s, L.m, L.b));
         TDI_TRY(launch(L.bt, 0, k_normal_eq_reduce, dim3(4, L.A()), dim3(NE_THREADS), 0, L.s, L.m, L.b));
     }
-    TDI_TRY(launch(L.bt, KID_BARRIER, k_barrier_full, dim3(L.A()), dim3(256), L.smem_bar(), L.s, L.m, L.b,
+    TDI_TRY(launch(L.bt, KID_BARRIER, L.bar_width() == NE_P8 ? k_barrier_full<NE_P8> : k_barrier_full<BAR_WIDE>, dim3(L.A()), dim3(256), L.smem_bar(), L.s, L.m, L.b,
                    (int)(stage == ST_FINETUNE)));
     TDI_TRY(launch(L.bt, KID_SOLVE, sv_blocks(L.m.KT) == 6 ? k_solve_t<6> : k_solve_t<8>, dim3(L.A()), dim3(SV_THREADS),
                    L.smem_solve(), L.s, L.m, L.b, c, stage));

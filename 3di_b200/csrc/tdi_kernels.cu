@@ -2155,25 +2155,45 @@ __global__ void __launch_bounds__(NE_THREADS) k_normal_eq_reduce(DModel m, DBatc
 // Log-barrier gradient and Gauss-Newton Hessian (logbarrier_initializer.cu:1272-1843) added
 // to the image system, one block per frame.
 
-// The barrier Hessian's tensor-core updates of warp W over the 4 x 51 constraint rows (FP32
-// in shared memory, pitch NE_P8), four consecutive rows per step.
-template <int W>
-__device__ __forceinline__ void bar_hessian(double (&acc)[NE_TPW][2], const float *Fm, int KTP, int kr, int fr8)
+// The constraint rows are P columns wide: 88 for up to 87 unknowns, 128 for the wider systems of the
+// tensor-core normal equations.
+constexpr int BAR_WIDE = 128;
+template <int P>
+struct BarTiles {
+    static constexpr int T8 = P / 8, NT8 = T8 * (T8 + 1) / 2, TPW = (NT8 + 7) / 8;
+    int bi[NT8], bj[NT8];
+};
+template <int P>
+__host__ __device__ constexpr BarTiles<P> make_bar_tiles()
 {
-    constexpr NeTiles TT = make_ne_tiles();
-    constexpr int NT = (NE_NT8 - W + 7) / 8;
+    BarTiles<P> t{};
+    int k = 0;
+    for (int i = 0; i < BarTiles<P>::T8; ++i)
+        for (int j = i; j < BarTiles<P>::T8; ++j) { t.bi[k] = i; t.bj[k] = j; ++k; }
+    return t;
+}
+
+// The barrier Hessian's tensor-core updates of warp W over the 4 x 51 constraint rows (FP32
+// in shared memory, pitch P), four consecutive rows per step.
+template <int P, int W>
+__device__ __forceinline__ void bar_hessian(double (&acc)[BarTiles<P>::TPW][2], const float *Fm, int kr, int fr8)
+{
+    constexpr BarTiles<P> TT = make_bar_tiles<P>();
+    constexpr int NT = (BarTiles<P>::NT8 - W + 7) / 8;
     for (int t = 0; t < 4 * NL; t += 4) {
-        const float *rk = Fm + (size_t)(t + kr) * KTP + fr8;
-        double v[NE_T8];
+        const float *rk = Fm + (size_t)(t + kr) * P + fr8;
+        double v[BarTiles<P>::T8];
 #pragma unroll
-        for (int c = 0; c < NE_T8; ++c) v[c] = (double)rk[8 * c];
+        for (int c = 0; c < BarTiles<P>::T8; ++c) v[c] = (double)rk[8 * c];
 #pragma unroll
         for (int j = 0; j < NT; ++j) dmma_884(acc[j][0], acc[j][1], v[TT.bi[W + 8 * j]], v[TT.bj[W + 8 * j]]);
     }
 }
 
+template <int P>
 __global__ void __launch_bounds__(256) k_barrier_full(DModel m, DBatch b, int ft_bounds)
 {
+    constexpr int NE_P8 = P, NE_NT8 = BarTiles<P>::NT8, NE_TPW = BarTiles<P>::TPW, NE_T8 = BarTiles<P>::T8;
     if ((int)blockIdx.x >= jac_n(b)) return;
     const int f = b.jlist[blockIdx.x];
     if (threadIdx.x == 0) prof_count(b, KID_BARRIER);
@@ -2308,21 +2328,22 @@ __global__ void __launch_bounds__(256) k_barrier_full(DModel m, DBatch b, int ft
 #pragma unroll
         for (int j = 0; j < NE_TPW; ++j) acc[j][0] = acc[j][1] = 0.0;
         switch (warp) {
-        case 0: bar_hessian<0>(acc, Fm, NE_P8, kr, fr8); break;
-        case 1: bar_hessian<1>(acc, Fm, NE_P8, kr, fr8); break;
-        case 2: bar_hessian<2>(acc, Fm, NE_P8, kr, fr8); break;
-        case 3: bar_hessian<3>(acc, Fm, NE_P8, kr, fr8); break;
-        case 4: bar_hessian<4>(acc, Fm, NE_P8, kr, fr8); break;
-        case 5: bar_hessian<5>(acc, Fm, NE_P8, kr, fr8); break;
-        case 6: bar_hessian<6>(acc, Fm, NE_P8, kr, fr8); break;
-        default: bar_hessian<7>(acc, Fm, NE_P8, kr, fr8); break;
+        case 0: bar_hessian<P, 0>(acc, Fm, kr, fr8); break;
+        case 1: bar_hessian<P, 1>(acc, Fm, kr, fr8); break;
+        case 2: bar_hessian<P, 2>(acc, Fm, kr, fr8); break;
+        case 3: bar_hessian<P, 3>(acc, Fm, kr, fr8); break;
+        case 4: bar_hessian<P, 4>(acc, Fm, kr, fr8); break;
+        case 5: bar_hessian<P, 5>(acc, Fm, kr, fr8); break;
+        case 6: bar_hessian<P, 6>(acc, Fm, kr, fr8); break;
+        default: bar_hessian<P, 7>(acc, Fm, kr, fr8); break;
         }
 #pragma unroll
         for (int j = 0; j < NE_TPW; ++j) {
             const int t = warp + 8 * j;
             if (t >= NE_NT8) continue;
-            int bi, bj;
-            ne_tile8(t, bi, bj);
+            int bi = 0, bj = t;                  // tile t: row by row of the upper triangle
+            while (bj >= NE_T8 - bi) { bj -= NE_T8 - bi; ++bi; }
+            bj += bi;
             const int a = 8 * bi + fr8;
 #pragma unroll
             for (int i = 0; i < 2; ++i) {
