@@ -143,7 +143,8 @@ struct tdi_model {
 // SMs that the other lane's per-frame kernels leave idle.
 struct tdi_lane {
     cudaStream_t s = nullptr;
-    cudaEvent_t ev = nullptr;
+    cudaStream_t side = nullptr;   // the barrier terms of a replayed round, beside the image's
+    cudaEvent_t ev = nullptr, fork = nullptr, join = nullptr;
     int *d_count = nullptr;        // [2]: active frames, error word
     int *h_count = nullptr;        // pinned copy
     DBatch d{};                    // view of the lane's frames
@@ -379,6 +380,8 @@ DBatch batch_view(const tdi_batch *bt, int f0, int nf)
     v.dlam = a.dlam + F0 * 4; v.glam = a.glam + F0 * 4;
     v.d = a.d + F0 * KTP; v.g = a.g + F0 * KTP;
     v.H = a.H + F0 * KTP * KTP;
+    v.Hb = a.Hb + F0 * KTP * KTP;
+    v.gb = a.gb + F0 * KTP;
     v.R = a.R + F0 * 9; v.dR = a.dR + F0 * 27;
     v.ctl = a.ctl + F0;
     v.act = a.act + F0;
@@ -468,8 +471,18 @@ tdi_status render(const Launch &L, const Cfg &c, int stage)
                   RENDER_SMEM_FLOATS * sizeof(float), L.s, L.m, L.b, c, stage);
 }
 
-tdi_status normal_equations(const Launch &L, const Cfg &c, int stage)
+// Normal equations and solve of the accepted points. The barrier terms run on their own stream
+// beside the image terms when one is given (side, with fork and join events), else before them.
+tdi_status normal_equations(const Launch &L, const Cfg &c, int stage, const tdi_lane *side)
 {
+    const cudaStream_t bs = side ? side->side : L.s;
+    if (side) {
+        TDI_CUDA(cudaEventRecord(side->fork, L.s));
+        TDI_CUDA(cudaStreamWaitEvent(bs, side->fork, 0));
+    }
+    TDI_TRY(launch(L.bt, KID_BARRIER, L.bar_width() == NE_P8 ? k_barrier_full<NE_P8> : k_barrier_full<BAR_WIDE>, dim3(L.A()), dim3(256), L.smem_bar(), bs, L.m, L.b,
+                   (int)(stage == ST_FINETUNE)));
+    if (side) TDI_CUDA(cudaEventRecord(side->join, bs));
     TDI_TRY(launch(L.bt, KID_NEIGHBOURS, k_neighbours, dim3(L.A()), dim3(1024), L.smem_neigh(), L.s, L.b, 0));
     TDI_TRY(launch(L.bt, KID_JACOBIAN, k_jacobian, dim3(JAC_BPF, L.A()), dim3(JAC_THREADS), 0, L.s, L.m, L.b));
     if (c.normal_eq == 1) {
@@ -481,25 +494,27 @@ tdi_status normal_equations(const Launch &L, const Cfg &c, int stage)
         else
             TDI_TRY(launch(L.bt, KID_NORMAL_EQ, k_normal_eq_tc<TC_MAXN / 8>, dim3(TC_BPF, L.A()), dim3(TC_THREADS),
                            (size_t)TC_SMEM, L.s, L.m, L.b));
-        TDI_TRY(launch(L.bt, 0, k_normal_eq_tc_reduce, dim3(TC_RBLOCKS, L.A()), dim3(256), 0, L.s, L.m, L.b));
     } else {
         TDI_TRY(launch(L.bt, KID_NORMAL_EQ, k_normal_eq, dim3(NE_BPF, L.A()), dim3(NE_THREADS), L.smem_ne(), L.s, L.m, L.b));
-        TDI_TRY(launch(L.bt, 0, k_normal_eq_reduce, dim3(4, L.A()), dim3(NE_THREADS), 0, L.s, L.m, L.b));
     }
-    TDI_TRY(launch(L.bt, KID_BARRIER, L.bar_width() == NE_P8 ? k_barrier_full<NE_P8> : k_barrier_full<BAR_WIDE>, dim3(L.A()), dim3(256), L.smem_bar(), L.s, L.m, L.b,
-                   (int)(stage == ST_FINETUNE)));
+    if (side) TDI_CUDA(cudaStreamWaitEvent(L.s, side->join, 0));
+    if (c.normal_eq == 1)
+        TDI_TRY(launch(L.bt, 0, k_normal_eq_tc_reduce, dim3(TC_RBLOCKS, L.A()), dim3(256), 0, L.s, L.m, L.b));
+    else
+        TDI_TRY(launch(L.bt, 0, k_normal_eq_reduce, dim3(4, L.A()), dim3(NE_THREADS), 0, L.s, L.m, L.b));
     TDI_TRY(launch(L.bt, KID_SOLVE, sv_blocks(L.m.KT) == 6 ? k_solve_t<6> : k_solve_t<8>, dim3(L.A()), dim3(SV_THREADS),
                    L.smem_solve(), L.s, L.m, L.b, c, stage));
     return TDI_OK;
 }
 
 // One round of a shape stage for the frames of b (launched on s).
-tdi_status stage_round(tdi_batch *bt, const Cfg &c, int stage, const DBatch &b, cudaStream_t s)
+tdi_status stage_round(tdi_batch *bt, const Cfg &c, int stage, const DBatch &b, cudaStream_t s,
+                       const tdi_lane *side = nullptr)
 {
     Launch L{bt, bt->m->d, b, s, b.F};
     TDI_TRY(geometry(L, c, stage));
     TDI_TRY(render(L, c, stage));
-    return normal_equations(L, c, stage);
+    return normal_equations(L, c, stage, side);
 }
 
 // The whole light fit of a lane's running frames: their raster and neighbour maps, then every
@@ -545,7 +560,7 @@ tdi_status stage_graph(tdi_batch *bt, const Cfg &c, int stage, int lane, int tie
     const int64_t before = bt->launches;
     TDI_CUDA(cudaStreamBeginCapture(ln.s, cudaStreamCaptureModeThreadLocal));
     tdi_status st = TDI_OK;
-    for (int r = 0; r < GRAPH_ROUNDS && st == TDI_OK; ++r) st = stage_round(bt, c, stage, gv, ln.s);
+    for (int r = 0; r < GRAPH_ROUNDS && st == TDI_OK; ++r) st = stage_round(bt, c, stage, gv, ln.s, &ln);
     if (st == TDI_OK) st = launch(bt, 0, k_compact_active, dim3(1), dim3(1024), 0, ln.s, (const DBatch)gv, ln.d_count);
     cudaGraph_t graph = nullptr;
     const cudaError_t ec = cudaStreamEndCapture(ln.s, &graph);
@@ -808,7 +823,7 @@ tdi_status tdi_batch_create(tdi_model *m, int32_t max_frames, tdi_batch **out)
     A(bounds, F * 4 * NL); A(fs, F); A(cam, F * 4); A(x0y0, F * 2); A(Lint, F);
     A(d.x, F * KTP); A(d.x_ls, F * KTP); A(d.xe, F * KTP);
     A(d.lam, F * 4); A(d.lam_ls, F * 4); A(d.lame, F * 4); A(d.dlam, F * 4); A(d.glam, F * 4);
-    A(d.d, F * KTP); A(d.g, F * KTP); A(d.H, F * KTP * KTP); A(d.R, F * 9); A(d.dR, F * 27);
+    A(d.d, F * KTP); A(d.g, F * KTP); A(d.H, F * KTP * KTP); A(d.Hb, F * KTP * KTP); A(d.gb, F * KTP); A(d.R, F * 9); A(d.dR, F * 27);
     A(d.ctl, F); A(d.act, F); A(d.rlist, F); A(d.jlist, F); A(d.rcount, 2 * F); A(d.geo, F * (size_t)md.V); A(d.proj, F * (size_t)md.V); A(d.zbuf, F * NPIX); A(d.ccount, F); if (!resolve_smem(md.T)) A(d.tri_work, F * (size_t)resolve_words(md.T)); A(d.frag, F * NMAX);
     A(d.fgrad, F * 5 * NMAX); A(d.nb, F * 4 * NMAX); A(d.shc, F * NMAX); A(d.sht, F * NMAX);
     A(d.J, F * NMAX * KTP); b->ne_frame_doubles = NE_MAXCH * std::max((size_t)ne_part_stride((int)KTP), (tc_part_bytes(md.KT) + 7) / 8);
@@ -834,7 +849,10 @@ tdi_status tdi_batch_create(tdi_model *m, int32_t max_frames, tdi_batch **out)
     b->lanes.resize(max_frames >= 2 ? FIT_LANES : 1);
     for (auto &ln : b->lanes) {
         if (cudaStreamCreateWithFlags(&ln.s, cudaStreamNonBlocking) != cudaSuccess ||
+            cudaStreamCreateWithFlags(&ln.side, cudaStreamNonBlocking) != cudaSuccess ||
             cudaEventCreateWithFlags(&ln.ev, cudaEventDisableTiming) != cudaSuccess ||
+            cudaEventCreateWithFlags(&ln.fork, cudaEventDisableTiming) != cudaSuccess ||
+            cudaEventCreateWithFlags(&ln.join, cudaEventDisableTiming) != cudaSuccess ||
             cudaMallocHost(&ln.h_count, 2 * sizeof(int)) != cudaSuccess ||
             dalloc(b->allocs, &ln.d_count, 2) != TDI_OK) {
             tdi_batch_destroy(b);
@@ -852,7 +870,9 @@ tdi_status tdi_batch_destroy(tdi_batch *b)
     for (auto &e : b->prof_events) { cudaEventDestroy(e.first); cudaEventDestroy(e.second); }
     for (auto &ln : b->lanes) {
         if (ln.s) cudaStreamDestroy(ln.s);
-        if (ln.ev) cudaEventDestroy(ln.ev);
+        if (ln.side) cudaStreamDestroy(ln.side);
+        for (cudaEvent_t e : {ln.ev, ln.fork, ln.join})
+            if (e) cudaEventDestroy(e);
         if (ln.h_count) cudaFreeHost(ln.h_count);
     }
     for (void *p : b->allocs) cudaFree(p);
@@ -1092,7 +1112,7 @@ tdi_status tdi_batch_evaluate(tdi_batch *b, const tdi_fit_config *cfg, int32_t f
     if (n == 0) return TDI_OK;
     TDI_TRY(geometry(L, c, stage));
     TDI_TRY(render(L, c, stage));
-    TDI_TRY(normal_equations(L, c, stage));
+    TDI_TRY(normal_equations(L, c, stage, nullptr));
     TDI_TRY(launch(b, 0, k_scalars, L.fblocks(), dim3(128), 0, s, d, b->scalars));
     TDI_CUDA(cudaStreamSynchronize(s));
     return TDI_OK;

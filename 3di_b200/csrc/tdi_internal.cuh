@@ -118,6 +118,7 @@ struct DBatch {
     float *lam, *lam_ls, *lame, *dlam, *glam;   // [F][4]
     float *d, *g;            // [F][KTP]
     float *H;                // [F][KTP][KTP]
+    float *Hb, *gb;          // [F][KTP][KTP] (upper triangle), [F][KTP]: the barrier's part of H and g
     float *R, *dR;           // [F][9], [F][27] of the evaluation point
     FrameCtl *ctl;           // [F]
     int32_t *act;            // [F] frames running the stage at the start of the round, ascending

@@ -284,11 +284,11 @@ __global__ void __launch_bounds__(256) k_normal_eq_tc_reduce(DModel m, DBatch b)
         }
         for (; q < nch; ++q) s += (double)p[(size_t)q * pstride];
         if (c < KT) {
-            const float v = (float)(tau * s);
+            const float v = (float)(tau * s) + b.Hb[(size_t)f * KTP * KTP + (size_t)a * KTP + c];
             H[(size_t)a * KTP + c] = v;
             H[(size_t)c * KTP + a] = v;
         } else if (a < KT) {
-            b.g[(size_t)f * KTP + a] = (float)(-tau * s);
+            b.g[(size_t)f * KTP + a] = (float)(-tau * s) + b.gb[(size_t)f * KTP + a];
         }
     }
 }
