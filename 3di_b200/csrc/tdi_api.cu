@@ -1237,11 +1237,13 @@ tdi_status tdi_batch_landmark_init(tdi_batch *b, const float *p0L, int32_t *succ
     int32_t *dit = b->lm_ibuf, *drun = dit + cap, *dsucc = drun + cap, *dnewton = dsucc + cap;
     static bool attr = false;
     if (!attr) {
-        TDI_CUDA(cudaFuncSetAttribute(k_landmark_init, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+        TDI_CUDA(cudaFuncSetAttribute(k_landmark_init<6, 88>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
+        TDI_CUDA(cudaFuncSetAttribute(k_landmark_init<8, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
         attr = true;
     }
-    const size_t smem = lm_smem(m.K);
-    if (smem > 220 * 1024) return fail(TDI_ERR_INVALID, "too many expression components for the landmark fit");
+    if (!lm_accepts(m.K)) return fail(TDI_ERR_INVALID, "too many expression components for the landmark fit");
+    const bool narrow = lm_narrow(m.K);
+    const size_t smem = narrow ? lm_smem<6, 88>(m.K) : lm_smem<8, 128>(m.K);
     TDI_CUDA(cudaMemcpyAsync(dp, p0L, sizeof(float) * 3 * NL, cudaMemcpyHostToDevice, s));
     const unsigned ob = (unsigned)((F + OR_WARPS - 1) / OR_WARPS);
     TDI_TRY(launch(b, 0, k_orthographic, dim3(ob), dim3(OR_WARPS * 32), 0, s, (const float *)b->d.xl,
@@ -1250,7 +1252,7 @@ tdi_status tdi_batch_landmark_init(tdi_batch *b, const float *p0L, int32_t *succ
     TDI_TRY(launch(b, 0, k_lm_flip, dim3((F + 127) / 128), dim3(128), 0, s, F, xo, (const float *)Ro, drun));
     TDI_TRY(launch(b, 0, k_orthographic, dim3(ob), dim3(OR_WARPS * 32), 0, s, (const float *)b->d.xl,
                    (const float *)b->d.yl, (const float *)dp, F, xo, Ro, dit, (const float *)xo, (const int32_t *)drun));
-    TDI_TRY(launch(b, 0, k_landmark_init, dim3(F), dim3(LM_THREADS), smem, s, m, b->d, (const float *)xo, dsucc,
+    TDI_TRY(launch(b, 0, narrow ? k_landmark_init<6, 88> : k_landmark_init<8, 128>, dim3(F), dim3(LM_THREADS), smem, s, m, b->d, (const float *)xo, dsucc,
                    dslack, dnewton));
     if (success) TDI_CUDA(cudaMemcpyAsync(success, dsucc, sizeof(int32_t) * F, cudaMemcpyDeviceToHost, s));
     if (slack) TDI_CUDA(cudaMemcpyAsync(slack, dslack, sizeof(float) * F, cudaMemcpyDeviceToHost, s));

@@ -17,11 +17,18 @@
 // oracle (o_landmark_init_f): FP32 elementwise in the reference's operand order, sums over
 // landmarks and constraint rows in FP64 in a fixed order (rows G_x-, G_y-, G_x+, G_y+,
 // landmarks ascending), the Hessian as an FP64 fused multiply-add chain over those rows, the
-// Cholesky factor left-looking with dot products in increasing k.
+// Cholesky factor left-looking with dot products in increasing k (objective sums in a tree: FP64,
+// rounded to FP32 at the end).
+//
+// A Newton step is a chain of small parallel pieces, so what bounds it is latency. The Hessian's
+// chains run on the FP64 tensor cores (four rows per mma.sync, the barrier kernel's form), the
+// system through chol_solve, every logarithm in its own thread, basis rows loaded ahead of their
+// chains. One frame of two steps: 1,120 us with a thread per Hessian entry, left-looking columns and
+// the logarithms of an objective in one thread; 253 us in this form (500 frames 9.17 -> 1.54 ms).
 
 namespace tdi {
 
-constexpr int LM_THREADS = 256;
+constexpr int LM_THREADS = CH_THREADS;
 constexpr int LM_ROWS = 4 * NL;
 
 // Euler angles in degrees of a rotation (rotation_header.cu:421-449, RAD2DEG).
@@ -103,41 +110,82 @@ __global__ void k_lm_flip(int F, float *xo, const float *Ro, int32_t *run)
 }
 
 struct LmShared {
-    float G[LM_ROWS], invG[LM_ROWS], nlog[LM_ROWS];
+    float G[LM_ROWS], invG[LM_ROWS];
     float p[NL * 3], Rp[NL * 3];
     float R[9], dR[27];
-    float obj, ot, tau, t;
-    int flag;            // solve failure
+    float obj, tau, t;
+    int accept;
 };
 
 constexpr size_t LM_HDR = (sizeof(LmShared) + 15) / 16 * 16;   // keeps the FP64 factor 16-byte aligned
 constexpr int LM_MAXN = 136;                                      // unknowns (K + 7) at most
 
-__host__ __device__ __forceinline__ size_t lm_smem(int K)
+// Expression counts the initializer takes: what one block's shared memory held in its first layout
+// (z, zt, d, g; H; the constraint rows or the factor; projection derivatives).
+__host__ __device__ __forceinline__ bool lm_accepts(int K)
 {
     const int n = K + 7;
-    // z, zt, d, g [n]; H [n][n]; F [LM_ROWS][n] (reused as the FP64 factor [n][n]); nW [2][NL][n-1]
     const size_t fl = (size_t)4 * n + (size_t)n * n + (size_t)2 * NL * (n - 1);
-    const size_t fbytes = (size_t)LM_ROWS * n * sizeof(float);
-    const size_t lbytes = (size_t)n * n * sizeof(double);
-    return LM_HDR + ((fbytes > lbytes ? fbytes : lbytes) + 15) / 16 * 16 + fl * sizeof(float);
+    const size_t fbytes = (size_t)LM_ROWS * n * sizeof(float), lbytes = (size_t)n * n * sizeof(double);
+    const size_t hdr = (size_t)(3 * LM_ROWS + 6 * NL + 36 + 5) * sizeof(float);
+    return n <= LM_MAXN && (hdr + 15) / 16 * 16 + ((fbytes > lbytes ? fbytes : lbytes) + 15) / 16 * 16 +
+                                   fl * sizeof(float) <= 220 * 1024;
 }
 
-// Constraint terms at z (compute_nonrigid_shape + compute_Gs, :456-520, 2124-2140) and, with
-// deriv, the derivative rows (fill_optimization_dc_landmark, :587-697,
+// Register blocks and row width: 6 and 88 columns for up to 89 unknowns (the reference's 79
+// expressions have 86), else 8 and 128 (lm_accepts ends at 119).
+__host__ __device__ __forceinline__ bool lm_narrow(int K) { return K + 6 <= 88 && K + 7 < 96; }
+
+// Shared memory: the header; the constraint rows [LM_ROWS][P], later the solve; the projection
+// derivatives [2][NL][n - 1], later H [n][n]; z, zt, d, g [n]; the bound terms [2 K].
+template <int RB, int P>
+__host__ __device__ __forceinline__ size_t lm_rows_bytes(int K)
+{
+    const size_t f = (size_t)LM_ROWS * P * sizeof(float), c = chol_smem(K + 7, RB);
+    return ((f > c ? f : c) + 15) / 16 * 16;
+}
+__host__ __device__ __forceinline__ size_t lm_h_floats(int K)
+{
+    const size_t n = (size_t)K + 7, w = 2 * (size_t)NL * (n - 1);
+    return w > n * n ? w : n * n;
+}
+template <int RB, int P>
+__host__ __device__ __forceinline__ size_t lm_smem(int K)
+{
+    return LM_HDR + lm_rows_bytes<RB, P>(K) + (lm_h_floats(K) + 4 * (size_t)(K + 7) + 2 * (size_t)K) * sizeof(float);
+}
+
+// Constraint terms at z (compute_nonrigid_shape + compute_Gs, :456-520, 2124-2140), the objective
+// tau s + bound and constraint barrier terms (FP64, rounded; in s.obj after the last barrier, thread
+// 0 writes it) and, with deriv, the derivative rows (fill_optimization_dc_landmark, :587-697,
 // fill_optimization_dI_depsilon_landmark, :836-912).
+template <int P>
 __device__ void lm_terms(const DModel &m, const float *xl, const float *yl, const float *bd, float fs,
-                         const float *cam, const float *z, bool deriv, LmShared &s, float *F, float *nWx,
-                         float *nWy)
+                         const float *cam, const float *z, bool deriv, bool objective, LmShared &s, float *F,
+                         float *nWx, float *nWy, float *bnd, float *obj_out)
 {
     const int K = m.K, KP = m.KP, V = m.V, n = K + 7, nb = n - 1, tid = threadIdx.x;
-    if (tid == 0) rotation(z + K + 3, s.R, s.dR);
-    __syncthreads();
-    if (tid < NL * 3) {
+    const float *lb = m.eps_b, *ub = m.eps_b + K;
+    // the rotation in one warp, a landmark coordinate's chain per thread in the others
+    if (tid >= CH_WORKERS) {
+        if (tid == CH_WORKERS) rotation(z + K + 3, s.R, s.dR);
+    } else if (tid < NL * 3) {
         const int i = tid / 3, c = tid - 3 * i, v = m.lis[i];
-        const float *e = m.E + ((size_t)v * 3 + c) * KP;
+        const float4 *e4 = reinterpret_cast<const float4 *>(m.E + ((size_t)v * 3 + c) * KP);
         float acc = 0.0f;
-        for (int k = 0; k < K; ++k) acc = fmaf(e[k], z[k], acc);
+        for (int k0 = 0; k0 < K; k0 += 4 * PT_E4) {
+            float4 e[PT_E4];
+#pragma unroll
+            for (int u = 0; u < PT_E4; ++u) e[u] = k0 + 4 * u < K ? __ldg(e4 + (k0 >> 2) + u) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+#pragma unroll
+            for (int u = 0; u < PT_E4; ++u) {
+                const int k = k0 + 4 * u;
+                if (k < K) acc = fmaf(e[u].x, z[k], acc);
+                if (k + 1 < K) acc = fmaf(e[u].y, z[k + 1], acc);
+                if (k + 2 < K) acc = fmaf(e[u].z, z[k + 2], acc);
+                if (k + 3 < K) acc = fmaf(e[u].w, z[k + 3], acc);
+            }
+        }
         s.p[tid] = m.mean[(size_t)c * V + v] + acc;
     }
     __syncthreads();
@@ -154,18 +202,45 @@ __device__ void lm_terms(const DModel &m, const float *xl, const float *yl, cons
         s.G[1 * NL + i] = sl - ((yl[i] + bd[1 * NL + i] * fs) - yproj);
         s.G[2 * NL + i] = sl - ((xproj - bd[2 * NL + i] * fs) - xl[i]);
         s.G[3 * NL + i] = sl - ((yproj - bd[3 * NL + i] * fs) - yl[i]);
-        for (int q = 0; q < 4; ++q) {
-            const float G = s.G[q * NL + i];
-            s.invG[q * NL + i] = 1.0f / (0.000001f + G);
-            s.nlog[q * NL + i] = -(float)log((double)G);
-        }
     }
     __syncthreads();
+    if (!objective) return;
+    // every logarithm in its own thread: constraint rows into invG's place until the sums are formed
+    float *nlog = s.invG;
+    for (int q = tid; q < LM_ROWS + 2 * K; q += LM_THREADS) {
+        const int k = q - LM_ROWS;
+        const float arg = k < 0 ? s.G[q] : k < K ? -(lb[k] - z[k]) : -(z[k - K] - ub[k - K]);
+        const float t = -(float)log((double)arg);
+        if (k < 0) nlog[q] = t; else bnd[k] = t;
+    }
+    __syncthreads();
+    if (tid < 32) {
+        double sum[3] = {0.0, 0.0, 0.0};
+        for (int k = tid; k < K; k += 32) { sum[0] += (double)bnd[k]; sum[1] += (double)bnd[K + k]; }
+        for (int r = tid; r < LM_ROWS; r += 32) sum[2] += (double)nlog[r];
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) sum[q] += __shfl_xor_sync(0xffffffffu, sum[q], o);
+        if (tid == 0) {
+            double acc = (double)(s.tau * z[K + 6]);
+            acc += sum[0];
+            acc += sum[1];
+            acc += sum[2];
+            *obj_out = (float)acc;
+        }
+    }
     if (!deriv) return;
+    __syncthreads();
+    for (int r = tid; r < LM_ROWS; r += LM_THREADS) s.invG[r] = 1.0f / (0.000001f + s.G[r]);
     const float phix = cam[0], phiy = cam[1];
-    // projection derivatives: expression columns, then the six pose columns
-    for (int w = tid; w < NL * (K + 6); w += LM_THREADS) {
-        const int i = w / (K + 6), a = w - i * (K + 6);
+    // projection derivatives: expression columns, then the six pose columns; zeros up to P
+    for (int w = tid; w < NL * P; w += LM_THREADS) {
+        const int i = w / P, a = w - i * P;
+        if (a >= nb) {
+            for (int q = 0; q < 4; ++q) F[(size_t)(q * NL + i) * P + a] = 0.0f;
+            continue;
+        }
         const float vx = s.Rp[3 * i] + z[K], vy = s.Rp[3 * i + 1] + z[K + 1], vz = s.Rp[3 * i + 2] + z[K + 2];
         const float ivz = 1.0f / vz, ivz2 = ivz * ivz;
         float wx, wy;
@@ -194,45 +269,27 @@ __device__ void lm_terms(const DModel &m, const float *xl, const float *yl, cons
         }
         nWx[(size_t)i * nb + a] = wx;
         nWy[(size_t)i * nb + a] = wy;
-        F[(size_t)(0 * NL + i) * n + a] = (-wx) / s.G[0 * NL + i];
-        F[(size_t)(1 * NL + i) * n + a] = (-wy) / s.G[1 * NL + i];
-        F[(size_t)(2 * NL + i) * n + a] = wx / s.G[2 * NL + i];
-        F[(size_t)(3 * NL + i) * n + a] = wy / s.G[3 * NL + i];
+        F[(size_t)(0 * NL + i) * P + a] = (-wx) / s.G[0 * NL + i];
+        F[(size_t)(1 * NL + i) * P + a] = (-wy) / s.G[1 * NL + i];
+        F[(size_t)(2 * NL + i) * P + a] = wx / s.G[2 * NL + i];
+        F[(size_t)(3 * NL + i) * P + a] = wy / s.G[3 * NL + i];
     }
-    for (int r = tid; r < LM_ROWS; r += LM_THREADS) F[(size_t)r * n + nb] = 0.0f;
     __syncthreads();
 }
 
-// tau s + expression-bound and constraint barrier terms, FP64 sums, rounded (thread 0).
-__device__ float lm_objective(const DModel &m, const float *z, float tau, const LmShared &s)
-{
-    const int K = m.K;
-    const float *lb = m.eps_b, *ub = m.eps_b + K;
-    double acc = (double)(tau * z[K + 6]);
-    double sl = 0.0, su = 0.0, sg = 0.0;
-    for (int k = 0; k < K; ++k) sl += (double)(-(float)log((double)(-(lb[k] - z[k]))));
-    for (int k = 0; k < K; ++k) su += (double)(-(float)log((double)(-(z[k] - ub[k]))));
-    for (int r = 0; r < LM_ROWS; ++r) sg += (double)s.nlog[r];
-    acc += sl;
-    acc += su;
-    acc += sg;
-    return (float)acc;
-}
-
-__global__ void __launch_bounds__(LM_THREADS) k_landmark_init(DModel m, DBatch b, const float *xo,
-                                                              int32_t *success_out, float *slack_out,
-                                                              int32_t *iters_out)
+template <int RB, int P>
+__global__ void __launch_bounds__(LM_THREADS, RB == 6 ? 2 : 1) k_landmark_init(DModel m, DBatch b, const float *xo,
+                                                                               int32_t *success_out, float *slack_out,
+                                                                               int32_t *iters_out)
 {
     extern __shared__ __align__(16) unsigned char lm_raw[];
     LmShared &s = *reinterpret_cast<LmShared *>(lm_raw);
-    const int K = m.K, n = K + 7, nb = n - 1, tid = threadIdx.x;
-    const size_t fbytes = (size_t)LM_ROWS * n * sizeof(float), lbytes = (size_t)n * n * sizeof(double);
-    unsigned char *big = lm_raw + LM_HDR;
-    float *F = reinterpret_cast<float *>(big);
-    double *Lf = reinterpret_cast<double *>(big);            // the factor, after F is used
-    float *z = reinterpret_cast<float *>(big + ((fbytes > lbytes ? fbytes : lbytes) + 15) / 16 * 16);
-    float *zt = z + n, *d = zt + n, *g = d + n, *H = g + n;
-    float *nWx = H + (size_t)n * n, *nWy = nWx + (size_t)NL * nb;
+    const int K = m.K, n = K + 7, nb = n - 1, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    float *F = reinterpret_cast<float *>(lm_raw + LM_HDR);
+    double *chol = reinterpret_cast<double *>(lm_raw + LM_HDR);      // the solve, after F is used
+    float *nWx = reinterpret_cast<float *>(lm_raw + LM_HDR + lm_rows_bytes<RB, P>(K)), *nWy = nWx + (size_t)NL * nb;
+    float *H = nWx;                                                  // after the derivatives are used
+    float *z = nWx + lm_h_floats(K), *zt = z + n, *d = zt + n, *g = d + n, *bnd = g + n;
     const int f = blockIdx.x;
     const float *xl = b.xl + (size_t)f * NL, *yl = b.yl + (size_t)f * NL;
     const float *bd = b.bounds + (size_t)f * 4 * NL, *cam = b.cam + (size_t)f * 4;
@@ -244,6 +301,7 @@ __global__ void __launch_bounds__(LM_THREADS) k_landmark_init(DModel m, DBatch b
     if (tid == 0) {
         const float *x7 = xo + (size_t)f * 7;
         float xm = 0.0f, ym = 0.0f;
+#pragma unroll 17
         for (int i = 0; i < NL; ++i) { xm += xl[i]; ym += yl[i]; }
         xm = xm / (float)NL;
         ym = ym / (float)NL;
@@ -252,15 +310,16 @@ __global__ void __launch_bounds__(LM_THREADS) k_landmark_init(DModel m, DBatch b
         z[K + 0] = (tz * (xm - cam[2])) / cam[0];
         z[K + 1] = (tz * (ym - cam[3])) / cam[1];
         z[K + 3] = x7[4]; z[K + 4] = x7[5]; z[K + 5] = x7[6];
+        s.tau = 10.0f;
     }
     __syncthreads();
     // minimal slack: s0 = 5 - min G at s = 0
-    lm_terms(m, xl, yl, bd, fs, cam, z, false, s, F, nWx, nWy);
+    lm_terms<P>(m, xl, yl, bd, fs, cam, z, false, false, s, F, nWx, nWy, bnd, nullptr);
     if (tid == 0) {
         float gmin = s.G[0];
+#pragma unroll 12
         for (int r = 1; r < LM_ROWS; ++r) gmin = s.G[r] < gmin ? s.G[r] : gmin;
         z[nb] = 5.0f - gmin;
-        s.tau = 10.0f;
     }
     __syncthreads();
     int success = 0, iters = 0;
@@ -271,108 +330,107 @@ __global__ void __launch_bounds__(LM_THREADS) k_landmark_init(DModel m, DBatch b
         bool terminate = false;
         for (int it = 0; it < 100 && !terminate; ++it) {
             if (z[nb] < -0.01f) { success = 1; break; }
-            lm_terms(m, xl, yl, bd, fs, cam, z, true, s, F, nWx, nWy);
-            if (tid == 0) s.obj = lm_objective(m, z, tau, s);
-            // gradient
-            for (int a = tid; a < nb; a += LM_THREADS) {
-                double acc = 0.0;
-                for (int i = 0; i < NL; ++i) {
-                    float e = F[(size_t)(0 * NL + i) * n + a];
-                    e = e + F[(size_t)(1 * NL + i) * n + a];
-                    e = e + F[(size_t)(2 * NL + i) * n + a];
-                    e = e + F[(size_t)(3 * NL + i) * n + a];
-                    acc += (double)e;
+            lm_terms<P>(m, xl, yl, bd, fs, cam, z, true, true, s, F, nWx, nWy, bnd, &s.obj);
+            // the constraint block of the Hessian: one FP64 fused multiply-add chain over the 204 rows per
+            // entry, four rows per tensor-core step (warps 0-7); the slack's own entries in the last warp
+            double acc[BarTiles<P>::TPW][2];
+#pragma unroll
+            for (int j = 0; j < BarTiles<P>::TPW; ++j) acc[j][0] = acc[j][1] = 0.0;
+            const int kr = lane & 3, fr8 = lane >> 2;
+            double hss = 0.0;
+            switch (warp) {
+            case 0: bar_hessian<P, 0>(acc, F, kr, fr8); break;
+            case 1: bar_hessian<P, 1>(acc, F, kr, fr8); break;
+            case 2: bar_hessian<P, 2>(acc, F, kr, fr8); break;
+            case 3: bar_hessian<P, 3>(acc, F, kr, fr8); break;
+            case 4: bar_hessian<P, 4>(acc, F, kr, fr8); break;
+            case 5: bar_hessian<P, 5>(acc, F, kr, fr8); break;
+            case 6: bar_hessian<P, 6>(acc, F, kr, fr8); break;
+            case 7: bar_hessian<P, 7>(acc, F, kr, fr8); break;
+            default:
+                if (lane == 0) {
+                    double gs = 0.0;
+#pragma unroll 12
+                    for (int r = 0; r < LM_ROWS; ++r) gs += (double)s.invG[r];
+                    g[nb] = tau + (float)(-gs);
+                } else if (lane == 1) {
+#pragma unroll 12
+                    for (int r = 0; r < LM_ROWS; ++r) hss = fma((double)s.invG[r], (double)s.invG[r], hss);
                 }
-                float ga = (float)acc;
+            }
+            // gradient: column sums over the landmarks
+            for (int a = tid; a < nb; a += LM_THREADS) {
+                double ga_d = 0.0;
+#pragma unroll 3
+                for (int i = 0; i < NL; ++i) {
+                    float e = F[(size_t)(0 * NL + i) * P + a];
+                    e = e + F[(size_t)(1 * NL + i) * P + a];
+                    e = e + F[(size_t)(2 * NL + i) * P + a];
+                    e = e + F[(size_t)(3 * NL + i) * P + a];
+                    ga_d += (double)e;
+                }
+                float ga = (float)ga_d;
                 if (a < K) {
                     const float fub = z[a] - ub[a], flb = lb[a] - z[a];
                     ga = ga + (-1.0f / fub + 1.0f / flb);
                 }
                 g[a] = ga;
             }
-            if (tid == LM_THREADS - 1) {
-                double acc = 0.0;
-                for (int r = 0; r < LM_ROWS; ++r) acc += (double)s.invG[r];
-                const float gs = (float)(-acc);
-                g[nb] = tau + gs;
+            // the slack's row: its terms in place of nWx (all threads), then the column sums
+            for (int w = tid; w < NL * nb; w += LM_THREADS) {
+                const int i = w / nb;
+                const float gxm = s.G[i], gym = s.G[NL + i], gxp = s.G[2 * NL + i], gyp = s.G[3 * NL + i];
+                const float wx = nWx[w], wy = nWy[w];
+                float e = (-wx) / (gxp * gxp) - wy / (gyp * gyp);
+                e = e + wx / (gxm * gxm);
+                e = e + wy / (gym * gym);
+                nWx[w] = e;
             }
-            // Hessian: the lower triangle of the constraint block, one entry per item
-            const int ntri = nb * (nb + 1) / 2;
-            for (int w = tid; w < ntri; w += LM_THREADS) {
-                int a = (int)((sqrt(8.0 * w + 1.0) - 1.0) * 0.5);
-                while ((a + 1) * (a + 2) / 2 <= w) ++a;
-                while (a * (a + 1) / 2 > w) --a;
-                const int bcol = w - a * (a + 1) / 2;
-                double acc = 0.0;
-                for (int r = 0; r < LM_ROWS; ++r)
-                    acc = fma((double)F[(size_t)r * n + a], (double)F[(size_t)r * n + bcol], acc);
-                float hv = (float)acc;
-                if (a == bcol && a < K) {
-                    const float fub = z[a] - ub[a], flb = lb[a] - z[a];
-                    const float nu = (float)(-1.0 / ((double)fub + 1e-12));
-                    const float nl = (float)(1.0 / ((double)flb + 1e-12));
-                    hv = hv + (nu * nu + nl * nl);
+            __syncthreads();
+            float hrow = 0.0f;                               // H(nb, tid)
+            if (tid < nb) {
+                double h = 0.0;
+#pragma unroll 3
+                for (int i = 0; i < NL; ++i) h += (double)nWx[(size_t)i * nb + tid];
+                hrow = (float)h;
+            }
+            __syncthreads();                                 // nWx is read: H takes its place
+            if (tid < nb) H[(size_t)tid * n + nb] = hrow;
+            if (tid == CH_WORKERS + 1) H[(size_t)nb * n + nb] = (float)hss;
+            if (warp < 8) {
+#pragma unroll
+                for (int j = 0; j < BarTiles<P>::TPW; ++j) {
+                    const int t = warp + 8 * j;
+                    if (t >= BarTiles<P>::NT8) continue;
+                    int bi = 0, bj = t;
+                    while (bj >= BarTiles<P>::T8 - bi) { bj -= BarTiles<P>::T8 - bi; ++bi; }
+                    bj += bi;
+                    const int a = 8 * bi + fr8;
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        const int c = 8 * bj + 2 * kr + q;
+                        if (a > c || c >= nb) continue;
+                        float hv = (float)acc[j][q];
+                        if (a == c && a < K) {
+                            const float fub = z[a] - ub[a], flb = lb[a] - z[a];
+                            const float nu = (float)(-1.0 / ((double)fub + 1e-12));
+                            const float nl = (float)(1.0 / ((double)flb + 1e-12));
+                            hv = hv + (nu * nu + nl * nl);
+                        }
+                        H[(size_t)a * n + c] = hv;           // the upper triangle
+                    }
                 }
-                H[(size_t)a * n + bcol] = hv;
-                H[(size_t)bcol * n + a] = hv;
-            }
-            for (int a = tid; a < nb; a += LM_THREADS) {
-                double acc = 0.0;
-                for (int i = 0; i < NL; ++i) {
-                    const float gxm = s.G[i], gym = s.G[NL + i], gxp = s.G[2 * NL + i], gyp = s.G[3 * NL + i];
-                    const float wx = nWx[(size_t)i * nb + a], wy = nWy[(size_t)i * nb + a];
-                    float e = (-wx) / (gxp * gxp) - wy / (gyp * gyp);
-                    e = e + wx / (gxm * gxm);
-                    e = e + wy / (gym * gym);
-                    acc += (double)e;
-                }
-                H[(size_t)nb * n + a] = (float)acc;
-                H[(size_t)a * n + nb] = (float)acc;
-            }
-            if (tid == LM_THREADS - 2) {
-                double acc = 0.0;
-                for (int r = 0; r < LM_ROWS; ++r) acc = fma((double)s.invG[r], (double)s.invG[r], acc);
-                H[(size_t)nb * n + nb] = (float)acc;
             }
             __syncthreads();
             ++iters;
-            // FP64 Cholesky (solver.h:70-105), left-looking; the factor overwrites F
-            for (int i = tid; i < n * n; i += LM_THREADS) Lf[i] = (double)H[i];
-            if (tid == 0) s.flag = 0;
-            __syncthreads();
-            for (int j = 0; j < n; ++j) {
-                if (tid == 0) {
-                    double sj = Lf[(size_t)j * n + j];
-                    for (int k = 0; k < j; ++k) sj -= Lf[(size_t)k * n + j] * Lf[(size_t)k * n + j];
-                    if (!(sj > 0.0)) s.flag = 1;
-                    else Lf[(size_t)j * n + j] = sqrt(sj);
-                }
-                __syncthreads();
-                if (s.flag) break;
-                const double ljj = Lf[(size_t)j * n + j];
-                for (int i = j + 1 + tid; i < n; i += LM_THREADS) {
-                    double t = Lf[(size_t)j * n + i];
-                    for (int k = 0; k < j; ++k) t -= Lf[(size_t)k * n + i] * Lf[(size_t)k * n + j];
-                    Lf[(size_t)j * n + i] = t / ljj;
-                }
-                __syncthreads();
-            }
-            if (s.flag) { terminate = true; break; }
-            if (tid == 0) {
-                double y[LM_MAXN];
-                for (int i = 0; i < n; ++i) {
-                    double t = (double)g[i];
-                    for (int k = 0; k < i; ++k) t -= Lf[(size_t)k * n + i] * y[k];
-                    y[i] = t / Lf[(size_t)i * n + i];
-                }
-                for (int i = n - 1; i >= 0; --i) {
-                    double t = y[i];
-                    for (int k = n - 1; k > i; --k) t -= Lf[(size_t)i * n + k] * y[k];
-                    y[i] = t / Lf[(size_t)i * n + i];
-                }
-                for (int i = 0; i < n; ++i) d[i] = (float)(-y[i]);
-                s.t = 1.0f;
-            }
+            // FP64 Cholesky (solver.h:70-105); the factor takes F's place
+            double *xs;
+            const bool ok = chol_solve<RB, true>(
+                n, chol, [&](int i, int l) { return (double)H[(size_t)l * n + i]; }, [&](int l) { return (double)g[l]; },
+                xs);
+            if (!ok) { terminate = true; break; }
+            if (tid < n) d[tid] = (float)(-xs[tid]);
+            if (tid == 0) s.t = 1.0f;
             __syncthreads();
             // line search: halve t until the objective decreases
             for (int inner = 0; inner < 100; ++inner) {
@@ -380,14 +438,14 @@ __global__ void __launch_bounds__(LM_THREADS) k_landmark_init(DModel m, DBatch b
                 if (t < 0.01f) { terminate = true; break; }
                 for (int a = tid; a < n; a += LM_THREADS) zt[a] = z[a] + t * d[a];
                 __syncthreads();
-                lm_terms(m, xl, yl, bd, fs, cam, zt, false, s, F, nWx, nWy);
+                float ot = 0.0f;
+                lm_terms<P>(m, xl, yl, bd, fs, cam, zt, false, true, s, F, nWx, nWy, bnd, &ot);
                 if (tid == 0) {
-                    s.ot = lm_objective(m, zt, tau, s);
-                    s.flag = s.ot < s.obj;
+                    s.accept = ot < s.obj;
                     s.t = t * 0.5f;
                 }
                 __syncthreads();
-                if (s.flag) {
+                if (s.accept) {
                     for (int a = tid; a < n; a += LM_THREADS) z[a] = zt[a];
                     __syncthreads();
                     break;
