@@ -10,17 +10,21 @@
 //
 // Backward pass (every buffer is recomputed from the state, nothing is kept from the forward):
 //   1. per fragment: dL/d(normalised gradients) -> dL/d(gx, gy) through the normalisation ->
-//      scattered into dL/d(blurred image) at the four neighbour pixels (FP64 atomics);
+//      scattered into dL/d(blurred image) at the four neighbour pixels;
 //   2. the transposed blur (the taps are symmetric and the border zero, so the transpose is the
 //      same separable filter, applied in the opposite order);
 //   3. per owner fragment: dL/d(pixel value) through the shading to the light (lambda, L), the
 //      translation and rotation (through R^T (lambda - tau)), the object coordinates of its three
-//      corners (normal and interpolated point) and the barycentrics, and through those to the
-//      projected corners -- scattered to per-vertex accumulators with FP64 atomics, per-frame
-//      terms summed per warp first (warp-aggregated atomics);
-//   4. per vertex: projected position -> camera coordinates -> rotation, translation and object
-//      coordinates; 5. object coordinates -> expression coefficients by the basis-transpose
-//      product dL/deps_k = sum_v E[v][:,k] . dL/dP0[v]; 6. dL/dR -> dL/du through dR/du.
+//      corners (normal and interpolated point) and the barycentrics; through those to the projected
+//      corners, the camera coordinates and again the object coordinates. Everything after the
+//      pixel is linear in it, so each fragment carries its own 3 x 3 object-coordinate terms
+//      and nothing is accumulated per vertex (only about a fifth of the vertices have a fragment);
+//   4. object coordinates -> expression coefficients by the basis-transpose product
+//      dL/deps_k = sum_n sum_c E[v(n, c)][:,k] . dL/dP0(n, c); 5. dL/dR -> dL/du through dR/du.
+// Steps 1 and 2 and the forward's image run in one kernel with a block per frame and the image
+// region in shared memory (k_adj_image). 96 frames of the 53,490-vertex model, loss and gradients:
+// 4.55 ms of kernels with dense per-vertex passes and whole-crop FP64 blurs in global memory,
+// 1.49 ms in this form.
 // Rotation in FP64: the reference's formula (rotation_header.cu:46-151) evaluated in double.
 
 namespace tdi {
@@ -33,13 +37,6 @@ __device__ __forceinline__ double wsum(double v)
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
     return v;
-}
-
-// one atomic per warp for a value every lane contributes to
-__device__ __forceinline__ void warp_atomic_add(double *dst, double v)
-{
-    v = wsum(v);
-    if ((threadIdx.x & 31) == 0) atomicAdd(dst, v);
 }
 
 __device__ void rotation_d(const float *uf, double *R, double *dR)
@@ -86,94 +83,88 @@ __global__ void k_adj_rot(DModel m, DBatch b, const float *x, int F, double *R64
     rotation_d(x + (size_t)f * m.KT + m.K + 3, R64 + (size_t)f * 36, R64 + (size_t)f * 36 + 9);
 }
 
-// FP64 vertex stage: object coordinates P0 = mean + E eps, camera X = R P0 + tau, projections.
-// geo64 [F][V][8]: P0 (3), X (3), xp, yp.
-// The same per (frame, vertex), tiled: a block takes AV_V vertices x AV_F frames, stages their
-// basis rows and coefficients in shared memory once (instead of every thread reading its
-// vertex's rows from L2 for every frame), and each thread forms one vertex of AV_F / 8 frames;
-// the fused multiply-add chains over k are the same, in the same order.
-constexpr int AV_V = 32, AV_F = 32, AV_FPT = AV_F / 8;
+// FP64 vertex stage: object coordinates P0 = mean + E eps, geo64 [F][V][3]. (Camera coordinates and
+// projections are formed by the fragments that need them: 24 bytes per vertex instead of 64.)
+// A block takes AV_V vertices x 8 FPT frames with their basis rows and coefficients in shared
+// memory as doubles, converted once; a thread forms one vertex of FPT frames by fused
+// multiply-add chains over k. Bound by shared-memory reads (6 + FPT / 2 wavefronts per 3 FPT
+// multiply-adds), so FPT is 8 for batches that fill it.
+constexpr int AV_V = 32;
 
-__host__ __device__ __forceinline__ size_t adj_vertex_smem(int KP)
+__host__ __device__ __forceinline__ size_t adj_vertex_smem(int KP, int FPT)
 {
-    return ((size_t)AV_V * 3 + AV_F) * (size_t)(KP + 1) * sizeof(float);
+    return ((size_t)AV_V * 3 * (KP + 1) + (size_t)8 * FPT * KP) * sizeof(double);
 }
 
-__global__ void __launch_bounds__(256) k_adj_vertex_tiled(DModel m, const float *x, int F, const double *R64,
-                                                          const float *cam, double *geo64)
+template <int FPT>
+__global__ void __launch_bounds__(256) k_adj_vertex_tiled(DModel m, const float *x, int F, double *geo64)
 {
-    extern __shared__ float avs[];
+    extern __shared__ __align__(16) double avs[];
+    constexpr int NF = 8 * FPT;
     const int KP = m.KP, K = m.K, KT = m.KT, W = KP + 1;    // row pitch KP + 1: lanes (vertices) on distinct banks
-    float *Es = avs;                                          // [AV_V][3][W]
-    float *Xs = Es + (size_t)AV_V * 3 * W;                   // [AV_F][W]
-    const int v0 = blockIdx.x * AV_V, f0 = blockIdx.y * AV_F, tid = threadIdx.x;
-    for (int i = tid; i < AV_V * 3 * KP; i += 256) {
-        const int r = i / KP, k = i - r * KP, v = v0 + r / 3;
-        Es[(size_t)r * W + k] = v < m.V ? m.E[(size_t)v0 * 3 * KP + i] : 0.0f;
+    double *Xs = avs;                                         // [KP][NF]
+    double *Es = Xs + (size_t)NF * KP;                        // [AV_V][3][W]
+    const int v0 = blockIdx.x * AV_V, f0 = blockIdx.y * NF, tid = threadIdx.x;
+    const int nrow = min(AV_V, m.V - v0) * 3 * KP;
+    for (int i = tid; i < nrow; i += 256) {
+        const int r = i / KP, k = i - r * KP;
+        Es[(size_t)r * W + k] = (double)m.E[(size_t)v0 * 3 * KP + i];
     }
-    for (int i = tid; i < AV_F * KP; i += 256) {
+    for (int i = tid; i < NF * KP; i += 256) {
         const int fl = i / KP, k = i - fl * KP, f = f0 + fl;
-        Xs[(size_t)fl * W + k] = (f < F && k < K) ? x[(size_t)f * KT + k] : 0.0f;
+        Xs[(size_t)k * NF + fl] = (f < F && k < K) ? (double)x[(size_t)f * KT + k] : 0.0;
     }
     __syncthreads();
     const int vl = tid & 31, fg = tid >> 5, v = v0 + vl;
-    const float *e0 = Es + (size_t)vl * 3 * W, *e1 = e0 + W, *e2 = e1 + W;
-    double acc[AV_FPT][3];
+    if (f0 + fg * FPT >= F || v >= m.V) return;
+    const double *e0 = Es + (size_t)vl * 3 * W, *e1 = e0 + W, *e2 = e1 + W, *xk = Xs + fg * FPT;
+    double acc[FPT][3];
 #pragma unroll
-    for (int q = 0; q < AV_FPT; ++q) acc[q][0] = acc[q][1] = acc[q][2] = 0.0;
-    for (int k = 0; k < K; ++k) {
+    for (int q = 0; q < FPT; ++q) acc[q][0] = acc[q][1] = acc[q][2] = 0.0;
+#pragma unroll 2
+    for (int k = 0; k < K; ++k, xk += NF) {
         const double a0 = e0[k], a1 = e1[k], a2 = e2[k];
+        double xv[FPT];
+        if constexpr (FPT == 1) {
+            xv[0] = xk[0];
+        } else {
 #pragma unroll
-        for (int q = 0; q < AV_FPT; ++q) {
-            const double xv = Xs[(size_t)(fg * AV_FPT + q) * W + k];
-            acc[q][0] = fma(a0, xv, acc[q][0]);
-            acc[q][1] = fma(a1, xv, acc[q][1]);
-            acc[q][2] = fma(a2, xv, acc[q][2]);
+            for (int q = 0; q < FPT; q += 2) {
+                const double2 t = *reinterpret_cast<const double2 *>(xk + q);
+                xv[q] = t.x; xv[q + 1] = t.y;
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < FPT; ++q) {
+            acc[q][0] = fma(a0, xv[q], acc[q][0]);
+            acc[q][1] = fma(a1, xv[q], acc[q][1]);
+            acc[q][2] = fma(a2, xv[q], acc[q][2]);
         }
     }
-    if (v >= m.V) return;
     const double mean[3] = {(double)m.mean[v], (double)m.mean[(size_t)m.V + v], (double)m.mean[2 * (size_t)m.V + v]};
 #pragma unroll
-    for (int q = 0; q < AV_FPT; ++q) {
-        const int f = f0 + fg * AV_FPT + q;
+    for (int q = 0; q < FPT; ++q) {
+        const int f = f0 + fg * FPT + q;
         if (f >= F) break;
-        const float *xf = x + (size_t)f * KT;
-        double P[3];
-        for (int c = 0; c < 3; ++c) P[c] = mean[c] + acc[q][c];
-        const double *R = R64 + (size_t)f * 36;
-        double X[3];
-        for (int i = 0; i < 3; ++i) X[i] = (R[i] * P[0] + R[3 + i] * P[1]) + R[6 + i] * P[2] + (double)xf[K + i];
-        const float *cm = cam + (size_t)f * 4;
-        double *g = geo64 + ((size_t)f * m.V + v) * 8;
-        g[0] = P[0]; g[1] = P[1]; g[2] = P[2];
-        g[3] = X[0]; g[4] = X[1]; g[5] = X[2];
-        g[6] = (double)cm[0] * X[0] / X[2] + (double)cm[2];
-        g[7] = (double)cm[1] * X[1] / X[2] + (double)cm[3];
+        double *g = geo64 + ((size_t)f * m.V + v) * 3;
+        for (int c = 0; c < 3; ++c) g[c] = mean[c] + acc[q][c];
     }
 }
 
-__global__ void k_adj_vertex(DModel m, const float *x, int F, const double *R64, const float *cam, double *geo64)
+// The same without staging, for bases too wide for shared memory.
+__global__ void k_adj_vertex(DModel m, const float *x, int F, double *geo64)
 {
     const int f = blockIdx.y;
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (f >= F || v >= m.V) return;
     const float *xf = x + (size_t)f * m.KT;
-    double P[3];
+    double *g = geo64 + ((size_t)f * m.V + v) * 3;
     for (int c = 0; c < 3; ++c) {
         const float *e = m.E + ((size_t)v * 3 + c) * m.KP;
         double acc = 0.0;
         for (int k = 0; k < m.K; ++k) acc = fma((double)e[k], (double)xf[k], acc);
-        P[c] = (double)m.mean[(size_t)c * m.V + v] + acc;
+        g[c] = (double)m.mean[(size_t)c * m.V + v] + acc;
     }
-    const double *R = R64 + (size_t)f * 36;
-    double X[3];
-    for (int i = 0; i < 3; ++i) X[i] = (R[i] * P[0] + R[3 + i] * P[1]) + R[6 + i] * P[2] + (double)xf[m.K + i];
-    const float *cm = cam + (size_t)f * 4;
-    double *g = geo64 + ((size_t)f * m.V + v) * 8;
-    g[0] = P[0]; g[1] = P[1]; g[2] = P[2];
-    g[3] = X[0]; g[4] = X[1]; g[5] = X[2];
-    g[6] = (double)cm[0] * X[0] / X[2] + (double)cm[2];
-    g[7] = (double)cm[1] * X[1] / X[2] + (double)cm[3];
 }
 
 // Barycentrics of sample s in triangle (b, c, a) by Cramer's rule: s - a = alpha (b - a) + beta (c - a)
@@ -201,10 +192,10 @@ __device__ __forceinline__ void bary_d(const double *pb, const double *pc, const
 }
 
 struct AdjFrame {                 // a frame's inputs to the FP64 render
-    const double *geo, *R;        // [V][8], [9]
-    const float *x, *lam;         // state [KT], light [3]
+    const double *geo, *R;        // [V][3], [9] (then dR [27])
+    const float *x, *lam, *cam;   // state [KT], light [3], camera [4]
     float L;
-    int x0, y0, N;
+    int x0, y0, N, K;
     const Fragment *fr;
 };
 
@@ -212,293 +203,396 @@ __device__ __forceinline__ AdjFrame adj_frame(const DModel &m, const DBatch &b, 
                                               const float *Lint, const double *geo64, const double *R64, int f)
 {
     AdjFrame a;
-    a.geo = geo64 + (size_t)f * m.V * 8;
+    a.geo = geo64 + (size_t)f * m.V * 3;
     a.R = R64 + (size_t)f * 36;
     a.x = x + (size_t)f * m.KT;
     a.lam = lam + (size_t)f * 3;
+    a.cam = b.cam + (size_t)f * 4;
     a.L = Lint[f];
     a.x0 = b.x0y0[2 * f];
     a.y0 = b.x0y0[2 * f + 1];
     a.N = b.ctl[f].N;
+    a.K = m.K;
     a.fr = b.frag + (size_t)f * NMAX;
     return a;
 }
 
-// FP64 shading of the owner fragments painted into a zero image (fill_diffuse_component...,
-// newfuncs.cu:18-167, and fill_tex_im1, funcs.cu:800-817).
-__global__ void k_adj_shade(DModel m, DBatch b, const float *x, const float *lam, const float *Lint, int F,
-                            const double *geo64, const double *R64, double *img)
+// A fragment's corner: object coordinates, camera coordinates X = R P + tau, projection.
+struct AdjCorner {
+    double P[3], X[3], s[2];
+};
+
+__device__ __forceinline__ AdjCorner adj_corner(const AdjFrame &a, int v)
 {
-    const int f = blockIdx.y;
-    if (f >= F) return;
+    AdjCorner c;
+    const double *g = a.geo + (size_t)v * 3;
+    for (int k = 0; k < 3; ++k) c.P[k] = g[k];
+    for (int i = 0; i < 3; ++i)
+        c.X[i] = (a.R[i] * c.P[0] + a.R[3 + i] * c.P[1]) + a.R[6 + i] * c.P[2] + (double)a.x[a.K + i];
+    c.s[0] = (double)a.cam[0] * c.X[0] / c.X[2] + (double)a.cam[2];
+    c.s[1] = (double)a.cam[1] * c.X[1] / c.X[2] + (double)a.cam[3];
+    return c;
+}
+
+// The image of one frame in FP64 and its loss, one block per frame, the region around the fragments
+// (their box + 8 px; beyond it the render is zero and the target does not reach a fragment's
+// gradient) in shared memory, in the layout of the fit's render: A [rw][pb + 2 RPAD] with zero
+// columns left and right, B [KRAD + rw + KRAD][pb] with zero lines above and below.
+//   shading of the owner fragments painted into a zero image (fill_diffuse_component...,
+//   newfuncs.cu:18-167, fill_tex_im1, funcs.cu:800-817), the 15-tap blur, the gradients of render
+//   and target at every fragment (fill_grads, funcs.cu:842-897), the loss; with BACK the adjoint of
+//   the gradients scattered into dL/d(blurred image), the transposed blur, and dL/d(pixel value)
+//   of every fragment's pixel out in dI.
+constexpr int AI_THREADS = 1024;
+constexpr int AI_SMEM = 216 * 1024;
+constexpr size_t AI_GLOBAL = 2 * (size_t)DIM * (DIM + 2 * RPAD);   // doubles of a frame's region that does not fit
+constexpr int AI_RUN_Y = 5, AI_RUN_X = 4;                          // blur outputs per thread along the taps
+
+struct RegionD {
+    int rx0, ry0, rw, rh, pb, ph;
+    double *A, *B;
+    __device__ __forceinline__ int at(int p) const { return ((p >> 8) - rx0) * ph + RPAD + ((p & 255) - ry0); }
+    __device__ __forceinline__ int bt(int p) const { return (KRAD + (p >> 8) - rx0) * pb + ((p & 255) - ry0); }
+};
+
+// along y: A -> B
+__device__ __forceinline__ void adj_blur_rows(const RegionD &r, const double (&tap)[NTAPS])
+{
+    const int nrun = (r.rh + AI_RUN_Y - 1) / AI_RUN_Y;
+    for (int i = threadIdx.x; i < r.rw * nrun; i += AI_THREADS) {
+        const int xl = i / nrun, y0 = min((i - xl * nrun) * AI_RUN_Y, r.rh - AI_RUN_Y);
+        const double *a = r.A + xl * r.ph + RPAD - KRAD + y0;
+        double s[AI_RUN_Y];
+#pragma unroll
+        for (int o = 0; o < AI_RUN_Y; ++o) s[o] = 0.0;
+#pragma unroll
+        for (int t = 0; t < AI_RUN_Y + 2 * KRAD; ++t) {
+            const double v = a[t];
+#pragma unroll
+            for (int o = 0; o < AI_RUN_Y; ++o)
+                if (t >= o && t - o <= 2 * KRAD) s[o] = fma(tap[t - o], v, s[o]);
+        }
+#pragma unroll
+        for (int o = 0; o < AI_RUN_Y; ++o) r.B[(KRAD + xl) * r.pb + y0 + o] = s[o];
+    }
+    __syncthreads();
+}
+
+// along x: B -> A
+__device__ __forceinline__ void adj_blur_cols(const RegionD &r, const double (&tap)[NTAPS])
+{
+    const int nrun = (r.rw + AI_RUN_X - 1) / AI_RUN_X;
+    for (int i = threadIdx.x; i < r.rh * nrun; i += AI_THREADS) {
+        const int g = i / r.rh, yl = i - g * r.rh, x0 = min(g * AI_RUN_X, r.rw - AI_RUN_X);
+        const double *bp = r.B + x0 * r.pb + yl;
+        double s[AI_RUN_X];
+#pragma unroll
+        for (int o = 0; o < AI_RUN_X; ++o) s[o] = 0.0;
+#pragma unroll
+        for (int t = 0; t < AI_RUN_X + 2 * KRAD; ++t) {
+            const double v = bp[t * r.pb];
+#pragma unroll
+            for (int o = 0; o < AI_RUN_X; ++o)
+                if (t >= o && t - o <= 2 * KRAD) s[o] = fma(tap[t - o], v, s[o]);
+        }
+#pragma unroll
+        for (int o = 0; o < AI_RUN_X; ++o) r.A[(x0 + o) * r.ph + RPAD + yl] = s[o];
+    }
+    __syncthreads();
+}
+
+template <bool BACK>
+__global__ void __launch_bounds__(AI_THREADS, 1) k_adj_image(DModel m, DBatch b, Cfg c, const float *x, const float *lam,
+                                                             const float *Lint, const double *geo64, const double *R64,
+                                                             const float *target, double *region, double *grads,
+                                                             const double *gloss, double *loss, double *dI)
+{
+    extern __shared__ __align__(16) double ais[];
+    __shared__ double s_red[AI_THREADS / 32];
+    __shared__ double s_q[3];
+    const int f = blockIdx.x, tid = threadIdx.x;
     const AdjFrame a = adj_frame(m, b, x, lam, Lint, geo64, R64, f);
-    double *im = img + (size_t)f * NPIX;
-    for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < a.N; n += gridDim.x * blockDim.x) {
+    const int N = a.N;
+    if (N == 0) {
+        if (tid == 0 && loss) loss[f] = 0.0;
+        return;
+    }
+    const Region rf = make_region(b.ctl[f], nullptr, nullptr);
+    RegionD r{rf.rx0, rf.ry0, rf.rw, rf.rh, rf.pb, rf.ph, nullptr, nullptr};
+    const size_t need = (size_t)r.rw * r.ph + (size_t)(r.rw + 2 * KRAD) * r.pb;
+    r.A = need * sizeof(double) <= AI_SMEM ? ais : region + (size_t)f * AI_GLOBAL;
+    r.B = r.A + (size_t)r.rw * r.ph;
+    double tap[NTAPS];
+#pragma unroll
+    for (int j = 0; j < NTAPS; ++j) tap[j] = (double)c.taps[2 * KRAD - j];
+    auto clear = [&](double *p, int n) { for (int i = tid; i < n; i += AI_THREADS) p[i] = 0.0; };
+    clear(r.A, (int)need);                               // A and B, zero lines included
+    if (tid < 3) {
+        double q = 0.0;
+        for (int j = 0; j < 3; ++j) q += a.R[3 * tid + j] * ((double)a.lam[j] - (double)a.x[a.K + j]);
+        s_q[tid] = q;
+    }
+    __syncthreads();
+    for (int n = tid; n < N; n += AI_THREADS) {
         const Fragment fr = a.fr[n];
         if (!(fr.pix_owner >> 31)) continue;
-        const int pix = fr.pix_owner & 0xFFFF, tri = fr.tri;
-        const int ib = m.tl[tri], ic = m.tl[m.T + tri], ia = m.tl[2 * m.T + tri];
-        const double *gb = a.geo + (size_t)ib * 8, *gc = a.geo + (size_t)ic * 8, *ga = a.geo + (size_t)ia * 8;
+        const int pix = fr.pix_owner & 0xFFFF;
+        const int4 tq = __ldg(m.tl4 + fr.tri);
+        const AdjCorner cb = adj_corner(a, tq.x), cc = adj_corner(a, tq.y), ca = adj_corner(a, tq.z);
         double al, be;
-        bary_d(gb + 6, gc + 6, ga + 6, (double)(a.x0 + (pix >> 8)), (double)(a.y0 + (pix & 255)), al, be, nullptr);
+        bary_d(cb.s, cc.s, ca.s, (double)(a.x0 + (pix >> 8)), (double)(a.y0 + (pix & 255)), al, be, nullptr);
         const double gm = 1.0 - al - be;
         double v[3], w[3], nr[3];
-        for (int c = 0; c < 3; ++c) { v[c] = gb[c] - ga[c]; w[c] = gc[c] - ga[c]; }
+        for (int k = 0; k < 3; ++k) { v[k] = cb.P[k] - ca.P[k]; w[k] = cc.P[k] - ca.P[k]; }
         nr[0] = v[1] * w[2] - v[2] * w[1]; nr[1] = v[2] * w[0] - v[0] * w[2]; nr[2] = v[0] * w[1] - v[1] * w[0];
         const double nn = sqrt(nr[0] * nr[0] + nr[1] * nr[1] + nr[2] * nr[2]);
         double Id = 0.0;
-        for (int k = 0; k < 3; ++k) {
-            double q = 0.0;
-            for (int j = 0; j < 3; ++j) q += a.R[3 * k + j] * ((double)a.lam[j] - (double)a.x[m.K + j]);
-            const double p = gb[k] * al + gc[k] * be + ga[k] * gm;
-            Id += nr[k] / nn * (q - p);
-        }
-        const double t = (double)m.tex[ib] * al + (double)m.tex[ic] * be + (double)m.tex[ia] * gm;
-        im[pix] = t + (double)a.L * t * Id;
+        for (int k = 0; k < 3; ++k) Id += nr[k] / nn * (s_q[k] - (cb.P[k] * al + cc.P[k] * be + ca.P[k] * gm));
+        const double t = (double)m.tex[tq.x] * al + (double)m.tex[tq.y] * be + (double)m.tex[tq.z] * gm;
+        r.A[r.at(pix)] = t + (double)a.L * t * Id;
     }
-}
-
-// FP64 separable blur pass (the 15 taps of the fit, zero border): along y (dir 0) or x (dir 1).
-__global__ void k_adj_blur(const double *src, double *dst, Cfg c, int F, int dir)
-{
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (size_t)F * NPIX) return;
-    const size_t f = i / NPIX;
-    const int p = (int)(i - f * NPIX), xx = p >> 8, yy = p & 255;
-    const double *s = src + f * NPIX;
-    double acc = 0.0;
-    for (int j = -KRAD; j <= KRAD; ++j) {
-        const int u = (dir == 0 ? yy : xx) + j;
-        if (u < 0 || u >= DIM) continue;
-        acc += (double)c.taps[KRAD - j] * s[dir == 0 ? xx * DIM + u : u * DIM + yy];
+    __syncthreads();
+    adj_blur_rows(r, tap);
+    adj_blur_cols(r, tap);
+    // the render's gradients, kept while the target takes the region
+    double *gr = grads + (size_t)f * 2 * NMAX;
+    for (int n = tid; n < N; n += AI_THREADS) {
+        int kr, kl, kd, ku;
+        neighbour_pixels((int)(a.fr[n].pix_owner & 0xFFFF), kr, kl, kd, ku);
+        gr[n] = 0.5 * (r.A[r.at(kr)] - r.A[r.at(kl)]);
+        gr[NMAX + n] = 0.5 * (r.A[r.at(kd)] - r.A[r.at(ku)]);
     }
-    dst[i] = acc;
-}
-
-// FP32 crops to FP64 (the target before its blur).
-__global__ void k_adj_widen(const float *src, double *dst, size_t n)
-{
-    const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) dst[i] = (double)src[i];
-}
-
-// Normalised central-difference gradients at every fragment (fill_grads, funcs.cu:842-897) of
-// the blurred render B and target T; loss sums into loss[f]; with adjB, the adjoint of the
-// gradients scattered into dL/dB (gloss[f] scales the frame's loss gradient).
-__global__ void k_adj_grad(DBatch b, int F, const double *B, const double *T, double *loss, const double *gloss,
-                           double *adjB)
-{
-    const int f = blockIdx.y;
-    if (f >= F) return;
-    const int N = b.ctl[f].N;
-    const Fragment *frs = b.frag + (size_t)f * NMAX;
-    const double *Bf = B + (size_t)f * NPIX, *Tf = T + (size_t)f * NPIX;
+    __syncthreads();
+    const float *tg = target + (size_t)f * NPIX;
+    for (int i = tid; i < r.rw * r.rh; i += AI_THREADS) {
+        const int xl = i / r.rh, yl = i - xl * r.rh;
+        r.A[xl * r.ph + RPAD + yl] = (double)tg[(r.rx0 + xl) * DIM + r.ry0 + yl];
+    }
+    __syncthreads();
+    adj_blur_rows(r, tap);
+    adj_blur_cols(r, tap);
+    if (BACK) {
+        clear(r.B + KRAD * r.pb, r.rw * r.pb);           // dL/d(blurred image) is collected here
+        __syncthreads();
+    }
     double part = 0.0;
-    for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < N; n += gridDim.x * blockDim.x) {
-        const int p = frs[n].pix_owner & 0xFFFF, x = p >> 8, y = p & 255;
-        const int kr = x < DIM - 1 ? p + DIM : 0, kl = x > 0 ? p - DIM : 0;
-        const int kb = y < DIM - 1 ? p + 1 : 0, ka = y > 0 ? p - 1 : 0;
-        const double gx = 0.5 * (Bf[kr] - Bf[kl]), gy = 0.5 * (Bf[kb] - Bf[ka]);
-        const double r = sqrt(4.0 * gx * gx + 4.0 * gy * gy), h = 1e-16 + r;
-        const double sx = 0.5 * (Tf[kr] - Tf[kl]), sy = 0.5 * (Tf[kb] - Tf[ka]);
+    const double gl = BACK ? gloss[f] : 0.0;
+    for (int n = tid; n < N; n += AI_THREADS) {
+        int kr, kl, kd, ku;
+        neighbour_pixels((int)(a.fr[n].pix_owner & 0xFFFF), kr, kl, kd, ku);
+        const double gx = gr[n], gy = gr[NMAX + n];
+        const double rr = sqrt(4.0 * gx * gx + 4.0 * gy * gy), h = 1e-16 + rr;
+        const double sx = 0.5 * (r.A[r.at(kr)] - r.A[r.at(kl)]), sy = 0.5 * (r.A[r.at(kd)] - r.A[r.at(ku)]);
         const double hs = 1e-16 + sqrt(4.0 * sx * sx + 4.0 * sy * sy);
         const double sxn = 2.0 * sx / hs, syn = 2.0 * sy / hs;
         part += -((2.0 * gx / h) * sxn + (2.0 * gy / h) * syn);
-        if (adjB) {
-            const double gl = gloss[f];
+        if (BACK) {
             const double dgxn = -gl * sxn, dgyn = -gl * syn;         // dL/d(2 gx / h), dL/d(2 gy / h)
-            const double dh = r > 0.0 ? 1.0 / r : 0.0;
+            const double dh = rr > 0.0 ? 1.0 / rr : 0.0;
             const double hx = 4.0 * gx * dh, hy = 4.0 * gy * dh;     // dh/dgx, dh/dgy
             const double dgx = dgxn * (2.0 / h - 2.0 * gx * hx / (h * h)) + dgyn * (-2.0 * gy * hx / (h * h));
             const double dgy = dgxn * (-2.0 * gx * hy / (h * h)) + dgyn * (2.0 / h - 2.0 * gy * hy / (h * h));
-            double *A = adjB + (size_t)f * NPIX;
-            atomicAdd(A + kr, 0.5 * dgx);
-            atomicAdd(A + kl, -0.5 * dgx);
-            atomicAdd(A + kb, 0.5 * dgy);
-            atomicAdd(A + ka, -0.5 * dgy);
+            atomicAdd(r.B + r.bt(kr), 0.5 * dgx);
+            atomicAdd(r.B + r.bt(kl), -0.5 * dgx);
+            atomicAdd(r.B + r.bt(kd), 0.5 * dgy);
+            atomicAdd(r.B + r.bt(ku), -0.5 * dgy);
         }
     }
-    warp_atomic_add(loss + f, part);
+    if (loss) {
+        part = wsum(part);
+        if ((tid & 31) == 0) s_red[tid >> 5] = part;
+        __syncthreads();
+        if (tid < 32) {
+            const double t = wsum(s_red[tid]);
+            if (tid == 0) loss[f] = t;
+        }
+    }
+    if (!BACK) return;
+    __syncthreads();
+    // transposed blur: the column pass first, then the row pass (A's zero columns are still zero)
+    adj_blur_cols(r, tap);
+    adj_blur_rows(r, tap);
+    double *out = dI + (size_t)f * NMAX;
+    for (int n = tid; n < N; n += AI_THREADS) {
+        const uint32_t po = a.fr[n].pix_owner;
+        out[n] = (po >> 31) ? r.B[r.bt(po & 0xFFFF)] : 0.0;
+    }
 }
 
-// Adjoint of the shading of the owner fragments: dL/dpixel -> light, pose (through R^T (lam - tau)),
-// object coordinates of the corners (normal, interpolated point) and projected corners
-// (barycentrics). Per-vertex terms by FP64 atomics, per-frame terms summed per warp.
-__global__ void k_adj_frag_back(DModel m, DBatch b, const float *x, const float *lam, const float *Lint, int F,
-                                const double *geo64, const double *R64, const double *adjI, double *dP0, double *dpos,
-                                double *glob)
+// Adjoint of the shading of the owner fragments: dL/dpixel -> light, pose, and the object coordinates
+// of the three corners (dP [N][9]: corners b, c, a), through the normal and the interpolated point,
+// and through the barycentrics, the projections and the camera coordinates. Per-frame terms
+// (glob: dR[9], dtau[3], dlam[3], dL) summed per block, one atomic per block and entry.
+__global__ void __launch_bounds__(AD_THREADS) k_adj_frag_back(DModel m, DBatch b, const float *x, const float *lam,
+                                                              const float *Lint, const double *geo64, const double *R64,
+                                                              const double *dI, double *dP0, double *glob)
 {
+    __shared__ double s_acc[AD_THREADS / 32][AD_GLOB];
     const int f = blockIdx.y;
-    if (f >= F) return;
     const AdjFrame a = adj_frame(m, b, x, lam, Lint, geo64, R64, f);
-    const double *AI = adjI + (size_t)f * NPIX;
+    if ((int)(blockIdx.x * AD_THREADS) >= a.N) return;
     double acc[AD_GLOB];
 #pragma unroll
     for (int i = 0; i < AD_GLOB; ++i) acc[i] = 0.0;
     double dl[3];
     for (int j = 0; j < 3; ++j) dl[j] = (double)a.lam[j] - (double)a.x[m.K + j];
-    for (int n = blockIdx.x * blockDim.x + threadIdx.x; n < a.N; n += gridDim.x * blockDim.x) {
-        const Fragment fr = a.fr[n];
-        if (!(fr.pix_owner >> 31)) continue;
-        const int pix = fr.pix_owner & 0xFFFF, tri = fr.tri;
-        const double dI = AI[pix];
-        if (dI == 0.0) continue;
-        const int iv[3] = {m.tl[tri], m.tl[m.T + tri], m.tl[2 * m.T + tri]};        // b, c, a
-        const double *gb = a.geo + (size_t)iv[0] * 8, *gc = a.geo + (size_t)iv[1] * 8, *ga = a.geo + (size_t)iv[2] * 8;
-        double al, be, db[12];
-        bary_d(gb + 6, gc + 6, ga + 6, (double)(a.x0 + (pix >> 8)), (double)(a.y0 + (pix & 255)), al, be, db);
-        const double gm = 1.0 - al - be;
-        double v[3], w[3], nr[3], nh[3], q[3], p[3];
-        for (int c = 0; c < 3; ++c) { v[c] = gb[c] - ga[c]; w[c] = gc[c] - ga[c]; }
-        nr[0] = v[1] * w[2] - v[2] * w[1]; nr[1] = v[2] * w[0] - v[0] * w[2]; nr[2] = v[0] * w[1] - v[1] * w[0];
-        const double nn = sqrt(nr[0] * nr[0] + nr[1] * nr[1] + nr[2] * nr[2]);
-        double Id = 0.0;
-        for (int k = 0; k < 3; ++k) {
-            nh[k] = nr[k] / nn;
-            q[k] = 0.0;
-            for (int j = 0; j < 3; ++j) q[k] += a.R[3 * k + j] * dl[j];
-            p[k] = gb[k] * al + gc[k] * be + ga[k] * gm;
-            Id += nh[k] * (q[k] - p[k]);
-        }
-        const double tb = m.tex[iv[0]], tc = m.tex[iv[1]], ta = m.tex[iv[2]];
-        const double t = tb * al + tc * be + ta * gm, L = a.L;
-        const double dt = dI * (1.0 + L * Id), dId = dI * L * t;
-        acc[15] += dI * t * Id;                                          // dL/dL_intensity
-        double dal = dt * (tb - ta), dbe = dt * (tc - ta);
-        double dn[3], dP[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
-        for (int k = 0; k < 3; ++k) {
-            dn[k] = dId * (q[k] - p[k]);
-            const double dq = dId * nh[k], dp = -dId * nh[k];
-            for (int j = 0; j < 3; ++j) {
-                acc[3 * k + j] += dq * dl[j];                            // dR[3k + j]
-                const double dd = dq * a.R[3 * k + j];
-                acc[12 + j] += dd;                                       // dlambda_j
-                acc[9 + j] -= dd;                                        // dtau_j
+    for (int n = blockIdx.x * AD_THREADS + threadIdx.x; n < a.N; n += gridDim.x * AD_THREADS) {
+        double dP[3][3] = {{0, 0, 0}, {0, 0, 0}, {0, 0, 0}};
+        const double dIn = dI[(size_t)f * NMAX + n];
+        if (dIn != 0.0) {
+            const Fragment fr = a.fr[n];
+            const int pix = fr.pix_owner & 0xFFFF;
+            const int4 tq = __ldg(m.tl4 + fr.tri);
+            const AdjCorner cr[3] = {adj_corner(a, tq.x), adj_corner(a, tq.y), adj_corner(a, tq.z)};    // b, c, a
+            double al, be, db[12];
+            bary_d(cr[0].s, cr[1].s, cr[2].s, (double)(a.x0 + (pix >> 8)), (double)(a.y0 + (pix & 255)), al, be, db);
+            const double gm = 1.0 - al - be;
+            double v[3], w[3], nr[3], nh[3], q[3], p[3];
+            for (int k = 0; k < 3; ++k) { v[k] = cr[0].P[k] - cr[2].P[k]; w[k] = cr[1].P[k] - cr[2].P[k]; }
+            nr[0] = v[1] * w[2] - v[2] * w[1]; nr[1] = v[2] * w[0] - v[0] * w[2]; nr[2] = v[0] * w[1] - v[1] * w[0];
+            const double nn = sqrt(nr[0] * nr[0] + nr[1] * nr[1] + nr[2] * nr[2]);
+            double Id = 0.0;
+            for (int k = 0; k < 3; ++k) {
+                nh[k] = nr[k] / nn;
+                q[k] = 0.0;
+                for (int j = 0; j < 3; ++j) q[k] += a.R[3 * k + j] * dl[j];
+                p[k] = cr[0].P[k] * al + cr[1].P[k] * be + cr[2].P[k] * gm;
+                Id += nh[k] * (q[k] - p[k]);
             }
-            dal += dp * (gb[k] - ga[k]);
-            dbe += dp * (gc[k] - ga[k]);
-            dP[0][k] += al * dp; dP[1][k] += be * dp; dP[2][k] += gm * dp;
+            const double tb = m.tex[tq.x], tc = m.tex[tq.y], ta = m.tex[tq.z];
+            const double t = tb * al + tc * be + ta * gm, L = a.L;
+            const double dt = dIn * (1.0 + L * Id), dId = dIn * L * t;
+            acc[15] += dIn * t * Id;                                         // dL/dL_intensity
+            double dal = dt * (tb - ta), dbe = dt * (tc - ta);
+            double dn[3];
+            for (int k = 0; k < 3; ++k) {
+                dn[k] = dId * (q[k] - p[k]);
+                const double dq = dId * nh[k], dp = -dId * nh[k];
+                for (int j = 0; j < 3; ++j) {
+                    acc[3 * k + j] += dq * dl[j];                            // dR[3k + j]
+                    const double dd = dq * a.R[3 * k + j];
+                    acc[12 + j] += dd;                                       // dlambda_j
+                    acc[9 + j] -= dd;                                        // dtau_j
+                }
+                dal += dp * (cr[0].P[k] - cr[2].P[k]);
+                dbe += dp * (cr[1].P[k] - cr[2].P[k]);
+                dP[0][k] += al * dp; dP[1][k] += be * dp; dP[2][k] += gm * dp;
+            }
+            const double nd = nh[0] * dn[0] + nh[1] * dn[1] + nh[2] * dn[2];
+            double dnr[3];
+            for (int k = 0; k < 3; ++k) dnr[k] = (dn[k] - nh[k] * nd) / nn;
+            // nr = v x w: dL/dv = w x dnr, dL/dw = dnr x v
+            const double dv[3] = {w[1] * dnr[2] - w[2] * dnr[1], w[2] * dnr[0] - w[0] * dnr[2], w[0] * dnr[1] - w[1] * dnr[0]};
+            const double dw[3] = {dnr[1] * v[2] - dnr[2] * v[1], dnr[2] * v[0] - dnr[0] * v[2], dnr[0] * v[1] - dnr[1] * v[0]};
+            for (int k = 0; k < 3; ++k) {
+                dP[0][k] += dv[k];
+                dP[1][k] += dw[k];
+                dP[2][k] -= dv[k] + dw[k];
+            }
+            // projected corners -> camera coordinates -> translation, rotation, object coordinates
+            for (int ci = 0; ci < 3; ++ci) {
+                const double sx = dal * db[2 * ci] + dbe * db[6 + 2 * ci], sy = dal * db[2 * ci + 1] + dbe * db[6 + 2 * ci + 1];
+                const double X = cr[ci].X[0], Y = cr[ci].X[1], Z = cr[ci].X[2];
+                const double gx = sx * a.cam[0], gy = sy * a.cam[1];
+                const double gc[3] = {gx / Z, gy / Z, -(gx * X + gy * Y) / (Z * Z)};
+                for (int j = 0; j < 3; ++j) {
+                    double s = 0.0;
+                    for (int i = 0; i < 3; ++i) {
+                        acc[i + 3 * j] += gc[i] * cr[ci].P[j];               // dR[i + 3j] (X = R P0 + tau)
+                        s += gc[i] * a.R[i + 3 * j];
+                    }
+                    dP[ci][j] += s;
+                    acc[9 + j] += gc[j];
+                }
+            }
         }
-        const double nd = nh[0] * dn[0] + nh[1] * dn[1] + nh[2] * dn[2];
-        double dnr[3];
-        for (int k = 0; k < 3; ++k) dnr[k] = (dn[k] - nh[k] * nd) / nn;
-        // nr = v x w: dL/dv = w x dnr, dL/dw = dnr x v
-        const double dv[3] = {w[1] * dnr[2] - w[2] * dnr[1], w[2] * dnr[0] - w[0] * dnr[2], w[0] * dnr[1] - w[1] * dnr[0]};
-        const double dw[3] = {dnr[1] * v[2] - dnr[2] * v[1], dnr[2] * v[0] - dnr[0] * v[2], dnr[0] * v[1] - dnr[1] * v[0]};
-        for (int k = 0; k < 3; ++k) {
-            dP[0][k] += dv[k];
-            dP[1][k] += dw[k];
-            dP[2][k] -= dv[k] + dw[k];
-        }
-        double *P0f = dP0 + (size_t)f * m.V * 3, *pf = dpos + (size_t)f * m.V * 2;
-        for (int c = 0; c < 3; ++c) {
-            for (int k = 0; k < 3; ++k) atomicAdd(P0f + (size_t)iv[c] * 3 + k, dP[c][k]);
-            atomicAdd(pf + (size_t)iv[c] * 2 + 0, dal * db[2 * c] + dbe * db[6 + 2 * c]);
-            atomicAdd(pf + (size_t)iv[c] * 2 + 1, dal * db[2 * c + 1] + dbe * db[6 + 2 * c + 1]);
-        }
+        double *o = dP0 + ((size_t)f * NMAX + n) * 9;
+        for (int ci = 0; ci < 3; ++ci)
+            for (int j = 0; j < 3; ++j) o[3 * ci + j] = dP[ci][j];
     }
 #pragma unroll
-    for (int i = 0; i < AD_GLOB; ++i) warp_atomic_add(glob + (size_t)f * AD_GLOB + i, acc[i]);
-}
-
-// Per vertex: dL/d(xp, yp) -> camera coordinates -> translation, rotation and object coordinates
-// (added to dP0 in place).
-__global__ void k_adj_vertex_back(DModel m, int F, const double *geo64, const double *R64, const float *cam,
-                                  const double *dpos, double *dP0, double *glob)
-{
-    const int f = blockIdx.y;
-    if (f >= F) return;
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    double acc[12];
-#pragma unroll
-    for (int i = 0; i < 12; ++i) acc[i] = 0.0;
-    if (v < m.V) {
-        const double *g = geo64 + ((size_t)f * m.V + v) * 8, *R = R64 + (size_t)f * 36;
-        const float *cm = cam + (size_t)f * 4;
-        const double gx = dpos[((size_t)f * m.V + v) * 2], gy = dpos[((size_t)f * m.V + v) * 2 + 1];
-        const double X = g[3], Y = g[4], Z = g[5];
-        const double gc[3] = {gx * cm[0] / Z, gy * cm[1] / Z, -(gx * cm[0] * X + gy * cm[1] * Y) / (Z * Z)};
-        double *P = dP0 + ((size_t)f * m.V + v) * 3;
-        for (int j = 0; j < 3; ++j) {
-            double s = 0.0;
-            for (int i = 0; i < 3; ++i) {
-                acc[i + 3 * j] += gc[i] * g[j];                          // dR[i + 3j] (X = R P0 + tau)
-                s += gc[i] * R[i + 3 * j];
-            }
-            P[j] += s;
-            acc[9 + j] += gc[j];                                         // dtau_j
-        }
-    }
-    // the per-fragment rotation terms are indexed by q_k = sum_j R[3k + j] (lam - tau)_j: both
-    // index the same storage, so they add up entry by entry; summed per warp, then per block,
-    // one atomic per block and entry
-    __shared__ double s_acc[8][12];
-#pragma unroll
-    for (int i = 0; i < 12; ++i) {
+    for (int i = 0; i < AD_GLOB; ++i) {
         const double w = wsum(acc[i]);
         if ((threadIdx.x & 31) == 0) s_acc[threadIdx.x >> 5][i] = w;
     }
     __syncthreads();
-    if (threadIdx.x < 12) {
+    if (threadIdx.x < AD_GLOB) {
         double t = 0.0;
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) t += s_acc[w][threadIdx.x];
+        for (int w = 0; w < AD_THREADS / 32; ++w) t += s_acc[w][threadIdx.x];
         atomicAdd(glob + (size_t)f * AD_GLOB + threadIdx.x, t);
     }
 }
 
-// Basis-transpose product dL/deps_k = sum_v sum_c E[v][c][k] dL/dP0[v][c] over a tile of vertices.
-constexpr int AD_VT = 256;
-// A block takes AD_VT vertices x AE_F frames (threads = expression columns), so that each
-// basis row is read once per AE_F frames; per frame and column the vertex terms are summed in
-// vertex order, the block's partial added with one atomic.
-constexpr int AE_F = 16;
+// Basis-transpose product dL/deps_k = sum_n sum_c sum_j E[v(n, c)][j][k] dP0[n][c][j]: a block takes a
+// share of one frame's fragments, a thread four columns of every FL-th fragment (nine 16-byte
+// basis loads in flight); the block's sums are added with one atomic per column. Bound by the
+// basis rows' reads (2.8 KB per fragment, mostly from L2) and the conversions to FP64.
+constexpr int AE_THREADS = 256, AE_CH = 64, AE_PARTS = 16;
 
-__global__ void k_adj_eps(DModel m, int F, const double *dP0, double *geps)
+__global__ void __launch_bounds__(AE_THREADS) k_adj_eps(DModel m, DBatch b, const double *dP0, double *geps)
 {
-    const int k = threadIdx.x, f0 = blockIdx.y * AE_F;
-    const int v0 = blockIdx.x * AD_VT, v1 = min(m.V, v0 + AD_VT);
-    const bool live = k < m.K;
-    double acc[AE_F];
-#pragma unroll
-    for (int q = 0; q < AE_F; ++q) acc[q] = 0.0;
-    for (int v = v0; v < v1; ++v) {
-        const float *e = m.E + (size_t)v * 3 * m.KP + (live ? k : 0);
-        const double e0 = e[0], e1 = e[m.KP], e2 = e[2 * m.KP];
-#pragma unroll
-        for (int q = 0; q < AE_F; ++q) {
-            const int f = f0 + q;
-            if (f >= F) break;
-            const double *P = dP0 + ((size_t)f * m.V + v) * 3;
-            acc[q] += e0 * P[0] + e1 * P[1] + e2 * P[2];
+    extern __shared__ __align__(16) double aes[];        // [FL][KP] the threads' sums
+    __shared__ double s_d[AE_CH * 9];
+    __shared__ int s_v[AE_CH * 3];
+    const int f = blockIdx.y, tid = threadIdx.x, N = b.ctl[f].N;
+    const int Q = m.KP >> 2, FL = AE_THREADS / Q;        // column groups; fragments taken side by side
+    const int kq = tid % Q, fl = tid / Q;
+    const Fragment *frs = b.frag + (size_t)f * NMAX;
+    if ((int)blockIdx.x * AE_CH >= N) return;
+    double acc[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int c0 = blockIdx.x * AE_CH; c0 < N; c0 += gridDim.x * AE_CH) {
+        const int cnt = min(AE_CH, N - c0);
+        for (int i = tid; i < cnt * 9; i += AE_THREADS) s_d[i] = dP0[((size_t)f * NMAX + c0) * 9 + i];
+        if (tid < cnt) {
+            const int4 tq = __ldg(m.tl4 + frs[c0 + tid].tri);
+            s_v[3 * tid] = tq.x; s_v[3 * tid + 1] = tq.y; s_v[3 * tid + 2] = tq.z;
         }
-    }
-    if (!live) return;
+        __syncthreads();
+        if (fl < FL)
+            for (int n = fl; n < cnt; n += FL) {
+                float4 e[9];
 #pragma unroll
-    for (int q = 0; q < AE_F; ++q) {
-        const int f = f0 + q;
-        if (f >= F) break;
-        atomicAdd(geps + (size_t)f * m.K + k, acc[q]);
+                for (int q = 0; q < 9; ++q)
+                    e[q] = __ldg(reinterpret_cast<const float4 *>(m.E + ((size_t)s_v[3 * n + q / 3] * 3 + q % 3) * m.KP) + kq);
+#pragma unroll
+                for (int q = 0; q < 9; ++q) {
+                    const double d = s_d[9 * n + q];
+                    acc[0] = fma((double)e[q].x, d, acc[0]);
+                    acc[1] = fma((double)e[q].y, d, acc[1]);
+                    acc[2] = fma((double)e[q].z, d, acc[2]);
+                    acc[3] = fma((double)e[q].w, d, acc[3]);
+                }
+            }
+        __syncthreads();
+    }
+    if (fl < FL) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) aes[(size_t)fl * m.KP + 4 * kq + j] = acc[j];
+    }
+    __syncthreads();
+    for (int k = tid; k < m.K; k += AE_THREADS) {
+        double t = 0.0;
+        for (int q = 0; q < FL; ++q) t += aes[(size_t)q * m.KP + k];
+        atomicAdd(geps + (size_t)f * m.K + k, t);
     }
 }
 
-// Gradients out: x [F][K+6] (epsilon, tau, u through dR/du), lambda [F][3], L [F].
-__global__ void k_adj_final(DModel m, int F, const double *R64, const double *glob, const double *geps, double *gx,
+// Gradients out: x [F][K+6] (epsilon, tau, u through dR/du), lambda [F][3], L [F]; one block per frame.
+__global__ void k_adj_final(DModel m, const double *R64, const double *glob, const double *geps, double *gx,
                             double *glam, double *gL)
 {
-    const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= F) return;
+    const int f = blockIdx.x, tid = threadIdx.x;
     const double *G = glob + (size_t)f * AD_GLOB, *dR = R64 + (size_t)f * 36 + 9;
     double *o = gx + (size_t)f * m.KT;
-    for (int k = 0; k < m.K; ++k) o[k] = geps[(size_t)f * m.K + k];
-    for (int j = 0; j < 3; ++j) o[m.K + j] = G[9 + j];
-    for (int a = 0; a < 3; ++a) {
+    for (int k = tid; k < m.K; k += blockDim.x) o[k] = geps[(size_t)f * m.K + k];
+    if (tid < 3) {
+        o[m.K + tid] = G[9 + tid];
         double s = 0.0;
-        for (int i = 0; i < 9; ++i) s += G[i] * dR[9 * a + i];
-        o[m.K + 3 + a] = s;
+        for (int i = 0; i < 9; ++i) s += G[i] * dR[9 * tid + i];
+        o[m.K + 3 + tid] = s;
+        if (glam) glam[(size_t)f * 3 + tid] = G[12 + tid];
     }
-    if (glam)
-        for (int j = 0; j < 3; ++j) glam[(size_t)f * 3 + j] = G[12 + j];
-    if (gL) gL[f] = G[15];
+    if (tid == 0 && gL) gL[f] = G[15];
 }
 
 // The caller's states [F][K+6] into the batch's evaluation states (pitch KTP).

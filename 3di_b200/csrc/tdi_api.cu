@@ -267,7 +267,7 @@ float face_size_of(const float *xl, const float *yl)
 }
 
 
-constexpr int ADJ_VERTEX_SMEM_MAX = 100 * 1024;   // the tiled FP64 vertex stage of the loss (K up to ~190)
+constexpr int ADJ_VERTEX_SMEM_MAX = 200 * 1024;   // the tiled FP64 vertex stage of the loss (K up to ~235)
 
 tdi_status set_attrs()
 {
@@ -291,7 +291,11 @@ tdi_status set_attrs()
     TDI_CUDA(cudaFuncSetAttribute(k_normal_eq_tc<NE_GRP>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM));
     TDI_CUDA(cudaFuncSetAttribute(k_normal_eq_tc<TC_MAXN / 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, TC_SMEM));
     TDI_CUDA(cudaFuncSetAttribute(k_vertex_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vc_smem(VC_MAXK)));
-    TDI_CUDA(cudaFuncSetAttribute(k_adj_vertex_tiled, cudaFuncAttributeMaxDynamicSharedMemorySize, ADJ_VERTEX_SMEM_MAX));
+    TDI_CUDA(cudaFuncSetAttribute(k_adj_vertex_tiled<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, ADJ_VERTEX_SMEM_MAX));
+    TDI_CUDA(cudaFuncSetAttribute(k_adj_vertex_tiled<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, ADJ_VERTEX_SMEM_MAX));
+    TDI_CUDA(cudaFuncSetAttribute(k_adj_vertex_tiled<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, ADJ_VERTEX_SMEM_MAX));
+    TDI_CUDA(cudaFuncSetAttribute(k_adj_image<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, AI_SMEM));
+    TDI_CUDA(cudaFuncSetAttribute(k_adj_image<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, AI_SMEM));
     done = true;
     return TDI_OK;
 }
@@ -582,7 +586,7 @@ tdi_status stage_begin(tdi_batch *bt, const Cfg &c, int stage, int nlanes)
 {
     for (int l = 0; l < nlanes; ++l) {
         tdi_lane &ln = bt->lanes[l];
-        TDI_TRY(launch(bt, 0, k_stage_start, dim3((ln.d.F + 127) / 128), dim3(128), 0, ln.s, bt->m->d, ln.d, c, stage));
+        TDI_TRY(launch(bt, 0, k_stage_start, dim3(ln.d.F), dim3(SS_THREADS), 0, ln.s, bt->m->d, ln.d, c, stage));
         TDI_TRY(lane_compact(bt, ln));
     }
     for (int l = 0; l < nlanes; ++l) TDI_TRY(lane_count(bt->lanes[l]));
@@ -1106,7 +1110,7 @@ tdi_status tdi_batch_evaluate(tdi_batch *b, const tdi_fit_config *cfg, int32_t f
     const int stage = finetune_bounds ? ST_FINETUNE : ST_RIGID;
     TDI_TRY(blur_targets(b, c, s));
     TDI_TRY(launch(b, 0, k_fit_begin, L.fblocks(), dim3(128), 0, s, d));
-    TDI_TRY(launch(b, 0, k_stage_start, L.fblocks(), dim3(128), 0, s, m, d, c, stage));
+    TDI_TRY(launch(b, 0, k_stage_start, dim3(d.F), dim3(SS_THREADS), 0, s, m, d, c, stage));
     int n = 0;
     TDI_TRY(compact_active(b, s, &n));
     if (n == 0) return TDI_OK;
@@ -1268,30 +1272,30 @@ tdi_status tdi_batch_landmark_init(tdi_batch *b, const float *p0L, int32_t *succ
 
 // Working set of the differentiable loss for cap frames, carved from one FP64 allocation.
 struct AdjBufs {
-    double *geo, *R, *img, *tmp, *B, *T, *adjB, *adjI, *dP0, *dpos, *glob, *geps, *loss;
+    double *geo, *R, *region, *grads, *dI, *dP0, *glob, *geps;
 };
 
 static tdi_status adj_bufs(tdi_batch *b, AdjBufs &o)
 {
     const DModel &m = b->m->d;
     const size_t F = (size_t)b->cap, V = (size_t)m.V;
-    const size_t sizes[13] = {F * V * 8, F * 36, F * NPIX, F * NPIX, F * NPIX, F * NPIX, F * NPIX, F * NPIX,
-                              F * V * 3, F * V * 2, F * AD_GLOB, F * (size_t)m.K, F};
+    constexpr int NB = 8;
+    const size_t sizes[NB] = {F * V * 3, F * 36, F * AI_GLOBAL, F * 2 * NMAX, F * NMAX, F * 9 * NMAX, F * AD_GLOB,
+                              F * (size_t)m.K};
     size_t total = 0;
     for (size_t s : sizes) total += (s + 31) / 32 * 32;
     if (!b->adj) {
         TDI_CUDA(cudaMalloc(&b->adj, total * sizeof(double)));
         b->adj_doubles = total;
     }
-    double **dst[13] = {&o.geo, &o.R, &o.img, &o.tmp, &o.B, &o.T, &o.adjB, &o.adjI, &o.dP0, &o.dpos, &o.glob, &o.geps, &o.loss};
+    double **dst[NB] = {&o.geo, &o.R, &o.region, &o.grads, &o.dI, &o.dP0, &o.glob, &o.geps};
     double *p = b->adj;
-    for (int i = 0; i < 13; ++i) { *dst[i] = p; p += (sizes[i] + 31) / 32 * 32; }
+    for (int i = 0; i < NB; ++i) { *dst[i] = p; p += (sizes[i] + 31) / 32 * 32; }
     return TDI_OK;
 }
 
-// The raster at the caller's states and the FP64 loss (the forward of the loss and of its adjoint).
-static tdi_status adj_forward(tdi_batch *b, const Cfg &c, const float *x, const float *lam, const float *L,
-                              cudaStream_t s, AdjBufs &o)
+// The raster at the caller's states and the FP64 geometry (the forward of the loss and of its adjoint).
+static tdi_status adj_forward(tdi_batch *b, const Cfg &c, const float *x, cudaStream_t s, AdjBufs &o)
 {
     const DModel &m = b->m->d;
     DBatch &d = b->d;
@@ -1300,7 +1304,7 @@ static tdi_status adj_forward(tdi_batch *b, const Cfg &c, const float *x, const 
     Launch Lc{b, m, d, s, F};
     TDI_TRY(launch(b, 0, k_adj_set_x, dim3((F * m.KT + 255) / 256), dim3(256), 0, s, m, d, x, F));
     TDI_TRY(launch(b, 0, k_fit_begin, Lc.fblocks(), dim3(128), 0, s, d));
-    TDI_TRY(launch(b, 0, k_stage_start, Lc.fblocks(), dim3(128), 0, s, m, d, c, (int)ST_RIGID));
+    TDI_TRY(launch(b, 0, k_stage_start, dim3(F), dim3(SS_THREADS), 0, s, m, d, c, (int)ST_RIGID));
     int n = 0;
     TDI_TRY(compact_active(b, s, &n));
     if (n > 0) {
@@ -1308,24 +1312,17 @@ static tdi_status adj_forward(tdi_batch *b, const Cfg &c, const float *x, const 
         TDI_TRY(launch_vertex(b, m, d, s, n));
         TDI_TRY(raster(Lc));
     }
-    const size_t np = (size_t)F * NPIX;
-    const dim3 pb((unsigned)((np + 255) / 256));
-    TDI_TRY(launch(b, 0, k_adj_rot, dim3((F + 127) / 128), dim3(128), 0, s, m, d, x, F, o.R));
-    if (adj_vertex_smem(m.KP) <= (size_t)ADJ_VERTEX_SMEM_MAX)
-        TDI_TRY(launch(b, 0, k_adj_vertex_tiled, dim3((m.V + AV_V - 1) / AV_V, (F + AV_F - 1) / AV_F), dim3(256),
-                       adj_vertex_smem(m.KP), s, m, x, F, (const double *)o.R, (const float *)d.cam, o.geo));
+    TDI_TRY(launch(b, 0, k_adj_rot, dim3((F + 31) / 32), dim3(32), 0, s, m, d, x, F, o.R));
+    // frames per thread of the FP64 vertex stage: as many as the batch and shared memory hold
+    const dim3 vb((m.V + AV_V - 1) / AV_V);
+    if (F > 32 && adj_vertex_smem(m.KP, 8) <= (size_t)ADJ_VERTEX_SMEM_MAX)
+        TDI_TRY(launch(b, 0, k_adj_vertex_tiled<8>, dim3(vb.x, (F + 63) / 64), dim3(256), adj_vertex_smem(m.KP, 8), s, m, x, F, o.geo));
+    else if (F > 8 && adj_vertex_smem(m.KP, 4) <= (size_t)ADJ_VERTEX_SMEM_MAX)
+        TDI_TRY(launch(b, 0, k_adj_vertex_tiled<4>, dim3(vb.x, (F + 31) / 32), dim3(256), adj_vertex_smem(m.KP, 4), s, m, x, F, o.geo));
+    else if (adj_vertex_smem(m.KP, 1) <= (size_t)ADJ_VERTEX_SMEM_MAX)
+        TDI_TRY(launch(b, 0, k_adj_vertex_tiled<1>, dim3(vb.x, (F + 7) / 8), dim3(256), adj_vertex_smem(m.KP, 1), s, m, x, F, o.geo));
     else
-        TDI_TRY(launch(b, 0, k_adj_vertex, dim3((m.V + 255) / 256, F), dim3(256), 0, s, m, x, F, (const double *)o.R,
-                       (const float *)d.cam, o.geo));
-    TDI_CUDA(cudaMemsetAsync(o.img, 0, np * sizeof(double), s));
-    TDI_TRY(launch(b, 0, k_adj_shade, dim3(16, F), dim3(AD_THREADS), 0, s, m, (const DBatch)d, x, lam, L, F,
-                   (const double *)o.geo, (const double *)o.R, o.img));
-    TDI_TRY(launch(b, 0, k_adj_blur, pb, dim3(256), 0, s, (const double *)o.img, o.tmp, c, F, 0));
-    TDI_TRY(launch(b, 0, k_adj_blur, pb, dim3(256), 0, s, (const double *)o.tmp, o.B, c, F, 1));
-    TDI_TRY(launch(b, 0, k_adj_widen, pb, dim3(256), 0, s, (const float *)b->target_raw, o.img, np));
-    TDI_TRY(launch(b, 0, k_adj_blur, pb, dim3(256), 0, s, (const double *)o.img, o.tmp, c, F, 0));
-    TDI_TRY(launch(b, 0, k_adj_blur, pb, dim3(256), 0, s, (const double *)o.tmp, o.T, c, F, 1));
-    TDI_CUDA(cudaMemsetAsync(o.loss, 0, F * sizeof(double), s));
+        TDI_TRY(launch(b, 0, k_adj_vertex, dim3((m.V + 255) / 256, F), dim3(256), 0, s, m, x, F, o.geo));
     return TDI_OK;
 }
 
@@ -1335,13 +1332,12 @@ tdi_status tdi_batch_loss(tdi_batch *b, const tdi_fit_config *cfg, const float *
     if (!b || !cfg || !x || !lam || !L || !loss) return fail(TDI_ERR_INVALID, "null argument");
     if (b->d.F <= 0) return fail(TDI_ERR_INVALID, "no frames: call tdi_batch_set_frames first");
     cudaStream_t s = (cudaStream_t)stream;
+    const Cfg c = to_cfg(*cfg);
     AdjBufs o;
-    TDI_TRY(adj_forward(b, to_cfg(*cfg), x, lam, L, s, o));
-    const int F = b->d.F;
-    TDI_TRY(launch(b, 0, k_adj_grad, dim3(16, F), dim3(AD_THREADS), 0, s, (const DBatch)b->d, F, (const double *)o.B,
-                   (const double *)o.T, o.loss, (const double *)nullptr, (double *)nullptr));
-    TDI_CUDA(cudaMemcpyAsync(loss, o.loss, F * sizeof(double), cudaMemcpyDeviceToDevice, s));
-    return TDI_OK;
+    TDI_TRY(adj_forward(b, c, x, s, o));
+    return launch(b, 0, k_adj_image<false>, dim3(b->d.F), dim3(AI_THREADS), (size_t)AI_SMEM, s, b->m->d, b->d, c, x, lam, L,
+                  (const double *)o.geo, (const double *)o.R, (const float *)b->target_raw, o.region, o.grads,
+                  (const double *)nullptr, loss, (double *)nullptr);
 }
 
 tdi_status tdi_batch_loss_backward(tdi_batch *b, const tdi_fit_config *cfg, const float *x, const float *lam,
@@ -1354,28 +1350,19 @@ tdi_status tdi_batch_loss_backward(tdi_batch *b, const tdi_fit_config *cfg, cons
     const DModel &m = b->m->d;
     const Cfg c = to_cfg(*cfg);
     AdjBufs o;
-    TDI_TRY(adj_forward(b, c, x, lam, L, s, o));   // recomputed: nothing is kept from the forward call
+    TDI_TRY(adj_forward(b, c, x, s, o));           // recomputed: nothing is kept from the forward call
     const int F = b->d.F;
-    const size_t np = (size_t)F * NPIX;
-    const dim3 pb((unsigned)((np + 255) / 256));
-    TDI_CUDA(cudaMemsetAsync(o.adjB, 0, np * sizeof(double), s));
-    TDI_CUDA(cudaMemsetAsync(o.dP0, 0, (size_t)F * m.V * 3 * sizeof(double), s));
-    TDI_CUDA(cudaMemsetAsync(o.dpos, 0, (size_t)F * m.V * 2 * sizeof(double), s));
-    TDI_CUDA(cudaMemsetAsync(o.glob, 0, (size_t)F * AD_GLOB * sizeof(double), s));
-    TDI_CUDA(cudaMemsetAsync(o.geps, 0, (size_t)F * m.K * sizeof(double), s));
-    TDI_TRY(launch(b, 0, k_adj_grad, dim3(16, F), dim3(AD_THREADS), 0, s, (const DBatch)b->d, F, (const double *)o.B,
-                   (const double *)o.T, o.loss, gloss, o.adjB));
-    // transposed blur: the column pass first, then the row pass
-    TDI_TRY(launch(b, 0, k_adj_blur, pb, dim3(256), 0, s, (const double *)o.adjB, o.tmp, c, F, 1));
-    TDI_TRY(launch(b, 0, k_adj_blur, pb, dim3(256), 0, s, (const double *)o.tmp, o.adjI, c, F, 0));
-    TDI_TRY(launch(b, 0, k_adj_frag_back, dim3(16, F), dim3(AD_THREADS), 0, s, m, (const DBatch)b->d, x, lam, L, F,
-                   (const double *)o.geo, (const double *)o.R, (const double *)o.adjI, o.dP0, o.dpos, o.glob));
-    TDI_TRY(launch(b, 0, k_adj_vertex_back, dim3((m.V + 255) / 256, F), dim3(256), 0, s, m, F, (const double *)o.geo,
-                   (const double *)o.R, (const float *)b->d.cam, (const double *)o.dpos, o.dP0, o.glob));
-    TDI_TRY(launch(b, 0, k_adj_eps, dim3((m.V + AD_VT - 1) / AD_VT, (F + AE_F - 1) / AE_F), dim3(128), 0, s, m, F, (const double *)o.dP0,
-                   o.geps));
-    TDI_TRY(launch(b, 0, k_adj_final, dim3((F + 127) / 128), dim3(128), 0, s, m, F, (const double *)o.R,
-                   (const double *)o.glob, (const double *)o.geps, gx, glam, gL));
+    TDI_CUDA(cudaMemsetAsync(o.glob, 0, (size_t)((o.geps - o.glob) + (size_t)F * m.K) * sizeof(double), s));
+    TDI_TRY(launch(b, 0, k_adj_image<true>, dim3(F), dim3(AI_THREADS), (size_t)AI_SMEM, s, m, b->d, c, x, lam, L,
+                   (const double *)o.geo, (const double *)o.R, (const float *)b->target_raw, o.region, o.grads, gloss,
+                   (double *)nullptr, o.dI));
+    TDI_TRY(launch(b, 0, k_adj_frag_back, dim3(16, F), dim3(AD_THREADS), 0, s, m, (const DBatch)b->d, x, lam, L,
+                   (const double *)o.geo, (const double *)o.R, (const double *)o.dI, o.dP0, o.glob));
+    TDI_TRY(launch(b, 0, k_adj_eps, dim3(AE_PARTS, F), dim3(AE_THREADS),
+                   (size_t)(AE_THREADS / (m.KP >> 2)) * m.KP * sizeof(double), s, m, (const DBatch)b->d,
+                   (const double *)o.dP0, o.geps));
+    TDI_TRY(launch(b, 0, k_adj_final, dim3(F), dim3(96), 0, s, m, (const double *)o.R, (const double *)o.glob,
+                   (const double *)o.geps, gx, glam, gL));
     return TDI_OK;
 }
 
@@ -1508,7 +1495,7 @@ tdi_status tdi_batch_render(tdi_batch *b, float *images, int32_t *tri_map, void 
     c.ref_face_size = 78.0f;
     // evaluation point = x (shape-fit full evaluation), no fitting
     TDI_TRY(launch(b, 0, k_fit_begin, L.fblocks(), dim3(128), 0, s, d));
-    TDI_TRY(launch(b, 0, k_stage_start, L.fblocks(), dim3(128), 0, s, m, d, c, (int)ST_RIGID));
+    TDI_TRY(launch(b, 0, k_stage_start, dim3(d.F), dim3(SS_THREADS), 0, s, m, d, c, (int)ST_RIGID));
     int n = 0;
     TDI_TRY(compact_active(b, s, &n));
     if (n > 0) {

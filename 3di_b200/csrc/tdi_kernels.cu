@@ -135,29 +135,30 @@ __device__ void shape_reject(const DModel &m, const DBatch &b, const Cfg &c, int
 __device__ __forceinline__ int render_n(const DBatch &b) { return b.rcount[0]; }
 __device__ __forceinline__ int jac_n(const DBatch &b) { return b.rcount[1]; }
 
-__global__ void k_stage_start(DModel m, DBatch b, Cfg c, int stage)
+constexpr int SS_THREADS = 96;                   // start of a stage: a block per frame copies its states
+
+__global__ void __launch_bounds__(SS_THREADS) k_stage_start(DModel m, DBatch b, Cfg c, int stage)
 {
-    int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f == 0) b.rcount[0] = b.rcount[1] = 0;
+    const int f = blockIdx.x, tid = threadIdx.x;
+    if (f == 0 && tid == 0) b.rcount[0] = b.rcount[1] = 0;
     if (f >= b.F) return;
-    FrameCtl &ctl = b.ctl[f];
-    const bool dead = (ctl.flags & (FLAG_RENDER_SKIPPED | FLAG_OVERFLOW)) != 0;
-    ctl.active = dead ? 0 : 1;
-    ctl.mode = M_FULL;
-    ctl.render = 0;
-    ctl.need_jac = 0;
-    ctl.t = 1.0f;
-    ctl.inner = 0;
-    ctl.outer = 1;
-    if (stage == ST_LAMBDA) {
-        for (int j = 0; j < 3; ++j) b.lam_ls[f * 4 + j] = b.lam[f * 4 + j];
+    if (tid == 0) {
+        FrameCtl &ctl = b.ctl[f];
+        const bool dead = (ctl.flags & (FLAG_RENDER_SKIPPED | FLAG_OVERFLOW)) != 0;
+        ctl.active = dead ? 0 : 1;
+        ctl.mode = M_FULL;
+        ctl.render = 0;
+        ctl.need_jac = 0;
+        ctl.t = 1.0f;
+        ctl.inner = 0;
+        ctl.outer = 1;
     }
+    if (stage == ST_LAMBDA && tid < 3) b.lam_ls[f * 4 + tid] = b.lam[f * 4 + tid];
     // fit_3DMM_lambdas copies ov.betas into ov_linesearch (model_fitter.cu:991) and so
     // does fit_to_video_frame before each shape fit (video_fitter.cu:570-574); the
     // finetune keeps the line-search state the last shape fit left.
-    if (stage == ST_RIGID || stage == ST_LAMBDA) {
-        for (int a = 0; a < m.KT; ++a) b.x_ls[(size_t)f * m.KTP + a] = b.x[(size_t)f * m.KTP + a];
-    }
+    if (stage == ST_RIGID || stage == ST_LAMBDA)
+        for (int a = tid; a < m.KT; a += SS_THREADS) b.x_ls[(size_t)f * m.KTP + a] = b.x[(size_t)f * m.KTP + a];
 }
 
 // ------------------------------------------------------------------------------------------
