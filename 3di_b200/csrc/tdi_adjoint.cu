@@ -105,17 +105,27 @@ __global__ void __launch_bounds__(256) k_adj_vertex_tiled(DModel m, const float 
     double *Xs = avs;                                         // [KP][NF]
     double *Es = Xs + (size_t)NF * KP;                        // [AV_V][3][W]
     const int v0 = blockIdx.x * AV_V, f0 = blockIdx.y * NF, tid = threadIdx.x;
-    const int nrow = min(AV_V, m.V - v0) * 3 * KP;
-    for (int i = tid; i < nrow; i += 256) {
-        const int r = i / KP, k = i - r * KP;
-        Es[(size_t)r * W + k] = (double)m.E[(size_t)v0 * 3 * KP + i];
-    }
-    for (int i = tid; i < NF * KP; i += 256) {
-        const int fl = i / KP, k = i - fl * KP, f = f0 + fl;
-        Xs[(size_t)k * NF + fl] = (f < F && k < K) ? (double)x[(size_t)f * KT + k] : 0.0;
+    const int vl = tid & 31, fg = tid >> 5, v = v0 + vl;
+    const int nrow = min(AV_V, m.V - v0) * 3;
+    {
+        const int Q = KP >> 2;
+        const uint32_t mq = 0xFFFFFFFFu / (uint32_t)Q + 1u;      // i / Q = umulhi(i, mq) for i < 2^16
+        const float4 *e4 = reinterpret_cast<const float4 *>(m.E + (size_t)v0 * 3 * KP);
+#pragma unroll 4
+        for (int i = tid; i < nrow * Q; i += 256) {
+            const int r = Q > 1 ? (int)__umulhi((uint32_t)i, mq) : i, k = 4 * (i - r * Q);
+            const float4 e = __ldg(e4 + i);
+            double *o = Es + (size_t)r * W + k;
+            o[0] = e.x; o[1] = e.y; o[2] = e.z; o[3] = e.w;
+        }
+        // lanes take frames, so that the transposed coefficients are stored side by side
+        for (int fl = tid % NF; fl < NF; fl += 256) {
+            const float *xr = x + (size_t)min(f0 + fl, F - 1) * KT;
+#pragma unroll 4
+            for (int k = tid / NF; k < K; k += 256 / NF) Xs[(size_t)k * NF + fl] = (double)xr[k];
+        }
     }
     __syncthreads();
-    const int vl = tid & 31, fg = tid >> 5, v = v0 + vl;
     if (f0 + fg * FPT >= F || v >= m.V) return;
     const double *e0 = Es + (size_t)vl * 3 * W, *e1 = e0 + W, *e2 = e1 + W, *xk = Xs + fg * FPT;
     double acc[FPT][3];
@@ -236,104 +246,104 @@ __device__ __forceinline__ AdjCorner adj_corner(const AdjFrame &a, int v)
 
 // The image of one frame in FP64 and its loss, one block per frame, the region around the fragments
 // (their box + 8 px; beyond it the render is zero and the target does not reach a fragment's
-// gradient) in shared memory, in the layout of the fit's render: A [rw][pb + 2 RPAD] with zero
-// columns left and right, B [KRAD + rw + KRAD][pb] with zero lines above and below.
-//   shading of the owner fragments painted into a zero image (fill_diffuse_component...,
-//   newfuncs.cu:18-167, fill_tex_im1, funcs.cu:800-817), the 15-tap blur, the gradients of render
+// gradient) in shared memory with zero lines and columns around it:
+//   the owner fragments' values painted into a zero image (fill_tex_im1, funcs.cu:800-817), the
+//   15-tap blur, the gradients of render
 //   and target at every fragment (fill_grads, funcs.cu:842-897), the loss; with BACK the adjoint of
 //   the gradients scattered into dL/d(blurred image), the transposed blur, and dL/d(pixel value)
 //   of every fragment's pixel out in dI.
-constexpr int AI_THREADS = 1024;
+// Both blur passes work in place (a thread's inputs are in registers before any output of its lines is
+// written), so that one FP64 buffer of the region suffices: a face's region of up to 150 x 150 fits.
+constexpr int AI_THREADS = 512;
 constexpr int AI_SMEM = 216 * 1024;
-constexpr size_t AI_GLOBAL = 2 * (size_t)DIM * (DIM + 2 * RPAD);   // doubles of a frame's region that does not fit
-constexpr int AI_RUN_Y = 5, AI_RUN_X = 4;                          // blur outputs per thread along the taps
+constexpr size_t AI_GLOBAL = (size_t)(DIM + 2 * KRAD) * (DIM + 2 * RPAD);   // doubles of a region that does not fit
+constexpr int AI_RUN_Y = 5;                            // row pass: outputs per lane (odd: lanes on distinct banks)
+constexpr int AI_CHUNK = 32 * AI_RUN_Y;                // outputs of a line per warp and chunk; two chunks cover the crop
+constexpr int AI_RUN_X = 16;                           // column pass: outputs per thread
+static_assert(2 * AI_CHUNK >= DIM, "row pass covers a line in two chunks");
 
-struct RegionD {
-    int rx0, ry0, rw, rh, pb, ph;
-    double *A, *B;
-    __device__ __forceinline__ int at(int p) const { return ((p >> 8) - rx0) * ph + RPAD + ((p & 255) - ry0); }
-    __device__ __forceinline__ int bt(int p) const { return (KRAD + (p >> 8) - rx0) * pb + ((p & 255) - ry0); }
+struct RegionD {                                       // [KRAD + rw + KRAD][ph], the image at (KRAD + x, RPAD + y)
+    int rx0, ry0, rw, rh, ph;
+    double *A;
+    __device__ __forceinline__ int at(int p) const { return (KRAD + (p >> 8) - rx0) * ph + RPAD + ((p & 255) - ry0); }
 };
 
-// along y: A -> B
+// along y: a warp per line
 __device__ __forceinline__ void adj_blur_rows(const RegionD &r, const double (&tap)[NTAPS])
 {
-    const int nrun = (r.rh + AI_RUN_Y - 1) / AI_RUN_Y;
-    for (int i = threadIdx.x; i < r.rw * nrun; i += AI_THREADS) {
-        const int xl = i / nrun, y0 = min((i - xl * nrun) * AI_RUN_Y, r.rh - AI_RUN_Y);
-        const double *a = r.A + xl * r.ph + RPAD - KRAD + y0;
-        double s[AI_RUN_Y];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const bool two = r.rh > AI_CHUNK;
+    for (int xl = warp; xl < r.rw; xl += AI_THREADS / 32) {
+        double *line = r.A + (KRAD + xl) * r.ph + RPAD;
+        double s[2][AI_RUN_Y];
 #pragma unroll
-        for (int o = 0; o < AI_RUN_Y; ++o) s[o] = 0.0;
+        for (int h = 0; h < 2; ++h) {
+            const int y0 = h * AI_CHUNK + lane * AI_RUN_Y;
 #pragma unroll
-        for (int t = 0; t < AI_RUN_Y + 2 * KRAD; ++t) {
-            const double v = a[t];
+            for (int o = 0; o < AI_RUN_Y; ++o) s[h][o] = 0.0;
+            if (h == 0 ? y0 < r.rh : two && y0 < r.rh) {
 #pragma unroll
-            for (int o = 0; o < AI_RUN_Y; ++o)
-                if (t >= o && t - o <= 2 * KRAD) s[o] = fma(tap[t - o], v, s[o]);
+                for (int t = 0; t < AI_RUN_Y + 2 * KRAD; ++t) {
+                    // (a run that reaches past the line's padding reads zeros instead)
+                    const double v = y0 + t - KRAD < r.rh + RPAD ? line[y0 + t - KRAD] : 0.0;
+#pragma unroll
+                    for (int o = 0; o < AI_RUN_Y; ++o)
+                        if (t >= o && t - o <= 2 * KRAD) s[h][o] = fma(tap[t - o], v, s[h][o]);
+                }
+            }
         }
+        __syncwarp();
 #pragma unroll
-        for (int o = 0; o < AI_RUN_Y; ++o) r.B[(KRAD + xl) * r.pb + y0 + o] = s[o];
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int o = 0; o < AI_RUN_Y; ++o) {
+                const int y = h * AI_CHUNK + lane * AI_RUN_Y + o;
+                if (y < r.rh) line[y] = s[h][o];
+            }
     }
     __syncthreads();
 }
 
-// along x: B -> A
+// along x: a thread per column and segment, all segments of a column in the same step
 __device__ __forceinline__ void adj_blur_cols(const RegionD &r, const double (&tap)[NTAPS])
 {
-    const int nrun = (r.rw + AI_RUN_X - 1) / AI_RUN_X;
-    for (int i = threadIdx.x; i < r.rh * nrun; i += AI_THREADS) {
-        const int g = i / r.rh, yl = i - g * r.rh, x0 = min(g * AI_RUN_X, r.rw - AI_RUN_X);
-        const double *bp = r.B + x0 * r.pb + yl;
+    const int nseg = (r.rw + AI_RUN_X - 1) / AI_RUN_X, ncol = AI_THREADS / nseg;
+    const int seg = threadIdx.x / ncol, yl = threadIdx.x - seg * ncol, x0 = seg * AI_RUN_X;
+    for (int y0 = 0; y0 < r.rh; y0 += ncol) {
+        const bool live = seg < nseg && y0 + yl < r.rh;
+        double *col = r.A + x0 * r.ph + RPAD + y0 + yl;    // col[t ph]: the image at x0 - KRAD + t
         double s[AI_RUN_X];
+        if (live) {
 #pragma unroll
-        for (int o = 0; o < AI_RUN_X; ++o) s[o] = 0.0;
+            for (int o = 0; o < AI_RUN_X; ++o) s[o] = 0.0;
 #pragma unroll
-        for (int t = 0; t < AI_RUN_X + 2 * KRAD; ++t) {
-            const double v = bp[t * r.pb];
+            for (int t = 0; t < AI_RUN_X + 2 * KRAD; ++t) {
+                const double v = x0 + t < r.rw + 2 * KRAD ? col[t * r.ph] : 0.0;
+#pragma unroll
+                for (int o = 0; o < AI_RUN_X; ++o)
+                    if (t >= o && t - o <= 2 * KRAD) s[o] = fma(tap[t - o], v, s[o]);
+            }
+        }
+        __syncthreads();
+        if (live) {
 #pragma unroll
             for (int o = 0; o < AI_RUN_X; ++o)
-                if (t >= o && t - o <= 2 * KRAD) s[o] = fma(tap[t - o], v, s[o]);
+                if (x0 + o < r.rw) col[(KRAD + o) * r.ph] = s[o];
         }
-#pragma unroll
-        for (int o = 0; o < AI_RUN_X; ++o) r.A[(x0 + o) * r.ph + RPAD + yl] = s[o];
     }
     __syncthreads();
 }
 
-template <bool BACK>
-__global__ void __launch_bounds__(AI_THREADS, 1) k_adj_image(DModel m, DBatch b, Cfg c, const float *x, const float *lam,
-                                                             const float *Lint, const double *geo64, const double *R64,
-                                                             const float *target, double *region, double *grads,
-                                                             const double *gloss, double *loss, double *dI)
+// FP64 shading of the owner fragments (fill_diffuse_component..., newfuncs.cu:18-167), one value per
+// fragment: 13 scattered loads each, so spread over the SMs instead of the image kernel's one block
+// per frame (where they took 26 us of its 46).
+__global__ void __launch_bounds__(AD_THREADS) k_adj_shade(DModel m, DBatch b, const float *x, const float *lam,
+                                                          const float *Lint, const double *geo64, const double *R64,
+                                                          double *shade)
 {
-    extern __shared__ __align__(16) double ais[];
-    __shared__ double s_red[AI_THREADS / 32];
-    __shared__ double s_q[3];
-    const int f = blockIdx.x, tid = threadIdx.x;
+    const int f = blockIdx.y;
     const AdjFrame a = adj_frame(m, b, x, lam, Lint, geo64, R64, f);
-    const int N = a.N;
-    if (N == 0) {
-        if (tid == 0 && loss) loss[f] = 0.0;
-        return;
-    }
-    const Region rf = make_region(b.ctl[f], nullptr, nullptr);
-    RegionD r{rf.rx0, rf.ry0, rf.rw, rf.rh, rf.pb, rf.ph, nullptr, nullptr};
-    const size_t need = (size_t)r.rw * r.ph + (size_t)(r.rw + 2 * KRAD) * r.pb;
-    r.A = need * sizeof(double) <= AI_SMEM ? ais : region + (size_t)f * AI_GLOBAL;
-    r.B = r.A + (size_t)r.rw * r.ph;
-    double tap[NTAPS];
-#pragma unroll
-    for (int j = 0; j < NTAPS; ++j) tap[j] = (double)c.taps[2 * KRAD - j];
-    auto clear = [&](double *p, int n) { for (int i = tid; i < n; i += AI_THREADS) p[i] = 0.0; };
-    clear(r.A, (int)need);                               // A and B, zero lines included
-    if (tid < 3) {
-        double q = 0.0;
-        for (int j = 0; j < 3; ++j) q += a.R[3 * tid + j] * ((double)a.lam[j] - (double)a.x[a.K + j]);
-        s_q[tid] = q;
-    }
-    __syncthreads();
-    for (int n = tid; n < N; n += AI_THREADS) {
+    for (int n = blockIdx.x * AD_THREADS + threadIdx.x; n < a.N; n += gridDim.x * AD_THREADS) {
         const Fragment fr = a.fr[n];
         if (!(fr.pix_owner >> 31)) continue;
         const int pix = fr.pix_owner & 0xFFFF;
@@ -347,9 +357,46 @@ __global__ void __launch_bounds__(AI_THREADS, 1) k_adj_image(DModel m, DBatch b,
         nr[0] = v[1] * w[2] - v[2] * w[1]; nr[1] = v[2] * w[0] - v[0] * w[2]; nr[2] = v[0] * w[1] - v[1] * w[0];
         const double nn = sqrt(nr[0] * nr[0] + nr[1] * nr[1] + nr[2] * nr[2]);
         double Id = 0.0;
-        for (int k = 0; k < 3; ++k) Id += nr[k] / nn * (s_q[k] - (cb.P[k] * al + cc.P[k] * be + ca.P[k] * gm));
+        for (int k = 0; k < 3; ++k) {
+            double q = 0.0;
+            for (int j = 0; j < 3; ++j) q += a.R[3 * k + j] * ((double)a.lam[j] - (double)a.x[m.K + j]);
+            Id += nr[k] / nn * (q - (cb.P[k] * al + cc.P[k] * be + ca.P[k] * gm));
+        }
         const double t = (double)m.tex[tq.x] * al + (double)m.tex[tq.y] * be + (double)m.tex[tq.z] * gm;
-        r.A[r.at(pix)] = t + (double)a.L * t * Id;
+        shade[(size_t)f * NMAX + n] = t + (double)a.L * t * Id;
+    }
+}
+
+template <bool BACK>
+__global__ void __launch_bounds__(AI_THREADS, 1) k_adj_image(DBatch b, Cfg c, const double *shade,
+                                                             const float *target, double *region, double *grads,
+                                                             const double *gloss, double *loss, double *dI)
+{
+    extern __shared__ __align__(16) double ais[];
+    __shared__ double s_red[AI_THREADS / 32];
+    const int f = blockIdx.x, tid = threadIdx.x;
+    const int N = b.ctl[f].N;
+    const Fragment *frs = b.frag + (size_t)f * NMAX;
+    if (N == 0) {
+        if (tid == 0 && loss) loss[f] = 0.0;
+        return;
+    }
+    const Region rf = make_region(b.ctl[f], nullptr, nullptr);
+    RegionD r{rf.rx0, rf.ry0, rf.rw, rf.rh, rf.ph, nullptr};
+    const size_t need = (size_t)(r.rw + 2 * KRAD) * r.ph;
+    r.A = need * sizeof(double) <= AI_SMEM ? ais : region + (size_t)f * AI_GLOBAL;
+    double tap[NTAPS];
+#pragma unroll
+    for (int j = 0; j < NTAPS; ++j) tap[j] = (double)c.taps[2 * KRAD - j];
+    auto clear = [&](double *p, int n) { for (int i = tid; i < n; i += AI_THREADS) p[i] = 0.0; };
+    clear(r.A, (int)need);                               // the zero lines and columns stay zero
+    __syncthreads();
+    const double *sh = shade + (size_t)f * NMAX;
+#pragma unroll 4
+    for (int n = tid; n < N; n += AI_THREADS) {
+        const uint32_t po = frs[n].pix_owner;
+        const double v = sh[n];
+        if (po >> 31) r.A[r.at(po & 0xFFFF)] = v;
     }
     __syncthreads();
     adj_blur_rows(r, tap);
@@ -358,7 +405,7 @@ __global__ void __launch_bounds__(AI_THREADS, 1) k_adj_image(DModel m, DBatch b,
     double *gr = grads + (size_t)f * 2 * NMAX;
     for (int n = tid; n < N; n += AI_THREADS) {
         int kr, kl, kd, ku;
-        neighbour_pixels((int)(a.fr[n].pix_owner & 0xFFFF), kr, kl, kd, ku);
+        neighbour_pixels((int)(frs[n].pix_owner & 0xFFFF), kr, kl, kd, ku);
         gr[n] = 0.5 * (r.A[r.at(kr)] - r.A[r.at(kl)]);
         gr[NMAX + n] = 0.5 * (r.A[r.at(kd)] - r.A[r.at(ku)]);
     }
@@ -366,20 +413,16 @@ __global__ void __launch_bounds__(AI_THREADS, 1) k_adj_image(DModel m, DBatch b,
     const float *tg = target + (size_t)f * NPIX;
     for (int i = tid; i < r.rw * r.rh; i += AI_THREADS) {
         const int xl = i / r.rh, yl = i - xl * r.rh;
-        r.A[xl * r.ph + RPAD + yl] = (double)tg[(r.rx0 + xl) * DIM + r.ry0 + yl];
+        r.A[(KRAD + xl) * r.ph + RPAD + yl] = (double)tg[(r.rx0 + xl) * DIM + r.ry0 + yl];
     }
     __syncthreads();
     adj_blur_rows(r, tap);
     adj_blur_cols(r, tap);
-    if (BACK) {
-        clear(r.B + KRAD * r.pb, r.rw * r.pb);           // dL/d(blurred image) is collected here
-        __syncthreads();
-    }
     double part = 0.0;
     const double gl = BACK ? gloss[f] : 0.0;
     for (int n = tid; n < N; n += AI_THREADS) {
         int kr, kl, kd, ku;
-        neighbour_pixels((int)(a.fr[n].pix_owner & 0xFFFF), kr, kl, kd, ku);
+        neighbour_pixels((int)(frs[n].pix_owner & 0xFFFF), kr, kl, kd, ku);
         const double gx = gr[n], gy = gr[NMAX + n];
         const double rr = sqrt(4.0 * gx * gx + 4.0 * gy * gy), h = 1e-16 + rr;
         const double sx = 0.5 * (r.A[r.at(kr)] - r.A[r.at(kl)]), sy = 0.5 * (r.A[r.at(kd)] - r.A[r.at(ku)]);
@@ -392,10 +435,8 @@ __global__ void __launch_bounds__(AI_THREADS, 1) k_adj_image(DModel m, DBatch b,
             const double hx = 4.0 * gx * dh, hy = 4.0 * gy * dh;     // dh/dgx, dh/dgy
             const double dgx = dgxn * (2.0 / h - 2.0 * gx * hx / (h * h)) + dgyn * (-2.0 * gy * hx / (h * h));
             const double dgy = dgxn * (-2.0 * gx * hy / (h * h)) + dgyn * (2.0 / h - 2.0 * gy * hy / (h * h));
-            atomicAdd(r.B + r.bt(kr), 0.5 * dgx);
-            atomicAdd(r.B + r.bt(kl), -0.5 * dgx);
-            atomicAdd(r.B + r.bt(kd), 0.5 * dgy);
-            atomicAdd(r.B + r.bt(ku), -0.5 * dgy);
+            gr[n] = 0.5 * dgx;                           // in place of the render's gradient
+            gr[NMAX + n] = 0.5 * dgy;
         }
     }
     if (loss) {
@@ -403,19 +444,31 @@ __global__ void __launch_bounds__(AI_THREADS, 1) k_adj_image(DModel m, DBatch b,
         if ((tid & 31) == 0) s_red[tid >> 5] = part;
         __syncthreads();
         if (tid < 32) {
-            const double t = wsum(s_red[tid]);
+            const double t = wsum(tid < AI_THREADS / 32 ? s_red[tid] : 0.0);
             if (tid == 0) loss[f] = t;
         }
     }
     if (!BACK) return;
     __syncthreads();
-    // transposed blur: the column pass first, then the row pass (A's zero columns are still zero)
+    // dL/d(blurred image), then the transposed blur: the column pass first, then the row pass
+    clear(r.A, (int)need);
+    __syncthreads();
+    for (int n = tid; n < N; n += AI_THREADS) {
+        int kr, kl, kd, ku;
+        neighbour_pixels((int)(frs[n].pix_owner & 0xFFFF), kr, kl, kd, ku);
+        const double dgx = gr[n], dgy = gr[NMAX + n];
+        atomicAdd(r.A + r.at(kr), dgx);
+        atomicAdd(r.A + r.at(kl), -dgx);
+        atomicAdd(r.A + r.at(kd), dgy);
+        atomicAdd(r.A + r.at(ku), -dgy);
+    }
+    __syncthreads();
     adj_blur_cols(r, tap);
     adj_blur_rows(r, tap);
     double *out = dI + (size_t)f * NMAX;
     for (int n = tid; n < N; n += AI_THREADS) {
-        const uint32_t po = a.fr[n].pix_owner;
-        out[n] = (po >> 31) ? r.B[r.bt(po & 0xFFFF)] : 0.0;
+        const uint32_t po = frs[n].pix_owner;
+        out[n] = (po >> 31) ? r.A[r.at(po & 0xFFFF)] : 0.0;
     }
 }
 
@@ -527,7 +580,7 @@ __global__ void __launch_bounds__(AD_THREADS) k_adj_frag_back(DModel m, DBatch b
 // share of one frame's fragments, a thread four columns of every FL-th fragment (nine 16-byte
 // basis loads in flight); the block's sums are added with one atomic per column. Bound by the
 // basis rows' reads (2.8 KB per fragment, mostly from L2) and the conversions to FP64.
-constexpr int AE_THREADS = 256, AE_CH = 64, AE_PARTS = 16;
+constexpr int AE_THREADS = 256, AE_CH = 64;
 
 __global__ void __launch_bounds__(AE_THREADS) k_adj_eps(DModel m, DBatch b, const double *dP0, double *geps)
 {

@@ -1272,7 +1272,7 @@ tdi_status tdi_batch_landmark_init(tdi_batch *b, const float *p0L, int32_t *succ
 
 // Working set of the differentiable loss for cap frames, carved from one FP64 allocation.
 struct AdjBufs {
-    double *geo, *R, *region, *grads, *dI, *dP0, *glob, *geps;
+    double *geo, *R, *region, *grads, *dI, *dP0, *glob, *geps;   // dI: the shading values before the adjoint
 };
 
 static tdi_status adj_bufs(tdi_batch *b, AdjBufs &o)
@@ -1295,7 +1295,8 @@ static tdi_status adj_bufs(tdi_batch *b, AdjBufs &o)
 }
 
 // The raster at the caller's states and the FP64 geometry (the forward of the loss and of its adjoint).
-static tdi_status adj_forward(tdi_batch *b, const Cfg &c, const float *x, cudaStream_t s, AdjBufs &o)
+static tdi_status adj_forward(tdi_batch *b, const Cfg &c, const float *x, const float *lam, const float *L,
+                              cudaStream_t s, AdjBufs &o)
 {
     const DModel &m = b->m->d;
     DBatch &d = b->d;
@@ -1323,7 +1324,8 @@ static tdi_status adj_forward(tdi_batch *b, const Cfg &c, const float *x, cudaSt
         TDI_TRY(launch(b, 0, k_adj_vertex_tiled<1>, dim3(vb.x, (F + 7) / 8), dim3(256), adj_vertex_smem(m.KP, 1), s, m, x, F, o.geo));
     else
         TDI_TRY(launch(b, 0, k_adj_vertex, dim3((m.V + 255) / 256, F), dim3(256), 0, s, m, x, F, o.geo));
-    return TDI_OK;
+    return launch(b, 0, k_adj_shade, dim3(16, F), dim3(AD_THREADS), 0, s, m, (const DBatch)d, x, lam, L,
+                  (const double *)o.geo, (const double *)o.R, o.dI);
 }
 
 tdi_status tdi_batch_loss(tdi_batch *b, const tdi_fit_config *cfg, const float *x, const float *lam, const float *L,
@@ -1334,10 +1336,10 @@ tdi_status tdi_batch_loss(tdi_batch *b, const tdi_fit_config *cfg, const float *
     cudaStream_t s = (cudaStream_t)stream;
     const Cfg c = to_cfg(*cfg);
     AdjBufs o;
-    TDI_TRY(adj_forward(b, c, x, s, o));
-    return launch(b, 0, k_adj_image<false>, dim3(b->d.F), dim3(AI_THREADS), (size_t)AI_SMEM, s, b->m->d, b->d, c, x, lam, L,
-                  (const double *)o.geo, (const double *)o.R, (const float *)b->target_raw, o.region, o.grads,
-                  (const double *)nullptr, loss, (double *)nullptr);
+    TDI_TRY(adj_forward(b, c, x, lam, L, s, o));
+    return launch(b, 0, k_adj_image<false>, dim3(b->d.F), dim3(AI_THREADS), (size_t)AI_SMEM, s, (const DBatch)b->d, c,
+                  (const double *)o.dI, (const float *)b->target_raw, o.region, o.grads, (const double *)nullptr, loss,
+                  (double *)nullptr);
 }
 
 tdi_status tdi_batch_loss_backward(tdi_batch *b, const tdi_fit_config *cfg, const float *x, const float *lam,
@@ -1350,15 +1352,16 @@ tdi_status tdi_batch_loss_backward(tdi_batch *b, const tdi_fit_config *cfg, cons
     const DModel &m = b->m->d;
     const Cfg c = to_cfg(*cfg);
     AdjBufs o;
-    TDI_TRY(adj_forward(b, c, x, s, o));           // recomputed: nothing is kept from the forward call
+    TDI_TRY(adj_forward(b, c, x, lam, L, s, o));   // recomputed: nothing is kept from the forward call
     const int F = b->d.F;
     TDI_CUDA(cudaMemsetAsync(o.glob, 0, (size_t)((o.geps - o.glob) + (size_t)F * m.K) * sizeof(double), s));
-    TDI_TRY(launch(b, 0, k_adj_image<true>, dim3(F), dim3(AI_THREADS), (size_t)AI_SMEM, s, m, b->d, c, x, lam, L,
-                   (const double *)o.geo, (const double *)o.R, (const float *)b->target_raw, o.region, o.grads, gloss,
-                   (double *)nullptr, o.dI));
+    TDI_TRY(launch(b, 0, k_adj_image<true>, dim3(F), dim3(AI_THREADS), (size_t)AI_SMEM, s, (const DBatch)b->d, c,
+                   (const double *)o.dI, (const float *)b->target_raw, o.region, o.grads, gloss, (double *)nullptr, o.dI));
     TDI_TRY(launch(b, 0, k_adj_frag_back, dim3(16, F), dim3(AD_THREADS), 0, s, m, (const DBatch)b->d, x, lam, L,
                    (const double *)o.geo, (const double *)o.R, (const double *)o.dI, o.dP0, o.glob));
-    TDI_TRY(launch(b, 0, k_adj_eps, dim3(AE_PARTS, F), dim3(AE_THREADS),
+    // 16 blocks per frame, or up to one per 64 fragments of a face while the frames do not fill the SMs
+    const int eparts = std::max(16, std::min(64, 4 * sm_count() / F));
+    TDI_TRY(launch(b, 0, k_adj_eps, dim3(eparts, F), dim3(AE_THREADS),
                    (size_t)(AE_THREADS / (m.KP >> 2)) * m.KP * sizeof(double), s, m, (const DBatch)b->d,
                    (const double *)o.dP0, o.geps));
     TDI_TRY(launch(b, 0, k_adj_final, dim3(F), dim3(96), 0, s, m, (const double *)o.R, (const double *)o.glob,

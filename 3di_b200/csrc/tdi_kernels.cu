@@ -849,11 +849,13 @@ __device__ __forceinline__ bool no_sample_inside(float bx, float by, float cx, f
     return dom && g > RC_GAP && shape;
 }
 
-// Blocks per frame for rc rendering frames, and the largest grid up to `frames` of them can ask for.
-__host__ __device__ __forceinline__ int raster_parts(int rc)
+// Blocks per frame for rc rendering frames of T triangles (a block has at least one per thread), and
+// the largest grid that up to `frames` of them can ask for.
+__host__ __device__ __forceinline__ int raster_parts(int rc, int T)
 {
-    const int p = RD_SPREAD / rc;
-    return p < RD_BLOCKS ? RD_BLOCKS : p > RD_MAX_BLOCKS ? RD_MAX_BLOCKS : p;
+    const int p = RD_SPREAD / rc, most = T < RD_THREADS * RD_MAX_BLOCKS ? (T + RD_THREADS - 1) / RD_THREADS : RD_MAX_BLOCKS;
+    const int q = p < RD_BLOCKS ? RD_BLOCKS : p;
+    return q > most ? most : q;
 }
 inline int raster_grid(int frames)
 {
@@ -880,7 +882,7 @@ __global__ void __launch_bounds__(RD_THREADS) k_raster_depth(DModel m, DBatch b)
     // the blocks are split between the frames that render: RD_BLOCKS each, or more when few do
     const int rc = render_n(b);
     if (rc == 0) return;
-    const int parts = raster_parts(rc);
+    const int parts = raster_parts(rc, m.T);
     const int fi = blockIdx.x / parts, part = blockIdx.x - fi * parts;
     if (fi >= rc) return;
     const int f = b.rlist[fi];
@@ -939,11 +941,11 @@ __global__ void __launch_bounds__(RD_THREADS) k_raster_depth(DModel m, DBatch b)
                                    });
         if (nf && !(B.z > 0.0f)) flags |= FLAG_OUT_OF_DOMAIN;
     };
-    for (int base = s_begin + warp * 32 * RD_ILP; base < s_end; base += RD_THREADS * RD_ILP) {
+    for (int base = s_begin + (int)threadIdx.x; base - lane < s_end; base += RD_THREADS * RD_ILP) {
         int4 tq[RD_ILP];
         float4 pb[RD_ILP], pc[RD_ILP], pa[RD_ILP];
 #pragma unroll
-        for (int h = 0; h < RD_ILP; ++h) tq[h] = __ldg(m.tlo4 + min(base + 32 * h + lane, T - 1));
+        for (int h = 0; h < RD_ILP; ++h) tq[h] = __ldg(m.tlo4 + min(base + RD_THREADS * h, T - 1));
 #pragma unroll
         for (int h = 0; h < RD_ILP; ++h) {
             pb[h] = __ldg(pj + tq[h].x);
@@ -952,13 +954,13 @@ __global__ void __launch_bounds__(RD_THREADS) k_raster_depth(DModel m, DBatch b)
         }
 #pragma unroll
         for (int h = 0; h < RD_ILP; ++h) {
-            const bool take = base + 32 * h + lane < s_end &&
+            const bool take = base + RD_THREADS * h < s_end &&
                               !no_sample_inside(pb[h].x, pb[h].y, pc[h].x, pc[h].y, pa[h].x, pa[h].y);
             const unsigned msk = __ballot_sync(0xffffffffu, take);
             if (take) {
                 const int e = queued + __popc(msk & ((1u << lane) - 1u));
                 qa[e] = make_float4(pb[h].x, pb[h].y, pc[h].x, pc[h].y);
-                qb[e] = make_float4(pa[h].x, pa[h].y, pb[h].z, __int_as_float(base + 32 * h + lane));
+                qb[e] = make_float4(pa[h].x, pa[h].y, pb[h].z, __int_as_float(base + RD_THREADS * h));
             }
             queued += __popc(msk);
         }
