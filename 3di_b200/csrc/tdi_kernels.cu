@@ -713,26 +713,6 @@ __device__ __forceinline__ int tri_samples(float bx, float by, float cx, float c
     return ridx;
 }
 
-// Fragments of triangle idx into arrays, corners fetched through fetch(v) -> float2.
-template <class Fetch>
-__device__ __forceinline__ int tri_fragments_t(const DModel &m, Fetch fetch, int idx, int x0, int y0,
-                                               uint16_t pix[NTMP], float al[NTMP], float be[NTMP],
-                                               uint32_t &flags)
-{
-    const int T = m.T;
-    const float2 pb = fetch(m.tl[idx]), pc = fetch(m.tl[T + idx]), pa = fetch(m.tl[2 * T + idx]);
-    return tri_samples(pb.x, pb.y, pc.x, pc.y, pa.x, pa.y, x0, y0, flags,
-                       [&](int r, uint32_t px, float a, float b) { pix[r] = (uint16_t)px; al[r] = a; be[r] = b; });
-}
-
-// projections as separate planes (caller-owned arrays)
-__device__ __forceinline__ int tri_fragments(const DModel &m, const float *xp, const float *yp,
-                                             int idx, int x0, int y0, uint16_t pix[NTMP],
-                                             float al[NTMP], float be[NTMP], uint32_t &flags)
-{
-    return tri_fragments_t(m, [&](int v) { return make_float2(xp[v], yp[v]); }, idx, x0, y0, pix, al, be, flags);
-}
-
 // The geometry terms of a fragment's shading: unit normal of its triangle and barycentric
 // point p in model coordinates, interpolated albedo t (corners b, c, a as geometry records).
 __device__ __forceinline__ void shade_geometry(const float4 &gb, const float4 &gc, const float4 &ga4, float al,
