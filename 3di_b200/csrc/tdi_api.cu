@@ -14,6 +14,8 @@
 #include "tdi_landmark.cu"
 #include "tdi_adjoint.cu"
 
+#include "tdi_stage.h"
+
 #include "../../include/tdi.h"
 
 #include <algorithm>
@@ -807,6 +809,7 @@ tdi_status tdi_batch_create(tdi_model *m, int32_t max_frames, tdi_batch **out)
 {
     if (!m || !out || max_frames <= 0) return fail(TDI_ERR_INVALID, "bad batch arguments");
     tdi_batch *b = new tdi_batch();
+    stage_pool().retain();
     b->m = m;
     b->cap = max_frames;
     cudaGetDevice(&b->device);
@@ -817,6 +820,7 @@ tdi_status tdi_batch_create(tdi_model *m, int32_t max_frames, tdi_batch **out)
         for (void *p : b->allocs) cudaFree(p);
         if (b->h_count) cudaFreeHost(b->h_count);
         delete b;
+        stage_pool().release();
         return st;
     };
     float *target, *xl, *yl, *bounds, *fs, *cam, *Lint;
@@ -886,6 +890,7 @@ tdi_status tdi_batch_destroy(tdi_batch *b)
     if (b->adj) cudaFree(b->adj);
     if (b->h_count) cudaFreeHost(b->h_count);
     delete b;
+    stage_pool().release();
     return TDI_OK;
 }
 
@@ -919,16 +924,29 @@ tdi_status tdi_batch_set_frames(tdi_batch *b, const tdi_frames *fr, void *stream
     if (fr->n_frames <= 0) return fail(TDI_ERR_INVALID, "no frames");
     if (fr->n_frames > b->cap) return fail(TDI_ERR_CAPACITY, "more frames than the batch holds");
     cudaStream_t s = (cudaStream_t)stream;
-    TDI_CUDA(cudaMemcpyAsync(b->target_raw, fr->targets, sizeof(float) * NPIX * fr->n_frames, cudaMemcpyHostToDevice, s));
+    const size_t bytes = sizeof(float) * NPIX * fr->n_frames;
+    TDI_CUDA(stage_upload({{(const char *)fr->targets, bytes, bytes, 1, (char *)b->target_raw}}, s));
     return set_frames_meta(b, fr, s);
 }
 
 // Raw video frames (video_fitter.cu:520-550, input_data.cu:32-53, camera.h:162-174): each
 // frame is rescaled by c = ref_face_size / face_size (float division), landmarks and camera
 // by c (float products), the crop origin and face size are taken from the rescaled
-// landmarks, and the crop is formed on the device (k_preprocess). Frames are staged on the
-// device in groups that fit PP_STAGE_BYTES.
+// landmarks, and the crop is formed on the device (k_preprocess). Only the part of each frame that
+// its crop samples is sent (source_window: on average less than half of a 1080p frame at face
+// sizes of 120-600 pixels), staged on the device in groups that fit PP_STAGE_BYTES.
 constexpr size_t PP_STAGE_BYTES = (size_t)256 << 20;
+
+// Source rows or columns [lo, hi] that resized positions p0 ... p0 + 255 (below n_resized) read, with a
+// position to spare on either side for the kernel's rounding of the coordinates to float. Empty
+// (hi < lo) when the crop lies outside the resized image.
+static void source_window(int p0, int n_resized, double inv, int n, int &lo, int &hi)
+{
+    const int p1 = std::min(p0 + DIM, n_resized) - 1;
+    if (p1 < p0) { lo = 0; hi = -1; return; }
+    lo = (int)std::min((double)(n - 1), std::max(0.0, std::floor((p0 + 0.5) * inv - 0.5) - 1.0));
+    hi = (int)std::max(0.0, std::min((double)(n - 1), std::floor((p1 + 0.5) * inv - 0.5) + 2.0));
+}
 
 tdi_status tdi_batch_set_video_frames(tdi_batch *b, const tdi_video_frames *fr, void *stream)
 {
@@ -982,8 +1000,24 @@ tdi_status tdi_batch_set_video_frames(tdi_batch *b, const tdi_video_frames *fr, 
     }
     for (int f0 = 0; f0 < F; f0 += group) {
         const int n = std::min(group, F - f0);
-        TDI_CUDA(cudaMemcpyAsync(b->raw_stage, fr->bgr + (size_t)f0 * fbytes, fbytes * n, cudaMemcpyHostToDevice, s));
-        for (int f = f0; f < f0 + n; ++f) pf[f].bgr = b->raw_stage + (size_t)(f - f0) * fbytes;
+        std::vector<StagePiece> pieces;
+        size_t used = 0;
+        for (int f = f0; f < f0 + n; ++f) {
+            PrepFrame &p = pf[f];
+            int c0, c1, r0, r1;
+            source_window(p.x0, p.rw, p.inv, p.width, c0, c1);
+            source_window(p.y0, p.rh, p.inv, p.height, r0, r1);
+            p.bgr = b->raw_stage;
+            if (c1 < c0 || r1 < r0) continue;            // the crop lies outside the frame: nothing is read
+            const size_t rows = (size_t)(r1 - r0 + 1), width = 3 * (size_t)(c1 - c0 + 1);
+            pieces.push_back({(const char *)fr->bgr + (size_t)f * fbytes + (size_t)r0 * fr->row_bytes + 3 * (size_t)c0,
+                              (size_t)fr->row_bytes, width, rows, (char *)b->raw_stage + used});
+            // the kernel addresses the window with the frame's own row and column numbers
+            p.row_bytes = (int64_t)width;
+            p.bgr = b->raw_stage + used - ((size_t)r0 * width + 3 * (size_t)c0);
+            used += width * rows;
+        }
+        if (!pieces.empty()) TDI_CUDA(stage_upload(pieces, s));
         TDI_CUDA(cudaMemcpyAsync(b->prep + f0, pf.data() + f0, sizeof(PrepFrame) * n, cudaMemcpyHostToDevice, s));
         TDI_TRY(launch(b, 0, k_preprocess, dim3(DIM / PP_TILE, DIM / PP_TILE, n), dim3(PP_TILE, PP_ROWS), 0, s,
                        (const PrepFrame *)(b->prep + f0), b->target_raw + (size_t)f0 * NPIX));
@@ -1508,7 +1542,9 @@ tdi_status tdi_batch_render(tdi_batch *b, float *images, int32_t *tri_map, void 
     }
     float *img = d.img;                                   // [F][NPIX] image, then [F][NPIX] map
     int32_t *map = reinterpret_cast<int32_t *>(d.img + (size_t)d.F * NPIX);
-    TDI_TRY(launch(b, 0, k_paint, dim3(1, d.F), dim3(1024), 0, s, m, (const DBatch)d, img, map));
+    TDI_CUDA(cudaMemsetAsync(img, 0, sizeof(float) * NPIX * d.F, s));
+    TDI_CUDA(cudaMemsetAsync(map, 0xFF, sizeof(int32_t) * NPIX * d.F, s));    // -1
+    TDI_TRY(launch(b, 0, k_paint, dim3(8, d.F), dim3(256), 0, s, m, (const DBatch)d, img, map));
     if (images) TDI_CUDA(cudaMemcpyAsync(images, img, sizeof(float) * NPIX * d.F, cudaMemcpyDeviceToHost, s));
     if (tri_map) TDI_CUDA(cudaMemcpyAsync(tri_map, map, sizeof(int32_t) * NPIX * d.F, cudaMemcpyDeviceToHost, s));
     TDI_CUDA(cudaStreamSynchronize(s));

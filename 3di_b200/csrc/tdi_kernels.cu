@@ -1183,47 +1183,12 @@ __global__ void __launch_bounds__(RS_THREADS) k_raster_slots(DModel m, DBatch b)
 // normalised gradients of render and target at every fragment (fill_grads, funcs.cu:842-897)
 // and the correlation sum.
 
-struct Shading {
-    float tex, Id, t, nn[3], p[3], v[3];
-};
-
 __device__ __forceinline__ void camera_coords(const float *R, const float *tau, float X0, float Y0,
                                               float Z0, float &X, float &Y, float &Z)
 {
     X = ((R[0] * X0 + R[3] * Y0) + R[6] * Z0) + tau[0];
     Y = ((R[1] * X0 + R[4] * Y0) + R[7] * Z0) + tau[1];
     Z = ((R[2] * X0 + R[5] * Y0) + R[8] * Z0) + tau[2];
-}
-
-__device__ __forceinline__ Shading shade(const DModel &m, const float4 *geo, const Fragment &fr,
-                                         const float *R, const float *tau, const float *lam,
-                                         float Lint)
-{
-    const int4 tc = __ldg(m.tl4 + fr.tri);
-    const float al = fr.al, be = fr.be, ga = (1 - fr.al) - fr.be;
-    const float4 gb = geo[tc.x], gc = geo[tc.y], ga4 = geo[tc.z];
-    const float b0x = gb.x, b0y = gb.y, b0z = gb.z;
-    const float c0x = gc.x, c0y = gc.y, c0z = gc.z;
-    const float a0x = ga4.x, a0y = ga4.y, a0z = ga4.z;
-    Shading s;
-    float t;
-    shade_geometry(gb, gc, ga4, al, be, s.nn, s.p, t);
-    const float d0 = lam[0] - tau[0], d1 = lam[1] - tau[1], d2 = lam[2] - tau[2];
-    float Id = (s.nn[0] * ((R[0] * d0 + R[1] * d1) + R[2] * d2)
-                + s.nn[1] * ((R[3] * d0 + R[4] * d1) + R[5] * d2))
-               + s.nn[2] * ((R[6] * d0 + R[7] * d1) + R[8] * d2);
-    Id = Id - ((s.nn[0] * s.p[0] + s.nn[1] * s.p[1]) + s.nn[2] * s.p[2]);
-    s.t = t;
-    s.tex = t + (Lint * t) * Id;
-    s.Id = Id;
-    float bX, bY, bZ, cX, cY, cZ, aX, aY, aZ;
-    camera_coords(R, tau, b0x, b0y, b0z, bX, bY, bZ);
-    camera_coords(R, tau, c0x, c0y, c0z, cX, cY, cZ);
-    camera_coords(R, tau, a0x, a0y, a0z, aX, aY, aZ);
-    s.v[0] = (bX * al + cX * be) + aX * ga;
-    s.v[1] = (bY * al + cY * be) + aY * ga;
-    s.v[2] = (bZ * al + cZ * be) + aZ * ga;
-    return s;
 }
 
 // Normalised central-difference gradient of one pixel from its four neighbours as
@@ -1393,7 +1358,7 @@ __device__ __forceinline__ void light_terms(const float *R, const float *tau, co
 // Owners shaded into the cleared region. Each fragment's unit normal, n . p and interpolated
 // albedo depend only on the geometry of the raster: the resolve forms them (shc, sht) for every
 // raster that renders. A render forms the rotated light once and the same FP32 operations as
-// shade(): Id = (n0 q0 + n1 q1) + n2 q2 - n.p, I = t + (L t) Id. RENDER_SU fragments per thread:
+// the reference's shading: Id = (n0 q0 + n1 q1) + n2 q2 - n.p, I = t + (L t) Id. RENDER_SU fragments per thread:
 // each one's pixel word and shading terms are loaded together.
 template <int NT>
 __device__ __forceinline__ void region_shade(const Region &r, const Fragment *frags, const float4 *shc,
@@ -2720,30 +2685,25 @@ __global__ void __launch_bounds__(LIGHT_THREADS, 1) k_light_fit(DModel m, DBatch
     }
 }
 
-// Unblurred image and owner-triangle map of every rendering frame (renderer.cu:635-696).
-__global__ void k_paint(DModel m, DBatch b, float *images, int32_t *tri_map)
+// Unblurred image and owner-triangle map of every rendering frame (renderer.cu:635-696), into a zero
+// image and a map of -1. The shading terms are the raster's (shc, sht).
+__global__ void __launch_bounds__(256) k_paint(DModel m, DBatch b, float *images, int32_t *tri_map)
 {
     const int f = blockIdx.y;
     const FrameCtl &ctl = b.ctl[f];
-    for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < NPIX; p += gridDim.x * blockDim.x) {
-        images[(size_t)f * NPIX + p] = 0.0f;
-        tri_map[(size_t)f * NPIX + p] = -1;
-    }
     if (!ctl.render) return;
-    __syncthreads();
-    // the clear above and the writes below touch disjoint work of one frame only when the
-    // grid has a single block in x; the host launches it that way
-    const float4 *geo = b.geo + (size_t)f * m.V;
-    const float *R = b.R + f * 9;
-    const float *tau = b.xe + (size_t)f * m.KTP + m.K;
-    const float *lam = b.lam + f * 4;
-    const Fragment *frags = b.frag + (size_t)f * NMAX;
-    for (int n = threadIdx.x; n < ctl.N; n += blockDim.x) {
-        const Fragment fr = frags[n];
+    float q[3];
+    light_terms(b.R + f * 9, b.xe + (size_t)f * m.KTP + m.K, b.lam + f * 4, q);
+    const float Lint = b.Lint[f];
+    const size_t n0 = (size_t)f * NMAX;
+    for (int n = blockIdx.x * 256 + threadIdx.x; n < ctl.N; n += gridDim.x * 256) {
+        const Fragment fr = b.frag[n0 + n];
         if (!(fr.pix_owner & 0x80000000u)) continue;
-        const Shading s = shade(m, geo, fr, R, tau, lam, b.Lint[f]);
+        const float4 sn = b.shc[n0 + n];
+        const float t = b.sht[n0 + n];
+        const float Id = ((sn.x * q[0] + sn.y * q[1]) + sn.z * q[2]) - sn.w;
         const int p = fr.pix_owner & 0xFFFF;
-        images[(size_t)f * NPIX + p] = s.tex;
+        images[(size_t)f * NPIX + p] = t + (Lint * t) * Id;
         tri_map[(size_t)f * NPIX + p] = fr.tri;
     }
 }
