@@ -15,8 +15,8 @@
 // while the CH_WORKERS others update the triangle, which they hold in registers (thread (tr, tc) =
 // (tid % 16, tid / 16) owns the entries (tr + 16 a, tc + 16 b)): they scale column j, subtract its
 // products from their entries, and publish column j + 1 and the diagonal entry of column
-// j + 2. One barrier per column (two with DIV, whose column is divided once into shared
-// memory). Each entry receives its updates in increasing k, the sequence of the oracle's
+// j + 2. One barrier per column (with DIV another among the workers, whose column is divided once
+// into shared memory). A pivot that is not positive is noticed at the end of its group. Each entry receives its updates in increasing k, the sequence of the oracle's
 // left-looking dot products. Entries left of the current column or above the diagonal are
 // updated too, without tests: nothing reads them again. Columns run in groups of 16, one
 // instantiation each, so that every register block has a compile-time index.
@@ -26,8 +26,8 @@
 // One 85 x 85 system with the shape solve's trial point: the pivot formed by its owner among the
 // workers and both substitutions by shuffles took 58 us; panels of 16 columns factored by one
 // warp (shuffles or shifts) 60 to 146 us, their 30 products and differences per column issue at
-// one per 3.5 cycles from a single warp and delay the chain; this form 36 us
-// (1,024 frames in one launch 253 -> 156 us).
+// one per 3.5 cycles from a single warp and delay the chain; this form 33 us
+// (1,024 frames in one launch 253 -> 143 us).
 #pragma once
 #include <cuda_runtime.h>
 
@@ -42,17 +42,41 @@ constexpr int CH_BU = 8;                    // back substitution: steps whose co
 __host__ __device__ __forceinline__ int chol_ld(int n) { return (n + 1) | 1; }
 __host__ __device__ __forceinline__ size_t chol_smem(int n, int RB)
 {
-    return ((size_t)n * chol_ld(n) + 4 * 16 * RB + 2) * sizeof(double);
+    return ((size_t)n * chol_ld(n) + 5 * 16 * RB + 3) * sizeof(double);
 }
 
 struct CholMem {
     double *Lf;      // [n][LD] the factor, column-major, row n the right-hand side
     double *raw;     // [2][16 RB] column j before its scaling, by step parity
-    double *pv;      // [16 RB] pivots (DIV) or their reciprocals
+    double *rv;      // [16 RB] reciprocal pivots
+    double *lv;      // [16 RB] pivots
     double *xs;      // [16 RB] the solution
     double *dd;      // [2] diagonal entry of the column after next, by parity
+    int *fail;       // a pivot was not positive
 };
 
+// t / l, correctly rounded, from r = 1 / l correctly rounded: two residual corrections with fused
+// multiply-adds (Markstein, "Computation of elementary functions on the IBM RISC System/6000
+// processor", 1990): the first brings the quotient within one unit in the last place, the second
+// rounds it correctly. Five dependent operations (45 cycles) instead of a division's 127. Operands
+// far from the middle of the exponent range take the division.
+__device__ __noinline__ double chol_div_any(double t, double l) { return t / l; }
+
+__device__ __forceinline__ double chol_div(double t, double l, double r)
+{
+    const double at = fabs(t);
+    const double q0 = t * r;
+    const double q1 = fma(fma(-q0, l, t), r, q0);
+    const double q = fma(fma(-q1, l, t), r, q1);
+    if (at == 0.0) return t;                             // (l > 0)
+    if (!(at > 1e-150 && at < 1e150 && l > 1e-100 && l < 1e100)) return chol_div_any(t, l);
+    return q;
+}
+
+__device__ __forceinline__ void chol_worker_barrier() { asm volatile("bar.sync 1, %0;" ::"n"(CH_WORKERS) : "memory"); }
+
+// Steps of column group J (columns 16 J ... 16 J + 15), then the next group; false when a pivot was not
+// positive (its reciprocal is then NaN or infinite, what follows it is not used).
 template <int RB, bool DIV, int J>
 __device__ __forceinline__ bool chol_group(double (&v)[RB][RB], const CholMem &cm, int n, int LD, int tid, int tr,
                                            int tc)
@@ -61,29 +85,29 @@ __device__ __forceinline__ bool chol_group(double (&v)[RB][RB], const CholMem &c
     const int jend = min(n, 16 * J + 16);
     for (int j = 16 * J; j < jend; ++j) {
         const double *rj = cm.raw + (j & 1) * 16 * RB;
-        if (!(rj[j] > 0.0)) return false;                // every thread reads the same pivot
-        const double p = cm.pv[j];
-        double *col = cm.Lf + (size_t)j * LD;
+        const double p = cm.rv[j];
         if (tid >= CH_WORKERS) {
-            if constexpr (DIV) __syncthreads();
             if (j + 1 < n) {
-                const double c = DIV ? rj[j + 1] / p : rj[j + 1] * p;
-                const double s = cm.dd[(j + 1) & 1] - c * c;
-                if (s > 0.0) {
-                    const double l = sqrt(s);
-                    const double q = DIV ? l : __drcp_rn(l);
-                    if (tid == CH_WORKERS) cm.pv[j + 1] = q;
+                const double t = rj[j + 1], d = cm.dd[(j + 1) & 1];
+                const double c = DIV ? chol_div(t, cm.lv[j], p) : t * p;
+                const double s = d - c * c;
+                const double l = sqrt(s);
+                const double r = __drcp_rn(l);
+                if (tid == CH_WORKERS) {
+                    cm.rv[j + 1] = r;
+                    if (DIV) cm.lv[j + 1] = l;
+                    if (!(s > 0.0)) *cm.fail = 1;
                 }
             }
         } else {
+            double *col = cm.Lf + (size_t)j * LD;
             double ci[RB], cl[RB];
             if constexpr (DIV) {
-                if (tid > j && tid <= n) col[tid] = rj[tid] / p;
-                __syncthreads();
+                if (tid > j && tid <= n) col[tid] = chol_div(rj[tid], cm.lv[j], p);
+                chol_worker_barrier();
 #pragma unroll
                 for (int a = J; a < RB; ++a) { ci[a] = col[tr + 16 * a]; cl[a] = col[tc + 16 * a]; }
             } else {
-                if (tid > j && tid <= n) col[tid] = rj[tid] * p;
 #pragma unroll
                 for (int a = J; a < RB; ++a) { ci[a] = rj[tr + 16 * a] * p; cl[a] = rj[tc + 16 * a] * p; }
             }
@@ -109,9 +133,18 @@ __device__ __forceinline__ bool chol_group(double (&v)[RB][RB], const CholMem &c
                 }
             }
             if (tr == tc && tr == (j2 & 15)) cm.dd[j2 & 1] = (j < 16 * J + 14 || J + 1 >= RB) ? v[J][J] : v[J + 1 < RB ? J + 1 : J][J + 1 < RB ? J + 1 : J];
+            if constexpr (!DIV) {
+                // the scaled column, for the back substitution
+                if (tc == (j & 15)) {
+#pragma unroll
+                    for (int a = J; a < RB; ++a)
+                        if (tr + 16 * a <= n) col[tr + 16 * a] = ci[a];
+                }
+            }
         }
         __syncthreads();
     }
+    if (*cm.fail) return false;
     if constexpr (J + 1 < RB) return chol_group<RB, DIV, J + 1>(v, cm, n, LD, tid, tr, tc);
     else return true;
 }
@@ -126,9 +159,11 @@ __device__ __forceinline__ bool chol_solve(int n, double *sm, A a_of, G rhs, dou
     CholMem cm;
     cm.Lf = sm;
     cm.raw = cm.Lf + (size_t)n * LD;
-    cm.pv = cm.raw + 2 * 16 * RB;
-    cm.xs = cm.pv + 16 * RB;
+    cm.rv = cm.raw + 2 * 16 * RB;
+    cm.lv = cm.rv + 16 * RB;
+    cm.xs = cm.lv + 16 * RB;
     cm.dd = cm.xs + 16 * RB;
+    cm.fail = reinterpret_cast<int *>(cm.dd + 2);
     xs = cm.xs;
     double v[RB][RB];
 #pragma unroll
@@ -136,11 +171,10 @@ __device__ __forceinline__ bool chol_solve(int n, double *sm, A a_of, G rhs, dou
 #pragma unroll
         for (int b = 0; b <= a; ++b) {
             const int i = tr + 16 * a, l = tc + 16 * b;
-            v[a][b] = 0.0;
-            if (tid < CH_WORKERS && l < n) {
-                if (i < n) { if (i >= l) v[a][b] = a_of(i, l); }
-                else if (i == n) v[a][b] = rhs(l);
-            }
+            // (clamped, so that all of a thread's loads can be in flight together)
+            const int lc = min(l, n - 1), ic = max(min(i, n - 1), lc);
+            const double e = a_of(ic, lc), g = a == n / 16 ? rhs(lc) : 0.0;
+            v[a][b] = l < n ? (i < n ? e : i == n ? g : 0.0) : 0.0;
         }
     // column 0, and the diagonal of column 1
     if (tid < CH_WORKERS) {
@@ -149,9 +183,11 @@ __device__ __forceinline__ bool chol_solve(int n, double *sm, A a_of, G rhs, dou
             for (int a = 0; a < RB; ++a) cm.raw[tr + 16 * a] = v[a][0];
         }
         if (tr == 1 && tc == 1) cm.dd[1] = v[0][0];
-        if (tid == 0 && v[0][0] > 0.0) {
+        if (tid == 0) {
             const double l = sqrt(v[0][0]);
-            cm.pv[0] = DIV ? l : __drcp_rn(l);
+            cm.lv[0] = l;
+            cm.rv[0] = __drcp_rn(l);
+            *cm.fail = !(v[0][0] > 0.0);
         }
     }
     __syncthreads();
@@ -160,12 +196,13 @@ __device__ __forceinline__ bool chol_solve(int n, double *sm, A a_of, G rhs, dou
     if (tid < 32) {
         constexpr int TQ = (RB + 1) / 2;
         const double *Lf = cm.Lf;
-        double t[TQ], po[TQ];
+        double t[TQ], po[TQ], lo[TQ];
 #pragma unroll
         for (int q = 0; q < TQ; ++q) {
             const int i = tid + 32 * q;
             t[q] = i < n ? Lf[(size_t)i * LD + n] : 0.0;
-            po[q] = i < n ? cm.pv[i] : 1.0;
+            po[q] = i < n ? cm.rv[i] : 1.0;
+            lo[q] = DIV && i < n ? cm.lv[i] : 1.0;
         }
 #pragma unroll
         for (int q = TQ - 1; q >= 0; --q) {              // unknowns 32 q + 31 ... 32 q
@@ -185,7 +222,7 @@ __device__ __forceinline__ bool chol_solve(int n, double *sm, A a_of, G rhs, dou
 #pragma unroll
                 for (int u = CH_BU - 1; u >= 0; --u) {
                     if (k0 + u >= n) continue;
-                    const double xo = DIV ? t[q] / po[q] : t[q] * po[q];     // meaningful in the owner's lane
+                    const double xo = DIV ? chol_div(t[q], lo[q], po[q]) : t[q] * po[q];     // meaningful in the owner's lane
                     const double xk = __shfl_sync(0xffffffffu, xo, u0 + u);
                     if (tid == u0 + u) cm.xs[k0 + u] = xo;
 #pragma unroll

@@ -24,7 +24,7 @@
 // chains run on the FP64 tensor cores (four rows per mma.sync, the barrier kernel's form), the
 // system through chol_solve, every logarithm in its own thread, basis rows loaded ahead of their
 // chains. One frame of two steps: 1,120 us with a thread per Hessian entry, left-looking columns and
-// the logarithms of an objective in one thread; 253 us in this form (500 frames 9.17 -> 1.54 ms).
+// the logarithms of an objective in one thread; 219 us in this form (500 frames 9.17 -> 1.33 ms).
 
 namespace tdi {
 
