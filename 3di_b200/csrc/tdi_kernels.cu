@@ -187,6 +187,25 @@ __device__ __forceinline__ float2 ffma2(float2 a, float2 b, float2 c)
     return d;
 }
 
+__device__ __forceinline__ float2 fmul2(float2 a, float2 b)
+{
+    float2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;"
+        : "=l"(reinterpret_cast<unsigned long long &>(d))
+        : "l"(reinterpret_cast<const unsigned long long &>(a)), "l"(reinterpret_cast<const unsigned long long &>(b)));
+    return d;
+}
+
+// 1 in both halves, from a zero the compiler does not know to be one. Packed products and
+// packed sums are contracted into packed fused multiply-adds by the assembler, .rn or not (measured:
+// every result equals fma's); a sum written as fma(p, 1, s) with an unknown 1 keeps the product's
+// own rounding and rounds as p + s.
+__device__ __forceinline__ float2 packed_one(int zero)
+{
+    const float u = __int_as_float(0x3f800000 | zero);
+    return make_float2(u, u);
+}
+
 constexpr int VT_V = 32;                                   // vertices per tile (one per lane)
 constexpr int VT_FPT = 8, VT_F = 8 * VT_FPT;               // frames per thread, per block (full rounds)
 constexpr int VT_FPT_SMALL = 2;                             // frames per thread when few frames render
@@ -1270,31 +1289,12 @@ __device__ __forceinline__ void region_clear(const Region &r, bool pads)
         }
 }
 
-__device__ __forceinline__ float2 fmul2(float2 a, float2 b)
-{
-    float2 d;
-    asm("mul.rn.f32x2 %0, %1, %2;"
-        : "=l"(reinterpret_cast<unsigned long long &>(d))
-        : "l"(reinterpret_cast<const unsigned long long &>(a)), "l"(reinterpret_cast<const unsigned long long &>(b)));
-    return d;
-}
-
-// 1 in both halves, from a value the compiler cannot know (normal_eq is 0 or 1). Packed products and
-// packed sums are contracted into packed fused multiply-adds by the assembler, .rn or not (measured:
-// every result equals fma's); a sum written as fma(p, 1, s) with an unknown 1 keeps the product's
-// own rounding and rounds as p + s.
-__device__ __forceinline__ float2 packed_one(const Cfg &c)
-{
-    const float u = __int_as_float(0x3f800000 | (c.normal_eq & 2));
-    return make_float2(u, u);
-}
-
 // Row pass A -> B, column pass B -> A (the shaded image in A, then the blurred one).
 template <int NT>
 __device__ __forceinline__ void region_blur(const Region &r, const Cfg &c)
 {
     const int tid = threadIdx.x;
-    const float2 one = packed_one(c);
+    const float2 one = packed_one(c.normal_eq & 2);      // (normal_eq is 0 or 1)
     float2 tap[NTAPS];                                   // tap[j]: the weight of offset j - KRAD, in both halves
 #pragma unroll
     for (int j = 0; j < NTAPS; ++j) tap[j] = make_float2(c.taps[2 * KRAD - j], c.taps[2 * KRAD - j]);
@@ -1723,14 +1723,43 @@ __global__ void __launch_bounds__(1024) k_neighbours(DBatch b, int all_frames)
 // Jacobian rows dI/dtheta (newfuncs.cu:173-299, funcs.cu:224-282). A block takes chunks of
 // JAC_CH fragments of one frame: one thread per fragment forms the interpolated point, its
 // camera coordinates and the pose columns, and leaves the per-fragment factors in shared
-// memory; then the chunk's (fragment, expression column) items are spread over all threads,
-// consecutive items being consecutive columns of a fragment, so that the three basis rows
-// are read coalesced and no lane idles on a short last pass. (Taking the chunks in pixel
-// order, so that a chunk's triangles share corners, measured 3% slower.)
+// memory (each twice, as the operand of a packed operation); then the chunk's (fragment, four
+// expression columns) items are spread over all threads, consecutive items being consecutive
+// columns of a fragment, so that the nine basis rows of an item are read in 16-byte loads,
+// coalesced and in flight together. Two columns per packed FP32 instruction, each half rounding as
+// the scalar operation (products and sums kept apart, see packed_one).
+// It was bound by issue (one column per item: 922,000 warp instructions per frame, 62% issue active,
+// 1,389 us for 1,024 frames); now by the reads of the basis rows (10.6 MB per frame, mostly L2):
+// 1,087 us (3 blocks per SM 1,153, 2 blocks 1,417). (Taking the chunks in pixel order, so that a chunk's triangles share corners, measured
+// 3% slower before.)
 
 constexpr int JAC_THREADS = 256;
 constexpr int JAC_CH = 128;                  // fragments per chunk
 constexpr int JAC_BPF = 32;                  // blocks per frame
+
+__device__ __forceinline__ float2 dup2(float v) { return make_float2(v, v); }
+
+// two columns of a Jacobian row from the basis pairs of the three corners (b, c, a; x, y, z each)
+struct JacFactors {
+    float2 al, be, ga, gx, vx, vy, vz, gy, cx, cy;
+};
+
+__device__ __forceinline__ float2 jac_pair(const float2 (&e)[3][3], const JacFactors &q, const float2 (&R)[9], float2 one,
+                                           float2 mone)
+{
+    float2 t[3];
+#pragma unroll
+    for (int j = 0; j < 3; ++j)
+        t[j] = ffma2(ffma2(fmul2(e[0][j], q.al), one, fmul2(e[1][j], q.be)), one, fmul2(e[2][j], q.ga));
+    float2 r[3];                             // (tx R[i] + ty R[3 + i]) + tz R[6 + i]
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        r[i] = ffma2(ffma2(fmul2(t[0], R[i]), one, fmul2(t[1], R[3 + i])), one, fmul2(t[2], R[6 + i]));
+    const float2 nwx = fmul2(q.cx, ffma2(fmul2(r[2], q.vx), mone, fmul2(r[0], q.vz)));
+    const float2 nwy = fmul2(q.cy, ffma2(fmul2(r[2], q.vy), mone, fmul2(r[1], q.vz)));
+    const float2 s = ffma2(fmul2(q.gx, nwx), one, fmul2(q.gy, nwy));
+    return make_float2(-s.x, -s.y);
+}
 
 __global__ void __launch_bounds__(JAC_THREADS, 4) k_jacobian(DModel m, DBatch b)
 {
@@ -1738,10 +1767,8 @@ __global__ void __launch_bounds__(JAC_THREADS, 4) k_jacobian(DModel m, DBatch b)
     const int f = b.jlist[blockIdx.y];
     const FrameCtl &ctl = b.ctl[f];
     if (blockIdx.x == 0 && threadIdx.x == 0) prof_count(b, KID_JACOBIAN);
-    __shared__ float4 s_w[JAC_CH];           // al, be, ga, gx
-    __shared__ float4 s_v[JAC_CH];           // vx, vy, vz, gy
-    __shared__ float2 s_c[JAC_CH];           // phix / vz^2, phiy / vz^2
-    __shared__ int4 s_e[JAC_CH];             // basis row offsets of b, c, a; Jacobian row offset
+    __shared__ float4 s_f[5][JAC_CH];        // factor pairs: (al, be), (ga, gx), (vx, vy), (vz, gy), (cx, cy), each twice
+    __shared__ int4 s_e[JAC_CH];             // basis row offsets of b, c, a (16-byte units); Jacobian row offset
     const int N = ctl.N, K = m.K, KP = m.KP, V = m.V, KTP = m.KTP;
     const int tid = threadIdx.x;
     const float4 *geo = b.geo + (size_t)f * V;
@@ -1751,10 +1778,13 @@ __global__ void __launch_bounds__(JAC_THREADS, 4) k_jacobian(DModel m, DBatch b)
     const Fragment *frags = b.frag + (size_t)f * NMAX;
     const float *fg = b.fgrad + (size_t)f * 5 * NMAX;
     float *Jf = b.J + (size_t)f * NMAX * KTP;
-    float R[9];
+    const float2 one = packed_one(ctl.need_jac & 2), mone = make_float2(-one.x, -one.y);   // (need_jac is 1)
+    float2 R2[9];
 #pragma unroll
-    for (int i = 0; i < 9; ++i) R[i] = Rg[i];
-    const uint32_t mg = 0xFFFFFFFFu / (uint32_t)K + 1u;   // i / K = umulhi(i, mg) for i < 2^16
+    for (int i = 0; i < 9; ++i) R2[i] = dup2(Rg[i]);
+    const int Q = KP >> 2;                               // column quads of a row
+    const uint32_t mg = Q > 1 ? 0xFFFFFFFFu / (uint32_t)Q + 1u : 0u;   // i / Q = umulhi(i, mg) for i < 2^16
+    const float4 *E4 = reinterpret_cast<const float4 *>(m.E);
     for (int c0 = blockIdx.x * JAC_CH; c0 < N; c0 += gridDim.x * JAC_CH) {
         const int cnt = min(JAC_CH, N - c0);
         if (tid < cnt) {
@@ -1767,6 +1797,9 @@ __global__ void __launch_bounds__(JAC_THREADS, 4) k_jacobian(DModel m, DBatch b)
             const float px = (gb.x * al + gc.x * be) + ga4.x * ga;
             const float py = (gb.y * al + gc.y * be) + ga4.y * ga;
             const float pz = (gb.z * al + gc.z * be) + ga4.z * ga;
+            float R[9];
+#pragma unroll
+            for (int i = 0; i < 9; ++i) R[i] = R2[i].x;
             float bX, bY, bZ, cX, cY, cZ, aX, aY, aZ;
             camera_coords(R, tau, gb.x, gb.y, gb.z, bX, bY, bZ);
             camera_coords(R, tau, gc.x, gc.y, gc.z, cX, cY, cZ);
@@ -1776,10 +1809,13 @@ __global__ void __launch_bounds__(JAC_THREADS, 4) k_jacobian(DModel m, DBatch b)
             const float vz = (bZ * al + cZ * be) + aZ * ga;
             const float ivz = 1.0f / vz, ivz2 = ivz * ivz;
             const float gx = fg[n], gy = fg[NMAX + n];
-            s_w[tid] = make_float4(al, be, ga, gx);
-            s_v[tid] = make_float4(vx, vy, vz, gy);
-            s_c[tid] = make_float2(phix * ivz2, phiy * ivz2);
-            s_e[tid] = make_int4(ib * 3 * KP, ic * 3 * KP, ia * 3 * KP, n * KTP);
+            const float cx = phix * ivz2, cy = phiy * ivz2;
+            s_f[0][tid] = make_float4(al, al, be, be);
+            s_f[1][tid] = make_float4(ga, ga, gx, gx);
+            s_f[2][tid] = make_float4(vx, vx, vy, vy);
+            s_f[3][tid] = make_float4(vz, vz, gy, gy);
+            s_f[4][tid] = make_float4(cx, cx, cy, cy);
+            s_e[tid] = make_int4(ib * 3 * Q, ic * 3 * Q, ia * 3 * Q, n * KTP);
             float *row = Jf + (size_t)n * KTP;
             row[K + 0] = -(gx * (phix * ivz) + gy * 0.0f);
             row[K + 1] = -(gx * 0.0f + gy * (phiy * ivz));
@@ -1797,22 +1833,38 @@ __global__ void __launch_bounds__(JAC_THREADS, 4) k_jacobian(DModel m, DBatch b)
             for (int j = m.KT; j < KTP; ++j) row[j] = 0.0f;
         }
         __syncthreads();
-#pragma unroll 2
-        for (int i = tid; i < cnt * K; i += JAC_THREADS) {
-            const int nl = (int)__umulhi((uint32_t)i, mg), k = i - nl * K;
-            const float4 w = s_w[nl], v = s_v[nl];
-            const float2 cc = s_c[nl];
-            const int4 e = s_e[nl];
-            const float *eb = m.E + e.x + k, *ec = m.E + e.y + k, *ea = m.E + e.z + k;
-            const float tx = (__ldg(eb) * w.x + __ldg(ec) * w.y) + __ldg(ea) * w.z;
-            const float ty = (__ldg(eb + KP) * w.x + __ldg(ec + KP) * w.y) + __ldg(ea + KP) * w.z;
-            const float tz = (__ldg(eb + 2 * KP) * w.x + __ldg(ec + 2 * KP) * w.y) + __ldg(ea + 2 * KP) * w.z;
-            const float REX = (tx * R[0] + ty * R[3]) + tz * R[6];
-            const float REY = (tx * R[1] + ty * R[4]) + tz * R[7];
-            const float REZ = (tx * R[2] + ty * R[5]) + tz * R[8];
-            const float nwx = cc.x * (REX * v.z - REZ * v.x);
-            const float nwy = cc.y * (REY * v.z - REZ * v.y);
-            Jf[e.w + k] = -(w.w * nwx + v.w * nwy);
+        for (int i = tid; i < cnt * Q; i += JAC_THREADS) {
+            const int nl = Q > 1 ? (int)__umulhi((uint32_t)i, mg) : i, kq = i - nl * Q;
+            const int4 o = s_e[nl];
+            float4 e[3][3];
+#pragma unroll
+            for (int j = 0; j < 3; ++j) {
+                e[0][j] = __ldg(E4 + o.x + j * Q + kq);
+                e[1][j] = __ldg(E4 + o.y + j * Q + kq);
+                e[2][j] = __ldg(E4 + o.z + j * Q + kq);
+            }
+            const float4 f0 = s_f[0][nl], f1 = s_f[1][nl], f2 = s_f[2][nl], f3 = s_f[3][nl], f4 = s_f[4][nl];
+            const JacFactors q{make_float2(f0.x, f0.y), make_float2(f0.z, f0.w), make_float2(f1.x, f1.y),
+                               make_float2(f1.z, f1.w), make_float2(f2.x, f2.y), make_float2(f2.z, f2.w),
+                               make_float2(f3.x, f3.y), make_float2(f3.z, f3.w), make_float2(f4.x, f4.y),
+                               make_float2(f4.z, f4.w)};
+            float2 lo[3][3], hi[3][3];
+#pragma unroll
+            for (int c = 0; c < 3; ++c)
+#pragma unroll
+                for (int j = 0; j < 3; ++j) {
+                    lo[c][j] = make_float2(e[c][j].x, e[c][j].y);
+                    hi[c][j] = make_float2(e[c][j].z, e[c][j].w);
+                }
+            const float2 r0 = jac_pair(lo, q, R2, one, mone), r1 = jac_pair(hi, q, R2, one, mone);
+            float *dst = Jf + o.w + 4 * kq;
+            if (4 * kq + 3 < K) {
+                *reinterpret_cast<float4 *>(dst) = make_float4(r0.x, r0.y, r1.x, r1.y);
+            } else {                                     // the last quad: columns from K on are the pose's
+                if (4 * kq < K) dst[0] = r0.x;
+                if (4 * kq + 1 < K) dst[1] = r0.y;
+                if (4 * kq + 2 < K) dst[2] = r1.x;
+            }
         }
         __syncthreads();
     }
