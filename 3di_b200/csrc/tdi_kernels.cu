@@ -1878,14 +1878,15 @@ __global__ void __launch_bounds__(JAC_THREADS, 4) k_jacobian(DModel m, DBatch b)
 // FP64 fused multiply-add per row and entry in fragment order (x row, then y row), the chunk
 // sums then added in chunk order. The rows are floats, so every product is exact in FP64.
 // k_normal_eq writes one partial per chunk (NE_BPF blocks per frame, each looping over
-// chunks); rows are staged 32 fragments at a time in shared memory as doubles and every
-// thread owns a 4x4 block of the upper triangle. k_normal_eq_reduce adds the chunk partials.
+// chunks); rows are staged 32 fragments at a time in shared memory as doubles. k_normal_eq_reduce
+// adds the chunk partials.
 
 constexpr int NE_THREADS = 256;
 constexpr int NE_CH = 256;                   // fragments per chunk (the unit of the sum order)
 constexpr int NE_SUB = 32;                   // fragments staged in shared memory at a time
 constexpr int NE_BPF = 32;                   // blocks per frame
 constexpr int NE_MAXCH = NMAX / NE_CH;       // chunk partials per frame at most
+constexpr int NE_SPREAD = 148;               // chunks of a round up to which their tiles are split over two blocks
 static_assert(NE_THREADS == NE_CH && NE_SUB == 32 && NE_THREADS == 8 * 32, "thread mapping of the row build");
 
 // Chunk partials are sized for the widest layout the normal-equation kernels have used:
@@ -1909,9 +1910,9 @@ struct ChunkHead {
     double w[2 * NE_CH];
 };
 
-__device__ __forceinline__ void chunk_head(ChunkHead &hd, const float *fg, const int32_t *nb, int c0, int cnt)
+__device__ __forceinline__ void chunk_head(ChunkHead &hd, const float *fg, const int32_t *nb, int c0, int cnt, int q)
 {
-    const int q = threadIdx.x, n = c0 + q;
+    const int n = c0 + q;
     float pre = 0.0f, dx = 0.0f, dy = 0.0f, wx = 0.0f, wy = 0.0f;
     int k0 = 0, k1 = 0, k2 = 0, k3 = 0;
     if (q < cnt) {
@@ -1939,10 +1940,10 @@ __device__ __forceinline__ void chunk_prefetch(float (&v)[GRP][4], const ChunkHe
     for (int g = 0; g < GRP; ++g) {
         const int a = 8 * g + a_low;
         const bool use = live && a < KT;
-        v[g][0] = use ? Jf[(size_t)r0 * KTP + a] : 0.0f;
-        v[g][1] = use ? Jf[(size_t)r1 * KTP + a] : 0.0f;
-        v[g][2] = use ? Jf[(size_t)r2 * KTP + a] : 0.0f;
-        v[g][3] = use ? Jf[(size_t)r3 * KTP + a] : 0.0f;
+        v[g][0] = use ? __ldg(Jf + (size_t)r0 * KTP + a) : 0.0f;
+        v[g][1] = use ? __ldg(Jf + (size_t)r1 * KTP + a) : 0.0f;
+        v[g][2] = use ? __ldg(Jf + (size_t)r2 * KTP + a) : 0.0f;
+        v[g][3] = use ? __ldg(Jf + (size_t)r3 * KTP + a) : 0.0f;
     }
 }
 
@@ -2000,28 +2001,132 @@ __host__ __device__ constexpr NeTiles make_ne_tiles()
     return t;
 }
 
-// The tensor-core updates of warp W (tiles W, W + 8, ...) over the fragment pairs of one
-// stage: a lane loads its row's value in each of the 11 column blocks once per pair and
-// feeds every tile from those registers.
-template <int W>
-__device__ __forceinline__ void ne_pairs(double (&acc)[NE_TPW][2], const double *rows, int cn, int kr, int fr8)
+// Half of a block's warps build rows, the other half run the tensor cores, two stages of rows
+// between them (named barriers: full and empty per stage), so that the neighbour rows' gathers, the
+// chain rule and the conversions of one stage hide behind the updates of the one before. With
+// one updating warp per SM sub-partition a row value loaded once feeds 16 tiles instead of 8 (the
+// shared-memory reads were 0.67 of the tensor time). All warps building, then all updating, took 2,874 us
+// for 1,024 frames; this form 2,498 us (26.6 TFLOP/s in the tiles; the pipe gives 37 measured alone).
+// With few frames a chunk's tiles are split over NE_SPLIT blocks, each building all rows: one frame is
+// 15 chunks, and 148 SMs (38 -> 24 us).
+constexpr int NE_MMA_WARPS = 4;              // one per SM sub-partition
+constexpr int NE_BUILDERS = NE_THREADS - 32 * NE_MMA_WARPS;
+constexpr int NE_SPLIT = 2;
+constexpr int NE_FULL = 1, NE_EMPTY = 3, NE_HEAD = 5;   // named barriers: full and empty by stage, the builders' own
+
+__device__ __forceinline__ void bar_sync(int id, int n) { asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+__device__ __forceinline__ void bar_arrive(int id, int n) { asm volatile("bar.arrive %0, %1;" ::"r"(id), "r"(n) : "memory"); }
+
+// Share W of the upper triangle's tiles. For whole blocks (S = 1) the four shares are cut so that each
+// touches few of the 11 column blocks (6, 6, 9 and 8 instead of 11 each, for 17, 17, 16 and 16 tiles),
+// since every column block touched is a shared-memory read per fragment pair; split blocks take
+// every 4 S-th tile.
+__host__ __device__ constexpr int ne_share(int t, int bi, int bj, int S)
 {
+    if (S > 1) return t % (NE_MMA_WARPS * S);
+    if (bj <= 4) return 0;
+    if (bi >= 6) return 1;
+    if (bj == 5) return bi <= 1 ? 0 : bi == 2 ? 2 : 3;
+    if (bi == 5) return bj <= 7 ? 1 : 3;
+    return bi <= 2 ? 2 : 3;
+}
+constexpr int NE_SHARE = 17;                 // tiles of a share at most
+struct NeList {
+    int n, t[NE_SHARE], bi[NE_SHARE], bj[NE_SHARE];
+    unsigned used;                           // column blocks touched
+};
+__host__ __device__ constexpr NeList make_ne_list(int W, int S)
+{
+    NeList l{};
     constexpr NeTiles TT = make_ne_tiles();
-    constexpr int NT = (NE_NT8 - W + 7) / 8;
+    for (int t = 0; t < NE_NT8; ++t)
+        if (ne_share(t, TT.bi[t], TT.bj[t], S) == W) {
+            l.t[l.n] = t; l.bi[l.n] = TT.bi[t]; l.bj[l.n] = TT.bj[t];
+            l.used |= 1u << TT.bi[t] | 1u << TT.bj[t];
+            ++l.n;
+        }
+    return l;
+}
+
+// The updates of one stage's fragment pairs for the tiles of share W: a lane loads its row's value in
+// each column block of the share once per pair and feeds every tile from those registers.
+template <int W, int S>
+__device__ __forceinline__ void ne_pairs(double (&acc)[NE_SHARE][2], const double *rows, int cn, int kr, int fr8)
+{
+    constexpr NeList LS = make_ne_list(W, S);
     for (int q = 0; q + 2 <= cn; q += 2) {
         const double *rk = rows + (size_t)(2 * q + kr) * NE_PD + fr8;
         double v[NE_T8];
 #pragma unroll
-        for (int c = 0; c < NE_T8; ++c) v[c] = rk[8 * c];
+        for (int c = 0; c < NE_T8; ++c)
+            if (LS.used >> c & 1u) v[c] = rk[8 * c];
 #pragma unroll
-        for (int j = 0; j < NT; ++j) dmma_884(acc[j][0], acc[j][1], v[TT.bi[W + 8 * j]], v[TT.bj[W + 8 * j]]);
+        for (int j = 0; j < LS.n; ++j) dmma_884(acc[j][0], acc[j][1], v[LS.bi[j]], v[LS.bj[j]]);
+    }
+    // an odd last fragment: this thread's two entries of each tile, the same chain
+    if (cn & 1) {
+        const double *rx = rows + (size_t)(2 * (cn - 1)) * NE_PD, *ry = rx + NE_PD;
+#pragma unroll
+        for (int j = 0; j < LS.n; ++j) {
+            const int r = 8 * LS.bi[j] + fr8, c = 8 * LS.bj[j] + 2 * kr;
+#pragma unroll
+            for (int i = 0; i < 2; ++i) acc[j][i] = fma(ry[r], ry[c + i], fma(rx[r], rx[c + i], acc[j][i]));
+        }
     }
 }
 
+template <int W, int S>
+__device__ __forceinline__ void ne_update(const double *rows, double *parts, int N, int ch0, int step, int total, int lane)
+{
+    constexpr NeList LS = make_ne_list(W, S);
+    const int kr = lane & 3, fr8 = lane >> 2;            // fragment row k and tile row/column
+    int g = 0;                                           // stages so far
+    for (int ch = ch0; ch * NE_CH < N; ch += step) {
+        double acc[NE_SHARE][2];
+#pragma unroll
+        for (int j = 0; j < LS.n; ++j) acc[j][0] = acc[j][1] = 0.0;
+        const int cnt = min(N - ch * NE_CH, NE_CH), nsub = (cnt + NE_SUB - 1) / NE_SUB;
+        for (int it = 0; it < nsub; ++it, ++g) {
+            bar_sync(NE_FULL + (g & 1), NE_THREADS);
+            ne_pairs<W, S>(acc, rows + (size_t)(g & 1) * 2 * NE_SUB * NE_PD, min(NE_SUB, cnt - it * NE_SUB), kr, fr8);
+            if (g + 2 < total) bar_arrive(NE_EMPTY + (g & 1), NE_THREADS);
+        }
+        double *part = parts + (size_t)ch * (NE_NT8 * 64);
+#pragma unroll
+        for (int j = 0; j < LS.n; ++j)
+            *reinterpret_cast<double2 *>(part + LS.t[j] * 64 + fr8 * 8 + 2 * kr) = make_double2(acc[j][0], acc[j][1]);
+    }
+}
+
+// Rows of one fragment's x and y gradients at four consecutive columns a0 ... a0 + 3, from its
+// neighbours' Jacobian rows; the weight in column KT, zeros right of it.
+__device__ __forceinline__ void ne_build4(double *rx, double *ry, const float4 (&v)[4], int a0, int KT, bool live, float pre,
+                                          float diffx, float diffy, float wx, float wy)
+{
+    const float e[4][4] = {{v[0].x, v[1].x, v[2].x, v[3].x}, {v[0].y, v[1].y, v[2].y, v[3].y},
+                           {v[0].z, v[1].z, v[2].z, v[3].z}, {v[0].w, v[1].w, v[2].w, v[3].w}};
+    double ox[4], oy[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        float x, y;
+        chain_value(e[i], pre, diffx, diffy, x, y);
+        const bool col = live && a0 + i < KT;
+        x = col ? x : 0.0f;
+        y = col ? y : 0.0f;
+        if (live && a0 + i == KT) { x = wx; y = wy; }
+        ox[i] = (double)x;
+        oy[i] = (double)y;
+    }
+    *reinterpret_cast<double2 *>(rx) = make_double2(ox[0], ox[1]);
+    *reinterpret_cast<double2 *>(rx + 2) = make_double2(ox[2], ox[3]);
+    *reinterpret_cast<double2 *>(ry) = make_double2(oy[0], oy[1]);
+    *reinterpret_cast<double2 *>(ry + 2) = make_double2(oy[2], oy[3]);
+}
 
 __global__ void __launch_bounds__(NE_THREADS, 2) k_normal_eq(DModel m, DBatch b)
 {
-    if ((int)blockIdx.y >= jac_n(b)) return;
+    const int jn = jac_n(b);
+    if ((int)blockIdx.y >= jn) return;
     const int f = b.jlist[blockIdx.y];
     const FrameCtl &ctl = b.ctl[f];
     if (blockIdx.x == 0 && threadIdx.x == 0) prof_count(b, KID_NORMAL_EQ);
@@ -2029,84 +2134,84 @@ __global__ void __launch_bounds__(NE_THREADS, 2) k_normal_eq(DModel m, DBatch b)
     const int KTP = m.KTP, KT = m.KT;
     __shared__ ChunkHead hd;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int a_low = lane & 7, q_me = 4 * warp + (lane >> 3);
     const int N = ctl.N;
     const int nch = (N + NE_CH - 1) / NE_CH;
+    // the blocks of a frame: all of a chunk's tiles each, or half of them while the chunks of the round
+    // are fewer than half the blocks that fit (NE_SPREAD)
+    const bool split = jn * nch <= NE_SPREAD;
+    const int ch0 = split ? blockIdx.x / NE_SPLIT : blockIdx.x, half = split ? blockIdx.x % NE_SPLIT : 0;
+    const int step = split ? gridDim.x / NE_SPLIT : gridDim.x;
+    if (ch0 >= nch) return;
+    int total = 0;                                   // stages of this block
+    for (int ch = ch0; ch < nch; ch += step) total += (min(N - ch * NE_CH, NE_CH) + NE_SUB - 1) / NE_SUB;
+    if (tid < 32 * NE_MMA_WARPS) {
+        double *parts = b.ne_part + (size_t)f * NE_MAXCH * ne_part_stride8();
+        if (!split) {
+            switch (warp) {
+            case 0: ne_update<0, 1>(nesd, parts, N, ch0, step, total, lane); break;
+            case 1: ne_update<1, 1>(nesd, parts, N, ch0, step, total, lane); break;
+            case 2: ne_update<2, 1>(nesd, parts, N, ch0, step, total, lane); break;
+            default: ne_update<3, 1>(nesd, parts, N, ch0, step, total, lane); break;
+            }
+        } else {
+            switch (warp + NE_MMA_WARPS * half) {
+            case 0: ne_update<0, 2>(nesd, parts, N, ch0, step, total, lane); break;
+            case 1: ne_update<1, 2>(nesd, parts, N, ch0, step, total, lane); break;
+            case 2: ne_update<2, 2>(nesd, parts, N, ch0, step, total, lane); break;
+            case 3: ne_update<3, 2>(nesd, parts, N, ch0, step, total, lane); break;
+            case 4: ne_update<4, 2>(nesd, parts, N, ch0, step, total, lane); break;
+            case 5: ne_update<5, 2>(nesd, parts, N, ch0, step, total, lane); break;
+            case 6: ne_update<6, 2>(nesd, parts, N, ch0, step, total, lane); break;
+            default: ne_update<7, 2>(nesd, parts, N, ch0, step, total, lane); break;
+            }
+        }
+        return;
+    }
+    // a builder lane forms four columns (of every 32) of one fragment: its neighbours' rows come in
+    // 16-byte loads, all of a fragment's in flight together
+    constexpr int NG = (NE_P8 + 31) / 32, NF = NE_BUILDERS / 8;   // column groups; fragments built side by side
+    const int bt = tid - 32 * NE_MMA_WARPS, a_low = 4 * (lane & 7), q_me = 4 * (bt >> 5) + (lane >> 3);
     const float *Jf = b.J + (size_t)f * NMAX * KTP;
     const int32_t *nb = b.nb + (size_t)f * 4 * NMAX;
     const float *fg = b.fgrad + (size_t)f * 5 * NMAX;
-    const int stride = ne_part_stride8();
-    // this warp's tiles: t = warp + 8 * j
-    int tbi[NE_TPW], tbj[NE_TPW];
-#pragma unroll
-    for (int j = 0; j < NE_TPW; ++j) {
-        const int t = warp + 8 * j;
-        if (t < NE_NT8) ne_tile8(t, tbi[j], tbj[j]); else { tbi[j] = -1; tbj[j] = -1; }
-    }
-    const int kr = lane & 3, fr8 = lane >> 2;        // fragment row k and tile row/column
-    for (int ch = blockIdx.x; ch < nch; ch += gridDim.x) {
-        double acc[NE_TPW][2];
-#pragma unroll
-        for (int j = 0; j < NE_TPW; ++j) acc[j][0] = acc[j][1] = 0.0;
+    int g = 0;
+    for (int ch = ch0; ch < nch; ch += step) {
         const int c0 = ch * NE_CH, cnt = min(N, c0 + NE_CH) - c0;
         const int nsub = (cnt + NE_SUB - 1) / NE_SUB;
-        __syncthreads();                          // the previous chunk is done with hd and the rows
-        chunk_head(hd, fg, nb, c0, cnt);
-        __syncthreads();
-        for (int it = 0; it < nsub; ++it) {
-            double *rows = nesd + (size_t)(it & 1) * 2 * NE_SUB * NE_PD;
-            {
-                float v[NE_GRP][4];
-                const int ql = q_me, q = it * NE_SUB + ql;
-                chunk_prefetch<NE_GRP>(v, hd, Jf, KT, KTP, q, cnt, a_low);
-                const float pre = hd.pre[q], diffx = hd.dx[q], diffy = hd.dy[q];
-                const bool live = q < cnt;
+        bar_sync(NE_HEAD, NE_BUILDERS);              // the previous chunk's rows are built
+        for (int q = bt; q < NE_CH; q += NE_BUILDERS) chunk_head(hd, fg, nb, c0, cnt, q);
+        bar_sync(NE_HEAD, NE_BUILDERS);
+        for (int it = 0; it < nsub; ++it, ++g) {
+            double *rows = nesd + (size_t)(g & 1) * 2 * NE_SUB * NE_PD;
+            float4 v[NE_SUB / NF][NG][4];
 #pragma unroll
-                for (int g = 0; g < NE_GRP; ++g) {
-                    const int a = 8 * g + a_low;
-                    if (a >= NE_P8) continue;
-                    float ox = 0.0f, oy = 0.0f;
-                    if (live) {
-                        if (a < KT) chain_value(v[g], pre, diffx, diffy, ox, oy);
-                        else if (a == KT) { ox = (float)hd.w[2 * q]; oy = (float)hd.w[2 * q + 1]; }
+            for (int h = 0; h < NE_SUB / NF; ++h) {
+                const int q = it * NE_SUB + q_me + h * NF;
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const float *row = Jf + (size_t)hd.nb[u][q] * KTP;
+#pragma unroll
+                    for (int gg = 0; gg < NG; ++gg) {
+                        const int a = 32 * gg + a_low;
+                        v[h][gg][u] = a < KTP ? __ldg(reinterpret_cast<const float4 *>(row + a)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     }
-                    rows[(2 * ql) * NE_PD + a] = (double)ox;
-                    rows[(2 * ql + 1) * NE_PD + a] = (double)oy;
                 }
             }
-            __syncthreads();
-            const int cn = min(NE_SUB, cnt - it * NE_SUB);
-            // pairs of fragments on the tensor cores
-            switch (warp) {
-            case 0: ne_pairs<0>(acc, rows, cn, kr, fr8); break;
-            case 1: ne_pairs<1>(acc, rows, cn, kr, fr8); break;
-            case 2: ne_pairs<2>(acc, rows, cn, kr, fr8); break;
-            case 3: ne_pairs<3>(acc, rows, cn, kr, fr8); break;
-            case 4: ne_pairs<4>(acc, rows, cn, kr, fr8); break;
-            case 5: ne_pairs<5>(acc, rows, cn, kr, fr8); break;
-            case 6: ne_pairs<6>(acc, rows, cn, kr, fr8); break;
-            default: ne_pairs<7>(acc, rows, cn, kr, fr8); break;
-            }
-            // an odd last fragment: this thread's two entries of each tile, same chain
-            if (cn & 1) {
-                const int q = cn - 1;
-                const double *rx = rows + (size_t)(2 * q) * NE_PD, *ry = rx + NE_PD;
+            if (g >= 2) bar_sync(NE_EMPTY + (g & 1), NE_THREADS);
 #pragma unroll
-                for (int j = 0; j < NE_TPW; ++j) {
-                    if (tbi[j] < 0) continue;
-                    const int r = 8 * tbi[j] + fr8, c = 8 * tbj[j] + 2 * kr;
+            for (int h = 0; h < NE_SUB / NF; ++h) {
+                const int ql = q_me + h * NF, q = it * NE_SUB + ql;
+                const float pre = hd.pre[q], diffx = hd.dx[q], diffy = hd.dy[q];
+                const float wx = (float)hd.w[2 * q], wy = (float)hd.w[2 * q + 1];
 #pragma unroll
-                    for (int i = 0; i < 2; ++i)
-                        acc[j][i] = fma(ry[r], ry[c + i], fma(rx[r], rx[c + i], acc[j][i]));
+                for (int gg = 0; gg < NG; ++gg) {
+                    const int a = 32 * gg + a_low;
+                    if (a < NE_P8)
+                        ne_build4(rows + (2 * ql) * NE_PD + a, rows + (2 * ql + 1) * NE_PD + a, v[h][gg], a, KT, q < cnt, pre,
+                                  diffx, diffy, wx, wy);
                 }
             }
-        }
-        double *part = b.ne_part + ((size_t)f * NE_MAXCH + ch) * stride;
-#pragma unroll
-        for (int j = 0; j < NE_TPW; ++j) {
-            if (tbi[j] < 0) continue;
-            const int t = warp + 8 * j;
-            *reinterpret_cast<double2 *>(part + t * 64 + fr8 * 8 + 2 * kr) = make_double2(acc[j][0], acc[j][1]);
+            bar_arrive(NE_FULL + (g & 1), NE_THREADS);
         }
     }
 }

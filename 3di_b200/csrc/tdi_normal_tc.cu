@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(TC_THREADS, 3) k_normal_eq_tc(DModel m, DBatch
         const int c0 = ch * NE_CH, cnt = min(N, c0 + NE_CH) - c0;
         const int nsub = (cnt + TC_SUB - 1) / TC_SUB;
         __syncthreads();                          // the previous chunk is done with hd
-        chunk_head(hd, fg, nb, c0, cnt);
+        chunk_head(hd, fg, nb, c0, cnt, threadIdx.x);
         __syncthreads();
         for (int it = 0; it < nsub; ++it) {
             const int ql = q_me, q = it * TC_SUB + ql;
