@@ -35,6 +35,21 @@ __device__ __forceinline__ void skew(float *S, const float *u)
     S[6] = u[1]; S[7] = -u[0]; S[8] = 0;
 }
 
+// R(u) alone, by the operations of rotation() (a line search's trials need no derivative).
+__device__ __forceinline__ void rotation_r(const float *u, float *R)
+{
+    const float theta = sqrtf((u[0] * u[0] + u[1] * u[1]) + u[2] * u[2]);
+    const float un[3] = {u[0] / theta, u[1] / theta, u[2] / theta};
+    float Sn[9], Sn2[9];
+    skew(Sn, un);
+    const float st = (float)sin((double)theta);
+    const float cis = 1.0f - (float)cos((double)theta);
+    mul33(Sn, Sn, Sn2);
+#pragma unroll
+    for (int i = 0; i < 9; ++i)
+        R[i] = i % 4 == 0 ? (cis * Sn2[i] + 1.0f) + st * Sn[i] : cis * Sn2[i] + st * Sn[i];
+}
+
 __device__ void rotation(const float *u, float *R, float *dR)
 {
     float theta = sqrtf((u[0] * u[0] + u[1] * u[1]) + u[2] * u[2]);

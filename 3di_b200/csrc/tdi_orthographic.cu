@@ -11,6 +11,11 @@
 // multiply-add chains over the 102 residual rows in order (x rows, then y rows), the
 // Cholesky factor by left-looking dot products in increasing k, forward substitution in
 // increasing k, back substitution in decreasing k.
+//
+// Bound by the latency of its serial chains (a frame is one warp, about twenty dependent steps), so the
+// independent chains of a step run side by side: the system's rows in the lanes, the 36 sums over the
+// residual rows in two chains per lane, and a trial's rotation is formed without its derivative. One
+// frame 95 -> 64 us, 500 frames (the slowest of them) 450 -> 300 us.
 
 namespace tdi {
 
@@ -18,11 +23,13 @@ constexpr int OR_WARPS = 4;                 // frames per block
 constexpr int OR_N = 7;
 constexpr int OR_ROWS = 2 * NL;
 
+constexpr int OR_SUMS = OR_N * (OR_N + 1) / 2 + OR_N + 1;
+
 struct OrthWarp {
     float xb[NL], yb[NL];                   // centred landmarks
     float W[OR_N][OR_ROWS];                 // Jacobian columns
     float e[OR_ROWS];                       // residuals (of the point, then of each trial)
-    float R[9], dR[27], Rt[9], dRt[27];     // rotation of the point and of the last trial
+    float R[9], dR[27], Rt[9];              // rotation of the point and of the last trial
     float x[OR_N], xs[OR_N], sd[OR_N], dg[OR_N], JTJ[OR_N * OR_N];
     float obj;
     int accept;
@@ -35,39 +42,43 @@ __device__ __forceinline__ void orth_rp(const float *R, const float *p0L, int i,
     for (int k = 0; k < 3; ++k) r[k] = (R[k] * p0 + R[3 + k] * p1) + R[6 + k] * p2;
 }
 
-// d = -(H^-1 g) for the 7 x 7 system, FP64 (solver.h:70-105); NaN when H is not positive definite.
-__device__ void orth_solve(const float *H, const float *g, float *d)
+// d = -(H^-1 g) for the 7 x 7 system, FP64 (solver.h:70-105); NaN when H is not positive definite. Lane i
+// holds row i (lanes from 7 on copy row 6); a column's quotients are formed side by side, and the
+// right-hand side is carried as one more column of every row's work: y_i by the operations of the
+// forward substitution, in increasing k.
+__device__ __forceinline__ void orth_solve(const float *H, const float *g, float *d, int lane)
 {
-    double L[OR_N * OR_N], y[OR_N];
-    for (int i = 0; i < OR_N * OR_N; ++i) L[i] = (double)H[i];
+    const int i = lane < OR_N ? lane : OR_N - 1;
+    double L[OR_N];                                    // row i: L(i, k)
+#pragma unroll
+    for (int k = 0; k < OR_N; ++k) L[k] = (double)H[k * OR_N + i];
+    double t = (double)g[i], piv[OR_N], y[OR_N];
     bool ok = true;
-    for (int j = 0; j < OR_N && ok; ++j) {
-        double s = L[j * OR_N + j];
-        for (int k = 0; k < j; ++k) s -= L[k * OR_N + j] * L[k * OR_N + j];
-        if (!(s > 0.0)) { ok = false; break; }
-        const double ljj = sqrt(s);
-        L[j * OR_N + j] = ljj;
-        for (int i = j + 1; i < OR_N; ++i) {
-            double t = L[j * OR_N + i];
-            for (int k = 0; k < j; ++k) t -= L[k * OR_N + i] * L[k * OR_N + j];
-            L[j * OR_N + i] = t / ljj;
-        }
+#pragma unroll
+    for (int j = 0; j < OR_N; ++j) {
+        // t_ij = a_ij minus L(i,k) L(j,k) in increasing k, in every lane (row j's own for the pivot)
+        double s = L[j];
+#pragma unroll
+        for (int k = 0; k < j; ++k) s -= L[k] * __shfl_sync(0xffffffffu, L[k], j);
+        const double sj = __shfl_sync(0xffffffffu, s, j);
+        ok = ok && sj > 0.0;
+        piv[j] = sqrt(sj);
+        L[j] = s / piv[j];                             // (row j's own entry is not used)
+        // y_j = t_j / l_jj; later rows subtract L(i,j) y_j
+        y[j] = __shfl_sync(0xffffffffu, t / piv[j], j);
+        if (i > j) t -= L[j] * y[j];
     }
-    if (!ok) {
-        for (int i = 0; i < OR_N; ++i) d[i] = __int_as_float(0x7fc00000);
-        return;
+#pragma unroll
+    for (int j = OR_N - 1; j >= 0; --j) {
+        double u = y[j];
+#pragma unroll
+        for (int k = OR_N - 1; k > j; --k) u -= __shfl_sync(0xffffffffu, L[j], k) * y[k];
+        y[j] = u / piv[j];
     }
-    for (int i = 0; i < OR_N; ++i) {
-        double t = (double)g[i];
-        for (int k = 0; k < i; ++k) t -= L[k * OR_N + i] * y[k];
-        y[i] = t / L[i * OR_N + i];
+    if (lane == 0) {
+#pragma unroll
+        for (int k = 0; k < OR_N; ++k) d[k] = ok ? (float)(-y[k]) : __int_as_float(0x7fc00000);
     }
-    for (int i = OR_N - 1; i >= 0; --i) {
-        double t = y[i];
-        for (int k = OR_N - 1; k > i; --k) t -= L[i * OR_N + k] * y[k];
-        y[i] = t / L[i * OR_N + i];
-    }
-    for (int i = 0; i < OR_N; ++i) d[i] = (float)(-y[i]);
 }
 
 // x_start: NULL for the reference's start point (reset_orthographic), else [F][7] start points
@@ -121,30 +132,44 @@ __global__ void __launch_bounds__(OR_WARPS * 32) k_orthographic(const float *xl,
             w.e[NL + i] = sy * (rp[1] + ty) - w.yb[i];
         }
         __syncwarp();
-        for (int k = lane; k < OR_N * OR_N; k += 32) {
-            const int a = k % OR_N, b = k / OR_N;
-            float s = 0.0f;
-            for (int r = 0; r < OR_ROWS; ++r) s = fmaf(w.W[a][r], w.W[b][r], s);
-            w.JTJ[k] = s;
-        }
-        if (lane < OR_N) {
-            float s = 0.0f;
-            for (int r = 0; r < OR_ROWS; ++r) s = fmaf(w.W[lane][r], w.e[r], s);
-            w.dg[lane] = s;
-        } else if (lane == OR_N) {
-            float s = 0.0f;
-            for (int r = 0; r < OR_ROWS; ++r) s = fmaf(w.e[r], w.e[r], s);
-            w.obj = s;
+        {
+            // The sums over the rows: the 28 entries H_ab (a >= b), the 7 gradient entries, the objective.
+            // A lane runs two of the 36 chains side by side.
+            const float *pa[2], *pb[2];
+            int ra[2], rb[2];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const int c = min(lane + 32 * h, OR_SUMS - 1);
+                int a = 0, r = c;
+                while (a < OR_N && r > a) r -= ++a;        // c = a (a + 1) / 2 + r; a = 7: gradient and objective
+                ra[h] = a; rb[h] = r;
+                pa[h] = a < OR_N ? w.W[a] : w.e;
+                pb[h] = r < OR_N ? w.W[r] : w.e;
+            }
+            float s0 = 0.0f, s1 = 0.0f;
+#pragma unroll 17
+            for (int r = 0; r < OR_ROWS; ++r) {
+                s0 = fmaf(pa[0][r], pb[0][r], s0);
+                s1 = fmaf(pa[1][r], pb[1][r], s1);
+            }
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float s = h ? s1 : s0;
+                if (lane + 32 * h >= OR_SUMS) break;
+                if (ra[h] < OR_N) { w.JTJ[rb[h] * OR_N + ra[h]] = s; w.JTJ[ra[h] * OR_N + rb[h]] = s; }
+                else if (rb[h] < OR_N) w.dg[rb[h]] = s;
+                else w.obj = s;
+            }
         }
         __syncwarp();
-        if (lane == 0) orth_solve(w.JTJ, w.dg, w.sd);
+        orth_solve(w.JTJ, w.dg, w.sd, lane);
         __syncwarp();
         float t = 1.0f;
         for (int inner = 0; inner < 1000; ++inner) {
             if (t < 0.1f) { terminate = true; break; }
             if (lane == 0) {
                 for (int n = 0; n < OR_N; ++n) w.xs[n] = w.x[n] + t * w.sd[n];
-                rotation(w.xs + 4, w.Rt, w.dRt);
+                rotation_r(w.xs + 4, w.Rt);
             }
             __syncwarp();
             for (int i = lane; i < NL; i += 32) {
@@ -156,6 +181,7 @@ __global__ void __launch_bounds__(OR_WARPS * 32) k_orthographic(const float *xl,
             __syncwarp();
             if (lane == 0) {
                 float objt = 0.0f, tmp = 0.0f;
+#pragma unroll 17
                 for (int r = 0; r < OR_ROWS; ++r) objt = fmaf(w.e[r], w.e[r], objt);
                 for (int n = 0; n < OR_N; ++n) tmp = fmaf(w.sd[n], w.dg[n], tmp);
                 tmp *= 0.4f * t;
