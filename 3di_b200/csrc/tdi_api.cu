@@ -283,8 +283,7 @@ tdi_status set_attrs()
     TDI_CUDA(cudaFuncSetAttribute(k_raster_resolve, cudaFuncAttributeMaxDynamicSharedMemorySize, RR_SMEM));
     TDI_CUDA(cudaFuncSetAttribute(k_neighbours, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)neigh_smem()));
-    TDI_CUDA(cudaFuncSetAttribute(k_vertex_t<VT_FPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    TDI_CUDA(cudaFuncSetAttribute(k_vertex_t<VT_FPT_SMALL>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    TDI_CUDA(cudaFuncSetAttribute(k_vertex, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     TDI_CUDA(cudaFuncSetAttribute(k_barrier_full<NE_P8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     TDI_CUDA(cudaFuncSetAttribute(k_barrier_full<BAR_WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     TDI_CUDA(cudaFuncSetAttribute(k_solve_t<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
@@ -314,31 +313,22 @@ int sm_count()
     return sms;
 }
 
-// Vertex stage grid: frame tiles of nf frames x vertex-tile groups, about VT_BLOCKS_PER_SM
-// blocks per SM.
-dim3 vertex_grid(const DModel &m, int frames, int nf = VT_F)
+// Vertex stage grid: frame tiles x vertex-tile groups, about VT_BLOCKS_PER_SM blocks per SM. The kernel
+// splits the blocks between frame tiles and vertex stripes by the number of frames that render, which is
+// at most `frames`.
+dim3 vertex_grid(const DModel &m, int frames)
 {
     const int sms = sm_count();
-    // the kernel splits the blocks between frame tiles and vertex stripes by the number of
-    // frames that render, which is at most `frames`
-    const long ftiles = std::max(1, (frames + nf - 1) / nf);
+    const long ftiles = std::max(1, (frames + VT_F - 1) / VT_F);
     const long ntiles = (m.V + VT_V - 1) / VT_V;
     return dim3((unsigned)std::max(ftiles, std::min((long)VT_BLOCKS_PER_SM * sms, ftiles * ntiles)));
 }
 
-// The exact vertex stage for at most `frames` rendering frames: 8 frames per thread (64-frame
-// tiles) for full rounds; 2 per thread (16-frame tiles) when at most VT_SMALL frames can render,
-// where a 64-frame tile would carry mostly idle frames through every multiply-add.
-constexpr int VT_SMALL = 32;
-
+// The exact vertex stage for at most `frames` rendering frames.
 template <class B>
 tdi_status launch_vertex(B *bt, const DModel &m, const DBatch &d, cudaStream_t s, int frames)
 {
-    if (frames <= VT_SMALL)
-        return launch(bt, KID_VERTEX, k_vertex_t<VT_FPT_SMALL>, vertex_grid(m, frames, 8 * VT_FPT_SMALL),
-                      dim3(32, VT_WARPS + 1), vt_smem(m.KP, 8 * VT_FPT_SMALL), s, m, d);
-    return launch(bt, KID_VERTEX, k_vertex_t<VT_FPT>, vertex_grid(m, frames), dim3(32, VT_WARPS + 1),
-                  vt_smem(m.KP), s, m, d);
+    return launch(bt, KID_VERTEX, k_vertex, vertex_grid(m, frames), dim3(32, VT_WARPS + 1), vt_smem(m.KP), s, m, d);
 }
 
 // Tensor-core vertex stage: one block per SM, split between frame tiles and vertex stripes.

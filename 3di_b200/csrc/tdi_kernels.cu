@@ -178,17 +178,22 @@ __global__ void __launch_bounds__(SS_THREADS) k_stage_start(DModel m, DBatch b, 
 
 // ------------------------------------------------------------------------------------------
 // Vertex stage: X0 = mean + E*eps (sequential fmaf over k), camera transform and
-// projection (renderer.cu:806-861, funcs.cu:395-453). A block owns 64 frames (coefficients,
+// projection (renderer.cu:806-861, funcs.cu:395-453). A block owns up to 96 frames (coefficients,
 // rotations, translations, cameras and render flags staged in shared memory) and walks a
 // strided set of 32-vertex tiles; each tile's basis rows (32 x 3 x KP floats, contiguous in
 // HBM) are brought into shared memory by the TMA engine, one bulk copy per vertex row,
 // double-buffered so that the next tile streams in while this one is computed. A thread
-// owns one vertex x 8 frames (24 FMA chains). geo[f][slot] = (X0, Y0, Z0, albedo);
+// owns one vertex x 2 to 12 frames (3 FMA chains each). geo[f][slot] = (X0, Y0, Z0, albedo);
 // proj[f][slot] = (xp, yp, camera Z, 0).
 // The grid is one-dimensional (about two blocks per SM) and is split on the device by the
 // number of frames that render this round (known only there): ftiles frame tiles x groups
 // vertex-tile stripes, so that every block has work whatever share of the active frames
-// the pre-render checks rejected.
+// the pre-render checks rejected. The frames are dealt evenly to the tiles and warps, and a warp
+// runs the loop compiled for its number of frame pairs: 77 frames are one tile of 10 per thread
+// (64-frame tiles carried 51 idle ones), and a warp without a frame only keeps the buffers moving.
+// Full rounds are bound by the packed multiply-adds and the projection's divisions (814 us for 1,024
+// frames, 16 per thread spill and take 869); 77 frames 112 -> 75 us, one frame 10.5 -> 6.9 us, where
+// the frames' coefficients, stored with all lanes in one bank, also took a part.
 
 // Two IEEE fused multiply-adds in one instruction (sm_100 packed FP32): d.x = fma(a.x, b.x, c.x),
 // d.y = fma(a.y, b.y, c.y), round to nearest, denormals kept -- the same results as two fmaf.
@@ -222,8 +227,7 @@ __device__ __forceinline__ float2 packed_one(int zero)
 }
 
 constexpr int VT_V = 32;                                   // vertices per tile (one per lane)
-constexpr int VT_FPT = 8, VT_F = 8 * VT_FPT;               // frames per thread, per block (full rounds)
-constexpr int VT_FPT_SMALL = 2;                             // frames per thread when few frames render
+constexpr int VT_F = 96;                                    // frames of a block, at most (12 per thread)
 constexpr int VT_FR = 16;                                   // per-frame floats: R(9), tau(3), cam(4)
 constexpr int VT_BLOCKS_PER_SM = 2;
 constexpr int VT_WARPS = 8;                                 // computing warps; one more issues the copies
@@ -235,37 +239,128 @@ __host__ __device__ __forceinline__ size_t vt_smem(int KP, int NF = VT_F)
     return ((size_t)2 * VT_V * vt_row(KP) + (size_t)NF * KP + (size_t)NF * VT_FR) * sizeof(float);
 }
 
-// A thread's FPT coefficients at one k as frame pairs (16-byte loads for 8, 8-byte for 2).
-template <int FPT>
-__device__ __forceinline__ void vt_load_x(float2 (&xv)[FPT / 2], const float *p)
+// A thread's coefficients at one k as NP frame pairs (16-byte loads, a last 8-byte one).
+template <int NP>
+__device__ __forceinline__ void vt_load_x(float2 (&xv)[NP], const float *p)
 {
-    if constexpr (FPT == 8) {
-        const float4 xa = *reinterpret_cast<const float4 *>(p), xb = *reinterpret_cast<const float4 *>(p + 4);
-        xv[0] = make_float2(xa.x, xa.y); xv[1] = make_float2(xa.z, xa.w);
-        xv[2] = make_float2(xb.x, xb.y); xv[3] = make_float2(xb.z, xb.w);
-    } else {
 #pragma unroll
-        for (int q = 0; q < FPT / 2; ++q) xv[q] = *reinterpret_cast<const float2 *>(p + 2 * q);
+    for (int q = 0; q + 1 < NP; q += 2) {
+        const float4 x = *reinterpret_cast<const float4 *>(p + 2 * q);
+        xv[q] = make_float2(x.x, x.y);
+        xv[q + 1] = make_float2(x.z, x.w);
+    }
+    if (NP & 1) xv[NP - 1] = *reinterpret_cast<const float2 *>(p + 2 * (NP - 1));
+}
+
+// Floats of a warp's coefficients at one k: its NP pairs, rounded up to 16 bytes.
+__device__ __forceinline__ constexpr int vt_pitch(int NP) { return 4 * ((NP + 1) / 2); }
+
+struct VtShared {
+    int any, issued;
+    volatile int abort;
+    int render[VT_F], frame[VT_F];
+    __align__(8) uint64_t full[2], empty[2];
+};
+
+// A computing warp's tiles: vertex v of the lane, 2 NP frames.
+template <int NP>
+__device__ __forceinline__ void vt_tiles(const DModel &m, const DBatch &b, VtShared &sh, const float *Eb, const float *Xs,
+                                         const float *Fs, int gy, int groups, int ntiles)
+{
+    constexpr int XP = VT_WARPS * vt_pitch(NP);
+    const int KP = m.KP, K = m.K, ER = vt_row(KP);
+    const int vl = threadIdx.x;
+    const float *xr = Xs + threadIdx.y * vt_pitch(NP);    // this warp's frames at k: xr[k * XP + q]
+    const int fl0 = threadIdx.y * 2 * NP;
+    bool busy = false;
+    for (int q = 0; q < 2 * NP; ++q) busy = busy || sh.render[fl0 + q];
+    for (int j = 0;; ++j) {
+        const int t = gy + j * groups;
+        if (t >= ntiles) break;
+        const int buf = j & 1;
+        const int v = t * VT_V + vl;
+        // the epilogue's per-vertex inputs, loaded before the wait
+        float mx = 0.0f, my = 0.0f, mz = 0.0f, tx = 0.0f;
+        if (busy && v < m.V) { mx = m.mean[v]; my = m.mean[m.V + v]; mz = m.mean[2 * m.V + v]; tx = m.tex[v]; }
+        const bool w = mbar_wait(smem_addr(&sh.full[buf]), (uint32_t)((j >> 1) & 1));
+        if (!__all_sync(0xffffffffu, w)) {
+            if (threadIdx.x == 0) { sh.abort = 1; atomicOr(b.err, 2); }
+            break;
+        }
+        // Sequential fused multiply-add over k for every output (the order the oracle uses),
+        // two frames per instruction: each half of fma.rn.f32x2 is an IEEE fused
+        // multiply-add, so every chain rounds exactly as fmaf would.
+        float2 acc[NP][3];
+#pragma unroll
+        for (int q = 0; q < NP; ++q) acc[q][0] = acc[q][1] = acc[q][2] = make_float2(0.0f, 0.0f);
+        if (busy) {
+            const float *er = Eb + (size_t)(buf * VT_V + vl) * ER;
+            int k = 0;
+#pragma unroll 1
+            for (; k + 4 <= K; k += 4) {
+                const float4 ex = *reinterpret_cast<const float4 *>(er + k);
+                const float4 ey = *reinterpret_cast<const float4 *>(er + KP + k);
+                const float4 ez = *reinterpret_cast<const float4 *>(er + 2 * KP + k);
+                const float exv[4] = {ex.x, ex.y, ex.z, ex.w}, eyv[4] = {ey.x, ey.y, ey.z, ey.w};
+                const float ezv[4] = {ez.x, ez.y, ez.z, ez.w};
+#pragma unroll
+                for (int jj = 0; jj < 4; ++jj) {
+                    float2 xv[NP];
+                    vt_load_x<NP>(xv, xr + (k + jj) * XP);
+                    const float2 e0 = make_float2(exv[jj], exv[jj]), e1 = make_float2(eyv[jj], eyv[jj]);
+                    const float2 e2 = make_float2(ezv[jj], ezv[jj]);
+#pragma unroll
+                    for (int q = 0; q < NP; ++q) {
+                        acc[q][0] = ffma2(e0, xv[q], acc[q][0]);
+                        acc[q][1] = ffma2(e1, xv[q], acc[q][1]);
+                        acc[q][2] = ffma2(e2, xv[q], acc[q][2]);
+                    }
+                }
+            }
+#pragma unroll 1
+            for (; k < K; ++k) {
+                const float ex = er[k], ey = er[KP + k], ez = er[2 * KP + k];
+                float2 xv[NP];
+                vt_load_x<NP>(xv, xr + k * XP);
+#pragma unroll
+                for (int q = 0; q < NP; ++q) {
+                    acc[q][0] = ffma2(make_float2(ex, ex), xv[q], acc[q][0]);
+                    acc[q][1] = ffma2(make_float2(ey, ey), xv[q], acc[q][1]);
+                    acc[q][2] = ffma2(make_float2(ez, ez), xv[q], acc[q][2]);
+                }
+            }
+        }
+        __syncwarp();                          // this warp is done with the buffer
+        if (threadIdx.x == 0) mbar_arrive(smem_addr(&sh.empty[buf]));
+        if (busy && v < m.V) {
+#pragma unroll
+            for (int q = 0; q < 2 * NP; ++q) {
+                if (!sh.render[fl0 + q]) continue;
+                const int f = sh.frame[fl0 + q];
+                const float *R = Fs + (fl0 + q) * VT_FR, *tau = R + 9, *cam = R + 12;
+                const float2 *a = acc[q >> 1];
+                const float X0 = mx + ((q & 1) ? a[0].y : a[0].x);
+                const float Y0 = my + ((q & 1) ? a[1].y : a[1].x);
+                const float Z0 = mz + ((q & 1) ? a[2].y : a[2].x);
+                const float X3 = ((R[0] * X0 + R[3] * Y0) + R[6] * Z0) + tau[0];
+                const float Y3 = ((R[1] * X0 + R[4] * Y0) + R[7] * Z0) + tau[1];
+                const float Z3 = ((R[2] * X0 + R[5] * Y0) + R[8] * Z0) + tau[2];
+                b.geo[(size_t)f * m.V + v] = make_float4(X0, Y0, Z0, tx);
+                b.proj[(size_t)f * m.V + v] = make_float4((cam[0] * X3) / Z3 + cam[2], (cam[1] * Y3) / Z3 + cam[3], Z3, 0.0f);
+            }
+        }
     }
 }
 
-// FPT frames per computing thread, 8 FPT per block: 8 for full rounds; 2 when few frames render
-// (a 64-frame tile then carries mostly idle frames through every multiply-add).
-template <int FPT>
-__global__ void __launch_bounds__(VT_THREADS, VT_BLOCKS_PER_SM) k_vertex_t(DModel m, DBatch b)
+// The round's frames are dealt evenly to tiles of at most VT_F, a tile's frames to the warps, 2 NP each.
+__global__ void __launch_bounds__(VT_THREADS, VT_BLOCKS_PER_SM) k_vertex(DModel m, DBatch b)
 {
-    constexpr int VT_F = 8 * FPT;              // frames of a block tile
-    constexpr int VT_FPT = FPT;
     extern __shared__ __align__(16) float vsm[];
     const int KP = m.KP, K = m.K, ER = vt_row(KP);
     float *Eb = vsm;                           // [2][VT_V][ER]: basis rows of two tiles
-    float *Xs = Eb + 2 * VT_V * ER;            // [KP][VT_F]: coefficients, the block's frames innermost
-    float *Fs = Xs + VT_F * KP;                // [VT_F][VT_FR]
-    __shared__ int s_any;
-    __shared__ volatile int s_abort;
-    __shared__ int s_issued;
-    __shared__ int s_render[VT_F], s_frame[VT_F];
-    __shared__ __align__(8) uint64_t s_full[2], s_empty[2];
+    float *Fs = Eb + 2 * VT_V * ER;            // [VT_F][VT_FR]
+    float *Xs = Fs + VT_F * VT_FR;             // [K][VT_WARPS][pitch]: coefficients, the frames innermost
+    __shared__ VtShared sh;
     const int ntiles = (m.V + VT_V - 1) / VT_V;
     const int rc = b.rcount[0];
     const int ftiles = (rc + VT_F - 1) / VT_F;
@@ -273,44 +368,57 @@ __global__ void __launch_bounds__(VT_THREADS, VT_BLOCKS_PER_SM) k_vertex_t(DMode
     const int groups = max(1, min(ntiles, (int)gridDim.x / ftiles));
     if ((int)blockIdx.x >= ftiles * groups) return;
     const int gy = blockIdx.x / ftiles;        // vertex-tile stripe
-    const int f0 = (blockIdx.x - gy * ftiles) * VT_F;
+    const int tf = (rc + ftiles - 1) / ftiles;                        // frames of a tile
+    const int np = (tf + 2 * VT_WARPS - 1) / (2 * VT_WARPS);          // frame pairs of a warp
+    const int f0 = (blockIdx.x - gy * ftiles) * tf;
     const int tid = threadIdx.y * 32 + threadIdx.x;
     const bool producer = threadIdx.y == VT_WARPS;
-    if (tid == 0) { s_any = 0; s_abort = 0; s_issued = 0; }
+    if (tid == 0) { sh.any = 0; sh.abort = 0; sh.issued = 0; }
     __syncthreads();
     if (tid < VT_F) {
         const int ai = f0 + tid;
-        const int f = ai < rc ? b.rlist[ai] : -1;
+        const int f = tid < tf && ai < rc ? b.rlist[ai] : -1;
         const int r = f >= 0 && b.ctl[f].render;
-        s_frame[tid] = f;
-        s_render[tid] = r;
+        sh.frame[tid] = f;
+        sh.render[tid] = r;
         if (r) {
-            s_any = 1;
+            sh.any = 1;
             if (gy == 0) prof_count(b, KID_VERTEX);
         }
     }
     if (tid == 0) {
-        mbar_init(smem_addr(&s_full[0]), 1);
-        mbar_init(smem_addr(&s_full[1]), 1);
-        mbar_init(smem_addr(&s_empty[0]), VT_WARPS);
-        mbar_init(smem_addr(&s_empty[1]), VT_WARPS);
+        mbar_init(smem_addr(&sh.full[0]), 1);
+        mbar_init(smem_addr(&sh.full[1]), 1);
+        mbar_init(smem_addr(&sh.empty[0]), VT_WARPS);
+        mbar_init(smem_addr(&sh.empty[1]), VT_WARPS);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     __syncthreads();
-    if (!s_any) return;
+    if (!sh.any) return;
     const int rowbytes = 3 * KP * (int)sizeof(float);
     const uint32_t eb_addr = smem_addr(Eb);
     if (!producer) {
-        for (int fl = threadIdx.y; fl < VT_F; fl += VT_WARPS) {
-            const int f = s_frame[fl];
-            const float *xr = f >= 0 ? b.xe + (size_t)f * m.KTP : nullptr;
-            for (int k = threadIdx.x; k < KP; k += 32) Xs[k * VT_F + fl] = (xr && k < K) ? xr[k] : 0.0f;
-            if (threadIdx.x < VT_FR) {
-                const int i = threadIdx.x;
-                float v = 0.0f;
-                if (f >= 0) v = i < 9 ? b.R[f * 9 + i] : i < 12 ? b.xe[(size_t)f * m.KTP + K + (i - 9)] : b.cam[f * 4 + (i - 12)];
-                Fs[fl * VT_FR + i] = v;
-            }
+        // lane = frame, four coefficients at a time: conflict-free stores
+        const int wp = vt_pitch(np), xp = VT_WARPS * wp;
+        const int fg = (tf + 31) / 32, kq = (K + 3) / 4;
+        for (int i = threadIdx.y; i < fg * kq; i += VT_WARPS) {
+            const int g = i / kq, k = 4 * (i - g * kq), fl = g * 32 + threadIdx.x;
+            if (fl >= 2 * VT_WARPS * np) continue;
+            const int f = fl < tf ? sh.frame[fl] : -1;
+            float4 x = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+            if (f >= 0) x = *reinterpret_cast<const float4 *>(b.xe + (size_t)f * m.KTP + k);
+            const int w = fl / (2 * np);
+            float *o = Xs + k * xp + w * wp + (fl - w * 2 * np);
+            o[0] = x.x;
+            o[xp] = x.y;
+            o[2 * xp] = x.z;
+            o[3 * xp] = x.w;
+        }
+        for (int i = tid; i < tf * VT_FR; i += VT_WARPS * 32) {
+            const int fl = i / VT_FR, e = i % VT_FR, f = sh.frame[fl];
+            float v = 0.0f;
+            if (f >= 0) v = e < 9 ? b.R[f * 9 + e] : e < 12 ? b.xe[(size_t)f * m.KTP + K + (e - 9)] : b.cam[f * 4 + (e - 12)];
+            Fs[i] = v;
         }
     } else if (threadIdx.x == 0) {
         // the first two tiles stream in while the coefficients are staged
@@ -318,7 +426,7 @@ __global__ void __launch_bounds__(VT_THREADS, VT_BLOCKS_PER_SM) k_vertex_t(DMode
             const int t = gy + j * groups;
             if (t >= ntiles) break;
             const int nv = min(VT_V, m.V - t * VT_V);
-            const uint32_t bar = smem_addr(&s_full[j]);
+            const uint32_t bar = smem_addr(&sh.full[j]);
             mbar_expect_tx(bar, (uint32_t)(nv * rowbytes));
             for (int r = 0; r < nv; ++r)
                 bulk_g2s(eb_addr + (uint32_t)((j * VT_V + r) * ER) * 4u, m.E + (size_t)(t * VT_V + r) * 3 * KP,
@@ -332,105 +440,38 @@ __global__ void __launch_bounds__(VT_THREADS, VT_BLOCKS_PER_SM) k_vertex_t(DMode
             int j = 2;
             for (;; ++j) {
                 const int t = gy + j * groups;
-                if (t >= ntiles || s_abort) break;
+                if (t >= ntiles || sh.abort) break;
                 const int buf = j & 1;
-                if (!mbar_wait(smem_addr(&s_empty[buf]), (uint32_t)(((j - 2) >> 1) & 1))) {
-                    s_abort = 1;
+                if (!mbar_wait(smem_addr(&sh.empty[buf]), (uint32_t)(((j - 2) >> 1) & 1))) {
+                    sh.abort = 1;
                     atomicOr(b.err, 2);
                     break;
                 }
                 const int nv = min(VT_V, m.V - t * VT_V);
-                const uint32_t bar = smem_addr(&s_full[buf]);
+                const uint32_t bar = smem_addr(&sh.full[buf]);
                 mbar_expect_tx(bar, (uint32_t)(nv * rowbytes));
                 for (int r = 0; r < nv; ++r)
                     bulk_g2s(eb_addr + (uint32_t)((buf * VT_V + r) * ER) * 4u, m.E + (size_t)(t * VT_V + r) * 3 * KP,
                              (uint32_t)rowbytes, bar);
             }
-            s_issued = min(j, (ntiles - gy + groups - 1) / groups);
+            sh.issued = min(j, (ntiles - gy + groups - 1) / groups);
         }
     } else {
-        const int vl = threadIdx.x;
-        const float *xr = Xs + threadIdx.y * VT_FPT;      // this warp's frames at k: xr[k * VT_F + q]
-        for (int j = 0;; ++j) {
-            const int t = gy + j * groups;
-            if (t >= ntiles) break;
-            const int buf = j & 1;
-            const int v = t * VT_V + vl;
-            // the epilogue's per-vertex inputs, loaded before the wait
-            float mx = 0.0f, my = 0.0f, mz = 0.0f, tx = 0.0f;
-            if (v < m.V) { mx = m.mean[v]; my = m.mean[m.V + v]; mz = m.mean[2 * m.V + v]; tx = m.tex[v]; }
-            const bool w = mbar_wait(smem_addr(&s_full[buf]), (uint32_t)((j >> 1) & 1));
-            if (!__all_sync(0xffffffffu, w)) {
-                if (threadIdx.x == 0) { s_abort = 1; atomicOr(b.err, 2); }
-                break;
-            }
-            const float *er = Eb + (size_t)(buf * VT_V + vl) * ER;
-            // Sequential fused multiply-add over k for every output (the order the oracle uses),
-            // two frames per instruction: each half of fma.rn.f32x2 is an IEEE fused
-            // multiply-add, so every chain rounds exactly as fmaf would.
-            float2 acc[VT_FPT / 2][3];
-#pragma unroll
-            for (int q = 0; q < VT_FPT / 2; ++q) acc[q][0] = acc[q][1] = acc[q][2] = make_float2(0.0f, 0.0f);
-            int k = 0;
-            for (; k + 4 <= K; k += 4) {
-                const float4 ex = *reinterpret_cast<const float4 *>(er + k);
-                const float4 ey = *reinterpret_cast<const float4 *>(er + KP + k);
-                const float4 ez = *reinterpret_cast<const float4 *>(er + 2 * KP + k);
-                const float exv[4] = {ex.x, ex.y, ex.z, ex.w}, eyv[4] = {ey.x, ey.y, ey.z, ey.w};
-                const float ezv[4] = {ez.x, ez.y, ez.z, ez.w};
-#pragma unroll
-                for (int jj = 0; jj < 4; ++jj) {
-                    float2 xv[VT_FPT / 2];
-                    vt_load_x<VT_FPT>(xv, xr + (k + jj) * VT_F);
-                    const float2 e0 = make_float2(exv[jj], exv[jj]), e1 = make_float2(eyv[jj], eyv[jj]);
-                    const float2 e2 = make_float2(ezv[jj], ezv[jj]);
-#pragma unroll
-                    for (int q = 0; q < VT_FPT / 2; ++q) {
-                        acc[q][0] = ffma2(e0, xv[q], acc[q][0]);
-                        acc[q][1] = ffma2(e1, xv[q], acc[q][1]);
-                        acc[q][2] = ffma2(e2, xv[q], acc[q][2]);
-                    }
-                }
-            }
-            for (; k < K; ++k) {
-                const float ex = er[k], ey = er[KP + k], ez = er[2 * KP + k];
-                float2 xv[VT_FPT / 2];
-                vt_load_x<VT_FPT>(xv, xr + k * VT_F);
-#pragma unroll
-                for (int q = 0; q < VT_FPT / 2; ++q) {
-                    acc[q][0] = ffma2(make_float2(ex, ex), xv[q], acc[q][0]);
-                    acc[q][1] = ffma2(make_float2(ey, ey), xv[q], acc[q][1]);
-                    acc[q][2] = ffma2(make_float2(ez, ez), xv[q], acc[q][2]);
-                }
-            }
-            __syncwarp();                          // this warp is done with the buffer
-            if (threadIdx.x == 0) mbar_arrive(smem_addr(&s_empty[buf]));
-            if (v < m.V) {
-#pragma unroll
-                for (int q = 0; q < VT_FPT; ++q) {
-                    const int fl = threadIdx.y * VT_FPT + q;
-                    if (!s_render[fl]) continue;
-                    const int f = s_frame[fl];
-                    const float *R = Fs + fl * VT_FR, *tau = R + 9, *cam = R + 12;
-                    const float2 *a = acc[q >> 1];
-                    const float X0 = mx + ((q & 1) ? a[0].y : a[0].x);
-                    const float Y0 = my + ((q & 1) ? a[1].y : a[1].x);
-                    const float Z0 = mz + ((q & 1) ? a[2].y : a[2].x);
-                    const float X3 = ((R[0] * X0 + R[3] * Y0) + R[6] * Z0) + tau[0];
-                    const float Y3 = ((R[1] * X0 + R[4] * Y0) + R[7] * Z0) + tau[1];
-                    const float Z3 = ((R[2] * X0 + R[5] * Y0) + R[8] * Z0) + tau[2];
-                    b.geo[(size_t)f * m.V + v] = make_float4(X0, Y0, Z0, tx);
-                    b.proj[(size_t)f * m.V + v] = make_float4((cam[0] * X3) / Z3 + cam[2], (cam[1] * Y3) / Z3 + cam[3], Z3, 0.0f);
-                }
-            }
+        switch (np) {
+        case 1: vt_tiles<1>(m, b, sh, Eb, Xs, Fs, gy, groups, ntiles); break;
+        case 2: vt_tiles<2>(m, b, sh, Eb, Xs, Fs, gy, groups, ntiles); break;
+        case 3: vt_tiles<3>(m, b, sh, Eb, Xs, Fs, gy, groups, ntiles); break;
+        case 4: vt_tiles<4>(m, b, sh, Eb, Xs, Fs, gy, groups, ntiles); break;
+        case 5: vt_tiles<5>(m, b, sh, Eb, Xs, Fs, gy, groups, ntiles); break;
+        default: vt_tiles<6>(m, b, sh, Eb, Xs, Fs, gy, groups, ntiles); break;
         }
     }
     __syncthreads();
-    if (s_abort && tid == VT_WARPS * 32) {
+    if (sh.abort && tid == VT_WARPS * 32) {
         // copies of the last two issued tiles may still be in flight: wait for them (bounded)
         // before the block's shared memory is released
-        for (int j = max(0, s_issued - 2); j < s_issued; ++j)
-            mbar_wait(smem_addr(&s_full[j & 1]), (uint32_t)((j >> 1) & 1));
+        for (int j = max(0, sh.issued - 2); j < sh.issued; ++j)
+            mbar_wait(smem_addr(&sh.full[j & 1]), (uint32_t)((j >> 1) & 1));
     }
 }
 
