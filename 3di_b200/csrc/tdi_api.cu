@@ -915,7 +915,7 @@ tdi_status tdi_batch_set_frames(tdi_batch *b, const tdi_frames *fr, void *stream
     if (fr->n_frames > b->cap) return fail(TDI_ERR_CAPACITY, "more frames than the batch holds");
     cudaStream_t s = (cudaStream_t)stream;
     const size_t bytes = sizeof(float) * NPIX * fr->n_frames;
-    TDI_CUDA(stage_upload({{(const char *)fr->targets, bytes, bytes, 1, (char *)b->target_raw}}, s));
+    TDI_CUDA(stage_upload({{(const char *)fr->targets, bytes, bytes, 1, (char *)b->target_raw}}, STAGE_PIN, s));
     return set_frames_meta(b, fr, s);
 }
 
@@ -1007,7 +1007,7 @@ tdi_status tdi_batch_set_video_frames(tdi_batch *b, const tdi_video_frames *fr, 
             p.bgr = b->raw_stage + used - ((size_t)r0 * width + 3 * (size_t)c0);
             used += width * rows;
         }
-        if (!pieces.empty()) TDI_CUDA(stage_upload(pieces, s));
+        if (!pieces.empty()) TDI_CUDA(stage_upload(pieces, STAGE_MIN, s));
         TDI_CUDA(cudaMemcpyAsync(b->prep + f0, pf.data() + f0, sizeof(PrepFrame) * n, cudaMemcpyHostToDevice, s));
         TDI_TRY(launch(b, 0, k_preprocess, dim3(DIM / PP_TILE, DIM / PP_TILE, n), dim3(PP_TILE, PP_ROWS), 0, s,
                        (const PrepFrame *)(b->prep + f0), b->target_raw + (size_t)f0 * NPIX));

@@ -105,8 +105,6 @@ __device__ __forceinline__ void prof_count(const DBatch &b, int id, unsigned lon
 // capacity; blocks past the count return at once).
 __device__ __forceinline__ int active_n(const DBatch &b) { return b.dnact ? *b.dnact : b.nact; }
 
-__device__ __forceinline__ bool shape_stage(int stage) { return stage != ST_LAMBDA; }
-
 __device__ void end_shape_stage(const Cfg &c, FrameCtl &ctl, int stage, int outer)
 {
     ctl.active = 0;
@@ -2023,7 +2021,6 @@ __device__ __forceinline__ void chain_value(const float (&vv)[4], float pre, flo
 constexpr int NE_P8 = 88;                    // padded width: parameters + weight column, <= 88
 constexpr int NE_T8 = NE_P8 / 8;             // 11 tile rows / columns
 constexpr int NE_NT8 = NE_T8 * (NE_T8 + 1) / 2;   // 66 tiles
-constexpr int NE_TPW = (NE_NT8 + 7) / 8;     // tiles per warp (8 warps)
 
 __device__ __forceinline__ void ne_tile8(int t, int &bi, int &bj)
 {

@@ -166,14 +166,13 @@ def algorithmic_bytes(kernel: str, V: int, T: int, K: int, n_frag: float):
         return 24.0 * V + 4.0 * K, 12.0 * V * K
     if kernel == "raster":
         # depth pass: projections (16 B per vertex), triangle corners and visiting order
-        # (16 B per triangle), one 8-byte depth key per visible fragment
-        return 16.0 * V + 16.0 * T + 8.0 * n_frag, 0.0
+        # (16 B per triangle), one 8-byte depth key per visible fragment; per fragment three
+        # vertices' object coordinates and albedo, its candidate record and shading inputs written
+        return 16.0 * V + 16.0 * T + n_frag * (8 + 3 * 16 + 16 + 24), 0.0
     if kernel == "raster_resolve":
-        # the frame's triangle mask, the corners and projections of the triangles with
-        # fragments (about one per fragment), their depth keys and the fragment records written;
-        # then per fragment its record, its triangle's corners, three vertices' object
-        # coordinates and albedo, and the shading records written (unit normal and n . p, albedo)
-        return T / 8.0 + n_frag * (16 + 3 * 16 + 8 + 16) + n_frag * (16 + 16 + 3 * 16 + 20), 0.0
+        # per fragment its candidate record and camera Z, its depth key, its mark in the bit sets (the
+        # records are placed by a kernel of their own)
+        return n_frag * (16 + 4 + 8 + 4), 0.0
     if kernel == "render":
         # fragments, their shading records, four target pixels, gradients
         return n_frag * (16 + 20 + 4 * 4 + 5 * 4), 0.0
