@@ -16,7 +16,10 @@
 // (tid % 16, tid / 16) owns the entries (tr + 16 a, tc + 16 b)): they scale column j, subtract its
 // products from their entries, and publish column j + 1 and the diagonal entry of column
 // j + 2. One barrier per column (with DIV another among the workers, whose column is divided once
-// into shared memory). A pivot that is not positive is noticed at the end of its group. Each entry receives its updates in increasing k, the sequence of the oracle's
+// into shared memory). A pivot that is not positive is noticed at the end of the group in which the chain
+// formed it, by every thread: the chain is a step ahead of what the workers have read, so group J's
+// mark has a slot by J's parity, read after the group's last barrier and written again 16 barriers later
+// at the earliest. Each entry receives its updates in increasing k, the sequence of the oracle's
 // left-looking dot products. Entries left of the current column or above the diagonal are
 // updated too, without tests: nothing reads them again. Columns run in groups of 16, one
 // instantiation each, so that every register block has a compile-time index.
@@ -52,7 +55,7 @@ struct CholMem {
     double *lv;      // [16 RB] pivots
     double *xs;      // [16 RB] the solution
     double *dd;      // [2] diagonal entry of the column after next, by parity
-    int *fail;       // a pivot was not positive
+    int *fail;       // [2] a pivot formed in a group was not positive, by group parity
 };
 
 // t / l, correctly rounded, from r = 1 / l correctly rounded: two residual corrections with fused
@@ -96,7 +99,7 @@ __device__ __forceinline__ bool chol_group(double (&v)[RB][RB], const CholMem &c
                 if (tid == CH_WORKERS) {
                     cm.rv[j + 1] = r;
                     if (DIV) cm.lv[j + 1] = l;
-                    if (!(s > 0.0)) *cm.fail = 1;
+                    if (!(s > 0.0)) cm.fail[J & 1] = 1;
                 }
             }
         } else {
@@ -144,7 +147,7 @@ __device__ __forceinline__ bool chol_group(double (&v)[RB][RB], const CholMem &c
         }
         __syncthreads();
     }
-    if (*cm.fail) return false;
+    if (cm.fail[J & 1]) return false;
     if constexpr (J + 1 < RB) return chol_group<RB, DIV, J + 1>(v, cm, n, LD, tid, tr, tc);
     else return true;
 }
@@ -187,7 +190,8 @@ __device__ __forceinline__ bool chol_solve(int n, double *sm, A a_of, G rhs, dou
             const double l = sqrt(v[0][0]);
             cm.lv[0] = l;
             cm.rv[0] = __drcp_rn(l);
-            *cm.fail = !(v[0][0] > 0.0);
+            cm.fail[0] = !(v[0][0] > 0.0);
+            cm.fail[1] = 0;
         }
     }
     __syncthreads();
