@@ -283,7 +283,7 @@ tdi_status set_attrs()
     TDI_CUDA(cudaFuncSetAttribute(k_raster_resolve, cudaFuncAttributeMaxDynamicSharedMemorySize, RR_SMEM));
     TDI_CUDA(cudaFuncSetAttribute(k_neighbours, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                   (int)neigh_smem()));
-    TDI_CUDA(cudaFuncSetAttribute(k_vertex, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    TDI_CUDA(cudaFuncSetAttribute(k_vertex, cudaFuncAttributeMaxDynamicSharedMemorySize, VT_SMEM));
     TDI_CUDA(cudaFuncSetAttribute(k_barrier_full<NE_P8>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     TDI_CUDA(cudaFuncSetAttribute(k_barrier_full<BAR_WIDE>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     TDI_CUDA(cudaFuncSetAttribute(k_solve_t<6>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
@@ -313,13 +313,13 @@ int sm_count()
     return sms;
 }
 
-// Vertex stage grid: frame tiles x vertex-tile groups, about VT_BLOCKS_PER_SM blocks per SM. The kernel
+// Vertex stage grid: frame tiles (of nf frames) x vertex-tile groups, about VT_BLOCKS_PER_SM blocks per SM. The kernel
 // splits the blocks between frame tiles and vertex stripes by the number of frames that render, which is
 // at most `frames`.
-dim3 vertex_grid(const DModel &m, int frames)
+dim3 vertex_grid(const DModel &m, int frames, int nf)
 {
     const int sms = sm_count();
-    const long ftiles = std::max(1, (frames + VT_F - 1) / VT_F);
+    const long ftiles = std::max(1, (frames + nf - 1) / nf);
     const long ntiles = (m.V + VT_V - 1) / VT_V;
     return dim3((unsigned)std::max(ftiles, std::min((long)VT_BLOCKS_PER_SM * sms, ftiles * ntiles)));
 }
@@ -328,7 +328,9 @@ dim3 vertex_grid(const DModel &m, int frames)
 template <class B>
 tdi_status launch_vertex(B *bt, const DModel &m, const DBatch &d, cudaStream_t s, int frames)
 {
-    return launch(bt, KID_VERTEX, k_vertex, vertex_grid(m, frames), dim3(32, VT_WARPS + 1), vt_smem(m.KP), s, m, d);
+    const int nf = vt_frames(m.KP);
+    if (!nf) return fail(TDI_ERR_INVALID, "the vertex stage takes at most 240 expression components");
+    return launch(bt, KID_VERTEX, k_vertex, vertex_grid(m, frames, nf), dim3(32, VT_WARPS + 1), vt_smem(m.KP, nf), s, m, d, nf);
 }
 
 // Tensor-core vertex stage: one block per SM, split between frame tiles and vertex stripes.

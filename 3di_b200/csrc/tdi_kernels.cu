@@ -176,8 +176,8 @@ __global__ void __launch_bounds__(SS_THREADS) k_stage_start(DModel m, DBatch b, 
 
 // ------------------------------------------------------------------------------------------
 // Vertex stage: X0 = mean + E*eps (sequential fmaf over k), camera transform and
-// projection (renderer.cu:806-861, funcs.cu:395-453). A block owns up to 96 frames (coefficients,
-// rotations, translations, cameras and render flags staged in shared memory) and walks a
+// projection (renderer.cu:806-861, funcs.cu:395-453). A block owns up to 96 frames (fewer
+// for bases too wide for that, vt_frames; coefficients, rotations, translations, cameras and render flags staged in shared memory) and walks a
 // strided set of 32-vertex tiles; each tile's basis rows (32 x 3 x KP floats, contiguous in
 // HBM) are brought into shared memory by the TMA engine, one bulk copy per vertex row,
 // double-buffered so that the next tile streams in while this one is computed. A thread
@@ -226,15 +226,26 @@ __device__ __forceinline__ float2 packed_one(int zero)
 
 constexpr int VT_V = 32;                                   // vertices per tile (one per lane)
 constexpr int VT_F = 96;                                    // frames of a block, at most (12 per thread)
+constexpr int VT_SMEM = 200 * 1024;                         // shared memory of a block, at most
 constexpr int VT_FR = 16;                                   // per-frame floats: R(9), tau(3), cam(4)
 constexpr int VT_BLOCKS_PER_SM = 2;
 constexpr int VT_WARPS = 8;                                 // computing warps; one more issues the copies
 constexpr int VT_THREADS = (VT_WARPS + 1) * 32;
 
 __host__ __device__ __forceinline__ int vt_row(int KP) { return 3 * KP + 4; }   // basis row pitch (floats)
-__host__ __device__ __forceinline__ size_t vt_smem(int KP, int NF = VT_F)
+__host__ __device__ __forceinline__ size_t vt_smem(int KP, int NF)
 {
     return ((size_t)2 * VT_V * vt_row(KP) + (size_t)NF * KP + (size_t)NF * VT_FR) * sizeof(float);
+}
+
+// Frames of a tile: what shared memory holds beside two tiles of basis rows, 96 up to 168 expressions,
+// 64 up to 192, 32 up to 224, 16 up to 240; 0 when the rows leave no room. (Counts at which the warps'
+// coefficients take no more than their frames': 2, 4, 8 or 12 per warp.)
+inline int vt_frames(int KP)
+{
+    for (int nf : {VT_F, 64, 32, 16})
+        if (vt_smem(KP, nf) <= VT_SMEM) return nf;
+    return 0;
 }
 
 // A thread's coefficients at one k as NP frame pairs (16-byte loads, a last 8-byte one).
@@ -250,8 +261,9 @@ __device__ __forceinline__ void vt_load_x(float2 (&xv)[NP], const float *p)
     if (NP & 1) xv[NP - 1] = *reinterpret_cast<const float2 *>(p + 2 * (NP - 1));
 }
 
-// Floats of a warp's coefficients at one k: its NP pairs, rounded up to 16 bytes.
-__device__ __forceinline__ constexpr int vt_pitch(int NP) { return 4 * ((NP + 1) / 2); }
+// Floats of a warp's coefficients at one k: its NP pairs, rounded up to 16 bytes (a single pair is read
+// in 8-byte loads).
+__device__ __forceinline__ constexpr int vt_pitch(int NP) { return NP == 1 ? 2 : 4 * ((NP + 1) / 2); }
 
 struct VtShared {
     int any, issued;
@@ -350,18 +362,19 @@ __device__ __forceinline__ void vt_tiles(const DModel &m, const DBatch &b, VtSha
     }
 }
 
-// The round's frames are dealt evenly to tiles of at most VT_F, a tile's frames to the warps, 2 NP each.
-__global__ void __launch_bounds__(VT_THREADS, VT_BLOCKS_PER_SM) k_vertex(DModel m, DBatch b)
+// The round's frames are dealt evenly to tiles of at most nf (vt_frames), a tile's frames to the warps,
+// 2 NP each.
+__global__ void __launch_bounds__(VT_THREADS, VT_BLOCKS_PER_SM) k_vertex(DModel m, DBatch b, int nf)
 {
     extern __shared__ __align__(16) float vsm[];
     const int KP = m.KP, K = m.K, ER = vt_row(KP);
     float *Eb = vsm;                           // [2][VT_V][ER]: basis rows of two tiles
-    float *Fs = Eb + 2 * VT_V * ER;            // [VT_F][VT_FR]
-    float *Xs = Fs + VT_F * VT_FR;             // [K][VT_WARPS][pitch]: coefficients, the frames innermost
+    float *Fs = Eb + 2 * VT_V * ER;            // [nf][VT_FR]
+    float *Xs = Fs + nf * VT_FR;               // [K][VT_WARPS][pitch]: coefficients, the frames innermost
     __shared__ VtShared sh;
     const int ntiles = (m.V + VT_V - 1) / VT_V;
     const int rc = b.rcount[0];
-    const int ftiles = (rc + VT_F - 1) / VT_F;
+    const int ftiles = (rc + nf - 1) / nf;
     if (ftiles == 0) return;
     const int groups = max(1, min(ntiles, (int)gridDim.x / ftiles));
     if ((int)blockIdx.x >= ftiles * groups) return;
