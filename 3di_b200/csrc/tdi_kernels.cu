@@ -1454,16 +1454,22 @@ __device__ __forceinline__ void region_shade(const Region &r, const Fragment *fr
     }
 }
 
-// FP64 sum of a block's values: shuffles, then the warps in order; the total in thread 0.
+// FP64 sum of a block's values: shuffles, then the warps in order; the total in thread 0. The order is
+// that of RENDER_SUMS threads with one value each, whatever the block: thread t of a smaller one holds
+// the values of threads t, t + NT, ..., so that a frame's sum does not depend on the block size.
+constexpr int RENDER_SUMS = 1024;
 template <int NT>
-__device__ __forceinline__ double render_sum(double v, double *s_red)
+__device__ __forceinline__ double render_sum(double (&v)[RENDER_SUMS / NT], double *s_red)
 {
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
-    if ((threadIdx.x & 31) == 0) s_red[threadIdx.x >> 5] = v;
+#pragma unroll
+    for (int h = 0; h < RENDER_SUMS / NT; ++h) {
+        for (int o = 16; o > 0; o >>= 1) v[h] += __shfl_down_sync(0xffffffffu, v[h], o);
+        if ((threadIdx.x & 31) == 0) s_red[(threadIdx.x >> 5) + h * (NT / 32)] = v[h];
+    }
     __syncthreads();
     double s = 0.0;
     if (threadIdx.x == 0)
-        for (int w = 0; w < NT / 32; ++w) s += s_red[w];
+        for (int w = 0; w < RENDER_SUMS / 32; ++w) s += s_red[w];
     return s;
 }
 
@@ -1484,7 +1490,7 @@ __global__ void k_target_grad(const float *target, float2 *tgn, int F)
 }
 
 // NT threads per frame: 512 (two blocks per SM) for full rounds, 1,024 when the frames do not
-// fill the SMs and a block's own latency is the round's.
+// fill the SMs and a block's own latency is the round's. Both give the same bits (render_sum).
 template <int NT>
 __global__ void __launch_bounds__(NT, 1024 / NT) k_render_t(DModel m, DBatch b, Cfg c, int stage)
 {
@@ -1498,7 +1504,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_render_t(DModel m, DBatch b, 
     }
     if (tid == 0) prof_count(b, KID_RENDER);
     extern __shared__ __align__(16) float rsm[];
-    __shared__ double s_red[NT / 32];
+    __shared__ double s_red[RENDER_SUMS / 32];
     __shared__ int s_take;
     __shared__ float s_t;
     const Region r = make_region(ctl, rsm, b.img + (size_t)f * RIMG);
@@ -1513,7 +1519,9 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_render_t(DModel m, DBatch b, 
     region_blur<NT>(r, c);
     const float2 *tgn = b.tgn + (size_t)f * NPIX;
     float *fg = b.fgrad + (size_t)f * 5 * NMAX;
-    double corr = 0.0;
+    constexpr int NS = RENDER_SUMS / NT;         // sums per thread: of the fragments tid + NT h modulo RENDER_SUMS
+    static_assert(RENDER_GU % NS == 0, "a thread's u-th fragment belongs to its sum u % NS");
+    double corr[NS] = {};
     for (int n0 = tid; n0 < N; n0 += NT * RENDER_GU) {
         int pv[RENDER_GU];
         float2 tg[RENDER_GU];
@@ -1534,7 +1542,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_render_t(DModel m, DBatch b, 
             grad_of(r.A[r.at(kr)], r.A[r.at(kl)], r.A[r.at(kd)], r.A[r.at(ku)], gx, gy, h, gxn, gyn);
             fg[n] = gx; fg[NMAX + n] = gy; fg[2 * NMAX + n] = h;
             fg[3 * NMAX + n] = tg[u].x; fg[4 * NMAX + n] = tg[u].y;
-            corr += (double)gxn * (double)tg[u].x + (double)gyn * (double)tg[u].y;
+            corr[u % NS] += (double)gxn * (double)tg[u].x + (double)gyn * (double)tg[u].y;
         }
     }
     const double total = render_sum<NT>(corr, s_red);
