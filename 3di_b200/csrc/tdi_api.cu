@@ -686,6 +686,7 @@ tdi_status tdi_model_create(const tdi_model_desc *desc, tdi_model **out)
     cudaGetDevice(&m->device);
     DModel &d = m->d;
     d.V = V; d.T = T; d.K = K; d.KP = round4(K); d.KT = K + 6; d.KTP = round4(K + 6);
+    d.KC = std::min(d.KTP, CAND_COLS);
     float *mean, *E, *tex, *epsb;
     int32_t *tl, *lis, *order, *tlo;
     int4 *tl4, *tlo4;

@@ -19,6 +19,7 @@ constexpr int NTMP = 4;           // fragments kept per triangle (src/lib/consta
 constexpr int KRAD = 7;           // blur radius (src/CMakeLists.txt:1)
 constexpr int NTAPS = 2 * KRAD + 1;
 constexpr int NMAX = 32768;       // fragment capacity per frame (reference domain: 25,600)
+constexpr int CAND_COLS = 32;     // a raster's candidates: floats per fragment of capacity, at most
 constexpr int TRI_BITS = 20;      // z-buffer key: [13-bit epoch tag | 31-bit depth | 20-bit triangle]
 constexpr int TAG_BITS = 64 - 31 - TRI_BITS;
 constexpr uint32_t TAG_MAX = (1u << TAG_BITS) - 1;
@@ -87,6 +88,7 @@ struct Cfg {
 struct DModel {
     int32_t V, T, K, KP;     // KP: K rounded up to a multiple of 4 (row pitch of E)
     int32_t KT, KTP;         // K + 6 unknowns, and its pitch (multiple of 4)
+    int32_t KC;              // KTP, CAND_COLS at most: sizes a raster's candidates
     const float *mean;       // [3][V]
     const float *E;          // [V][3][KP]
     const float *tex;        // [V]
@@ -140,7 +142,8 @@ struct DBatch {
     float4 *shc;             // [F][NMAX]: unit normal and n . p of each fragment
     float *sht;              // [F][NMAX]: interpolated albedo of each fragment
     float *J;                // [F][NMAX][KTP]
-    double *ne_part;         // [F][NMAX/256][part stride] chunk partials of the normal equations
+    double *ne_part;         // [F][NMAX/256][part stride] chunk partials of the normal equations; before
+                             // them a raster's slots and candidates (RASTER_WORK bytes per frame)
     float *img;              // [F][2][NPIX] blur scratch for frames too large for shared memory
     // live profiling: frames processed by the kernel being timed (kernel ids as in tdi.h)
     unsigned long long *prof_frames;

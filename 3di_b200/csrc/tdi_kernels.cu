@@ -851,9 +851,11 @@ constexpr int RR_WARPS = RR_THREADS / 32;
 constexpr int RR_U = 4;                     // resolve: candidates per thread in flight together
 constexpr int RD_CAND = 640;                // depth pass: candidates a block collects before it appends them
 
-// A fragment of the raster in flight. Candidates of a frame lie in its Jacobian buffer (idle
-// between the solve and the next accepted point), CandidateSpan of them at most; a frame with more
-// takes the resolve's general path.
+// A fragment of the raster in flight. A raster's working set lies in the frame's chunk partials of the
+// normal equations (idle but between the normal equations and their reduction): the candidate of every
+// slot, then the candidates, in the room of KC floats per fragment of capacity (104,857 candidates from 23
+// expressions on); a frame with more takes the resolve's general path. What an evaluation leaves for
+// tdi_batch_read (neighbours, gradients, Jacobian) is not touched.
 struct __align__(16) Candidate {
     uint32_t pix_row;                       // pixel | row << 16
     int32_t tri;
@@ -868,12 +870,19 @@ struct CandidateSpan {
     int cap;
 };
 
+constexpr size_t RASTER_WORK = (size_t)NMAX * (CAND_COLS + 1) * sizeof(float);    // bytes per frame (4.1 MB)
+
+__device__ __forceinline__ uint32_t *raster_slots(const DBatch &b, int f)
+{
+    return reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(b.ne_part) + (size_t)f * RASTER_WORK);   // [NMAX]
+}
+
 __device__ __forceinline__ CandidateSpan candidates(const DModel &m, const DBatch &b, int f)
 {
     CandidateSpan s;
-    const size_t bytes = (size_t)NMAX * m.KTP * sizeof(float);
+    const size_t bytes = (size_t)NMAX * m.KC * sizeof(float);
     s.cap = (int)(bytes / (sizeof(Candidate) + sizeof(float4) + 2 * sizeof(float)));
-    s.c = reinterpret_cast<Candidate *>(b.J + (size_t)f * NMAX * m.KTP);
+    s.c = reinterpret_cast<Candidate *>(raster_slots(b, f) + NMAX);
     s.sn = reinterpret_cast<float4 *>(s.c + s.cap);
     s.t = reinterpret_cast<float *>(s.sn + s.cap);
     s.z = s.t + s.cap;
@@ -935,7 +944,8 @@ inline int raster_grid(int frames)
 // instructions instead of about 230) and queues the others' corners in shared memory (12-15% of the
 // 53,490-vertex mesh's); a full warp's worth of queued triangles is then evaluated densely. RD_ILP
 // triangles per lane have their gathers in flight together (1,024 frames in one launch: 1 875 us,
-// 2 707, 3 671; a fifth block per SM needs 48 registers and spills, 953).
+// 2 707, 3 671). 64 registers and 47 KB of shared memory are four blocks per SM (at 70 registers, three
+// blocks, 795 us; at 48 registers it spills, 953).
 // 1,024 frames of the 53,490-vertex model in one launch: 1,192 us with every sample evaluated in
 // place, 671 with the queue, the candidates and their shading inputs included (which the resolve
 // formed before). What is left is issue (0.68 per cycle) and the latency of the gathers.
@@ -1192,7 +1202,7 @@ __global__ void __launch_bounds__(RR_THREADS) k_raster_resolve(DModel m, DBatch 
     Fragment *out = b.frag + (size_t)f * NMAX;
     float4 *shc = b.shc + (size_t)f * NMAX;
     float *sht = b.sht + (size_t)f * NMAX;
-    uint32_t *slot = reinterpret_cast<uint32_t *>(b.nb + (size_t)f * 4 * NMAX);
+    uint32_t *slot = raster_slots(b, f);
     for_candidates([&](const Candidate &c, float z, unsigned long long key, int i) {
         if (!survivor(c, z, key)) return;
         const int w = (int)(c.pix_row >> 16) * W + (c.tri >> 5);
@@ -1246,7 +1256,7 @@ __global__ void __launch_bounds__(RS_THREADS) k_raster_slots(DModel m, DBatch b)
         if (!ctl.slots) continue;
         const int N = ctl.N;
         const CandidateSpan cs = candidates(m, b, f);
-        const uint32_t *slot = reinterpret_cast<const uint32_t *>(b.nb + (size_t)f * 4 * NMAX);
+        const uint32_t *slot = raster_slots(b, f);
         for (int p = (it % RS_PARTS) * RS_THREADS + threadIdx.x; p < N; p += RS_PARTS * RS_THREADS) {
             const uint32_t s = slot[p];
             const int i = (int)(s & 0x7FFFFFFFu);
@@ -2050,7 +2060,8 @@ __device__ __forceinline__ void ne_tile8(int t, int &bi, int &bj)
     bj = bi + t;
 }
 
-__host__ __device__ __forceinline__ int ne_part_stride8() { return NE_NT8 * 64; }
+__host__ __device__ constexpr inline int ne_part_stride8() { return NE_NT8 * 64; }
+static_assert(RASTER_WORK <= (size_t)NE_MAXCH * ne_part_stride8() * sizeof(double), "a raster's working set lies there");
 
 __device__ __forceinline__ void dmma_884(double &d0, double &d1, double a, double b)
 {

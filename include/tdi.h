@@ -227,6 +227,10 @@ tdi_status tdi_batch_evaluate(tdi_batch *b, const tdi_fit_config *cfg, int32_t f
  *  6 geometry    float [6][V]: X0, Y0, Z0, xp, yp, camera Z
  *  7 crop        float [65536]: the unblurred crop, x-major (after set_frames / set_video_frames)
  *  8 frame data  float [109]: xl [51], yl [51], camera [4], face size, crop origin x0, y0
+ * Fragments, geometry and the count N are the last raster's (tdi_batch_raster, a render or the
+ * differentiable loss among them); items 1 to 5 stay the last evaluation's.
+ * Fragments, geometry and the count N are the last raster's (tdi_batch_raster, a render or the
+ * differentiable loss among them); items 1 to 5 stay the last evaluation's.
  * Returns the number of elements written through *count. Synchronous. */
 tdi_status tdi_batch_read(tdi_batch *b, int32_t frame, int32_t what, void *dst, int64_t capacity,
                           int64_t *count);
