@@ -85,7 +85,9 @@ inline cudaError_t stage_upload(const std::vector<StagePiece> &pieces, size_t pi
 {
     size_t total = 0;
     for (const StagePiece &p : pieces) total += p.width * p.rows;
-    if (total < STAGE_MIN || !stage_pageable(pieces[0].host)) return stage_plain(pieces, s);
+    // (the per-thread default stream is another stream in each staging thread: their copies would not wait
+    // for the caller's earlier work)
+    if (total < STAGE_MIN || s == cudaStreamPerThread || !stage_pageable(pieces[0].host)) return stage_plain(pieces, s);
     StagePool &pool = stage_pool();
     std::unique_lock<std::mutex> lk(pool.mu, std::try_to_lock);
     if (!lk.owns_lock()) return stage_plain(pieces, s);
