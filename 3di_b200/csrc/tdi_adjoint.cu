@@ -161,22 +161,6 @@ __global__ void __launch_bounds__(256) k_adj_vertex_tiled(DModel m, const float 
     }
 }
 
-// The same without staging, for bases too wide for shared memory.
-__global__ void k_adj_vertex(DModel m, const float *x, int F, double *geo64)
-{
-    const int f = blockIdx.y;
-    const int v = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= F || v >= m.V) return;
-    const float *xf = x + (size_t)f * m.KT;
-    double *g = geo64 + ((size_t)f * m.V + v) * 3;
-    for (int c = 0; c < 3; ++c) {
-        const float *e = m.E + ((size_t)v * 3 + c) * m.KP;
-        double acc = 0.0;
-        for (int k = 0; k < m.K; ++k) acc = fma((double)e[k], (double)xf[k], acc);
-        g[c] = (double)m.mean[(size_t)c * m.V + v] + acc;
-    }
-}
-
 // Barycentrics of sample s in triangle (b, c, a) by Cramer's rule: s - a = alpha (b - a) + beta (c - a)
 // (the same values as the reference's dot-product form, funcs.cu:961-977, in exact arithmetic),
 // and their derivatives with respect to the three projected corners when d != nullptr:

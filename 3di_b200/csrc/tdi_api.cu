@@ -167,8 +167,6 @@ struct tdi_batch {
     float *lm_buf = nullptr;       // landmark initialisation: p0L [3][51], orthographic x [cap][7], R [cap][9], slack [cap]
     int32_t *lm_ibuf = nullptr;    // its iterations, run flags, successes, Newton steps [4][cap]
     double *adj = nullptr;         // differentiable loss: FP64 geometry, images, adjoints (tdi_batch_loss)
-    size_t adj_doubles = 0;
-    float *ctrl_scratch = nullptr;
     double *scalars = nullptr;     // [cap][4]
     int *d_count = nullptr;
     int *h_count = nullptr;        // pinned
@@ -269,7 +267,7 @@ float face_size_of(const float *xl, const float *yl)
 }
 
 
-constexpr int ADJ_VERTEX_SMEM_MAX = 200 * 1024;   // the tiled FP64 vertex stage of the loss (K up to ~235)
+constexpr int ADJ_VERTEX_SMEM_MAX = 200 * 1024;   // the FP64 vertex stage of the loss (K up to 240, as the raster's)
 
 tdi_status set_attrs()
 {
@@ -374,7 +372,7 @@ DBatch batch_view(const tdi_batch *bt, int f0, int nf)
     v.x0y0 = a.x0y0 + F0 * 2;
     v.Lint = a.Lint + F0;
     v.x = a.x + F0 * KTP; v.x_ls = a.x_ls + F0 * KTP; v.xe = a.xe + F0 * KTP;
-    v.lam = a.lam + F0 * 4; v.lam_ls = a.lam_ls + F0 * 4; v.lame = a.lame + F0 * 4;
+    v.lam = a.lam + F0 * 4; v.lam_ls = a.lam_ls + F0 * 4;
     v.dlam = a.dlam + F0 * 4; v.glam = a.glam + F0 * 4;
     v.d = a.d + F0 * KTP; v.g = a.g + F0 * KTP;
     v.H = a.H + F0 * KTP * KTP;
@@ -688,14 +686,13 @@ tdi_status tdi_model_create(const tdi_model_desc *desc, tdi_model **out)
     d.V = V; d.T = T; d.K = K; d.KP = round4(K); d.KT = K + 6; d.KTP = round4(K + 6);
     d.KC = std::min(d.KTP, CAND_COLS);
     float *mean, *E, *tex, *epsb;
-    int32_t *tl, *lis, *order, *tlo;
+    int32_t *lis;
     int4 *tl4, *tlo4;
     auto cleanup = [&](tdi_status st) { for (void *p : m->allocs) cudaFree(p); delete m; return st; };
     tdi_status st;
     if ((st = dalloc(m->allocs, &mean, 3 * (size_t)V)) || (st = dalloc(m->allocs, &E, (size_t)V * 3 * d.KP)) ||
-        (st = dalloc(m->allocs, &tex, (size_t)V)) || (st = dalloc(m->allocs, &tl, 3 * (size_t)T)) ||
-        (st = dalloc(m->allocs, &lis, (size_t)NL)) || (st = dalloc(m->allocs, &epsb, 4 * (size_t)K)) ||
-        (st = dalloc(m->allocs, &order, (size_t)T)) || (st = dalloc(m->allocs, &tlo, 3 * (size_t)T)) ||
+        (st = dalloc(m->allocs, &tex, (size_t)V)) || (st = dalloc(m->allocs, &lis, (size_t)NL)) ||
+        (st = dalloc(m->allocs, &epsb, 4 * (size_t)K)) ||
         (st = dalloc(m->allocs, &tl4, (size_t)T)) || (st = dalloc(m->allocs, &tlo4, (size_t)T)))
         return cleanup(st);
     // Internal vertex numbering: vertices are stored in Morton order of their mean-shape (x, y)
@@ -703,7 +700,7 @@ tdi_status tdi_model_create(const tdi_model_desc *desc, tdi_model **out)
     // memory. Every per-vertex quantity is computed independently of the numbering; the
     // entry points that take or return per-vertex arrays translate at the boundary.
     // The raster's depth pass visits triangles in Morton order of their centroids (the
-    // z-buffer result does not depend on the order); tlo holds their corners as slots.
+    // z-buffer result does not depend on the order); tlo4 holds their corners as slots.
     float xmin = desc->mean[0], xmax = xmin, ymin = desc->mean[V], ymax = ymin;
     for (int v = 0; v < V; ++v) {
         xmin = std::min(xmin, desc->mean[v]); xmax = std::max(xmax, desc->mean[v]);
@@ -767,15 +764,12 @@ tdi_status tdi_model_create(const tdi_model_desc *desc, tdi_model **out)
     if (cudaMemcpy(mean, mean_h.data(), sizeof(float) * 3 * V, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(E, Ep.data(), sizeof(float) * Ep.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(tex, tex_h.data(), sizeof(float) * V, cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(tl, tls.data(), sizeof(int32_t) * 3 * T, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(lis, lis_h.data(), sizeof(int32_t) * NL, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(epsb, eb.data(), sizeof(float) * eb.size(), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(order, tord.data(), sizeof(int32_t) * T, cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMemcpy(tlo, tlo_h.data(), sizeof(int32_t) * 3 * T, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(tl4, tl4_h.data(), sizeof(int4) * T, cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMemcpy(tlo4, tlo4_h.data(), sizeof(int4) * T, cudaMemcpyHostToDevice) != cudaSuccess)
         return cleanup(fail(TDI_ERR_CUDA, "model upload failed"));
-    d.mean = mean; d.E = E; d.tex = tex; d.tl = tl; d.lis = lis; d.eps_b = epsb; d.tri_order = order; d.tlo = tlo; d.tl4 = tl4; d.tlo4 = tlo4;
+    d.mean = mean; d.E = E; d.tex = tex; d.lis = lis; d.eps_b = epsb; d.tl4 = tl4; d.tlo4 = tlo4;
     if (K <= VC_MAXK) {
         // the basis split into BF16 pieces once, in the tensor-core vertex stage's tile layout
         const int ntiles = (V + VC_V - 1) / VC_V;
@@ -823,7 +817,7 @@ tdi_status tdi_batch_create(tdi_model *m, int32_t max_frames, tdi_batch **out)
     A(target, F * NPIX); A(d.tgn, F * NPIX); A(b->target_raw, F * NPIX); A(b->prep, F); A(xl, F * NL); A(yl, F * NL);
     A(bounds, F * 4 * NL); A(fs, F); A(cam, F * 4); A(x0y0, F * 2); A(Lint, F);
     A(d.x, F * KTP); A(d.x_ls, F * KTP); A(d.xe, F * KTP);
-    A(d.lam, F * 4); A(d.lam_ls, F * 4); A(d.lame, F * 4); A(d.dlam, F * 4); A(d.glam, F * 4);
+    A(d.lam, F * 4); A(d.lam_ls, F * 4); A(d.dlam, F * 4); A(d.glam, F * 4);
     A(d.d, F * KTP); A(d.g, F * KTP); A(d.H, F * KTP * KTP); A(d.Hb, F * KTP * KTP); A(d.gb, F * KTP); A(d.R, F * 9); A(d.dR, F * 27);
     A(d.ctl, F); A(d.act, F); A(d.rlist, F); A(d.jlist, F); A(d.rcount, 2 * F); A(d.geo, F * (size_t)md.V); A(d.proj, F * (size_t)md.V); A(d.zbuf, F * NPIX); A(d.ccount, F); if (!resolve_smem(md.T)) A(d.tri_work, F * (size_t)resolve_words(md.T)); A(d.frag, F * NMAX);
     A(d.fgrad, F * 5 * NMAX); A(d.nb, F * 4 * NMAX); A(d.shc, F * NMAX); A(d.sht, F * NMAX);
@@ -1311,10 +1305,7 @@ static tdi_status adj_bufs(tdi_batch *b, AdjBufs &o)
                               F * (size_t)m.K};
     size_t total = 0;
     for (size_t s : sizes) total += (s + 31) / 32 * 32;
-    if (!b->adj) {
-        TDI_CUDA(cudaMalloc(&b->adj, total * sizeof(double)));
-        b->adj_doubles = total;
-    }
+    if (!b->adj) TDI_CUDA(cudaMalloc(&b->adj, total * sizeof(double)));
     double **dst[NB] = {&o.geo, &o.R, &o.region, &o.grads, &o.dI, &o.dP0, &o.glob, &o.geps};
     double *p = b->adj;
     for (int i = 0; i < NB; ++i) { *dst[i] = p; p += (sizes[i] + 31) / 32 * 32; }
@@ -1347,10 +1338,8 @@ static tdi_status adj_forward(tdi_batch *b, const Cfg &c, const float *x, const 
         TDI_TRY(launch(b, 0, k_adj_vertex_tiled<8>, dim3(vb.x, (F + 63) / 64), dim3(256), adj_vertex_smem(m.KP, 8), s, m, x, F, o.geo));
     else if (F > 8 && adj_vertex_smem(m.KP, 4) <= (size_t)ADJ_VERTEX_SMEM_MAX)
         TDI_TRY(launch(b, 0, k_adj_vertex_tiled<4>, dim3(vb.x, (F + 31) / 32), dim3(256), adj_vertex_smem(m.KP, 4), s, m, x, F, o.geo));
-    else if (adj_vertex_smem(m.KP, 1) <= (size_t)ADJ_VERTEX_SMEM_MAX)
-        TDI_TRY(launch(b, 0, k_adj_vertex_tiled<1>, dim3(vb.x, (F + 7) / 8), dim3(256), adj_vertex_smem(m.KP, 1), s, m, x, F, o.geo));
     else
-        TDI_TRY(launch(b, 0, k_adj_vertex, dim3((m.V + 255) / 256, F), dim3(256), 0, s, m, x, F, o.geo));
+        TDI_TRY(launch(b, 0, k_adj_vertex_tiled<1>, dim3(vb.x, (F + 7) / 8), dim3(256), adj_vertex_smem(m.KP, 1), s, m, x, F, o.geo));
     return launch(b, 0, k_adj_shade, dim3(16, F), dim3(AD_THREADS), 0, s, m, (const DBatch)d, x, lam, L,
                   (const double *)o.geo, (const double *)o.R, o.dI);
 }

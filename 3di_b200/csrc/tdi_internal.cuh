@@ -84,7 +84,7 @@ struct Cfg {
 
 // Device view of the model.
 // Vertices are numbered internally by slot (Morton order of the mean shape's x-y position);
-// tl and lis hold slots. Triangles keep the caller's numbering.
+// tl4, tlo4 and lis hold slots. Triangles keep the caller's numbering.
 struct DModel {
     int32_t V, T, K, KP;     // KP: K rounded up to a multiple of 4 (row pitch of E)
     int32_t KT, KTP;         // K + 6 unknowns, and its pitch (multiple of 4)
@@ -92,13 +92,11 @@ struct DModel {
     const float *mean;       // [3][V]
     const float *E;          // [V][3][KP]
     const float *tex;        // [V]
-    const int32_t *tl;       // [3][T] corner slots
     const int32_t *lis;      // [NL] landmark slots
     const float *eps_b;      // [4][K]: lb, ub, lb_ft, ub_ft
-    const int32_t *tri_order;// [T] triangles in Morton order of their mean-shape centroids
-    const int32_t *tlo;      // [3][T] corner slots of the triangles in tri_order
     const int4 *tl4;         // [T] corner slots (b, c, a, 0): one 16-byte gather per triangle
-    const int4 *tlo4;        // [T] in tri_order: corner slots and the triangle id (b, c, a, tri)
+    const int4 *tlo4;        // [T] in Morton order of the mean-shape centroids: corner slots and the triangle
+                             // id (b, c, a, tri)
     const void *Etc;         // the basis split into BF16 pieces in the tensor-core vertex stage's
                              // tile layout (null when K is above that stage's limit)
 };
@@ -117,7 +115,7 @@ struct DBatch {
     const float *Lint;       // [F]
     // state
     float *x, *x_ls, *xe;    // [F][KTP]: accepted, line-search, evaluation point
-    float *lam, *lam_ls, *lame, *dlam, *glam;   // [F][4]
+    float *lam, *lam_ls, *dlam, *glam;          // [F][4]
     float *d, *g;            // [F][KTP]
     float *H;                // [F][KTP][KTP]
     float *Hb, *gb;          // [F][KTP][KTP] (upper triangle), [F][KTP]: the barrier's part of H and g
