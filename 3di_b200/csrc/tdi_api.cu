@@ -188,7 +188,7 @@ struct tdi_batch {
 
 namespace {
 
-// Streams a batched fit runs on: lanes are parts of the batch with their own stream, active
+// Lanes of a batched fit: lanes are parts of the batch with their own stream, active
 // list and round graphs, replayed side by side so that one lane's latency-bound rounds (few
 // frames still running, one block per frame) overlap the other's work.
 #ifndef TDI_FIT_LANES
@@ -400,7 +400,7 @@ DBatch batch_view(const tdi_batch *bt, int f0, int nf)
 }
 
 // Compacts a lane's list of frames running the stage; the count arrives with the lane's
-// next synchronisation (one 8-byte read-back per round and lane).
+// next synchronisation (one 8-byte read-back per replay, or per host-driven round, and lane).
 tdi_status lane_compact(tdi_batch *bt, tdi_lane &ln)
 {
     TDI_TRY(launch(bt, 0, k_compact_active, dim3(1), dim3(1024), 0, ln.s, (const DBatch)ln.d, ln.d_count));
@@ -840,7 +840,7 @@ tdi_status tdi_batch_create(tdi_model *m, int32_t max_frames, tdi_batch **out)
     d.target = target; d.xl = xl; d.yl = yl; d.bounds = bounds; d.face_size = fs; d.cam = cam;
     d.x0y0 = x0y0; d.Lint = Lint;
     d.prof_id = 0;
-    // lanes: two for batches that can be halved, each with a non-blocking stream
+    // lanes: FIT_LANES for batches that can be split, each with non-blocking streams
     b->lanes.resize(max_frames >= 2 ? FIT_LANES : 1);
     for (auto &ln : b->lanes) {
         if (cudaStreamCreateWithFlags(&ln.s, cudaStreamNonBlocking) != cudaSuccess ||
@@ -1245,7 +1245,7 @@ tdi_status tdi_batch_landmark_init(tdi_batch *b, const float *p0L, int32_t *succ
 {
     if (!b || !p0L) return fail(TDI_ERR_INVALID, "null argument");
     const DModel &m = b->m->d;
-    if (m.K + 7 > LM_MAXN) return fail(TDI_ERR_INVALID, "landmark initialisation takes at most 129 expression components");
+    if (!lm_accepts(m.K)) return fail(TDI_ERR_INVALID, "landmark initialisation takes at most 112 expression components");
     const int F = b->d.F;
     if (F <= 0) return fail(TDI_ERR_INVALID, "no frames: call tdi_batch_set_frames first");
     cudaStream_t s = (cudaStream_t)stream;
@@ -1266,7 +1266,6 @@ tdi_status tdi_batch_landmark_init(tdi_batch *b, const float *p0L, int32_t *succ
         TDI_CUDA(cudaFuncSetAttribute(k_landmark_init<8, 128>, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
         attr = true;
     }
-    if (!lm_accepts(m.K)) return fail(TDI_ERR_INVALID, "too many expression components for the landmark fit");
     const bool narrow = lm_narrow(m.K);
     const size_t smem = narrow ? lm_smem<6, 88>(m.K) : lm_smem<8, 128>(m.K);
     TDI_CUDA(cudaMemcpyAsync(dp, p0L, sizeof(float) * 3 * NL, cudaMemcpyHostToDevice, s));

@@ -490,8 +490,9 @@ __global__ void __launch_bounds__(VT_THREADS, VT_BLOCKS_PER_SM) k_vertex(DModel 
 // Barrier objective of a state (logbarrier_initializer.cu:1921-2093 with compute_Gs :456-520):
 // expression bounds, then the four landmark box constraints. Landmark 3D points are the
 // vertex-stage object coordinates at the landmark vertices (same formula as the reference's
-// p0L + EL*eps). One warp per frame: lanes evaluate the -log terms (FP64 log rounded to FP32),
-// lane 0 sums them sequentially in FP64 in the oracle's order.
+// p0L + EL*eps). The -log terms are FP64 logarithms rounded to FP32, summed in FP64: strides of the
+// block, then a tree over the lanes, then the warps. The oracle adds them one after the other; the two
+// sums agree to FP64 rounding, and the objective is their FP32 rounding.
 
 __device__ __forceinline__ void landmark_G(const DModel &m, const DBatch &b, int f, const float *x,
                                            const float *R, int i, const float *p, float G[4])
@@ -845,7 +846,7 @@ __device__ __forceinline__ bool survives(unsigned long long k, uint32_t tag, uin
 constexpr int RD_THREADS = 256;             // depth pass: threads per block
 constexpr int RD_BLOCKS = 8;                // depth pass: blocks per frame (at least)
 constexpr int RD_MAX_BLOCKS = 128;          // depth pass: blocks per frame when few frames render
-constexpr int RD_SPREAD = 2400;             // blocks that fill the SMs twice over
+constexpr int RD_SPREAD = 2400;             // blocks of a launch of few frames: four waves of four per SM
 constexpr int RR_THREADS = 1024;            // resolve: one block per frame
 constexpr int RR_WARPS = RR_THREADS / 32;
 constexpr int RR_U = 4;                     // resolve: candidates per thread in flight together
@@ -945,7 +946,7 @@ inline int raster_grid(int frames)
 // 53,490-vertex mesh's); a full warp's worth of queued triangles is then evaluated densely. RD_ILP
 // triangles per lane have their gathers in flight together (1,024 frames in one launch: 1 875 us,
 // 2 707, 3 671). 64 registers and 47 KB of shared memory are four blocks per SM (at 70 registers, three
-// blocks, 795 us; at 48 registers it spills, 953).
+// blocks, 795 us); shared memory admits no fifth.
 // 1,024 frames of the 53,490-vertex model in one launch: 1,192 us with every sample evaluated in
 // place, 671 with the queue, the candidates and their shading inputs included (which the resolve
 // formed before). What is left is issue (0.68 per cycle) and the latency of the gathers.
@@ -1325,7 +1326,7 @@ __device__ __forceinline__ void neighbour_pixels(int p, int &kr, int &kl, int &k
 constexpr int LIGHT_THREADS = 1024;               // the light fit's renders
 constexpr int RENDER_SMEM_FLOATS = 27 * 1024;     // padded region buffers (108 KB)
 constexpr int RENDER_GU = 4;                      // fragments in flight in the gradient pass
-constexpr int RENDER_SU = 4;                      // the same when shading from the resolve's terms
+constexpr int RENDER_SU = 4;                      // and in the shading
 constexpr int RPAD = 8;                           // zero columns left and right of A's lines (KRAD used)
 constexpr int RUN_Y = 9, RUN_X = 8;               // outputs per thread and line of the row and column pass
 constexpr int RIMG = 2 * DIM * (DIM + 2 * RPAD);  // per-frame floats of the global fallback
@@ -1433,8 +1434,8 @@ __device__ __forceinline__ void light_terms(const float *R, const float *tau, co
 }
 
 // Owners shaded into the cleared region. Each fragment's unit normal, n . p and interpolated
-// albedo depend only on the geometry of the raster: the resolve forms them (shc, sht) for every
-// raster that renders. A render forms the rotated light once and the same FP32 operations as
+// albedo depend only on the geometry of the raster: the depth pass forms them for every
+// raster (k_raster_slots places them, shc and sht). A render forms the rotated light once and the same FP32 operations as
 // the reference's shading: Id = (n0 q0 + n1 q1) + n2 q2 - n.p, I = t + (L t) Id. RENDER_SU fragments per thread:
 // each one's pixel word and shading terms are loaded together.
 template <int NT>

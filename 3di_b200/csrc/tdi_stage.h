@@ -9,7 +9,8 @@
 // STAGE_PIN bytes (24 frames' crops, 6 MB: 0.7 ms plain, 4.5 ms when the slots are pinned for them; a
 // plain copy of 64 MB takes as long as pinning and staging it), and given back when the last
 // batch is destroyed. One upload uses them at a time and has left them when it returns; an
-// upload that finds them busy (another thread's batch) makes plain copies instead.
+// upload that finds them busy (another thread's batch), or is on the per-thread default stream, makes
+// plain copies instead.
 #pragma once
 #include <cuda_runtime.h>
 

@@ -53,7 +53,8 @@ typedef struct tdi_batch tdi_batch;
 typedef struct {
     int32_t n_vertices;          /* V */
     int32_t n_triangles;         /* T (the reference's 16-bit indices cap T at 65,535) */
-    int32_t n_expr;              /* K, 79 for the GLOBAL79 basis */
+    int32_t n_expr;              /* K, 79 for the GLOBAL79 basis (exact fits take at most 81, fits with
+                                    tensor-core normal equations 121, renders and the loss 240) */
     const float *mean;           /* [3][V] X0_mean, Y0_mean, Z0_mean (identity applied) */
     const float *expr_basis;     /* [V][3][K] rows of EX_79/EY_79/EZ_79.dat per vertex */
     const float *tex;            /* [V] albedo (tex_mu with the identity texture) */
@@ -200,8 +201,8 @@ tdi_status tdi_batch_set_state(tdi_batch *b, const float *x, const float *lam, c
 tdi_status tdi_batch_landmark_init(tdi_batch *b, const float *p0L, int32_t *success, float *slack,
                                    int32_t *iters, void *stream);
 
-/* Fit every frame of the batch on the device (asynchronous on the stream apart from one
- * 4-byte read-back per round). Replaces fit_to_video_frame's fitting calls. */
+/* Fit every frame of the batch on the device (asynchronous on the stream apart from an
+ * 8-byte read-back per 16 rounds). Replaces fit_to_video_frame's fitting calls. */
 tdi_status tdi_batch_fit(tdi_batch *b, const tdi_fit_config *cfg, void *stream);
 /* Download states and reports. Synchronous. */
 tdi_status tdi_batch_get_state(tdi_batch *b, float *x, float *lam, tdi_report *rep, void *stream);
