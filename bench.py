@@ -174,8 +174,8 @@ def algorithmic_bytes(kernel: str, V: int, T: int, K: int, n_frag: float):
         # records are placed by a kernel of their own)
         return n_frag * (16 + 4 + 8 + 4), 0.0
     if kernel == "render":
-        # fragments, their shading records, four target pixels, gradients
-        return n_frag * (16 + 20 + 4 * 4 + 5 * 4), 0.0
+        # fragments, their shading records, the target's gradients at their pixels, gradients written
+        return n_frag * (16 + 20 + 8 + 5 * 4), 0.0
     if kernel == "neighbours":
         # fragment pixels in, four neighbour indices out
         return n_frag * (16 + 16), 0.0
